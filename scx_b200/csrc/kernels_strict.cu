@@ -1,11 +1,11 @@
 // CUDA-core SpMM pair with FP32 products and a fixed summation order (the
 // strict FP32 path, and the CUDA-core path of 16-bit values when the tensor
 // cores cannot take a matrix).  Both kernels read their dense operand from
-// shared memory and accumulate in registers; neither uses atomics, so every
-// result is bit-identical from run to run.
+// shared memory and accumulate in registers; neither uses floating-point
+// atomics, so every result is bit-identical from run to run.
 //
 //   forward    Y = P V - 1 mc^T   (CSR rows, V staged in gene chunks)
-//   transposed W_part = P^T Q     (tile-CSC copy, Q staged one row tile at a time)
+//   transposed W_part = P^T Q     (chunk-CSC copy, Q staged one row chunk at a time)
 //
 // Restate spmm_forward_row (scx-accel/src/pca/cpu.rs:1500-1523) with the mean
 // correction of forward_mean_prefactor (scx-gpu/src/gpu_pca.rs:218-237), and
@@ -13,20 +13,49 @@
 // partitioned reduction of spmm_transpose_into (cpu.rs:1330-1389).
 //
 // Layouts (device memory):
-//   CSR      : int64 indptr[n+1], int32 idx[nnz], values[nnz], rows sorted by gene
-//   V        : float [n_vars][ld] gene-major;  Y, Q: float [n_obs][ld] cell-major
-//   tile CSC : for row tile t (kStrictTile rows, entries indptr[t T] .. indptr[(t+1) T]),
-//              the same entries reordered by (slot, row): cell[p] = row within the
-//              tile (uint8), cval[p] = value; tptr[t (S + 1) + s] = offset of slot
-//              s's first entry from indptr[t T] (S + 1 offsets per tile).  Genes are
-//              relabelled to slots (gene2slot) so that each warp of the transposed
-//              product owns GPW consecutive slots of about equal stored-entry count.
-//   partial  : float [ranges][n_vars][ld], summed in range order by k_reduce_rows
+//   CSR       : int64 indptr[n+1], int32 idx[nnz], values[nnz], rows sorted by gene
+//   V         : float [n_vars][ld] gene-major;  Y, Q: float [n_obs][ld] cell-major
+//   chunk CSC : for row chunk t (geo.rows rows, entries indptr[t T] .. indptr[(t+1) T]),
+//               the same entries reordered by (slot, row): row[p] = row within the
+//               chunk (uint16), cval[p] = value; tptr[t (g + 1) + s] = offset of slot
+//               s's first entry from indptr[t T].  Slots are the genes in decreasing
+//               order of stored entries (gene2slot / slot2gene), so neighbouring
+//               slots have lists of about the same length.
+//   partial   : float [ranges][n_vars][ld], summed in range order by k_reduce_rows
+//
+// What bounds the pair, and the layout that follows.  An entry costs one row of
+// the dense operand out of shared memory, ld x 4 bytes: 2 clocks of an SM's
+// 128 bytes per clock at ld 64, 323 us for 47M entries on 148 SMs.  Everything
+// else has to hide under that.  So
+//   * a block owns a SLICE of 64 or 32 columns and keeps a table of dense rows
+//     of that slice, as many as shared memory holds (800 or 1,600), so a list
+//     is long, a barrier rare, and one block per SM stages a table a few times
+//     per product;
+//   * four lanes walk one LIST (a cell's entries inside the table's genes, or a
+//     gene's entries inside the table's cells) straight from global memory,
+//     eight entries per 32-byte load of indices and of values (the lanes read
+//     the same address: a whole sector, so nothing depends on what little L1
+//     is left staying there), two steps loaded ahead.  Nothing is exchanged
+//     between lanes: no shuffles, ballots or barriers in the walk.  The load
+//     delivers a copy of the entry to every lane, which the same pipe pays
+//     for: four lanes with 16 columns each cost half of eight lanes with 8;
+//   * a lane reads its columns 16 bytes at a time, and the two lists that share
+//     a wavefront take the 64-byte halves of a line in opposite order, so no
+//     read conflicts;
+//   * the eight lists of a warp have about the same length (cells ordered by
+//     length in the kernel, genes by slot), and the warps of a block take
+//     groups of eight lists in that order.
+// With 64 columns the entries are read once and a step has half the overhead
+// per column; with 32 there are twice as many blocks per range, so a range is
+// twice as long, its partial half the traffic, and a table holds twice the
+// rows.  Measured (forward / transposed / sum of partials, us): 250,000 cells
+// 554 / 512 / 14 with 64 columns, 569 / 586 / 9 with 32; 50,000 cells 136 / 124
+// / 14 and 137 / 134 / 8; 10,000 cells 53 / 48 / 13 and 49 / 44 / 8.  The line
+// lies at 256 cells per SM.
+// Against the layout before (a 128-row dense window per block, entries
+// broadcast with shuffles, 14.6 instructions per entry): 1,304 / 923 us at
+// 250,000 x 2,000 (47M entries), 370 / 200 at 50,000, 167 / 62 at 10,000.
 #include <algorithm>
-#include <functional>
-#include <queue>
-#include <utility>
-#include <vector>
 
 #include "common.cuh"
 #include "launch.h"
@@ -35,363 +64,505 @@ namespace scx {
 
 namespace {
 
+constexpr int kThreads = 512;      // threads of a product block (one block per SM)
+constexpr int kLanes = 4;          // lanes that walk a list together
+constexpr int kLists = kThreads / kLanes;
+constexpr int kRowBlock = 4096;    // cells a forward block orders and walks at a time
+constexpr int kBuckets = 256;      // length classes of that order
+constexpr size_t kSmemMax = 231424;  // 227 KB less the static variables' share
+// forward: the cells' order (uint16) and their cursors (uint32), the length classes
+constexpr size_t kFwdSmemFixed = kRowBlock * 2 + kRowBlock * 4 + kBuckets * 4;
+// Columns a block holds: 64 where the panel is a multiple of 64 and there are
+// cells enough, else 32.
+int slice_cols(int ld, int64_t n, int num_sms) {
+  return ld % 64 == 0 && n >= (int64_t)256 * num_sms ? 64 : 32;
+}
+// rows of the table (one more, all zeros, follows them)
+constexpr int fwd_table_rows(int cols) { return (int)((kSmemMax - kFwdSmemFixed) / (cols * 4)) - 1; }
+constexpr int rmat_table_rows(int cols) { return (int)(kSmemMax / (cols * 4)) - 1; }
+
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+__device__ __forceinline__ void cp_async_wait_all() {
+  asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;\n" ::: "memory");
 }
 
-// Copy `bytes` (a multiple of 16, both addresses 16-byte aligned) with the
-// whole block, as 16-byte asynchronous copies.
-__device__ __forceinline__ void block_copy_async(void* smem, const void* gmem, int bytes) {
-  for (int o = threadIdx.x * 16; o < bytes; o += blockDim.x * 16)
-    cp_async16(static_cast<char*>(smem) + o, static_cast<const char*>(gmem) + o);
+// Stage `rows` rows of one slice (row stride lds floats) with the block, and
+// the row of zeros behind them.
+template <int NV>
+__device__ __forceinline__ void stage_table(float* tab, const float* src, int rows, int lds) {
+  constexpr int Q = kLanes * NV;  // 16-byte pieces per row
+  for (int o = threadIdx.x; o < rows * Q; o += kThreads) {
+    const int r = o / Q, q = o % Q;
+    cp_async16(tab + r * (4 * Q) + 4 * q, src + (int64_t)r * lds + 4 * q);
+  }
+  if (threadIdx.x < 4 * Q) tab[rows * (4 * Q) + threadIdx.x] = 0.f;
+  cp_async_wait_all();
 }
 
-// Copy `rows` rows of LD floats, row stride `lds` floats in global memory
-// (a column panel of a wider matrix), to consecutive rows in shared memory.
-// With lds == LD it is the contiguous copy.
-template <int LD>
-__device__ __forceinline__ void block_copy_rows_async(float* smem, const float* gmem, int rows, int lds) {
-  if (lds == LD) {
-    block_copy_async(smem, gmem, rows * LD * 4);
-    return;
+// Eight consecutive list entries, their position a multiple of eight: whole
+// 32-byte sectors of an int32 or FP32 array, in one 256-bit load.
+template <typename T>
+struct Oct {
+  alignas(32) T v[8];
+};
+
+__device__ __forceinline__ void load_oct(Oct<float>& d, const float* p) {
+  asm("ld.global.nc.L2::256B.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=f"(d.v[0]), "=f"(d.v[1]), "=f"(d.v[2]), "=f"(d.v[3]), "=f"(d.v[4]), "=f"(d.v[5]), "=f"(d.v[6]), "=f"(d.v[7])
+      : "l"(p));
+}
+__device__ __forceinline__ void load_oct(Oct<int32_t>& d, const int32_t* p) {
+  asm("ld.global.nc.L2::256B.v8.s32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(d.v[0]), "=r"(d.v[1]), "=r"(d.v[2]), "=r"(d.v[3]), "=r"(d.v[4]), "=r"(d.v[5]), "=r"(d.v[6]), "=r"(d.v[7])
+      : "l"(p));
+}
+template <typename T>  // 16-bit types
+__device__ __forceinline__ void load_oct(Oct<T>& d, const T* p) {
+  static_assert(sizeof(T) == 2, "16-bit entries");
+  *reinterpret_cast<uint4*>(d.v) = __ldg(reinterpret_cast<const uint4*>(p));
+}
+
+// VEC: the array allows the aligned vector load; positions at or past `lim`
+// (the array's length) are not read.
+template <bool VEC, typename T>
+__device__ __forceinline__ void load_oct(Oct<T>& d, const T* a, int64_t p, int64_t lim) {
+  if (VEC && p + 8 <= lim) {
+    load_oct(d, a + p);
+  } else {
+#pragma unroll
+    for (int u = 0; u < 8; ++u) d.v[u] = p + u < lim ? a[p + u] : T();
   }
-  constexpr int Q = LD / 4;  // 16-byte pieces per row
-  for (int o = threadIdx.x; o < rows * Q; o += blockDim.x) {
-    const int r = o / Q, q = o - r * Q;
-    cp_async16(smem + r * LD + 4 * q, gmem + (int64_t)r * lds + 4 * q);
+}
+
+__device__ __forceinline__ float4 lds128(unsigned addr) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+  return v;
+}
+
+// acc += sum over the entries [s, e) of val[p] * table row (idx[p] - j0), in
+// position order; with LIMIT it stops at the first entry whose row is not in
+// the table (idx[p] >= j0 + rows; the list is sorted).  Returns where it
+// stopped.  `tab` is the shared address of the lane's first piece of row 0.
+// Entries of a step that are not the list's read the row of zeros behind the
+// table, so a step is the same instructions for a full and for a ragged one
+// and the lists of a warp stay together.  (Indices are validated when
+// the plan is built; one that is out of range reads that row as well.)
+template <bool VEC, bool LIMIT, int NV, typename IdxT, typename ValT>
+__device__ __forceinline__ int64_t walk(float (&acc)[4 * NV], const IdxT* __restrict__ idx,
+                                        const ValT* __restrict__ val, int64_t s, int64_t e, int64_t lim, int j0,
+                                        int rows, unsigned tab) {
+  if (s >= e) return e;
+  int64_t p = s & ~int64_t(7);
+  unsigned valid = 0xffu << (int)(s - p);
+  Oct<IdxT> j1, j2;  // the next two steps' entries
+  Oct<ValT> x1, x2;
+  load_oct<VEC>(j1, idx, p, lim);
+  load_oct<VEC>(x1, val, p, lim);
+  if (p + 8 < e) {
+    load_oct<VEC>(j2, idx, p + 8, lim);
+    load_oct<VEC>(x2, val, p + 8, lim);
   }
+  while (true) {
+    Oct<IdxT> cj = j1;
+    const Oct<ValT> cx = x1;
+    j1 = j2;
+    x1 = x2;
+    const int64_t left = e - p;  // entries from the step's first position to the list's end
+    if (left > 16) {
+      load_oct<VEC>(j2, idx, p + 16, lim);
+      load_oct<VEC>(x2, val, p + 16, lim);
+    } else if (left < 8) {
+      valid &= (1u << (int)left) - 1u;
+    }
+    bool stop = false;
+    // (past the list's end the last entry is another list's and says nothing)
+    if (LIMIT && (left < 8 || (int)cj.v[7] >= j0 + rows)) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if ((int)cj.v[u] >= j0 + rows && (valid >> u & 1)) {
+          valid &= (1u << u) - 1u;
+          stop = true;
+        }
+    }
+    if (valid != 0xffu) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (!(valid >> u & 1)) cj.v[u] = (IdxT)(j0 + rows);
+    }
+#pragma unroll
+    for (int half = 0; half < 8; half += 4) {
+      if (LIMIT || (valid >> half & 0xfu)) {
+#pragma unroll
+        for (int u = half; u < half + 4; ++u) {
+          const unsigned r = tab + min((unsigned)((int)cj.v[u] - j0), (unsigned)rows) * (64 * NV);
+          const float x = to_f32(cx.v[u]);
+#pragma unroll
+          for (int h = 0; h < NV; ++h) {
+            const float4 v = lds128((h & 1 ? r ^ 64u : r) + (h >> 1) * 128);
+            acc[4 * h + 0] = fmaf(x, v.x, acc[4 * h + 0]);
+            acc[4 * h + 1] = fmaf(x, v.y, acc[4 * h + 1]);
+            acc[4 * h + 2] = fmaf(x, v.z, acc[4 * h + 2]);
+            acc[4 * h + 3] = fmaf(x, v.w, acc[4 * h + 3]);
+          }
+        }
+      }
+    }
+    if (LIMIT && stop) return max(s, p + 32 - __clz(valid));  // past the last entry taken
+    if (left <= 8) return e;
+    p += 8;
+    valid = 0xffu;
+  }
+}
+
+// A lane's columns of a row: piece h is 4 floats at 16 ((h & ~1) + ((h ^ list) & 1)) + 4 l.
+// Lists of odd and even number in the block take the two 64-byte pieces of a
+// 128-byte line in opposite order, so the two lists of a shared-memory
+// wavefront (8 lanes) never meet in a bank.
+__device__ __forceinline__ int piece_col(int h, int odd) { return 16 * ((h & ~1) + ((h & 1) ^ odd)); }
+
+template <int NV>
+__device__ __forceinline__ void load_cols(float (&a)[4 * NV], const float* src, int odd) {
+#pragma unroll
+  for (int h = 0; h < NV; ++h)
+    *reinterpret_cast<float4*>(a + 4 * h) = *reinterpret_cast<const float4*>(src + piece_col(h, odd));
+}
+template <int NV>
+__device__ __forceinline__ void store_cols(float* dst, const float (&a)[4 * NV], int odd) {
+#pragma unroll
+  for (int h = 0; h < NV; ++h)
+    *reinterpret_cast<float4*>(dst + piece_col(h, odd)) =
+        make_float4(a[4 * h], a[4 * h + 1], a[4 * h + 2], a[4 * h + 3]);
 }
 
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Tile-CSC build, one warp per row tile (once per plan).  Counting sort of
-// the tile's entries by slot (the relabelled gene); rows are visited in
-// order, so within a slot the entries keep row order.  Within one 32-entry
+// Stored entries per gene.  Each block counts its share in shared memory and
+// adds its counts to the global ones (integers: the order does not matter).
+// Matrices with more genes than a block's counters go to global memory directly.
+// (100,000 x 2,000, 18M entries: 26 us, against 606 us with one global
+// atomic per entry, which a few frequent genes serialise.)
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(512) k_gene_counts(const int32_t* __restrict__ idx, int64_t nnz, int32_t g,
+                                                     int32_t* __restrict__ counts) {
+  extern __shared__ int32_t hist[];
+  for (int j = threadIdx.x; j < g; j += blockDim.x) hist[j] = 0;
+  __syncthreads();
+  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t j = (uint32_t)__ldg(idx + p);
+    if (j < (uint32_t)g) atomicAdd(hist + j, 1);  // a streamed shard is counted before its flags are read
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < g; j += blockDim.x) {
+    const int32_t c = hist[j];
+    if (c) atomicAdd(counts + j, c);
+  }
+}
+
+__global__ void k_gene_counts_global(const int32_t* __restrict__ idx, int64_t nnz, int32_t g,
+                                     int32_t* __restrict__ counts) {
+  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t j = (uint32_t)__ldg(idx + p);
+    if (j < (uint32_t)g) atomicAdd(counts + j, 1);
+  }
+}
+
+// Slots: genes in decreasing order of stored entries, ties by gene.  One warp
+// per gene counts the genes in front of it, so the order needs no host round
+// trip (2,000 genes: a few us, against two copies, a synchronisation and a
+// host sort).
+__global__ void __launch_bounds__(256) k_rank_genes(const int32_t* __restrict__ counts, int32_t g,
+                                                    int32_t* __restrict__ gene2slot, int32_t* __restrict__ slot2gene) {
+  const int lane = threadIdx.x & 31;
+  const int32_t j = (int32_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  if (j >= g) return;
+  const int32_t mine = __ldg(counts + j);
+  int32_t before = 0;
+  for (int32_t i = lane; i < g; i += 32) {
+    const int32_t c = __ldg(counts + i);
+    before += (c > mine || (c == mine && i < j)) ? 1 : 0;
+  }
+  before = (int32_t)__reduce_add_sync(0xffffffffu, (unsigned)before);
+  if (lane == 0) {
+    gene2slot[j] = before;
+    slot2gene[before] = j;
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Chunk-CSC build, one block per row chunk (once per plan).  Counting sort of
+// the chunk's entries by slot that keeps row order inside a slot: warp w takes
+// the w-th run of consecutive rows, counts its entries per slot in shared
+// memory, the block turns the counts into each warp's first position in every
+// slot, and each warp then places its rows in order.  Within one 32-entry
 // step two lanes can name the same gene only across a duplicate; the step is
 // cut into runs of strictly increasing gene, applied in lane order, which
 // keeps the placement (and so the later summation order) deterministic.
-// k_gene_counts gives the stored entries per gene that the slot assignment
-// balances.
+// The scattered stores bound it (each entry writes a part of two sectors: at
+// 100,000 x 2,000 the 115 MB copy causes 835 MB of DRAM writes); up to 16 warps
+// share a chunk and load four steps ahead.  10,000 x 2,000: 74 us against
+// 836 us for one warp per 128-row tile, 100,000: 723 against 1,171 us.
 // ---------------------------------------------------------------------------
-__global__ void k_gene_counts(const int32_t* __restrict__ idx, int64_t nnz, int32_t* __restrict__ counts) {
-  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += (int64_t)gridDim.x * blockDim.x)
-    atomicAdd(counts + __ldg(idx + p), 1);
-}
-
 template <typename ValT>
-__global__ void k_tile_csc(const int64_t* __restrict__ indptr, const int32_t* __restrict__ idx,
-                           const ValT* __restrict__ val, int64_t n, const int32_t* __restrict__ gene2slot,
-                           int32_t nslots, int64_t n_tiles, int32_t* __restrict__ tptr, uint8_t* __restrict__ cell,
-                           ValT* __restrict__ cval) {
-  extern __shared__ int32_t cur_all[];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int warps = blockDim.x >> 5;
-  int32_t* cur = cur_all + (int64_t)wib * (nslots + 1);
-  const unsigned lanemask_le = 0xffffffffu >> (31 - lane);
-  for (int64_t t = (int64_t)blockIdx.x * warps + wib; t < n_tiles; t += (int64_t)gridDim.x * warps) {
-    const int64_t r0 = t * kStrictTile;
-    const int64_t r1 = min(n, r0 + kStrictTile);
-    const int64_t base = indptr[r0];
-    const int64_t end = indptr[r1];
-    for (int j = lane; j <= nslots; j += 32) cur[j] = 0;
-    __syncwarp();
-    // counts (integer atomics: the counts do not depend on the order)
-    for (int64_t p = base + lane; p < end; p += 32) atomicAdd(&cur[__ldg(gene2slot + __ldg(idx + p))], 1);
-    __syncwarp();
-    // exclusive scan of cur[0..nslots] -> offsets; lane owns a contiguous segment
-    const int per = (nslots + 1 + 31) / 32;
-    const int j0 = min(nslots + 1, lane * per), j1 = min(nslots + 1, j0 + per);
-    int32_t sum = 0;
-    for (int j = j0; j < j1; ++j) sum += cur[j];
-    int32_t incl = sum;
+__global__ void __launch_bounds__(512) k_chunk_csc(const int64_t* __restrict__ indptr, const int32_t* __restrict__ idx,
+                                                   const ValT* __restrict__ val, int64_t n, int chunk_rows,
+                                                   const int32_t* __restrict__ gene2slot, int32_t g, bool map_in_smem,
+                                                   int32_t* __restrict__ tptr, uint16_t* __restrict__ row,
+                                                   ValT* __restrict__ cval) {
+  extern __shared__ int32_t cur_all[];  // [warps][g], then gene2slot
+  __shared__ int32_t warp_sum[16];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const int64_t t = blockIdx.x;
+  const int64_t c0 = t * chunk_rows, c1 = min(n, c0 + chunk_rows);
+  const int per_warp = (int)((c1 - c0 + warps - 1) / warps);
+  const int64_t r0 = min(c1, c0 + (int64_t)w * per_warp), r1 = min(c1, r0 + per_warp);
+  const int64_t base = indptr[c0];
+  int32_t* cur = cur_all + (int64_t)w * g;
+  const int32_t* map = gene2slot;
+  if (map_in_smem) {
+    int32_t* m = cur_all + (int64_t)warps * g;
+    for (int j = threadIdx.x; j < g; j += blockDim.x) m[j] = gene2slot[j];
+    map = m;
+  }
+  for (int64_t j = threadIdx.x; j < (int64_t)warps * g; j += blockDim.x) cur_all[j] = 0;
+  __syncthreads();
+  {  // counts (integer atomics: the counts do not depend on the order)
+    const int64_t b = indptr[r0], e = indptr[r1];
+#pragma unroll 4
+    for (int64_t p = b + lane; p < e; p += 32) atomicAdd(&cur[map[__ldg(idx + p)]], 1);
+  }
+  __syncthreads();
+  // exclusive scan over (slot, warp): thread i owns a run of slots
+  const int per = (g + (int)blockDim.x - 1) / (int)blockDim.x;
+  const int j0 = min(g, (int)threadIdx.x * per), j1 = min(g, j0 + per);
+  int32_t sum = 0;
+  for (int j = j0; j < j1; ++j)
+    for (int u = 0; u < warps; ++u) sum += cur_all[(int64_t)u * g + j];
+  int32_t incl = sum;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    int32_t run = incl - sum;
-    for (int j = j0; j < j1; ++j) {
-      const int32_t c = cur[j];
-      cur[j] = run;
-      tptr[t * (nslots + 1) + j] = run;
+  for (int o = 1; o < 32; o <<= 1) {
+    const int32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += y;
+  }
+  if (lane == 31) warp_sum[w] = incl;
+  __syncthreads();
+  int32_t run = incl - sum;
+  for (int u = 0; u < w; ++u) run += warp_sum[u];
+  for (int j = j0; j < j1; ++j) {
+    tptr[t * (g + 1) + j] = run;
+    for (int u = 0; u < warps; ++u) {
+      const int32_t c = cur_all[(int64_t)u * g + j];
+      cur_all[(int64_t)u * g + j] = run;
       run += c;
     }
-    __syncwarp();
-    // fill, rows in order
-    for (int64_t r = r0; r < r1; ++r) {
-      const int64_t s = indptr[r], e = indptr[r + 1];
-      const uint8_t rl = (uint8_t)(r - r0);
-      for (int64_t b = s; b < e; b += 32) {
-        const int64_t p = b + lane;
-        const bool ok = p < e;
-        const int32_t j = ok ? __ldg(idx + p) : -1;
-        const ValT x = ok ? val[p] : ValT();
-        const int32_t jl = __shfl_up_sync(0xffffffffu, j, 1);
-        const unsigned starts = __ballot_sync(0xffffffffu, lane > 0 && ok && j <= jl);
-        const int my_run = __popc(starts & lanemask_le);
-        const int runs = __popc(starts) + 1;
-        const int32_t slot = ok ? __ldg(gene2slot + j) : 0;
-        for (int rr = 0; rr < runs; ++rr) {
-          if (ok && my_run == rr) {
-            const int32_t q = cur[slot]++;
-            cell[base + q] = rl;
-            cval[base + q] = x;
-          }
-          __syncwarp();
+  }
+  if (threadIdx.x == 0) tptr[t * (g + 1) + g] = (int32_t)(indptr[c1] - base);
+  __syncthreads();
+  // placement, rows in order
+  const unsigned lanemask_le = 0xffffffffu >> (31 - lane);
+  if (r0 >= r1) return;
+  // the steps (32 entries of one row) are loaded kAhead steps before they are placed
+  constexpr int kAhead = 4;
+  int32_t sj[kAhead];
+  ValT sx[kAhead];
+  int sr[kAhead];  // row within the chunk, -1 past the last step
+  int64_t r = r0, b = indptr[r0], e = indptr[r0 + 1];
+  auto fetch = [&](int u) {
+    while (b >= e && ++r < r1) {  // the next row with entries
+      b = e;
+      e = indptr[r + 1];
+    }
+    sr[u] = r < r1 ? (int)(r - c0) : -1;
+    const bool ok = r < r1 && b + lane < e;
+    sj[u] = ok ? __ldg(idx + b + lane) : -1;
+    sx[u] = ok ? val[b + lane] : ValT();
+    b += 32;
+    if (b > e) b = e;
+  };
+#pragma unroll
+  for (int u = 0; u < kAhead; ++u) fetch(u);
+  while (sr[0] >= 0) {
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int32_t j = sj[u];
+      const ValT x = sx[u];
+      const int rl = sr[u];
+      fetch(u);
+      const bool ok = j >= 0;
+      const int32_t jl = __shfl_up_sync(0xffffffffu, j, 1);
+      const unsigned starts = __ballot_sync(0xffffffffu, lane > 0 && ok && j <= jl);
+      const int my_run = __popc(starts & lanemask_le);
+      const int runs = __popc(starts) + 1;
+      const int32_t slot = ok ? map[j] : 0;
+      for (int rr = 0; rr < runs; ++rr) {
+        if (ok && my_run == rr) {
+          const int32_t q = cur[slot];
+          cur[slot] = q + 1;
+          row[base + q] = (uint16_t)rl;
+          cval[base + q] = x;
         }
+        __syncwarp();
       }
     }
-    __syncwarp();
   }
 }
 
 // ---------------------------------------------------------------------------
-// Forward product, quarter-warp layout.  A quarter (8 lanes) owns RPQ rows and
-// lane l8 of it the columns 4 l8 + 32 s + e (s < LD / 32, e < 4) of each:
-// an entry's V row is read as LD / 32 16-byte loads per lane, the quarter's
-// eight lanes covering 128 consecutive bytes, so the four quarters of a warp
-// read four V rows in four shared-memory wavefronts, conflict-free.  Each
-// entry is broadcast to the 8 lanes of its quarter only (the four quarters
-// take four entries with one shuffle), and every lane does 4 LD / 32 FMAs per
-// entry, against 2 shuffles for LD / 32 FMAs when a whole warp owns a row
-// (measured at 250,000 cells, LD 64: 1.51 ms against 1.85 ms per launch).
-//
-// Per gene chunk and row, each quarter keeps an 8-entry window of the row
-// (one entry per lane; consumed entries marked -1, entries past the row's
-// end INT32_MAX), takes the entries whose gene falls in the chunk (the next
-// unconsumed ones: rows are sorted), and reloads the window once all 8 are
-// consumed.  The four quarters step together: a step runs the largest take
-// count of the four, and a quarter past its own count adds 0 x (a staged row
-// of V), so every shuffle is warp-uniform.  Entries are added in row order.
+// Forward product.  Block (slice, range) owns 32 columns of a contiguous range
+// of cells, kRowBlock of them at a time, and takes the genes in chunks of
+// `table_rows`: V's chunk is staged, every cell's entries inside the chunk are
+// walked, and the sums go to Y (read back by the same lanes for the next
+// chunk; the entries are added in row order whatever the chunks).  The cells
+// are ordered by length (a counting sort over kBuckets classes): the order
+// only decides which lanes take which cell, not any result.  A walk stops at
+// the first gene past the chunk (rows are sorted); where it stopped is kept in
+// shared memory for the next chunk.
 // ---------------------------------------------------------------------------
-template <int LD, int RPQ, int GC, typename ValT>
-__global__ void __launch_bounds__(256, 2) k_fwd_strict_q(const int64_t* __restrict__ indptr,
-                                                         const int32_t* __restrict__ idx,
-                                                         const ValT* __restrict__ val, int64_t n, int32_t g,
-                                                         const float* __restrict__ V, const float* __restrict__ mc,
-                                                         float* __restrict__ Y, int lds) {
-  constexpr int S4 = LD / 32;  // 16-byte column groups per lane
-  constexpr int32_t kDone = -1;
-  constexpr unsigned FULL = 0xffffffffu;
-  static_assert(RPQ <= 8, "a quarter holds the window bounds of its rows in its 8 lanes");
-  extern __shared__ __align__(16) float vs[];  // [2][GC][LD]
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int qw = lane >> 3, l8 = lane & 7;
-  const int64_t row0 = (int64_t)blockIdx.x * (32 * RPQ) + (int64_t)wib * (4 * RPQ) + qw * RPQ;
-  // lane l8 < RPQ of a quarter: window start and end of its row row0 + l8
-  int64_t my_base = 0, my_end = 0;
-  if (l8 < RPQ && row0 + l8 < n) {
-    my_base = indptr[row0 + l8];
-    my_end = indptr[row0 + l8 + 1];
-  }
-  float acc[RPQ][4 * S4];
-  int32_t wi[RPQ], ni[RPQ];  // the window, and the next 8 entries of the row already loaded
-  float wv[RPQ], nv[RPQ];
-#pragma unroll
-  for (int r = 0; r < RPQ; ++r) {
-#pragma unroll
-    for (int c = 0; c < 4 * S4; ++c) acc[r][c] = 0.f;
-    const int64_t base = __shfl_sync(FULL, my_base, r, 8);
-    const int64_t end = __shfl_sync(FULL, my_end, r, 8);
-    const int64_t p = base + l8;
-    wi[r] = p < end ? __ldg(idx + p) : INT32_MAX;
-    wv[r] = p < end ? to_f32(val[p]) : 0.f;
-    ni[r] = p + 8 < end ? __ldg(idx + p + 8) : INT32_MAX;
-    nv[r] = p + 8 < end ? to_f32(val[p + 8]) : 0.f;
-  }
-  const int nchunk = (g + GC - 1) / GC;
-  block_copy_rows_async<LD>(vs, V, min(GC, (int)g), lds);
-  cp_async_commit();
-  for (int ch = 0; ch < nchunk; ++ch) {
-    const int g0 = ch * GC;
-    const int g1 = min((int)g, g0 + GC);
-    if (ch + 1 < nchunk) {
-      const int n1 = min(GC, (int)g - g1);
-      block_copy_rows_async<LD>(vs + ((ch + 1) & 1) * GC * LD, V + (int64_t)g1 * lds, n1, lds);
-    }
-    cp_async_commit();
-    cp_async_wait<1>();
+template <bool VEC, int NV, typename ValT>
+__global__ void __launch_bounds__(kThreads, 1)
+    k_fwd_strict(const int64_t* __restrict__ indptr, const int32_t* __restrict__ idx, const ValT* __restrict__ val,
+                 int64_t n, int32_t g, int nslice, int64_t rows_per_range, int table_rows,
+                 const float* __restrict__ V, const float* __restrict__ mc, float* Y, int lds) {
+  extern __shared__ __align__(128) char smem[];
+  float* tab = reinterpret_cast<float*>(smem);
+  uint32_t* cursor = reinterpret_cast<uint32_t*>(smem + (size_t)(table_rows + 1) * (64 * NV));
+  int32_t* bucket = reinterpret_cast<int32_t*>(cursor + kRowBlock);
+  uint16_t* order = reinterpret_cast<uint16_t*>(bucket + kBuckets);
+  __shared__ int32_t longest;
+  const int tid = threadIdx.x, lane = tid & 31, l = tid % kLanes, list = tid / kLanes, odd = list & 1;
+  const int slice = blockIdx.x % nslice;
+  const int64_t range = blockIdx.x / nslice;
+  const int64_t r0 = range * rows_per_range, r1 = min(n, r0 + rows_per_range);
+  const int nch = (g + table_rows - 1) / table_rows;
+  const int64_t lim = indptr[n];
+  const int col = slice * (16 * NV) + 4 * l;
+  const unsigned tab_lane = (unsigned)__cvta_generic_to_shared(smem) + 16 * l + 64 * odd;
+  float m[4 * NV] = {};
+  if (mc) load_cols<NV>(m, mc + col, odd);
+  for (int64_t rb = r0; rb < r1; rb += kRowBlock) {
+    const int rows = (int)min((int64_t)kRowBlock, r1 - rb);
+    // order the cells by decreasing number of entries
+    if (tid == 0) longest = 1;
+    for (int b = tid; b < kBuckets; b += kThreads) bucket[b] = 0;
     __syncthreads();
-    const float* vc = vs + (ch & 1) * GC * LD + 4 * l8;
+    for (int i = tid; i < rows; i += kThreads) {
+      const int64_t len = indptr[rb + i + 1] - indptr[rb + i];
+      cursor[i] = (uint32_t)min(len, (int64_t)INT32_MAX);
+      atomicMax(&longest, (int)cursor[i]);
+    }
+    __syncthreads();
+    const float scale = (float)(kBuckets - 1) / (float)longest;
+    auto bucket_of = [&](int i) { return kBuckets - 1 - min(kBuckets - 1, (int)((float)cursor[i] * scale)); };
+    for (int i = tid; i < rows; i += kThreads) atomicAdd(&bucket[bucket_of(i)], 1);
+    __syncthreads();
+    if (tid < 32) {  // exclusive scan of the classes
+      int32_t run = 0;
+      for (int b = lane; b < kBuckets; b += 32) {
+        const int32_t c = bucket[b];
+        int32_t incl = c;
 #pragma unroll
-    for (int r = 0; r < RPQ; ++r) {
-      while (true) {
-        const bool take = (unsigned)wi[r] < (unsigned)g1;
-        const unsigned mq = (__ballot_sync(FULL, take) >> (8 * qw)) & 0xffu;
-        const int cnt = __popc(mq);
-        const int t0 = cnt ? __ffs(mq) - 1 : 0;
-        const int steps = (int)__reduce_max_sync(FULL, (unsigned)cnt);
-        for (int t = 0; t < steps; ++t) {
-          const int src = min(t0 + t, 7);
-          const int32_t j = __shfl_sync(FULL, wi[r], src, 8);
-          const float x = __shfl_sync(FULL, wv[r], src, 8);
-          const bool in = t < cnt;
-          const float xs = in ? x : 0.f;
-          // a taken gene is in [g0, g1); a step past the quarter's count
-          // reads row 0 of the chunk (always staged) and adds zero
-          const unsigned jl = in ? min((unsigned)(j - g0), (unsigned)(GC - 1)) : 0u;
-          const float* vr = vc + jl * LD;
-#pragma unroll
-          for (int s4 = 0; s4 < S4; ++s4) {
-            const float4 v = *reinterpret_cast<const float4*>(vr + 32 * s4);
-            acc[r][4 * s4 + 0] = fmaf(xs, v.x, acc[r][4 * s4 + 0]);
-            acc[r][4 * s4 + 1] = fmaf(xs, v.y, acc[r][4 * s4 + 1]);
-            acc[r][4 * s4 + 2] = fmaf(xs, v.z, acc[r][4 * s4 + 2]);
-            acc[r][4 * s4 + 3] = fmaf(xs, v.w, acc[r][4 * s4 + 3]);
-          }
+        for (int o = 1; o < 32; o <<= 1) {
+          const int32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += y;
         }
-        if (take) wi[r] = kDone;
-        // a quarter whose 8 window entries are all consumed loads the next 8
-        const unsigned dq = (__ballot_sync(FULL, wi[r] == kDone) >> (8 * qw)) & 0xffu;
-        const bool reload = dq == 0xffu;
-        if (!__any_sync(FULL, reload)) break;
-        if (reload && l8 == r) my_base += 8;
-        const int64_t base = __shfl_sync(FULL, my_base, r, 8);
-        const int64_t end = __shfl_sync(FULL, my_end, r, 8);
-        if (reload) {
-          // the next window was loaded a window ahead; fetch the one after it
-          wi[r] = ni[r];
-          wv[r] = nv[r];
-          const int64_t p = base + 8 + l8;
-          ni[r] = p < end ? __ldg(idx + p) : INT32_MAX;
-          nv[r] = p < end ? to_f32(val[p]) : 0.f;
-        }
+        bucket[b] = run + incl - c;
+        run += __shfl_sync(0xffffffffu, incl, 31);
       }
     }
-    __syncthreads();  // everyone is done with this buffer before it is refilled
-  }
-  cp_async_wait<0>();
-  float m[4 * S4];
+    __syncthreads();
+    for (int i = tid; i < rows; i += kThreads) order[atomicAdd(&bucket[bucket_of(i)], 1)] = (uint16_t)i;
+    __syncthreads();
+    for (int i = tid; i < rows; i += kThreads) cursor[i] = 0;
+    for (int ch = 0; ch < nch; ++ch) {
+      const int g0 = ch * table_rows, g1 = min((int)g, g0 + table_rows);
+      const bool last = ch + 1 == nch;
+      if (ch > 0 || nch > 1 || rb == r0) {  // one chunk: the table stays
+        __syncthreads();                    // everyone is done with the table
+        stage_table<NV>(tab, V + (int64_t)g0 * lds + slice * (16 * NV), g1 - g0, lds);
+      }
+      __syncthreads();
+      int64_t nbase = 0, nend = 0;  // the next cell's bounds, read one cell ahead
+      if (list < rows) {
+        nbase = indptr[rb + order[list]];
+        nend = indptr[rb + order[list] + 1];
+      }
+      for (int i = list; i < rows; i += kLists) {
+        const int rl = order[i];
+        const int64_t row = rb + rl;
+        const int64_t base = nbase, s = base + cursor[rl], e = nend;
+        if (i + kLists < rows) {
+          nbase = indptr[rb + order[i + kLists]];
+          nend = indptr[rb + order[i + kLists] + 1];
+        }
+        float* y = Y + row * lds + col;
+        float acc[4 * NV] = {};
+        if (ch > 0) load_cols<NV>(acc, y, odd);
+        const int64_t stop = walk<VEC, true, NV>(acc, idx, val, s, e, lim, g0, g1 - g0, tab_lane);
+        if (last) {
 #pragma unroll
-  for (int s4 = 0; s4 < S4; ++s4)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) m[4 * s4 + e] = mc ? mc[4 * l8 + 32 * s4 + e] : 0.f;
-#pragma unroll
-  for (int r = 0; r < RPQ; ++r) {
-    const int64_t row = row0 + r;
-    if (row < n) {
-#pragma unroll
-      for (int s4 = 0; s4 < S4; ++s4)
-        *reinterpret_cast<float4*>(Y + row * lds + 4 * l8 + 32 * s4) =
-            make_float4(acc[r][4 * s4 + 0] - m[4 * s4 + 0], acc[r][4 * s4 + 1] - m[4 * s4 + 1],
-                        acc[r][4 * s4 + 2] - m[4 * s4 + 2], acc[r][4 * s4 + 3] - m[4 * s4 + 3]);
+          for (int c = 0; c < 4 * NV; ++c) acc[c] -= m[c];
+        } else if (l == 0) {  // read next after the block's barrier
+          cursor[rl] = (uint32_t)(stop - base);
+        }
+        store_cols<NV>(y, acc, odd);
+      }
     }
+    __syncthreads();  // the order and the cursors are rewritten
   }
 }
 
 // ---------------------------------------------------------------------------
-// Transposed product, quarter-warp layout.  Block (range, b) owns the slots
-// [b 32 GPQ, (b + 1) 32 GPQ) and the row tiles of one contiguous range; warp
-// w owns the GPW = 4 GPQ slots of one group of the slot assignment
-// (strict_genes_per_warp), and its quarter qw the slots slot0 + 4 i + qw
-// (i < GPQ), so the group's heaviest genes, which fill its first slots,
-// spread over the four quarters.  For each tile, Q's rows (kStrictTile x LD
-// floats) are staged in shared memory (double-buffered, asynchronous
-// copies).  The block writes one partial row per gene it owns.  Lane l8 owns
-// the columns 4 l8 + 32 s + e: a cell's Q row is read as LD / 32 16-byte
-// loads per lane, the quarter covering 128 consecutive bytes, and each entry
-// is broadcast within its quarter only.  For each slot the four quarters walk
-// their entry lists 8 at a time in step (the longest list sets the count; a
-// lane past its list holds x = 0 and cell 0, a staged row).  Entries are added
-// in tile-CSC order, so the partials do not depend on the schedule.
+// Transposed product.  Block (slice, range) owns 32 columns of the row chunks
+// of one contiguous range; for each chunk it stages Q's rows and walks every
+// slot's list, a warp taking eight neighbouring slots.  The sums go
+// to the range's partial (read back by the same lanes for the next chunk).
+// Entries are added in (chunk, row) order.
 // ---------------------------------------------------------------------------
-template <int LD, int GPQ, typename ValT>
-__global__ void __launch_bounds__(256, 2) k_rmat_strict_q(const int64_t* __restrict__ indptr,
-                                                          const int32_t* __restrict__ tptr,
-                                                          const uint8_t* __restrict__ cell,
-                                                          const ValT* __restrict__ cval, int64_t n, int32_t g,
-                                                          int32_t nslots, const int32_t* __restrict__ slot2gene,
-                                                          int64_t tiles_per_range, const float* __restrict__ Q,
-                                                          int lds, float* __restrict__ part) {
-  constexpr int S4 = LD / 32;
-  constexpr int T = kStrictTile;
-  constexpr unsigned FULL = 0xffffffffu;
-  static_assert(GPQ <= 8, "a quarter holds the list bounds of its slots in its 8 lanes");
-  extern __shared__ __align__(16) float qs[];  // [2][T][LD]
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int qw = lane >> 3, l8 = lane & 7;
-  const int64_t n_tiles = (n + T - 1) / T;
-  const int64_t t0 = (int64_t)blockIdx.x * tiles_per_range;
-  const int64_t t1 = min(n_tiles, t0 + tiles_per_range);
-  const int slot0 = (blockIdx.y * 8 + wib) * (4 * GPQ);
-  // lane l8 < GPQ of a quarter reads the list bounds of its slot i = l8
-  const int my_slot = slot0 + 4 * (l8 % GPQ) + qw;
-  float acc[GPQ][4 * S4];
-#pragma unroll
-  for (int i = 0; i < GPQ; ++i)
-#pragma unroll
-    for (int c = 0; c < 4 * S4; ++c) acc[i][c] = 0.f;
-  if (t0 < t1) {
-    auto stage = [&](int64_t t, int buf) {
-      const int64_t r0 = t * T;
-      const int rows = (int)min((int64_t)T, n - r0);
-      block_copy_rows_async<LD>(qs + buf * T * LD, Q + r0 * lds, rows, lds);
-    };
-    stage(t0, 0);
-    cp_async_commit();
-    for (int64_t t = t0; t < t1; ++t) {
-      const int buf = (int)((t - t0) & 1);
-      if (t + 1 < t1) stage(t + 1, buf ^ 1);
-      cp_async_commit();
-      const int64_t tb = indptr[t * T];
-      int32_t p0 = 0, p1 = 0;
-      if (my_slot < nslots) {
-        p0 = __ldg(tptr + t * (nslots + 1) + my_slot);
-        p1 = __ldg(tptr + t * (nslots + 1) + my_slot + 1);
-      }
-      cp_async_wait<1>();
-      __syncthreads();
-      const float* qt = qs + buf * T * LD + 4 * l8;
-#pragma unroll
-      for (int i = 0; i < GPQ; ++i) {
-        const int32_t s = __shfl_sync(FULL, p0, i, 8);
-        const int32_t len = __shfl_sync(FULL, p1, i, 8) - s;
-        const int32_t longest = (int32_t)__reduce_max_sync(FULL, (unsigned)max(len, 0));
-        for (int32_t b = 0; b < longest; b += 8) {
-          const int32_t q = b + l8;
-          int cl = 0;
-          float x = 0.f;
-          if (q < len) {
-            cl = __ldg(cell + tb + s + q);
-            x = to_f32(cval[tb + s + q]);
-          }
-          const int steps = min(8, longest - b);
-          for (int u = 0; u < steps; ++u) {
-            const int cu = __shfl_sync(FULL, cl, u, 8) & (T - 1);
-            const float xu = __shfl_sync(FULL, x, u, 8);
-            const float* qr = qt + cu * LD;
-#pragma unroll
-            for (int s4 = 0; s4 < S4; ++s4) {
-              const float4 v = *reinterpret_cast<const float4*>(qr + 32 * s4);
-              acc[i][4 * s4 + 0] = fmaf(xu, v.x, acc[i][4 * s4 + 0]);
-              acc[i][4 * s4 + 1] = fmaf(xu, v.y, acc[i][4 * s4 + 1]);
-              acc[i][4 * s4 + 2] = fmaf(xu, v.z, acc[i][4 * s4 + 2]);
-              acc[i][4 * s4 + 3] = fmaf(xu, v.w, acc[i][4 * s4 + 3]);
-            }
-          }
-        }
-      }
-      __syncthreads();  // this buffer is read before it is refilled
+template <int NV, typename ValT>
+__global__ void __launch_bounds__(kThreads, 1)
+    k_rmat_strict(const int64_t* __restrict__ indptr, const int32_t* __restrict__ tptr,
+                  const uint16_t* __restrict__ row, const ValT* __restrict__ cval, int64_t n, int32_t g,
+                  const int32_t* __restrict__ slot2gene, int chunk_rows, int64_t n_chunks, int chunks_per_range,
+                  int nslice, const float* __restrict__ Q, int lds, float* part, int ldp) {
+  extern __shared__ __align__(128) char smem[];
+  float* tab = reinterpret_cast<float*>(smem);
+  const int tid = threadIdx.x, l = tid % kLanes, list = tid / kLanes, odd = list & 1;
+  const unsigned tab_lane = (unsigned)__cvta_generic_to_shared(smem) + 16 * l + 64 * odd;
+  const int slice = blockIdx.x % nslice;
+  const int64_t range = blockIdx.x / nslice;
+  const int64_t t0 = range * chunks_per_range, t1 = min(n_chunks, t0 + chunks_per_range);
+  float* out = part + range * g * ldp + slice * (16 * NV) + 4 * l;
+  for (int64_t t = t0; t < t1; ++t) {
+    const int64_t r0 = t * chunk_rows;
+    const int rows = (int)min((int64_t)chunk_rows, n - r0);
+    __syncthreads();  // everyone is done with the table
+    stage_table<NV>(tab, Q + r0 * lds + slice * (16 * NV), rows, lds);
+    __syncthreads();
+    const int64_t base = indptr[r0], lim = indptr[r0 + rows];
+    const int32_t* tp = tptr + t * (g + 1);
+    int nb = 0, ne = 0, ng = 0;  // the next list's bounds and gene, read one list ahead
+    if (list < g) {
+      nb = __ldg(tp + list);
+      ne = __ldg(tp + list + 1);
+      ng = __ldg(slot2gene + list);
     }
-    cp_async_wait<0>();
-  }
-  float* out = part + (int64_t)blockIdx.x * g * LD;
-#pragma unroll
-  for (int i = 0; i < GPQ; ++i) {
-    const int slot = slot0 + 4 * i + qw;
-    const int j = slot < nslots ? __ldg(slot2gene + slot) : -1;
-    if (j >= 0) {
-#pragma unroll
-      for (int s4 = 0; s4 < S4; ++s4)
-        *reinterpret_cast<float4*>(out + (int64_t)j * LD + 4 * l8 + 32 * s4) =
-            make_float4(acc[i][4 * s4 + 0], acc[i][4 * s4 + 1], acc[i][4 * s4 + 2], acc[i][4 * s4 + 3]);
+    for (int s = list; s < g; s += kLists) {
+      const int64_t b = base + nb, e = base + ne;
+      float* w = out + (int64_t)ng * ldp;
+      if (s + kLists < g) {
+        nb = __ldg(tp + s + kLists);
+        ne = __ldg(tp + s + kLists + 1);
+        ng = __ldg(slot2gene + s + kLists);
+      }
+      if (t > t0 && b >= e) continue;
+      float acc[4 * NV] = {};
+      if (t > t0) load_cols<NV>(acc, w, odd);
+      walk<true, false, NV>(acc, row, cval, b, e, lim, 0, rows, tab_lane);
+      store_cols<NV>(w, acc, odd);
     }
   }
 }
@@ -399,176 +570,149 @@ __global__ void __launch_bounds__(256, 2) k_rmat_strict_q(const int64_t* __restr
 // ---------------------------------------------------------------------------
 // Host launchers
 // ---------------------------------------------------------------------------
-int strict_genes_per_warp(int ld) { return ld <= 64 ? 32 : 16; }
 
-int strict_slot_count(int64_t g, int ld) {
-  const int per_block = 8 * strict_genes_per_warp(ld);
-  return (int)((g + per_block - 1) / per_block) * per_block;
+// The transposed product's row chunks: the ranges of all slices fill the SMs
+// once, a range is a whole number of equal chunks that fit the table, and a
+// chunk has at least 64 rows (below that a list is shorter than its set-up).
+StrictGeometry strict_geometry(int64_t n, int ld, int num_sms) {
+  StrictGeometry geo;
+  geo.cols = slice_cols(ld, n, num_sms);
+  const int nslice = ld / geo.cols, table_rows = rmat_table_rows(geo.cols);
+  const int64_t want = std::max<int64_t>(1, num_sms / nslice);
+  const int64_t per = std::max<int64_t>(64, (n + want - 1) / want);
+  const int64_t m = (per + table_rows - 1) / table_rows;
+  geo.rows = (int)((per + m - 1) / m);
+  geo.chunks = (n + geo.rows - 1) / geo.rows;
+  geo.per_range = (int)m;
+  geo.ranges = (int)((geo.chunks + m - 1) / m);
+  return geo;
 }
 
-// Longest-processing-time assignment of genes to the warps of the
-// transposed product: genes in decreasing stored-entry count (ties by gene
-// index) each go to the warp group with the smallest count so far that still
-// has a free slot (ties by group index).  slot2gene[s] = -1 marks an empty
-// slot.  Deterministic for given counts.
-void strict_assign_slots(const std::vector<int32_t>& counts, int ld, std::vector<int32_t>& gene2slot,
-                         std::vector<int32_t>& slot2gene) {
-  const int64_t g = (int64_t)counts.size();
-  const int gpw = strict_genes_per_warp(ld);
-  const int nslots = strict_slot_count(g, ld);
-  const int groups = nslots / gpw;
-  std::vector<int32_t> order(g);
-  for (int64_t j = 0; j < g; ++j) order[j] = (int32_t)j;
-  std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return counts[a] > counts[b]; });
-  // min-heap of (load, group) over groups with a free slot
-  using Item = std::pair<int64_t, int32_t>;
-  std::priority_queue<Item, std::vector<Item>, std::greater<Item>> heap;
-  for (int32_t q = 0; q < groups; ++q) heap.push({0, q});
-  std::vector<int32_t> fill(groups, 0);
-  gene2slot.assign(g, 0);
-  slot2gene.assign(nslots, -1);
-  for (int32_t j : order) {
-    Item it = heap.top();
-    heap.pop();
-    const int32_t q = it.second;
-    const int32_t slot = q * gpw + fill[q]++;
-    gene2slot[j] = slot;
-    slot2gene[slot] = j;
-    if (fill[q] < gpw) heap.push({it.first + counts[j], q});
-  }
+// The per-warp slot counters of the chunk-CSC build have to fit shared memory.
+bool strict_csc_fits(int64_t g, int ld) {
+  const int64_t unit = ld <= 64 ? 256 : 128;
+  return sizeof(int32_t) * (size_t)((g + unit - 1) / unit * unit + 1) <= kStatsSmemMax;
 }
 
-cudaError_t launch_gene_counts(const int32_t* idx, int64_t nnz, int32_t* counts, cudaStream_t st, int num_sms) {
+cudaError_t launch_gene_counts(const int32_t* idx, int64_t nnz, int32_t g, int32_t* counts, cudaStream_t st,
+                               int num_sms) {
   if (nnz == 0) return cudaSuccess;
-  k_gene_counts<<<grid_for(nnz, 256, num_sms), 256, 0, st>>>(idx, nnz, counts);
   note_launches(1);
+  const size_t smem = sizeof(int32_t) * (size_t)g;
+  if (smem <= 100 * 1024) {  // two blocks per SM
+    if (smem > 48 * 1024)
+      if (cudaError_t e = allow_smem(k_gene_counts, smem); e != cudaSuccess) return e;
+    k_gene_counts<<<grid_for(nnz, 8192, num_sms, 2), 512, smem, st>>>(idx, nnz, g, counts);
+  } else {
+    k_gene_counts_global<<<grid_for(nnz, 256, num_sms), 256, 0, st>>>(idx, nnz, g, counts);
+  }
   return cudaGetLastError();
 }
 
-size_t strict_tile_smem_bytes(int nslots) { return sizeof(int32_t) * (size_t)(nslots + 1); }
+cudaError_t launch_rank_genes(const int32_t* counts, int32_t g, int32_t* gene2slot, int32_t* slot2gene,
+                              cudaStream_t st) {
+  note_launches(1);
+  k_rank_genes<<<(unsigned)(((int64_t)g + 7) / 8), 256, 0, st>>>(counts, g, gene2slot, slot2gene);
+  return cudaGetLastError();
+}
 
 template <typename ValT>
-static cudaError_t tile_csc_t(const int64_t* indptr, const int32_t* idx, const void* val, int64_t n,
-                              const int32_t* gene2slot, int32_t nslots, int32_t* tptr, uint8_t* cell, void* cval,
-                              cudaStream_t st, int num_sms) {
-  const int64_t n_tiles = (n + kStrictTile - 1) / kStrictTile;
-  const size_t per_warp = strict_tile_smem_bytes(nslots);
+static cudaError_t chunk_csc_t(const int64_t* indptr, const int32_t* idx, const void* val, int64_t n,
+                               const StrictGeometry& geo, const int32_t* gene2slot, int32_t g, int32_t* tptr,
+                               uint16_t* row, void* cval, cudaStream_t st) {
+  const size_t per_warp = sizeof(int32_t) * (size_t)g;
   if (per_warp > kStatsSmemMax) return cudaErrorInvalidValue;
-  const int warps = (int)std::min<size_t>(8, kStatsSmemMax / per_warp);
-  const size_t smem = per_warp * warps;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_tile_csc<ValT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>((n_tiles + warps - 1) / warps, (int64_t)num_sms * 4));
-  k_tile_csc<ValT><<<grid, warps * 32, smem, st>>>(indptr, idx, static_cast<const ValT*>(val), n, gene2slot, nslots,
-                                                   n_tiles, tptr, cell, static_cast<ValT*>(cval));
+  int warps = (int)std::min<size_t>(16, kStatsSmemMax / per_warp);
+  warps = std::max(1, std::min(warps, (geo.rows + 3) / 4));
+  // the slot map beside the counters where it fits (a gather per entry from L1
+  // costs a tag lookup per line it touches)
+  const bool map_in_smem = per_warp * (warps + 1) <= kStatsSmemMax;
+  const size_t smem = per_warp * (warps + (map_in_smem ? 1 : 0));
+  if (smem > 48 * 1024)
+    if (cudaError_t e = allow_smem(k_chunk_csc<ValT>, smem); e != cudaSuccess) return e;
+  k_chunk_csc<ValT><<<(unsigned)geo.chunks, warps * 32, smem, st>>>(indptr, idx, static_cast<const ValT*>(val), n,
+                                                                    geo.rows, gene2slot, g, map_in_smem, tptr, row,
+                                                                    static_cast<ValT*>(cval));
   note_launches(1);
   return cudaGetLastError();
 }
 
-cudaError_t launch_tile_csc(int dtype, const int64_t* indptr, const int32_t* idx, const void* val, int64_t n,
-                            const int32_t* gene2slot, int32_t nslots, int32_t* tptr, uint8_t* cell, void* cval,
-                            cudaStream_t st, int num_sms) {
+cudaError_t launch_chunk_csc(int dtype, const int64_t* indptr, const int32_t* idx, const void* val, int64_t n,
+                             const StrictGeometry& geo, const int32_t* gene2slot, int32_t g, int32_t* tptr,
+                             uint16_t* row, void* cval, cudaStream_t st) {
   if (n == 0) return cudaSuccess;
   switch (dtype) {
-    case 0: return tile_csc_t<float>(indptr, idx, val, n, gene2slot, nslots, tptr, cell, cval, st, num_sms);
-    case 1: return tile_csc_t<__nv_bfloat16>(indptr, idx, val, n, gene2slot, nslots, tptr, cell, cval, st, num_sms);
-    default: return tile_csc_t<__half>(indptr, idx, val, n, gene2slot, nslots, tptr, cell, cval, st, num_sms);
+    case 0: return chunk_csc_t<float>(indptr, idx, val, n, geo, gene2slot, g, tptr, row, cval, st);
+    case 1: return chunk_csc_t<__nv_bfloat16>(indptr, idx, val, n, geo, gene2slot, g, tptr, row, cval, st);
+    default: return chunk_csc_t<__half>(indptr, idx, val, n, geo, gene2slot, g, tptr, row, cval, st);
   }
-}
-
-template <int LD, typename ValT>
-static cudaError_t fwd_strict_t(const int64_t* indptr, const int32_t* idx, const void* val, int64_t n, int32_t g,
-                                const float* V, const float* mc, float* Y, int lds, cudaStream_t st) {
-  constexpr int RPQ = LD <= 32 ? 8 : 4;  // rows per quarter-warp: RPQ x LD / 8 accumulators per lane
-  constexpr int GC = (8192 / LD) & ~7;
-  const size_t smem = (size_t)2 * GC * LD * sizeof(float);
-  auto kern = k_fwd_strict_q<LD, RPQ, GC, ValT>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  const int64_t rows_per_block = 32 * RPQ;
-  const int64_t grid = (n + rows_per_block - 1) / rows_per_block;
-  kern<<<(unsigned)grid, 256, smem, st>>>(indptr, idx, static_cast<const ValT*>(val), n, g, V, mc, Y, lds);
-  note_launches(1);
-  return cudaGetLastError();
 }
 
 template <typename ValT>
-static cudaError_t fwd_strict_v(int ld, const int64_t* indptr, const int32_t* idx, const void* val, int64_t n,
-                                int32_t g, const float* V, const float* mc, float* Y, int lds, cudaStream_t st) {
-  switch (ld) {
-    case 32: return fwd_strict_t<32, ValT>(indptr, idx, val, n, g, V, mc, Y, lds, st);
-    case 64: return fwd_strict_t<64, ValT>(indptr, idx, val, n, g, V, mc, Y, lds, st);
-    case 96: return fwd_strict_t<96, ValT>(indptr, idx, val, n, g, V, mc, Y, lds, st);
-    case 128: return fwd_strict_t<128, ValT>(indptr, idx, val, n, g, V, mc, Y, lds, st);
-    default: return cudaErrorInvalidValue;
-  }
+static cudaError_t fwd_strict_t(int ld, const int64_t* indptr, const int32_t* idx, const void* val, int64_t n,
+                                int32_t g, const float* V, const float* mc, float* Y, int lds, cudaStream_t st,
+                                int num_sms) {
+  const int cols = slice_cols(ld, n, num_sms), nslice = ld / cols;
+  const int nch = (g + fwd_table_rows(cols) - 1) / fwd_table_rows(cols);
+  const int table_rows = (g + nch - 1) / nch;
+  const size_t smem = (size_t)(table_rows + 1) * cols * 4 + kFwdSmemFixed;
+  const int64_t want = std::max<int64_t>(1, num_sms / nslice);
+  const int64_t per = std::max<int64_t>((n + want - 1) / want, 1);
+  const int64_t ranges = (n + per - 1) / per;
+  // a caller's matrix may sit at any element: vector loads need both arrays
+  // aligned to eight elements
+  const bool vec = (reinterpret_cast<uintptr_t>(idx) & 31) == 0 &&
+                   (reinterpret_cast<uintptr_t>(val) & (8 * sizeof(ValT) - 1)) == 0;
+  auto go = [&](auto kern) {
+    if (cudaError_t e = allow_smem(kern, smem); e != cudaSuccess) return e;
+    kern<<<(unsigned)(ranges * nslice), kThreads, smem, st>>>(indptr, idx, static_cast<const ValT*>(val), n, g,
+                                                              nslice, per, table_rows, V, mc, Y, lds);
+    note_launches(1);
+    return cudaGetLastError();
+  };
+  if (cols == 64) return vec ? go(k_fwd_strict<true, 4, ValT>) : go(k_fwd_strict<false, 4, ValT>);
+  return vec ? go(k_fwd_strict<true, 2, ValT>) : go(k_fwd_strict<false, 2, ValT>);
 }
 
 cudaError_t launch_fwd_strict(int dtype, int ld, const int64_t* indptr, const int32_t* idx, const void* val,
                               int64_t n, int32_t g, const float* V, const float* mc, float* Y, cudaStream_t st,
-                              int lds) {
+                              int num_sms, int lds) {
   if (n == 0) return cudaSuccess;
   if (lds == 0) lds = ld;
-  if (lds < ld || (lds & 3)) return cudaErrorInvalidValue;
+  if (lds < ld || (lds & 3) || ld % 32 || ld > kMaxK) return cudaErrorInvalidValue;
   switch (dtype) {
-    case 0: return fwd_strict_v<float>(ld, indptr, idx, val, n, g, V, mc, Y, lds, st);
-    case 1: return fwd_strict_v<__nv_bfloat16>(ld, indptr, idx, val, n, g, V, mc, Y, lds, st);
-    default: return fwd_strict_v<__half>(ld, indptr, idx, val, n, g, V, mc, Y, lds, st);
+    case 0: return fwd_strict_t<float>(ld, indptr, idx, val, n, g, V, mc, Y, lds, st, num_sms);
+    case 1: return fwd_strict_t<__nv_bfloat16>(ld, indptr, idx, val, n, g, V, mc, Y, lds, st, num_sms);
+    default: return fwd_strict_t<__half>(ld, indptr, idx, val, n, g, V, mc, Y, lds, st, num_sms);
   }
-}
-
-template <int LD, typename ValT>
-static cudaError_t rmat_strict_t(const int64_t* indptr, const int32_t* tptr, const uint8_t* cell, const void* cval,
-                                 int64_t n, int32_t g, int32_t nslots, const int32_t* slot2gene, int ranges,
-                                 const float* Q, int lds, float* part, cudaStream_t st) {
-  constexpr int GPW = LD <= 64 ? 32 : 16;  // slots per warp (strict_genes_per_warp)
-  const size_t smem = (size_t)2 * kStrictTile * LD * sizeof(float);
-  auto kern = k_rmat_strict_q<LD, GPW / 4, ValT>;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  if (nslots % (8 * GPW) != 0) return cudaErrorInvalidValue;
-  const int64_t n_tiles = (n + kStrictTile - 1) / kStrictTile;
-  const int64_t per = (n_tiles + ranges - 1) / ranges;
-  dim3 grid((unsigned)ranges, (unsigned)(nslots / (8 * GPW)));
-  kern<<<grid, 256, smem, st>>>(indptr, tptr, cell, static_cast<const ValT*>(cval), n, g, nslots, slot2gene, per, Q,
-                                lds, part);
-  note_launches(1);
-  return cudaGetLastError();
 }
 
 template <typename ValT>
-static cudaError_t rmat_strict_v(int ld, const int64_t* indptr, const int32_t* tptr, const uint8_t* cell,
-                                 const void* cval, int64_t n, int32_t g, int32_t nslots, const int32_t* slot2gene,
-                                 int ranges, const float* Q, int lds, float* part, cudaStream_t st) {
-  switch (ld) {
-    case 32: return rmat_strict_t<32, ValT>(indptr, tptr, cell, cval, n, g, nslots, slot2gene, ranges, Q, lds, part, st);
-    case 64: return rmat_strict_t<64, ValT>(indptr, tptr, cell, cval, n, g, nslots, slot2gene, ranges, Q, lds, part, st);
-    case 96: return rmat_strict_t<96, ValT>(indptr, tptr, cell, cval, n, g, nslots, slot2gene, ranges, Q, lds, part, st);
-    case 128:
-      return rmat_strict_t<128, ValT>(indptr, tptr, cell, cval, n, g, nslots, slot2gene, ranges, Q, lds, part, st);
-    default: return cudaErrorInvalidValue;
-  }
+static cudaError_t rmat_strict_t(int ld, const int64_t* indptr, const int32_t* tptr, const uint16_t* row,
+                                 const void* cval, int64_t n, int32_t g, const int32_t* slot2gene,
+                                 const StrictGeometry& geo, const float* Q, int lds, float* part, cudaStream_t st) {
+  const int cols = geo.cols, nslice = ld / cols;
+  const size_t smem = (size_t)(geo.rows + 1) * cols * 4;
+  auto go = [&](auto kern) {
+    if (cudaError_t e = allow_smem(kern, smem); e != cudaSuccess) return e;
+    kern<<<(unsigned)(geo.ranges * nslice), kThreads, smem, st>>>(indptr, tptr, row, static_cast<const ValT*>(cval), n,
+                                                                  g, slot2gene, geo.rows, geo.chunks, geo.per_range,
+                                                                  nslice, Q, lds, part, ld);
+    note_launches(1);
+    return cudaGetLastError();
+  };
+  return cols == 64 ? go(k_rmat_strict<4, ValT>) : go(k_rmat_strict<2, ValT>);
 }
 
-cudaError_t launch_rmat_strict(int dtype, int ld, const int64_t* indptr, const int32_t* tptr, const uint8_t* cell,
-                               const void* cval, int64_t n, int32_t g, int32_t nslots, const int32_t* slot2gene,
-                               int ranges, const float* Q, float* part, cudaStream_t st, int lds) {
+cudaError_t launch_rmat_strict(int dtype, int ld, const int64_t* indptr, const int32_t* tptr, const uint16_t* row,
+                               const void* cval, int64_t n, int32_t g, const int32_t* slot2gene,
+                               const StrictGeometry& geo, const float* Q, float* part, cudaStream_t st, int lds) {
   if (lds == 0) lds = ld;
-  if (lds < ld || (lds & 3)) return cudaErrorInvalidValue;
+  if (lds < ld || (lds & 3) || ld % 32 || ld > kMaxK) return cudaErrorInvalidValue;
   switch (dtype) {
-    case 0:
-      return rmat_strict_v<float>(ld, indptr, tptr, cell, cval, n, g, nslots, slot2gene, ranges, Q, lds, part, st);
-    case 1:
-      return rmat_strict_v<__nv_bfloat16>(ld, indptr, tptr, cell, cval, n, g, nslots, slot2gene, ranges, Q, lds,
-                                          part, st);
-    default:
-      return rmat_strict_v<__half>(ld, indptr, tptr, cell, cval, n, g, nslots, slot2gene, ranges, Q, lds, part, st);
+    case 0: return rmat_strict_t<float>(ld, indptr, tptr, row, cval, n, g, slot2gene, geo, Q, lds, part, st);
+    case 1: return rmat_strict_t<__nv_bfloat16>(ld, indptr, tptr, row, cval, n, g, slot2gene, geo, Q, lds, part, st);
+    default: return rmat_strict_t<__half>(ld, indptr, tptr, row, cval, n, g, slot2gene, geo, Q, lds, part, st);
   }
 }
 

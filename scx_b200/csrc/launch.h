@@ -56,31 +56,38 @@ cudaError_t launch_reduce_panel_f32(const float* part, int nparts, int64_t rows,
                                     cudaStream_t st, int num_sms);
 
 // ---- CUDA-core SpMM pair in a fixed summation order (kernels_strict.cu) ----
-constexpr int kStrictTile = 128;  // rows per tile of the tile-CSC copy (a power of two <= 256)
-int strict_genes_per_warp(int ld);
-// Slots of the tile-CSC copy: n_vars rounded up to whole blocks of the transposed product.
-int strict_slot_count(int64_t g, int ld);
-// Balanced gene -> slot assignment from per-gene stored-entry counts.
-void strict_assign_slots(const std::vector<int32_t>& counts, int ld, std::vector<int32_t>& gene2slot,
-                         std::vector<int32_t>& slot2gene);
-size_t strict_tile_smem_bytes(int nslots);
-cudaError_t launch_gene_counts(const int32_t* idx, int64_t nnz, int32_t* counts, cudaStream_t st, int num_sms);
-// Tile-CSC copy of a row-sorted CSR: tptr [n_tiles][nslots + 1], cell/cval [nnz].
-cudaError_t launch_tile_csc(int dtype, const int64_t* indptr, const int32_t* idx, const void* val, int64_t n,
-                            const int32_t* gene2slot, int32_t nslots, int32_t* tptr, uint8_t* cell, void* cval,
-                            cudaStream_t st, int num_sms);
+// Row chunks of the transposed product: `chunks` chunks of `rows` cells, a
+// range (one partial) of `per_range` consecutive ones.
+struct StrictGeometry {
+  int cols = 32;  // columns a block takes
+  int rows = 0, per_range = 1, ranges = 1;
+  int64_t chunks = 0;
+};
+// Geometry for n cells and a column panel of width ld.
+StrictGeometry strict_geometry(int64_t n, int ld, int num_sms);
+// Whether the chunk-CSC copy can be built for g genes at panel width ld.
+bool strict_csc_fits(int64_t g, int ld);
+cudaError_t launch_gene_counts(const int32_t* idx, int64_t nnz, int32_t g, int32_t* counts, cudaStream_t st,
+                               int num_sms);
+// Genes in decreasing order of stored entries: gene -> slot and slot -> gene.
+cudaError_t launch_rank_genes(const int32_t* counts, int32_t g, int32_t* gene2slot, int32_t* slot2gene,
+                              cudaStream_t st);
+// Chunk-CSC copy of a row-sorted CSR: tptr [chunks][g + 1], row/cval [nnz].
+cudaError_t launch_chunk_csc(int dtype, const int64_t* indptr, const int32_t* idx, const void* val, int64_t n,
+                             const StrictGeometry& geo, const int32_t* gene2slot, int32_t g, int32_t* tptr,
+                             uint16_t* row, void* cval, cudaStream_t st);
 // Y (n x ld) = P V - 1 mc^T (mc may be null) from a row-sorted CSR.  `ld` is
 // the width of the column panel taken (32, 64, 96 or 128); V, mc and Y point
 // at its first column and `lds` is the row stride of V and Y in floats
 // (0: lds = ld, the whole matrix).
 cudaError_t launch_fwd_strict(int dtype, int ld, const int64_t* indptr, const int32_t* idx, const void* val,
                               int64_t n, int32_t g, const float* V, const float* mc, float* Y, cudaStream_t st,
-                              int lds = 0);
-// part[range][g][ld] = partial P^T Q over the row tiles of each of `ranges`
-// contiguous ranges; Q is a column panel of width ld and row stride lds (0: ld).
-cudaError_t launch_rmat_strict(int dtype, int ld, const int64_t* indptr, const int32_t* tptr, const uint8_t* cell,
-                               const void* cval, int64_t n, int32_t g, int32_t nslots, const int32_t* slot2gene,
-                               int ranges, const float* Q, float* part, cudaStream_t st, int lds = 0);
+                              int num_sms, int lds = 0);
+// part[range][g][ld] = partial P^T Q over the row chunks of each range; Q is a
+// column panel of width ld and row stride lds (0: ld).
+cudaError_t launch_rmat_strict(int dtype, int ld, const int64_t* indptr, const int32_t* tptr, const uint16_t* row,
+                               const void* cval, int64_t n, int32_t g, const int32_t* slot2gene,
+                               const StrictGeometry& geo, const float* Q, float* part, cudaStream_t st, int lds = 0);
 cudaError_t launch_reduce_rows_f64(const double* part, int nparts, int64_t len, double* out,
                                    int accumulate, cudaStream_t st, int num_sms);
 

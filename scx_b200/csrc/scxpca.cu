@@ -276,13 +276,13 @@ struct scxpca_plan {
   double total_var = 0.0;
   bool total_var_recomputed = false;
 
-  // CUDA-core transposed product: the tile-CSC copy (slots balanced by
-  // stored-entry count) and its per-range partials; the row-block pointer
+  // CUDA-core transposed product: the chunk-CSC copy (slots in decreasing
+  // order of stored entries) and its per-range partials; the row-block pointer
   // table of the gradient's SDDMM (and of the atomic fallback for matrices
-  // too wide for the tile-CSC copy) is built on first use
+  // too wide for the chunk-CSC copy) is built on first use
   bool strict_csc = false;
-  int nslots = 0, strict_ranges = 0;
-  DevBuf csc_tptr, csc_cell, csc_val, d_slot2gene;
+  StrictGeometry geo;
+  DevBuf csc_tptr, csc_row, csc_val, d_slot2gene;
   int nb = 0, nchunks = 0;
   int64_t rows_per_chunk = 0;
   bool rbp_built = false;
@@ -328,10 +328,10 @@ struct scxpca_plan {
     int64_t r0, r1, p0, p1;  // rows [r0, r1), stored entries [p0, p1)
     CUtensorMap qmap;        // TMA map of the shard's rows of the tall image
     int row_groups;          // partials of its tensor-core transposed product
-    int ranges;              // partials of its CUDA-core transposed product
+    StrictGeometry geo;      // row chunks of its CUDA-core transposed product
   };
   struct Slot {
-    DevBuf ip, idx, vin, vwork, counts, seg, ent, meta, tptr, cell, cval;
+    DevBuf ip, idx, vin, vwork, counts, seg, ent, meta, tptr, row, cval;
   };
   bool streaming = false;
   bool stream_sort = false;       // re-sort every shard after its upload
@@ -518,7 +518,7 @@ std::vector<double> read_vec(const double* src, int64_t n, int32_t memory, doubl
 }
 
 // Row-block pointer table (the SDDMM of the gradient, and the transposed
-// product of matrices too wide for the tile-CSC copy), built on first use.
+// product of matrices too wide for the chunk-CSC copy), built on first use.
 void ensure_rbp(scxpca_plan* pl) {
   if (pl->rbp_built) return;
   PoolScope pool_scope(pl->device, pl->stream);
@@ -530,43 +530,31 @@ void ensure_rbp(scxpca_plan* pl) {
   pl->rbp_built = true;
 }
 
-// Tile-CSC copy of the working matrix for the CUDA-core transposed product:
-// per-gene stored-entry counts -> balanced slot assignment (host) -> the
-// copy, and the per-range partial buffer.
 // Column panel the CUDA-core SpMM pair takes per launch: the whole sketch up
 // to 128 columns, else 128-column panels of it.
 int panel_width(const scxpca_plan* pl) { return (int)std::min<int64_t>(pl->ld, kPanel); }
 
-void build_tile_csc(scxpca_plan* pl) {
+// Chunk-CSC copy of the working matrix for the CUDA-core transposed product:
+// per-gene stored-entry counts -> the slot order -> the copy, and the
+// per-range partial buffer.
+void build_chunk_csc(scxpca_plan* pl) {
   cudaStream_t st = pl->stream;
   const int64_t n = pl->n, g = pl->g, nnz = pl->nnz;
-  DevBuf counts;
-  counts.alloc(sizeof(int32_t) * g);
-  CK(cudaMemsetAsync(counts.p, 0, sizeof(int32_t) * g, st));
-  CK(launch_gene_counts(pl->idx, nnz, counts.as<int32_t>(), st, pl->num_sms));
-  std::vector<int32_t> hc(g);
-  CK(cudaMemcpyAsync(hc.data(), counts.p, sizeof(int32_t) * g, cudaMemcpyDeviceToHost, st));
-  CK(cudaStreamSynchronize(st));
-  std::vector<int32_t> gene2slot, slot2gene;
   const int pw = panel_width(pl);
-  strict_assign_slots(hc, pw, gene2slot, slot2gene);
-  DevBuf d_g2s;
+  DevBuf counts, d_g2s;
+  counts.alloc(sizeof(int32_t) * g);
   d_g2s.alloc(sizeof(int32_t) * g);
-  CK(cudaMemcpyAsync(d_g2s.p, gene2slot.data(), sizeof(int32_t) * g, cudaMemcpyHostToDevice, st));
-  pl->d_slot2gene.alloc(sizeof(int32_t) * pl->nslots);
-  CK(cudaMemcpyAsync(pl->d_slot2gene.p, slot2gene.data(), sizeof(int32_t) * pl->nslots, cudaMemcpyHostToDevice,
-                     st));
-  const int64_t n_tiles = (n + kStrictTile - 1) / kStrictTile;
-  pl->csc_tptr.alloc(sizeof(int32_t) * (size_t)n_tiles * (pl->nslots + 1));
-  pl->csc_cell.alloc(std::max<int64_t>(nnz, 1));
+  pl->d_slot2gene.alloc(sizeof(int32_t) * g);
+  CK(cudaMemsetAsync(counts.p, 0, sizeof(int32_t) * g, st));
+  CK(launch_gene_counts(pl->idx, nnz, (int32_t)g, counts.as<int32_t>(), st, pl->num_sms));
+  CK(launch_rank_genes(counts.as<int32_t>(), (int32_t)g, d_g2s.as<int32_t>(), pl->d_slot2gene.as<int32_t>(), st));
+  pl->geo = strict_geometry(n, pw, pl->num_sms);
+  pl->csc_tptr.alloc(sizeof(int32_t) * (size_t)pl->geo.chunks * (g + 1));
+  pl->csc_row.alloc(sizeof(uint16_t) * std::max<int64_t>(nnz, 1));
   pl->csc_val.alloc(dtype_size(pl->dtype) * std::max<int64_t>(nnz, 1));
-  CK(launch_tile_csc(pl->dtype, pl->indptr, pl->idx, pl->val, n, d_g2s.as<int32_t>(), pl->nslots,
-                     pl->csc_tptr.as<int32_t>(), pl->csc_cell.as<uint8_t>(), pl->csc_val.p, st, pl->num_sms));
-  // ranges: about four blocks per SM over all gene blocks, for balance
-  const int gblocks = pl->nslots / (8 * strict_genes_per_warp(pw));
-  pl->strict_ranges = (int)std::max<int64_t>(1, std::min<int64_t>(n_tiles, (4 * pl->num_sms + gblocks - 1) / gblocks));
-  pl->wpart.alloc(sizeof(float) * (size_t)pl->strict_ranges * g * pw);
-  CK(cudaStreamSynchronize(st));  // the host vectors above go out of scope
+  CK(launch_chunk_csc(pl->dtype, pl->indptr, pl->idx, pl->val, n, pl->geo, d_g2s.as<int32_t>(), (int32_t)g,
+                      pl->csc_tptr.as<int32_t>(), pl->csc_row.as<uint16_t>(), pl->csc_val.p, st));
+  pl->wpart.alloc(sizeof(float) * (size_t)pl->geo.ranges * g * pw);
 }
 
 // ---------------------------------------------------------------------------
@@ -587,7 +575,7 @@ void alloc_work_buffers(scxpca_plan* pl);
 // Bytes one device slot needs per stored entry and per row.
 double slot_bytes_per_entry(const scxpca_plan* pl, bool tc) {
   double b = 4.0 + (double)dtype_size(pl->in_dtype) + (double)dtype_size(pl->dtype);
-  b += tc ? 4.0 * 1.2 : 1.0 + (double)dtype_size(pl->dtype);
+  b += tc ? 4.0 * 1.2 : 2.0 + (double)dtype_size(pl->dtype);
   return b;
 }
 
@@ -609,7 +597,7 @@ void shard_upload(scxpca_plan* pl, size_t s, int k) {
 
 // Bring an uploaded shard to the working form on the plan's stream: the
 // rebased indptr, sorted rows when needed, working values (`work`), and, per
-// `pack` (0 none, 1 tensor-core tiles, 2 tile-CSC), the packed copy.
+// `pack` (0 none, 1 tensor-core tiles, 2 chunk-CSC), the packed copy.
 const void* shard_prepare(scxpca_plan* pl, size_t s, int k, bool work, int pack) {
   const scxpca_plan::Shard& sh = pl->shards[s];
   scxpca_plan::Slot& sl = pl->slot[k];
@@ -635,8 +623,9 @@ const void* shard_prepare(scxpca_plan* pl, size_t s, int k, bool work, int pack)
     CK(tile_format_fill(sl.ip.as<int64_t>(), sl.idx.as<int32_t>(), vals, rows, pl->n_chunks, sl.seg.as<int64_t>(),
                         sl.ent.as<uint32_t>(), sl.meta.p, st, pl->num_sms));
   } else if (pack == 2) {
-    CK(launch_tile_csc(pl->dtype, sl.ip.as<int64_t>(), sl.idx.as<int32_t>(), vals, rows, pl->d_gene2slot.as<int32_t>(),
-                       pl->nslots, sl.tptr.as<int32_t>(), sl.cell.as<uint8_t>(), sl.cval.p, st, pl->num_sms));
+    CK(launch_chunk_csc(pl->dtype, sl.ip.as<int64_t>(), sl.idx.as<int32_t>(), vals, rows, sh.geo,
+                        pl->d_gene2slot.as<int32_t>(), (int32_t)pl->g, sl.tptr.as<int32_t>(), sl.row.as<uint16_t>(),
+                        sl.cval.p, st));
   }
   return vals;
 }
@@ -675,7 +664,7 @@ void stream_stats(scxpca_plan* pl, bool work, std::vector<double>& sums, std::ve
     if (flags)
       CK(launch_validate_csr(pl->in_dtype, sl.ip.as<int64_t>(), sl.idx.as<int32_t>(), sl.vin.p, rows, g, cnt, flags,
                              st, pl->num_sms));
-    if (gene_counts) CK(launch_gene_counts(sl.idx.as<int32_t>(), cnt, gene_counts, st, pl->num_sms));
+    if (gene_counts) CK(launch_gene_counts(sl.idx.as<int32_t>(), cnt, (int32_t)g, gene_counts, st, pl->num_sms));
     CK(launch_col_stats(work ? pl->dtype : pl->in_dtype, sl.idx.as<int32_t>(), vals, cnt, (int32_t)g,
                         pl->stats_part.as<double>(), pl->stats_parts, pl->stats_out.as<double>(), st, pl->num_sms,
                         s > 0 ? 1 : 0));
@@ -703,7 +692,7 @@ void stream_forward(scxpca_plan* pl, bool f32) {
     } else {
       CK(launch_fwd_strict(pl->dtype, (int)ld, sl.ip.as<int64_t>(), sl.idx.as<int32_t>(), vals, rows, (int32_t)pl->g,
                            pl->V.as<float>(), pl->centered ? pl->mc.as<float>() : nullptr,
-                           pl->Y.as<float>() + sh.r0 * ld, st));
+                           pl->Y.as<float>() + sh.r0 * ld, st, pl->num_sms));
     }
   });
 }
@@ -722,10 +711,10 @@ void stream_rmat(scxpca_plan* pl, const float* A) {
       CK(launch_reduce_rows_f32(pl->tc_part.as<float>(), sh.row_groups, g * ld, pl->W.as<double>(), s > 0 ? 1 : 0,
                                 st, pl->num_sms));
     } else {
-      CK(launch_rmat_strict(pl->dtype, (int)ld, sl.ip.as<int64_t>(), sl.tptr.as<int32_t>(), sl.cell.as<uint8_t>(),
-                            sl.cval.p, rows, (int32_t)g, pl->nslots, pl->d_slot2gene.as<int32_t>(), sh.ranges,
-                            A + sh.r0 * ld, pl->wpart.as<float>(), st));
-      CK(launch_reduce_rows_f32(pl->wpart.as<float>(), sh.ranges, g * ld, pl->W.as<double>(), s > 0 ? 1 : 0, st,
+      CK(launch_rmat_strict(pl->dtype, (int)ld, sl.ip.as<int64_t>(), sl.tptr.as<int32_t>(), sl.row.as<uint16_t>(),
+                            sl.cval.p, rows, (int32_t)g, pl->d_slot2gene.as<int32_t>(), sh.geo, A + sh.r0 * ld,
+                            pl->wpart.as<float>(), st));
+      CK(launch_reduce_rows_f32(pl->wpart.as<float>(), sh.geo.ranges, g * ld, pl->W.as<double>(), s > 0 ? 1 : 0, st,
                                 pl->num_sms));
     }
   });
@@ -967,34 +956,27 @@ void setup_streaming(scxpca_plan* pl, const scxpca_csr* x, size_t limit) {
     if (r1 || r2)
       fail(SCXPCA_CUDA_ERROR, "cuTensorMapEncodeTiled failed (" + std::to_string(r1) + ", " + std::to_string(r2) + ")");
   } else {
-    pl->nslots = strict_slot_count(g, (int)ld);
-    if (strict_tile_smem_bytes(pl->nslots) > kStatsSmemMax)
+    if (!strict_csc_fits(g, (int)ld))
       fail(SCXPCA_UNSUPPORTED, "a streamed CUDA-core PCA takes at most " +
                                    std::to_string(kStatsSmemMax / sizeof(int32_t) - 1) + " genes");
-    std::vector<int32_t> hc(g), gene2slot, slot2gene;
-    CK(cudaMemcpyAsync(hc.data(), counts.p, sizeof(int32_t) * g, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    strict_assign_slots(hc, (int)ld, gene2slot, slot2gene);
     pl->d_gene2slot.alloc(sizeof(int32_t) * g);
-    pl->d_slot2gene.alloc(sizeof(int32_t) * pl->nslots);
-    CK(cudaMemcpyAsync(pl->d_gene2slot.p, gene2slot.data(), sizeof(int32_t) * g, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(pl->d_slot2gene.p, slot2gene.data(), sizeof(int32_t) * pl->nslots, cudaMemcpyHostToDevice,
-                       st));
-    for (auto& sl : pl->slot) {
-      sl.tptr.alloc(sizeof(int32_t) * (size_t)tiles_max * (pl->nslots + 1));
-      sl.cell.alloc(emax);
-      sl.cval.alloc(dtype_size(pl->dtype) * emax);
-    }
-    const int gblocks = pl->nslots / (8 * strict_genes_per_warp((int)ld));
+    pl->d_slot2gene.alloc(sizeof(int32_t) * g);
+    CK(launch_rank_genes(counts.as<int32_t>(), (int32_t)g, pl->d_gene2slot.as<int32_t>(),
+                         pl->d_slot2gene.as<int32_t>(), st));
     int ranges_max = 1;
+    int64_t chunks_max = 1;
     for (auto& sh : pl->shards) {
-      const int64_t nt = (sh.r1 - sh.r0 + kStrictTile - 1) / kStrictTile;
-      sh.ranges = (int)std::max<int64_t>(1, std::min<int64_t>(nt, (4 * pl->num_sms + gblocks - 1) / gblocks));
-      ranges_max = std::max(ranges_max, sh.ranges);
+      sh.geo = strict_geometry(sh.r1 - sh.r0, (int)ld, pl->num_sms);
+      ranges_max = std::max(ranges_max, sh.geo.ranges);
+      chunks_max = std::max(chunks_max, sh.geo.chunks);
+    }
+    for (auto& sl : pl->slot) {
+      sl.tptr.alloc(sizeof(int32_t) * (size_t)chunks_max * (g + 1));
+      sl.row.alloc(sizeof(uint16_t) * emax);
+      sl.cval.alloc(dtype_size(pl->dtype) * emax);
     }
     pl->strict_csc = true;
     pl->wpart.alloc(sizeof(float) * (size_t)ranges_max * g * ld);
-    CK(cudaStreamSynchronize(st));  // the host vectors above go out of scope
   }
   phase_mark(SCXPCA_PHASE_PACK, st);
   alloc_work_buffers(pl);
@@ -1104,7 +1086,7 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
                            pl->wpart.bytes + pl->gpart.bytes + pl->W.bytes + pl->Z.bytes + pl->V.bytes;
         for (auto& sl : pl->slot)
           pl->device_bytes += sl.ip.bytes + sl.idx.bytes + sl.vin.bytes + sl.vwork.bytes + sl.counts.bytes +
-                              sl.seg.bytes + sl.ent.bytes + sl.meta.bytes + sl.tptr.bytes + sl.cell.bytes +
+                              sl.seg.bytes + sl.ent.bytes + sl.meta.bytes + sl.tptr.bytes + sl.row.bytes +
                               sl.cval.bytes;
         return pl;
       }
@@ -1372,19 +1354,16 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
              "cuTensorMapEncodeTiled failed (" + std::to_string(r1) + ", " + std::to_string(r2) + ")");
     }
 
-    // ---- CUDA-core products: tile-CSC copy for the transposed product ----
+    // ---- CUDA-core products: chunk-CSC copy for the transposed product ----
     pl->nb = (int)((g + kTransposeGeneBlock - 1) / kTransposeGeneBlock);
     pl->nchunks = std::max(1, (2 * pl->num_sms + pl->nb - 1) / pl->nb);
     pl->nchunks = (int)std::min<int64_t>(pl->nchunks, n);
     pl->rows_per_chunk = (n + pl->nchunks - 1) / pl->nchunks;
-    if (!pl->use_tc) {
-      pl->nslots = strict_slot_count(g, panel_width(pl));
-      pl->strict_csc = strict_tile_smem_bytes(pl->nslots) <= kStatsSmemMax;
-    }
+    if (!pl->use_tc) pl->strict_csc = strict_csc_fits(g, panel_width(pl));
     if (pl->ld > kMaxK && !pl->strict_csc)
-      fail(SCXPCA_UNSUPPORTED, "a sketch wider than " + std::to_string(kMaxK) + " columns needs the tile-CSC "
+      fail(SCXPCA_UNSUPPORTED, "a sketch wider than " + std::to_string(kMaxK) + " columns needs the chunk-CSC "
                                "copy, whose per-gene offsets exceed shared memory at n_vars = " + std::to_string(g));
-    if (pl->strict_csc) build_tile_csc(pl);
+    if (pl->strict_csc) build_chunk_csc(pl);
     else if (!pl->use_tc) ensure_rbp(pl);
     phase_mark(SCXPCA_PHASE_PACK, st);
 
@@ -1396,7 +1375,7 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
     CK(cudaMemGetInfo(&fr, &tot));
     pl->device_bytes = pl->b_indptr.bytes + pl->b_idx.bytes + pl->b_val.bytes + pl->stats_part.bytes +
                        pl->rbp.bytes + pl->wpart.bytes + pl->Y.bytes + pl->gpart.bytes +
-                       pl->W.bytes + pl->Z.bytes + pl->V.bytes + pl->csc_tptr.bytes + pl->csc_cell.bytes +
+                       pl->W.bytes + pl->Z.bytes + pl->V.bytes + pl->csc_tptr.bytes + pl->csc_row.bytes +
                        pl->csc_val.bytes + pl->tf_ent.bytes + pl->Yimg.bytes + pl->tc_part.bytes;
     return pl;
   } catch (...) {
@@ -1546,12 +1525,12 @@ void rmatmat_raw(scxpca_plan* pl, float* A, int split) {
     const int ld = (int)pl->ld, pw = panel_width(pl);
     for (int c0 = 0; c0 < ld; c0 += pw) {
       int s = stage_begin(pl);
-      CK(launch_rmat_strict(pl->dtype, pw, pl->indptr, pl->csc_tptr.as<int32_t>(), pl->csc_cell.as<uint8_t>(),
-                            pl->csc_val.p, pl->n, (int32_t)pl->g, pl->nslots, pl->d_slot2gene.as<int32_t>(),
-                            pl->strict_ranges, A + c0, pl->wpart.as<float>(), st, ld));
+      CK(launch_rmat_strict(pl->dtype, pw, pl->indptr, pl->csc_tptr.as<int32_t>(), pl->csc_row.as<uint16_t>(),
+                            pl->csc_val.p, pl->n, (int32_t)pl->g, pl->d_slot2gene.as<int32_t>(), pl->geo, A + c0,
+                            pl->wpart.as<float>(), st, ld));
       stage_end(pl, SCXPCA_STAGE_TRANSPOSE, s);
       s = stage_begin(pl);
-      CK(launch_reduce_panel_f32(pl->wpart.as<float>(), pl->strict_ranges, pl->g, pw, pl->W.as<double>() + c0, ld,
+      CK(launch_reduce_panel_f32(pl->wpart.as<float>(), pl->geo.ranges, pl->g, pw, pl->W.as<double>() + c0, ld,
                                  st, pl->num_sms));
       stage_end(pl, SCXPCA_STAGE_REDUCE, s);
     }
@@ -1560,10 +1539,10 @@ void rmatmat_raw(scxpca_plan* pl, float* A, int split) {
   int s = stage_begin(pl);
   int parts = pl->nchunks;
   if (pl->strict_csc) {
-    CK(launch_rmat_strict(pl->dtype, (int)pl->ld, pl->indptr, pl->csc_tptr.as<int32_t>(), pl->csc_cell.as<uint8_t>(),
-                          pl->csc_val.p, pl->n, (int32_t)pl->g, pl->nslots, pl->d_slot2gene.as<int32_t>(),
-                          pl->strict_ranges, A, pl->wpart.as<float>(), st));
-    parts = pl->strict_ranges;
+    CK(launch_rmat_strict(pl->dtype, (int)pl->ld, pl->indptr, pl->csc_tptr.as<int32_t>(), pl->csc_row.as<uint16_t>(),
+                          pl->csc_val.p, pl->n, (int32_t)pl->g, pl->d_slot2gene.as<int32_t>(), pl->geo, A,
+                          pl->wpart.as<float>(), st));
+    parts = pl->geo.ranges;
   } else {
     CK(launch_spmm_t(pl->dtype, (int)pl->ld, pl->indptr, pl->idx, pl->val, pl->n, (int32_t)pl->g,
                      pl->rbp.as<int32_t>(), pl->nb, pl->nchunks, pl->rows_per_chunk, A,
@@ -1610,7 +1589,7 @@ void forward(scxpca_plan* pl, bool f32 = true, bool split_v = true) {
   const int ld = (int)pl->ld, pw = panel_width(pl);
   for (int c0 = 0; c0 < ld; c0 += pw)
     CK(launch_fwd_strict(pl->dtype, pw, pl->indptr, pl->idx, pl->val, pl->n, (int32_t)pl->g, pl->V.as<float>() + c0,
-                         pl->centered ? pl->mc.as<float>() + c0 : nullptr, pl->Y.as<float>() + c0, st, ld));
+                         pl->centered ? pl->mc.as<float>() + c0 : nullptr, pl->Y.as<float>() + c0, st, pl->num_sms, ld));
   stage_end(pl, SCXPCA_STAGE_FORWARD, s);
 }
 

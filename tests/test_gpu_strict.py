@@ -183,3 +183,40 @@ def test_householder_qr_orthonormal_on_ill_conditioned(mode):
     resid = np.linalg.norm(y64 - q @ (q.T @ y64)) / np.linalg.norm(y64)
     assert resid < 1e-5, resid
     plan.close()
+
+
+@pytest.mark.parametrize("n,g,k", [
+    (40000, 900, 60),    # cells enough for 64-column blocks; V in two gene chunks of them
+    (38016, 260, 120),   # two 64-column blocks per cell range
+    (500, 1700, 30),     # 32-column blocks, V in two gene chunks
+    (150, 3500, 90),     # three gene chunks, fewer cells than a block has lists
+])
+def test_strict_products_across_tables(n, g, k):
+    """Products whose dense operand takes several shared-memory tables, on
+    arrays that start at a vector boundary and on arrays that do not: the same
+    bits either way, and FP32 sums of a few hundred terms against FP64."""
+    import torch
+
+    c = _csr(n, g, seed=g, loc=-3.0)
+    nnz = len(c.indices)
+    ip = torch.from_numpy(c.indptr).cuda()
+    ix = torch.zeros(nnz + 1, dtype=torch.int32, device="cuda")
+    vv = torch.zeros(nnz + 1, dtype=torch.float32, device="cuda")
+    ix[1:] = torch.from_numpy(c.indices).cuda()
+    vv[1:] = torch.from_numpy(c.data).cuda()
+    rng = np.random.default_rng(5)
+    v = rng.standard_normal((g, k)).astype(np.float32)
+    q = rng.standard_normal((n, k)).astype(np.float32)
+    got = []
+    for idx, val in ((ix[1:].clone(), vv[1:].clone()), (ix[1:], vv[1:])):
+        torch.cuda.synchronize()
+        plan = accel.Plan(ip, idx, val, c.shape, n_components=k, n_oversamples=0, math_mode="strict_fp32")
+        got.append((plan.matmat(torch.from_numpy(v).cuda()).cpu().numpy(),
+                    plan.rmatmat(torch.from_numpy(q).cuda()).cpu().numpy()))
+        plan.close()
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1])
+    mu = rpca.col_sums_and_sum_sq(c)[0] / n
+    y_ref = rpca.spmm_forward(c, v.astype(np.float64), mu)
+    z_ref = rpca.spmm_transpose(c, q.astype(np.float64), mu)
+    assert np.linalg.norm(got[0][0] - y_ref) / np.linalg.norm(y_ref) < OP_RTOL
+    assert np.linalg.norm(got[0][1] - z_ref) / np.linalg.norm(z_ref) < OP_RTOL
