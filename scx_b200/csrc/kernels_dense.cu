@@ -131,11 +131,12 @@ cudaError_t launch_gram_f64(const double* A, int64_t n, int ld, double* part, in
 
 // ---------------------------------------------------------------------------
 // Cholesky of the leading k x k block of G (ld x ld) and the inverse of its
-// factor, one block of T x T threads.  A pivot j fails when its Schur
-// complement d_j <= tau * G_jj (the column is numerically dependent on the
-// previous ones) or is not finite.  With shift_on_fail the factorisation
-// restarts once on G + s I, s = 10 tau max_j G_jj, which always succeeds on
-// finite input.
+// factor, one block of 256 threads.  A pivot j fails when its Schur complement
+// d_j <= tau * G_jj (the column is numerically dependent on the previous ones)
+// or is not finite.  With shift_on_fail the factorisation restarts once on
+// G + s I, s = 10 tau max_j G_jj, which always succeeds on finite input.  With
+// CLAMP (the eigensolver's factor) no pivot fails: one below 1e-15 of the
+// largest diagonal, or 1e-300, is set there.
 //
 // Symmetric Gaussian elimination of the augmented matrix [A | I]: step j
 // subtracts (A_ja / d_j) times row j from every row a > j, which turns A's
@@ -143,41 +144,73 @@ cudaError_t launch_gram_f64(const double* A, int64_t n, int ld, double* part, in
 // triangular), where A = L D L^T.  Then R = D^{1/2} L^T and
 // R^{-1} = X^T D^{-1/2}: R_jc = A_jc / sqrt(d_j), R^{-1}_ca = X_ac / sqrt(d_a).
 // Every matrix entry lives in a register of its owner, thread (ty, tx) owning
-// rows ty + T u and columns tx + T v; one register holds A_ac above the
-// diagonal (c >= a) or X_ac below it.  Per step the owners of row j + 1
-// publish it (double-buffered rows in shared memory) and the owner of the
-// next diagonal entry computes the next pivot's reciprocals, so a step is
-// one barrier plus a short dependent chain.
+// rows ty + 16 u and columns tx + 16 v; one register holds A_ac above the
+// diagonal (c >= a) or X_ac below it.
+//
+// What bounds it is the chain of pivots: each needs a reciprocal and one
+// multiply-add of the pivot before it.  One pivot per block barrier cost 1,300
+// clocks (51 us at k = 60, 170 us at k = 110), so the rows go in panels of
+// eight: a panel's rows are handed to a few warps that eliminate inside the
+// panel without a barrier, one column per lane, and then all threads take the
+// panel's eight steps at once on their entries.  Measured: 17 us at k = 60, 59 us at k = 110.
 // ---------------------------------------------------------------------------
-// With `tasks` set, block b factors the matrix of tasks[b] (many segments'
-// factorisations in one launch, one block each) and the pointer arguments are
-// ignored.
-template <int U, int T>
-__global__ void __launch_bounds__(T * T) k_cholesky(const double* __restrict__ G, int k, int ld, double tau,
-                                                   int shift_on_fail, double* __restrict__ R,
-                                                   double* __restrict__ Rinv, float* __restrict__ Rinv_f,
-                                                   int* __restrict__ status, const CholTask* __restrict__ tasks) {
-  if (tasks) {
-    const CholTask t = tasks[blockIdx.x];
+constexpr int kCholThreads = 256;
+constexpr int kPanelRows = 8;
+
+// 1 / x for normal x: the hardware's approximation and two Newton steps
+// (y <- y (2 - x y), each doubling the correct bits).
+__device__ __forceinline__ double rcp_fast(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+// 1 / sqrt(x) for normal x > 0, in the same way (y <- y (3 - x y^2) / 2).
+__device__ __forceinline__ double rsqrt_fast(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double h = 0.5 * x;
+  y = fma(y, fma(-h * y, y, 0.5), y);
+  return fma(y, fma(-h * y, y, 0.5), y);
+}
+
+template <int KP>
+constexpr size_t chol_smem() {  // factored rows [KP][KP + 1]; a panel's rows and multipliers, X in its own columns
+  return sizeof(double) * ((size_t)KP * (KP + 1) + 2 * kPanelRows * KP + (size_t)kPanelRows * (KP + 1));
+}
+
+// With `tasks` set (CholTask, or JacobiTask with CLAMP), block b factors the
+// matrix of tasks[b] (many segments' factorisations in one launch, one block
+// each) and the pointer arguments are ignored.
+template <int KP, bool CLAMP>
+__global__ void __launch_bounds__(kCholThreads) k_cholesky(const double* __restrict__ G, int k, int ld, double tau,
+                                                           int shift_on_fail, double* __restrict__ R,
+                                                           double* __restrict__ Rinv, float* __restrict__ Rinv_f,
+                                                           int* __restrict__ status, const void* tasks) {
+  if (tasks && CLAMP) {
+    const JacobiTask t = static_cast<const JacobiTask*>(tasks)[blockIdx.x];
+    G = t.C;
+    R = t.evecs + (size_t)ld * ld;
+    Rinv = R + (size_t)ld * ld;
+  } else if (tasks) {
+    const CholTask t = static_cast<const CholTask*>(tasks)[blockIdx.x];
     G = t.G;
     R = t.R;
     Rinv = t.Rinv;
     Rinv_f = t.Rinv_f;
     status = t.status;
   }
-  __shared__ double rowA[2][kMaxK], rowX[2][kMaxK];
-  __shared__ double pv_rinv[kMaxK], pv_di[kMaxK], dg[kMaxK];
-  __shared__ int pv_ok[kMaxK];
+  constexpr int U = KP / 16, NT = kCholThreads, PR = kPanelRows, FS = KP + 1;
+  extern __shared__ double chol_sm[];
+  double* F = chol_sm;          // [KP][FS]: row j of D L^T (c >= j) and of X (c < j), once final
+  double* P = F + KP * FS;      // [PR][KP]: the panel's rows as their owners left them
+  double* M = P + PR * KP;      // [PR][KP]: multipliers A_ja / d_j
+  double* T = M + PR * KP;      // [PR][FS]: X in the panel's own columns
+  __shared__ double piv[KP], dg[KP];
   __shared__ double maxdiag_s;
   __shared__ int fail_s;
-  constexpr int NT = T * T;
-  const int tid = threadIdx.x, tx = tid % T, ty = tid / T;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, lane = tid & 31, warp = tid >> 5;
   for (int j = tid; j < k; j += NT) dg[j] = G[(int64_t)j * ld + j];
-  for (int t = tid; t < ld * ld; t += NT) {
-    R[t] = 0.0;
-    Rinv[t] = 0.0;
-    Rinv_f[t] = 0.f;
-  }
   __syncthreads();
   if (tid < 32) {
     double m = 0.0;
@@ -186,92 +219,141 @@ __global__ void __launch_bounds__(T * T) k_cholesky(const double* __restrict__ G
     if (tid == 0) maxdiag_s = m;
   }
   double shift = 0.0;
-  int fail = -1;
-  double val[U][U];
   for (int attempt = 0; attempt < 2; ++attempt) {
-    // Pivot j from its updated diagonal entry d (called by the entry's owner).
-    auto pivot = [&](int j, double d) {
-      const bool ok = isfinite(d) && d > 0.0 && (attempt == 1 || d > tau * (dg[j] + shift));
-      pv_ok[j] = ok ? 1 : 0;
-      if (ok) {
-        const double rinv = d >= 1e-300 ? rsqrt_nr(d) : rsqrt(d);
-        pv_rinv[j] = rinv;
-        pv_di[j] = rinv * rinv;
-      }
-    };
+    double val[U][U];
 #pragma unroll
     for (int u = 0; u < U; ++u)
 #pragma unroll
       for (int v = 0; v < U; ++v) {
-        const int a = ty + T * u, c = tx + T * v;
-        double x = 0.0;
-        if (a < k && c < k) {
-          if (c >= a) x = G[(int64_t)a * ld + c] + (a == c ? shift : 0.0);
-        }
-        val[u][v] = x;  // X starts as the identity; its unit diagonal is implicit
+        const int a = ty + 16 * u, c = tx + 16 * v;
+        double x = 0.0;  // X starts as the identity; its unit diagonal is implicit
+        if (c >= a && c < k) x = G[(int64_t)a * ld + c] + (a == c ? shift : 0.0);
+        val[u][v] = x;
       }
-    if (ty == 0) {
-#pragma unroll
-      for (int v = 0; v < U; ++v) {
-        const int c = tx + T * v;
-        if (c < k) {
-          rowA[0][c] = val[0][v];
-          rowX[0][c] = c == 0 ? 1.0 : 0.0;
-        }
-      }
-    }
-    if (tid == 0) {
-      fail_s = -1;
-      pivot(0, val[0][0]);
-    }
+    if (tid == 0) fail_s = -1;
     __syncthreads();
-    for (int j = 0; j < k; ++j) {
-      if (!pv_ok[j]) {  // every thread reads the same flag: uniform exit
-        if (tid == 0) fail_s = j;
-        break;
-      }
-      const int b = j & 1;
-      const double di = pv_di[j], rj = pv_rinv[j];
+    const double floor_d = fmax(1e-15 * maxdiag_s, 1e-300);
+    for (int j0 = 0; j0 < k; j0 += PR) {
+      // the panel's rows, from their owners
 #pragma unroll
       for (int u = 0; u < U; ++u) {
-        const int a = ty + T * u;
-        if (a == j) {  // row j is final: R_jc = A_jc / sqrt(d_j)
+        const int a = ty + 16 * u;
+        if ((unsigned)(a - j0) < (unsigned)PR) {
 #pragma unroll
-          for (int v = 0; v < U; ++v) {
-            const int c = tx + T * v;
-            if (c >= j && c < k) R[(int64_t)j * ld + c] = val[u][v] * rj;
+          for (int v = 0; v < U; ++v) P[(a - j0) * KP + tx + 16 * v] = val[u][v];
+        }
+      }
+      __syncthreads();
+      // elimination inside the panel, a column per lane: the panel's own columns
+      // of X, every column outside the panel, the panel's own columns of A.  Each
+      // lane repeats the 8 x 8 diagonal block's steps beside its column's, so
+      // nothing is exchanged and the chain of a step is a reciprocal, a product
+      // and a multiply-add.
+      const int i = tid;
+      if (warp < (KP + PR + 31) / 32) {
+        int c = i - PR;
+        if (c >= j0) c += PR;
+        const bool xdiag = i < PR, adiag = i >= KP && i < KP + PR;
+        if (xdiag) c = j0 + i;
+        if (adiag) c = j0 + i - KP;
+        const bool there = i < KP + PR;
+        const int steps = min(PR, k - j0);
+        double x[PR], D[PR][PR], di[PR], least[PR];
+#pragma unroll
+        for (int r = 0; r < PR; ++r) {
+          x[r] = xdiag ? (r == i ? 1.0 : 0.0) : there ? P[r * KP + c] : 0.0;
+#pragma unroll
+          for (int q = r; q < PR; ++q) D[r][q] = P[r * KP + j0 + q];
+          if (r >= steps) D[r][r] = 1.0;  // rows past the matrix: zero but for the pivot
+          least[r] = CLAMP ? floor_d : attempt == 0 && r < steps ? fmax(tau * (dg[j0 + r] + shift), 0.0) : 0.0;
+        }
+        // No branch on a pivot: one that fails is noted, and what follows from it
+        // is not used.  (Every lane of every warp sees the same pivots.)
+        unsigned bad = 0;
+#pragma unroll
+        for (int r = 0; r < PR; ++r) {
+          double d = D[r][r];
+          if (CLAMP) d = d > floor_d ? d : floor_d;
+          else if (!(d > least[r] && d < INFINITY)) bad |= 1u << r;
+          di[r] = rcp_fast(d);
+          D[r][r] = d;
+#pragma unroll
+          for (int q = r + 1; q < PR; ++q) {
+            const double m = -(D[r][q] * di[r]);
+#pragma unroll
+            for (int s = q; s < PR; ++s) D[q][s] = fma(m, D[r][s], D[q][s]);
+            x[q] = fma(m, x[r], x[q]);
           }
         }
-        if (a > j && a < k) {
-          const double m = rowA[b][a] * di;
+        const int fail = bad ? j0 + __ffs(bad) - 1 : -1;
+        if (tid == 0) {
 #pragma unroll
-          for (int v = 0; v < U; ++v) {
-            const int c = tx + T * v;
-            if (c < k) {
-              if (c >= a) val[u][v] -= m * rowA[b][c];
-              else if (c <= j) val[u][v] -= m * rowX[b][c];
-            }
+          for (int r = 0; r < PR; ++r)
+            if (r < steps) piv[j0 + r] = D[r][r];
+        }
+        if (fail >= 0) {
+          if (tid == 0) fail_s = fail;
+        } else if (xdiag) {
+#pragma unroll
+          for (int r = 0; r < PR; ++r) {
+            T[r * FS + c] = x[r];
+            if (r > i) F[(j0 + r) * FS + c] = x[r];
           }
-          if (a == j + 1) {  // publish row j + 1 for the next step
+        } else if (adiag) {
 #pragma unroll
-            for (int v = 0; v < U; ++v) {
-              const int c = tx + T * v;
-              if (c < k) {
-                if (c >= a) rowA[b ^ 1][c] = val[u][v];
-                if (c < a) rowX[b ^ 1][c] = val[u][v];
-                if (c == a) {
-                  rowX[b ^ 1][c] = 1.0;
-                  pivot(a, val[u][v]);
-                }
-              }
-            }
+          for (int r = 0; r < PR; ++r)
+            if (r <= i - KP) F[(j0 + r) * FS + c] = x[r];
+        } else if (there) {
+#pragma unroll
+          for (int r = 0; r < PR; ++r) {
+            F[(j0 + r) * FS + c] = x[r];
+            M[r * KP + c] = x[r] * di[r];
           }
         }
       }
       __syncthreads();
+      if (fail_s >= 0) break;
+      // the panel's steps on the rows behind it: A's entries (c >= a), and X's
+      // up to the panel's last column; four blocks of rows at a time
+      const int pe = j0 + PR;
+      if (pe < k) {
+        const double* src[U];
+#pragma unroll
+        for (int v = 0; v < U; ++v) {
+          const int c = tx + 16 * v;
+          src[v] = (unsigned)(c - j0) < (unsigned)PR ? T + c : F + j0 * FS + c;
+        }
+#pragma unroll
+        for (int ub = 0; ub < U; ub += 4) {
+          if (16 * (ub + 4) <= pe) continue;
+          double s[4][U] = {};
+#pragma unroll
+          for (int r = 0; r < PR; ++r) {
+            double t[U];
+#pragma unroll
+            for (int v = 0; v < U; ++v) t[v] = src[v][r * FS];
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+              if (16 * (ub + w + 1) <= pe) continue;
+              const double m = M[r * KP + ty + 16 * (ub + w)];
+#pragma unroll
+              for (int v = 0; v < U; ++v) s[w][v] = fma(m, t[v], s[w][v]);
+            }
+          }
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            const int a = ty + 16 * (ub + w);
+#pragma unroll
+            for (int v = 0; v < U; ++v) {
+              const int c = tx + 16 * v;
+              if (a >= pe && (c >= a || c < pe)) val[ub + w][v] -= s[w][v];
+            }
+          }
+        }
+      }
     }
     __syncthreads();
-    fail = fail_s;
+    const int fail = fail_s;
     if (fail < 0) break;
     if (!shift_on_fail || attempt == 1) {
       if (tid == 0) status[0] = -(fail + 1);
@@ -289,47 +371,49 @@ __global__ void __launch_bounds__(T * T) k_cholesky(const double* __restrict__ G
     shift = 10.0 * tau * fmax(maxdiag_s, 1e-300);
     __syncthreads();
   }
-  // R^{-1}_ca = X_ac / sqrt(d_a), c <= a.
-#pragma unroll
-  for (int u = 0; u < U; ++u)
-#pragma unroll
-    for (int v = 0; v < U; ++v) {
-      const int a = ty + T * u, c = tx + T * v;
-      if (a < k && c <= a) {
-        const double x = (c == a ? 1.0 : val[u][v]) * pv_rinv[a];
-        Rinv[(int64_t)c * ld + a] = x;
-        Rinv_f[(int64_t)c * ld + a] = (float)x;
-      }
+  // 1 / sqrt(d_j), then R_jc = A_jc / sqrt(d_j) and R^{-1}_ca = X_ac / sqrt(d_a), c <= a
+  if (tid < k) {
+    const double d = piv[tid];
+    dg[tid] = rsqrt_fast(d);
+  }
+  __syncthreads();
+  for (int t = tid; t < ld * ld; t += NT) {
+    const int r = t / ld, c = t - r * ld;
+    double up = 0.0, inv = 0.0;
+    if (c < k && r <= c) {
+      up = r == c && CLAMP ? piv[r] * dg[r] : F[r * FS + c] * dg[r];
+      inv = (r == c ? 1.0 : F[c * FS + r]) * dg[c];
     }
+    R[t] = up;
+    Rinv[t] = inv;
+    if (!CLAMP) Rinv_f[t] = (float)inv;
+  }
+}
+
+template <bool CLAMP>
+static cudaError_t chol_go(const double* G, int k, int ld, double tau, int shift_on_fail, double* R, double* Rinv,
+                           float* Rinv_f, int* status, const void* tasks, int nblocks, cudaStream_t st) {
+  if (k > kMaxK || ld > kMaxK) return cudaErrorInvalidValue;
+  note_launches(1);
+  auto go = [&](auto kern, size_t smem) {
+    if (cudaError_t e = allow_smem(kern, smem); e != cudaSuccess) return e;
+    kern<<<nblocks, kCholThreads, smem, st>>>(G, k, ld, tau, shift_on_fail, R, Rinv, Rinv_f, status, tasks);
+    return cudaGetLastError();
+  };
+  if (k <= 64) return go(k_cholesky<64, CLAMP>, chol_smem<64>());
+  return go(k_cholesky<128, CLAMP>, chol_smem<128>());
 }
 
 cudaError_t launch_cholesky(const double* G, int k, int ld, double tau, int shift_on_fail,
                             double* R, double* Rinv, float* Rinv_f, int* status, cudaStream_t st) {
   if (ld > kMaxK) return launch_cholesky_wide(G, k, ld, tau, shift_on_fail, R, Rinv, Rinv_f, status, st);
-  if (k > kMaxK) return cudaErrorInvalidValue;
-  note_launches(1);
-  // 32 x 32 threads, 2 x 2 entries each for k <= 64 (measured per 60 x 60
-  // factor: 51 us, against 61 us for 16 x 16 threads with 4 x 4 entries, and
-  // 94 us for 8 warps updating rows of the matrix held in shared memory)
-  if (k <= 64)
-    k_cholesky<2, 32><<<1, 1024, 0, st>>>(G, k, ld, tau, shift_on_fail, R, Rinv, Rinv_f, status, nullptr);
-  else
-    k_cholesky<4, 32><<<1, 1024, 0, st>>>(G, k, ld, tau, shift_on_fail, R, Rinv, Rinv_f, status, nullptr);
-  return cudaGetLastError();
+  return chol_go<false>(G, k, ld, tau, shift_on_fail, R, Rinv, Rinv_f, status, nullptr, 1, st);
 }
 
 cudaError_t launch_cholesky_batch(const CholTask* tasks, int ntasks, int k, int ld, double tau, int shift_on_fail,
                                   cudaStream_t st) {
-  if (k > kMaxK || ld > kMaxK) return cudaErrorInvalidValue;
   if (ntasks <= 0) return cudaSuccess;
-  note_launches(1);
-  if (k <= 64)
-    k_cholesky<2, 32><<<ntasks, 1024, 0, st>>>(nullptr, k, ld, tau, shift_on_fail, nullptr, nullptr, nullptr, nullptr,
-                                               tasks);
-  else
-    k_cholesky<4, 32><<<ntasks, 1024, 0, st>>>(nullptr, k, ld, tau, shift_on_fail, nullptr, nullptr, nullptr, nullptr,
-                                               tasks);
-  return cudaGetLastError();
+  return chol_go<false>(nullptr, k, ld, tau, shift_on_fail, nullptr, nullptr, nullptr, nullptr, tasks, ntasks, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -1041,39 +1125,21 @@ cudaError_t launch_round_v(const double* A, int64_t g, int ld, const double* mu,
 // the NB synthetic at k = 40 and 60: 3e-2 -> 2e-5 -> 9e-11), so stopping at
 // t < 1e-4 leaves every eigenvector within ~1e-9 of the next sweep's, below
 // the FP32 resolution of the components and embeddings, and the eigenvalues
-// (second order in the rotation) within ~1e-18.  FP64 issue bandwidth (one warp instruction per ~4 cycles per SM
-// sub-partition) bounds a round, so the work per round is kept minimal.
-// ---------------------------------------------------------------------------
-// V (use_eglob) and R (use_rglob) go to the scratch that follows evecs when
-// they do not fit shared memory.  With `tasks` set, block b solves tasks[b]
-// (one launch for many segments) and C, evals, evecs, sweeps_out are ignored.
+// (second order in the rotation) within ~1e-18.
+// This form serves sketches wider than one panel (k > 128): R, and V after it,
+// in the scratch that follows evecs.
 template <int NR>  // column entries a lane holds in registers: kk <= 16 NR
 __global__ void __launch_bounds__(1024) k_jacobi(const double* __restrict__ C, int k, int ld,
                                                  double* __restrict__ evals, double* __restrict__ evecs,
-                                                 int use_eglob, int use_rglob, int* sweeps_out,
-                                                 const JacobiTask* __restrict__ tasks) {
-  if (tasks) {
-    const JacobiTask t = tasks[blockIdx.x];
-    C = t.C;
-    evals = t.evals;
-    evecs = t.evecs;
-    sweeps_out = t.sweeps;
-  }
-  double* Eglob = use_eglob ? evecs + (size_t)ld * ld : nullptr;
-  double* Rglob = use_rglob ? evecs + (size_t)ld * ld + (size_t)ld * (ld + 1) : nullptr;
-  extern __shared__ double sm[];
+                                                 int* sweeps_out) {
+  extern __shared__ __align__(16) double sm[];
   const int kk = (k + 1) & ~1;  // even number of columns; column k (if odd) is a zero dummy
   const int S = kk + 1;
   const int npair = kk / 2, m = kk - 1;
-  // R, and V after it, in shared memory when they fit, else in the global
-  // scratch the launcher passes (a sketch wider than one panel)
-  double* R = Rglob != nullptr ? Rglob : sm;                   // [kk cols][S]: R[c * S + r]
-  double* sm_rest = Rglob != nullptr ? sm : sm + kk * S;
-  uint16_t* sched = reinterpret_cast<uint16_t*>(sm_rest);      // [m][npair]: p | q << 8
-  double* V = (Eglob != nullptr) ? Eglob : sm_rest + (m * npair + 3) / 4;  // [kk cols][S]: R0, then V
+  double* V = evecs + (size_t)ld * ld;                   // [kk cols][S]: R0, then V
+  double* R = V + (size_t)ld * (ld + 1);                 // [kk cols][S]: R[c * S + r]
+  uint16_t* sched = reinterpret_cast<uint16_t*>(sm);     // [m][npair]: p | q << 8
   __shared__ double colnorm[kMaxKWide];
-  __shared__ int done;
-  __shared__ unsigned long long maxt_bits;  // largest |t| of the sweep (non-negative doubles order as integers)
   const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
   const int hl = lane & 15, half = lane >> 4;  // lane within the half-warp, which half
   const unsigned hmask = half ? 0xffff0000u : 0x0000ffffu;
@@ -1112,11 +1178,7 @@ __global__ void __launch_bounds__(1024) k_jacobi(const double* __restrict__ C, i
     }
     __syncthreads();
   }
-  if (tid == 0) {
-    if (k > 0) R[(k - 1) * S + (k - 1)] = prev_diag;
-    done = 1;
-    maxt_bits = 0ull;
-  }
+  if (tid == 0 && k > 0) R[(k - 1) * S + (k - 1)] = prev_diag;
   __syncthreads();
   // R0, kept for the back substitution; a unit diagonal for the dummy column
   // (odd k) keeps it invertible
@@ -1134,6 +1196,7 @@ __global__ void __launch_bounds__(1024) k_jacobi(const double* __restrict__ C, i
       if (hl == 0) colnorm[col] = a;
     }
     __syncthreads();
+    bool large = false;  // this thread's pairs turned by a tangent of 1e-4 or more
     for (int round = 0; round < m; ++round) {
       const uint16_t* pr = sched + round * npair;
       for (int i = 2 * warp + half; i < npair; i += 2 * nw) {
@@ -1182,20 +1245,12 @@ __global__ void __launch_bounds__(1024) k_jacobi(const double* __restrict__ C, i
           const double cc = cs * cs, ss = sn * sn, x2 = 2.0 * cs * sn * c;
           colnorm[p] = fma(cc, a, fma(ss, b, -x2));
           colnorm[q] = fma(ss, a, fma(cc, b, x2));
-          done = 0;
-          atomicMax(&maxt_bits, (unsigned long long)__double_as_longlong(fabs(t)));
         }
+        large |= !(fabs(t) < 1e-4);
       }
       __syncthreads();
     }
-    const int converged = done || __longlong_as_double((long long)maxt_bits) < 1e-4;
-    __syncthreads();  // every thread has read the flags before they are reset
-    if (converged) break;
-    if (tid == 0) {
-      done = 1;
-      maxt_bits = 0ull;
-    }
-    __syncthreads();
+    if (!__syncthreads_or(large)) break;  // no rotation, or none of 1e-4
   }
   // eigenvalues: squared column norms of R0 V
   for (int col = 2 * warp + half; col < kk; col += 2 * nw) {
@@ -1244,36 +1299,278 @@ __global__ void __launch_bounds__(1024) k_jacobi(const double* __restrict__ C, i
   if (tid == 0 && sweeps_out) *sweeps_out = sweep;
 }
 
+// ---------------------------------------------------------------------------
+// The same for k <= 128: one-sided Jacobi on the columns of the factor R0 that
+// k_cholesky<., true> left in global memory with its inverse (the rotations,
+// their order, the angle and the stopping rule are those of k_jacobi).  R0 sits
+// in shared memory column by column; eight lanes own a pair and read a column
+// 16 bytes per lane (eight lanes cover 128 consecutive bytes: no conflicts for
+// any pair).
+//
+// A round is a chain: columns in, a dot product, the angle, the rotation,
+// columns out, a barrier.  A half-warp per pair took 2,600 clocks for it at
+// k = 60: the largest tangent went through a 64-bit shared-memory maximum by
+// every pair, which serialised them (a lane keeps its own now, and the block
+// votes once per sweep), and at k = 110 both columns of every pair through
+// shared memory were more than its bandwidth hid.  Of the round-robin's two
+// columns of a pair one can stay in its group's registers for half a sweep, so
+// only the other moves.  Eight lanes need one shuffle stage less than sixteen
+// and half the warps, so the angle's instructions are issued for four pairs at
+// once; the pair of a round is kept by counting instead of a table; square
+// roots and reciprocals are the hardware's approximations, with steps to
+// double precision where the rotation has to be orthogonal.  V = R0^{-1} (R0 V)
+// is a product with the stored inverse instead of a back substitution per
+// column.  A round now takes 1,300 clocks at k = 60, bound by the latency of
+// the chain.  Measured, factor included: 454 -> 295 us at k = 60,
+// 228 -> 162 at k = 40, 1,861 -> 977 at k = 110.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float rsqrt_approx(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float y;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+template <int NQ>  // 16-byte pieces of a column per lane: kk <= 16 NQ
+__global__ void __launch_bounds__(NQ <= 4 ? 256 : 512) k_jacobi8(int k, int ld, double* evals, double* evecs, int* sweeps_out,
+                                                 const JacobiTask* __restrict__ tasks) {
+  if (tasks) {
+    const JacobiTask t = tasks[blockIdx.x];
+    evals = t.evals;
+    evecs = t.evecs;
+    sweeps_out = t.sweeps;
+  }
+  // the scratch behind evecs: R0, then R0^{-1}
+  double* R0 = evecs + (size_t)ld * ld;
+  const double* R0inv = R0 + (size_t)ld * ld;
+  constexpr int H = 16 * NQ;  // rows held (zero past k)
+  constexpr int S = H + 2;    // column stride: even, so every column starts on 16 bytes
+  extern __shared__ __align__(16) double sm[];
+  double* R = sm;  // [kk][S]
+  __shared__ double colnorm[kMaxK], inv_norm[kMaxK];
+  __shared__ int rank_of[kMaxK];
+  const int kk = (k + 1) & ~1;  // even number of columns; column k (if odd) is a zero dummy
+  const int npair = kk / 2, m = kk - 1;
+  const int tid = threadIdx.x, nt = blockDim.x, l = tid & 7, group = tid >> 3, ngroup = nt >> 3;
+  for (int t = tid; t < kk * S; t += nt) R[t] = 0.0;
+  __syncthreads();
+#pragma unroll 8
+  for (int t = tid; t < k * ld; t += nt) {
+    const int r = t / ld, c = t - r * ld;
+    const double x = R0[t];
+    if (r <= c && c < k) R[c * S + r] = x;
+  }
+  __syncthreads();
+  auto column = [&](double (&x)[2 * NQ], int c) {
+#pragma unroll
+    for (int u = 0; u < NQ; ++u)
+      *reinterpret_cast<double2*>(x + 2 * u) = *reinterpret_cast<const double2*>(R + c * S + 16 * u + 2 * l);
+  };
+  auto dot8 = [&](const double (&x)[2 * NQ], const double (&y)[2 * NQ]) {
+    double a = 0.0, b = 0.0;
+#pragma unroll
+    for (int u = 0; u < NQ; ++u) {
+      a = fma(x[2 * u], y[2 * u], a);
+      b = fma(x[2 * u + 1], y[2 * u + 1], b);
+    }
+    a += b;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    return a;
+  };
+  auto put_back = [&](const double (&x)[2 * NQ], int c) {
+#pragma unroll
+    for (int u = 0; u < NQ; ++u)
+      *reinterpret_cast<double2*>(R + c * S + 16 * u + 2 * l) = make_double2(x[2 * u], x[2 * u + 1]);
+  };
+  auto norms = [&]() {
+    for (int c0 = 0; c0 < kk; c0 += ngroup) {  // whole warps: a group past the columns repeats the last one
+      const int c = min(c0 + group, kk - 1);
+      double x[2 * NQ];
+      column(x, c);
+      const double a = dot8(x, x);
+      if (l == 0) colnorm[c] = a;
+    }
+  };
+  const bool active = group < npair;  // a group past the pairs shadows pair 0 and writes nothing
+  int sweep = 0;
+  for (; sweep < 40; ++sweep) {
+    norms();  // from scratch once per sweep
+    __syncthreads();
+    bool large = false;  // this lane's pair turned by a tangent of 1e-4 or more
+    // Pair i of round t: columns (t + i) mod m and (t - i) mod m, and t and m for
+    // i = 0.  A group keeps the first of them, xa, in registers while i counts
+    // down from its start to 0; only the second moves through shared memory.
+    // After i = 0 column t goes back and the group takes column t + npair, the
+    // second column of the round's last pair.
+    int i = active ? group : 0, ca = i, cb = i ? m - i : 0;
+    bool take = true;
+    double xa[2 * NQ];
+    for (int round = 0; round < m; ++round) {
+      const int other = i == 0 ? m : cb;
+      double xb[2 * NQ];
+      if (take) column(xa, ca);
+      column(xb, other);
+      const double na = colnorm[ca], nb = colnorm[other];
+      // what the angle needs of the norms, while the dot product is on its way
+      const double sc = pow2_int(-exponent_of(na + nb));
+      const float tf = (float)((ca < other ? nb - na : na - nb) * sc);
+      const double least = 1e-30 * na * nb, sc2 = 2.0 * sc;
+      const double c = dot8(xa, xb);
+      if (active && fabs(c) > 1e-150 && c * c > least) {  // uniform over the pair's lanes
+        // t = tan of the angle that zeroes p.q (p the lower column), in single
+        // precision from inputs scaled by a power of two into range (k_jacobi);
+        // below its resolution t is 0 and the rotation the identity
+        const float cf = (float)(c * sc2);
+        const float den = fabsf(tf) + sqrt_approx(fmaf(tf, tf, cf * cf));
+        const float ts = __fdividef(tf >= 0.f ? cf : -cf, den);
+        // cs = 1 / sqrt(1 + t^2) to double precision: a single-precision seed y
+        // and one step y (1 + e / 2 + 3 e^2 / 8), e = 1 - (1 + t^2) y^2
+        const double t = (double)ts, y = (double)rsqrt_approx(fmaf(ts, ts, 1.f));
+        const double e = fma(-fma(t, t, 1.0), y * y, 1.0);
+        const double cs = fma(y * e, fma(0.375, e, 0.5), y), sn = ca < other ? t * cs : -t * cs;
+#pragma unroll
+        for (int u = 0; u < NQ; ++u) {
+          double2 z;
+          z.x = sn * xa[2 * u] + cs * xb[2 * u];
+          z.y = sn * xa[2 * u + 1] + cs * xb[2 * u + 1];
+          xa[2 * u] = cs * xa[2 * u] - sn * xb[2 * u];
+          xa[2 * u + 1] = cs * xa[2 * u + 1] - sn * xb[2 * u + 1];
+          *reinterpret_cast<double2*>(R + other * S + 16 * u + 2 * l) = z;
+        }
+        if (l == 0) {
+          const double cc = cs * cs, ss = sn * sn, x2 = 2.0 * cs * sn * c;
+          colnorm[ca] = fma(cc, na, fma(ss, nb, -x2));
+          colnorm[other] = fma(ss, na, fma(cc, nb, x2));
+        }
+        large |= !(fabsf(ts) < 1e-4f);
+      }
+      take = i == 0;
+      if (take) {
+        if (active) put_back(xa, ca);
+        i = npair - 1;
+        cb = ca + 2 - npair;
+        if (cb < 0) cb += m;
+        ca += npair;
+        if (ca >= m) ca -= m;
+      } else {
+        --i;
+        cb += 2;
+        if (cb >= m) cb -= m;
+      }
+      __syncthreads();
+    }
+    if (active && !take) put_back(xa, ca);
+    __syncthreads();
+    if (!__syncthreads_or(large)) break;
+  }
+  // eigenvalues: squared column norms of R0 V; V = R0^{-1} (R0 V), then unit columns
+  norms();
+  // R0^{-1}'s upper triangle, row by row, behind R
+  double* Ri = R + (size_t)kk * S;
+  auto row_at = [&](int r) { return Ri + r * k - r * (r + 1) / 2; };  // row_at(r)[j], j >= r
+#pragma unroll 8
+  for (int t = tid; t < k * ld; t += nt) {
+    const int r = t / ld, j = t - r * ld;
+    const double x = R0inv[t];
+    if (j >= r && j < k) row_at(r)[j] = x;
+  }
+  __syncthreads();
+  // four rows by four columns of V per thread, before scaling: behind both
+  // where they fit, else over R0
+  double* W = NQ <= 4 ? Ri + k * (k + 1) / 2 : R0;
+  const int t4 = (k + 3) / 4;
+  for (int t = tid; t < t4 * t4; t += nt) {
+    const int r0 = t / t4 * 4, c0 = t % t4;  // columns c0 + t4 f: neighbours in neighbouring lanes
+    double acc[4][4] = {};
+    const double* ri[4];
+    const double* cj[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      ri[e] = row_at(min(r0 + e, k - 1));
+      cj[e] = R + min(c0 + t4 * e, k - 1) * S;
+    }
+    for (int j = r0; j < k; ++j) {
+      double x[4], y[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        x[e] = j >= r0 + e ? ri[e][j] : 0.0;
+        y[e] = cj[e][j];
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+#pragma unroll
+        for (int f = 0; f < 4; ++f) acc[e][f] = fma(x[e], y[f], acc[e][f]);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+#pragma unroll
+      for (int f = 0; f < 4; ++f)
+        if (r0 + e < k && c0 + t4 * f < k) W[(r0 + e) * ld + c0 + t4 * f] = acc[e][f];
+  }
+  __syncthreads();
+  // column c's length and rank, eight lanes per column
+  for (int c0 = 0; c0 < k; c0 += ngroup) {
+    const int c = min(c0 + group, k - 1);
+    const double v = colnorm[c];
+    double a = 0.0;
+    int rank = 0;
+    for (int r = l; r < k; r += 8) {
+      const double w = W[r * ld + c], o = colnorm[r];
+      a = fma(w, w, a);
+      if (o > v || (o == v && r < c)) ++rank;
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+      a += __shfl_xor_sync(0xffffffffu, a, o);
+      rank += __shfl_xor_sync(0xffffffffu, rank, o);
+    }
+    if (l == 0) {
+      inv_norm[c] = a > 0.0 ? rsqrt_nr(a) : 0.0;
+      rank_of[c] = rank;
+      evals[rank] = v;
+    }
+  }
+  __syncthreads();
+  for (int t = tid; t < ld * ld; t += nt) {
+    const int r = t / ld, c = t - r * ld;
+    if (r < k && c < k) evecs[r * ld + rank_of[c]] = W[t] * inv_norm[c];
+    else evecs[t] = 0.0;
+  }
+  if (tid == 0 && sweeps_out) *sweeps_out = sweep;
+}
+
 static cudaError_t jacobi_go(const double* C, int k, int ld, double* evals, double* evecs, int* sweeps,
                              const JacobiTask* tasks, int nblocks, cudaStream_t st) {
   const int kk = (k + 1) & ~1;
-  const size_t one = (size_t)kk * (kk + 1) * sizeof(double);
-  const size_t sched = ((size_t)(kk - 1) * (kk / 2) + 3) / 4 * sizeof(double);
-  // V lives in shared memory when both matrices fit, else in the scratch that
-  // follows evecs (the plan allocates ld * ld + 2 ld (ld + 1) doubles there),
-  // and R too when even one does not fit (a sketch wider than one panel).
-  if (kk > 256) return cudaErrorInvalidValue;  // the schedule packs a column pair into 8 + 8 bits
-  int use_e = 0, use_r = 0;
-  size_t smem = 2 * one + sched;
-  if (smem > 200 * 1024) {
-    use_e = 1;
-    smem = one + sched;
-  }
-  if (smem > 200 * 1024) {
-    use_r = 1;
-    smem = sched;
-  }
-  const int warps = std::min(32, std::max(1, (kk / 2 + 1) / 2));  // one half-warp per column pair
-  auto go = [&](auto kern) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
+  auto go = [&](auto kern, int threads, size_t smem, auto... args) {
+    if (cudaError_t e = allow_smem(kern, smem); e != cudaSuccess) return e;
     note_launches(1);
-    kern<<<nblocks, 32 * warps, smem, st>>>(C, k, ld, evals, evecs, use_e, use_r, sweeps, tasks);
+    kern<<<nblocks, threads, smem, st>>>(args...);
     return cudaGetLastError();
   };
-  if (kk <= 64) return go(k_jacobi<4>);
-  if (kk <= 128) return go(k_jacobi<8>);
-  return go(k_jacobi<16>);
+  if (k <= kMaxK) {
+    // C = R0^T R0 and R0^{-1} into the scratch behind evecs (the plan allocates
+    // ld * ld + 2 ld (ld + 1) doubles there), then the rotations
+    double* R0 = tasks ? nullptr : evecs + (size_t)ld * ld;
+    cudaError_t e = chol_go<true>(C, k, ld, 0.0, 0, R0, tasks ? nullptr : R0 + (size_t)ld * ld, nullptr, nullptr,
+                                  tasks, nblocks, st);
+    if (e != cudaSuccess) return e;
+    const int threads = (kk / 2 * 8 + 31) / 32 * 32;
+    auto smem = [&](int nq) {
+      return sizeof(double) * ((size_t)kk * (16 * nq + 2) + (size_t)k * (k + 1) / 2 + (nq <= 4 ? (size_t)k * ld : 0));
+    };
+    if (kk <= 64) return go(k_jacobi8<4>, threads, smem(4), k, ld, evals, evecs, sweeps, tasks);
+    return go(k_jacobi8<8>, threads, smem(8), k, ld, evals, evecs, sweeps, tasks);
+  }
+  if (kk > 256) return cudaErrorInvalidValue;  // the schedule packs a column pair into 8 + 8 bits
+  const size_t sched = ((size_t)(kk - 1) * (kk / 2) + 3) / 4 * sizeof(double);
+  const int warps = std::min(32, std::max(1, (kk / 2 + 1) / 2));  // one half-warp per column pair
+  return go(k_jacobi<16>, 32 * warps, sched, C, k, ld, evals, evecs, sweeps);
 }
 
 cudaError_t launch_jacobi_eig(const double* C, int k, int ld, double* evals, double* evecs,
