@@ -91,7 +91,12 @@ cudaError_t launch_rmat_strict(int dtype, int ld, const int64_t* indptr, const i
 cudaError_t launch_reduce_rows_f64(const double* part, int nparts, int64_t len, double* out,
                                    int accumulate, cudaStream_t st, int num_sms);
 
-// ---- CSR validation (kernels_csr.cu) ----
+// ---- prefix sums, CSR validation (kernels_csr.cu) ----
+// out[0..n] = exclusive prefix sums of n counts (out[n] the total); in and out do not overlap.
+cudaError_t launch_exclusive_scan_i64(const int64_t* in, int64_t n, int64_t* out, cudaStream_t st);
+// flags[0] and flags[1] of launch_validate_csr alone.
+cudaError_t launch_check_indices(const int64_t* indptr, const int32_t* idx, int64_t n, int64_t g, int64_t nnz,
+                                 int32_t* flags, cudaStream_t st, int num_sms);
 // flags[0]: bad indptr (non-monotone / out of range), flags[1]: column index
 // out of range, flags[2]: a row not sorted strictly ascending (duplicates or
 // disorder), flags[3]: non-finite value.
@@ -400,12 +405,16 @@ cudaError_t launch_sddmm(int dtype, const int64_t* indptr, const int32_t* idx, c
 cudaError_t launch_normalize_log1p(const int64_t* indptr, const float* in, float* out, int64_t n,
                                    double target_sum, int do_log1p, const float* row_factor, cudaStream_t st,
                                    int num_sms);
-// Kept entries per row under col_map (new index or -1), then the compacted CSR.
-cudaError_t launch_project_count(const int64_t* indptr, const int32_t* idx, int64_t n, const int32_t* col_map,
-                                 int64_t* counts, cudaStream_t st, int num_sms);
-cudaError_t launch_project_fill(const int64_t* indptr, const int32_t* idx, const float* val, int64_t n,
-                                const int32_t* col_map, const int64_t* out_ptr, int32_t* out_idx, float* out_val,
-                                cudaStream_t st, int num_sms);
+// Column projection: the kept columns as a bit per column and the number kept
+// before each word of 32.  The count checks the CSR as launch_check_indices does
+// and gives the kept entries per row; the fill writes the compacted CSR of a
+// checked one.
+cudaError_t launch_project_count(const int64_t* indptr, const int32_t* idx, int64_t n, int64_t g, int64_t nnz,
+                                 const uint32_t* bits, const int32_t* before, int64_t* counts, int32_t* flags,
+                                 cudaStream_t st, int num_sms);
+cudaError_t launch_project_fill(const int64_t* indptr, const int32_t* idx, const float* val, int64_t n, int64_t g,
+                                const uint32_t* bits, const int32_t* before, const int64_t* out_ptr,
+                                int32_t* out_idx, float* out_val, cudaStream_t st, int num_sms);
 
 // PFlog: delta = log1p(four_alpha x), baseline b_i = -sum_j delta_ij / d (FP64);
 // flags[0] negative count, flags[1] non-finite count.
@@ -433,7 +442,5 @@ cudaError_t launch_synth_fill(uint64_t seed, int64_t n, int64_t g, double loc, d
                               int32_t* idx, float* val, cudaStream_t st, int num_sms);
 cudaError_t launch_synth_gene_means(uint64_t seed, int64_t g, double loc, float* mu_g,
                                     cudaStream_t st);
-cudaError_t launch_exclusive_scan_i64(const int64_t* in, int64_t n, int64_t* out,
-                                      cudaStream_t st);
 
 }  // namespace scx

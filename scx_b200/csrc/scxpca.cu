@@ -3147,24 +3147,32 @@ int32_t scxpca_wait_selftest(int32_t device_ordinal, char* err, size_t err_len) 
 // Shared argument checks of the device-CSR producers: a device CSR with FP32
 // values whose indptr is monotone within [0, nnz] and whose column indices
 // lie in [0, n_vars) (validated on the device before any kernel indexes with
-// them).
-void check_device_csr_f32(const scxpca_csr* x, cudaStream_t st, int sms) {
+// them): the arguments, and the entries' flags (written by the check, or by
+// the projection's count) once they are back on the host.
+void check_csr_args_f32(const scxpca_csr* x) {
   if (!x) fail(SCXPCA_INVALID_ARGUMENT, "null csr");
   if (x->memory != SCXPCA_MEM_DEVICE) fail(SCXPCA_INVALID_ARGUMENT, "a device CSR (memory = DEVICE) is required");
   if (x->values_dtype != SCXPCA_F32) fail(SCXPCA_INVALID_ARGUMENT, "values must be float32");
   if (x->n_obs < 0 || x->n_vars <= 0 || x->nnz < 0) fail(SCXPCA_INVALID_ARGUMENT, "bad matrix dimensions");
   if (x->n_vars > INT32_MAX) fail(SCXPCA_INVALID_ARGUMENT, "n_vars exceeds int32 index range");
   if (!x->indptr || (x->nnz > 0 && (!x->indices || !x->values))) fail(SCXPCA_INVALID_ARGUMENT, "null CSR arrays");
+}
+
+void check_csr_flags(const int32_t* hf) {
+  if (hf[0]) fail(SCXPCA_INVALID_CSR, "invalid CSR: indptr is not monotone within [0, nnz]");
+  if (hf[1]) fail(SCXPCA_INVALID_CSR, "invalid CSR: column index out of range [0, n_vars)");
+}
+
+void check_device_csr_f32(const scxpca_csr* x, cudaStream_t st, int sms) {
+  check_csr_args_f32(x);
   DevBuf flags;
   flags.alloc(16);
   CK(cudaMemsetAsync(flags.p, 0, 16, st));
-  CK(launch_validate_csr(SCXPCA_F32, x->indptr, x->indices, x->values, x->n_obs, x->n_vars, x->nnz,
-                         flags.as<int32_t>(), st, sms));
+  CK(launch_check_indices(x->indptr, x->indices, x->n_obs, x->n_vars, x->nnz, flags.as<int32_t>(), st, sms));
   int32_t hf[4];
   CK(cudaMemcpyAsync(hf, flags.p, 16, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  if (hf[0]) fail(SCXPCA_INVALID_CSR, "invalid CSR: indptr is not monotone within [0, nnz]");
-  if (hf[1]) fail(SCXPCA_INVALID_CSR, "invalid CSR: column index out of range [0, n_vars)");
+  check_csr_flags(hf);
 }
 
 int32_t scxpca_preprocess(int32_t device_ordinal, const scxpca_csr* x, float* values_out, double target_sum,
@@ -3192,32 +3200,49 @@ int32_t scxpca_project_columns(int32_t device_ordinal, const scxpca_csr* x, cons
     if ((out_indices == nullptr) != (out_values == nullptr))
       fail(SCXPCA_INVALID_ARGUMENT, "out_indices and out_values must both be given or both be NULL");
     if (!x) fail(SCXPCA_INVALID_ARGUMENT, "null csr");
-    // the kept columns: sorted, unique, in range (ProjectedShardSource's contract)
-    std::vector<int32_t> col_map(x->n_vars > 0 ? x->n_vars : 0, -1);
+    // the kept columns: sorted, unique, in range (ProjectedShardSource's contract),
+    // as a bit per column and the number kept before each word of 32
+    const int64_t words = x->n_vars > 0 ? (x->n_vars + 31) / 32 : 0;
+    std::vector<uint32_t> table(2 * words, 0);
     for (int64_t i = 0; i < n_cols; ++i) {
       if (cols[i] < 0 || cols[i] >= x->n_vars) fail(SCXPCA_INVALID_ARGUMENT, "column index out of range");
       if (i > 0 && cols[i] <= cols[i - 1]) fail(SCXPCA_INVALID_ARGUMENT, "cols must be sorted and unique");
-      col_map[cols[i]] = (int32_t)i;
+      table[cols[i] >> 5] |= 1u << (cols[i] & 31);
     }
+    for (int64_t w = 1; w < words; ++w)
+      table[words + w] = table[words + w - 1] + (uint32_t)__builtin_popcount(table[w - 1]);
     DeviceGuard dg(device_ordinal);
     int sms = 148;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device_ordinal));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     PoolScope pool_scope(device_ordinal, st);
-    check_device_csr_f32(x, st, sms);
+    check_csr_args_f32(x);
     const int64_t n = x->n_obs;
-    DevBuf d_map, counts;
-    d_map.alloc(sizeof(int32_t) * col_map.size());
-    CK(cudaMemcpyAsync(d_map.p, col_map.data(), sizeof(int32_t) * col_map.size(), cudaMemcpyHostToDevice, st));
+    DevBuf d_table, counts, flags;
+    d_table.alloc(sizeof(uint32_t) * table.size());
+    CK(cudaMemcpyAsync(d_table.p, table.data(), sizeof(uint32_t) * table.size(), cudaMemcpyHostToDevice, st));
+    const uint32_t* bits = d_table.as<uint32_t>();
+    const int32_t* before = d_table.as<int32_t>() + words;
     counts.alloc(sizeof(int64_t) * std::max<int64_t>(n, 1));
-    CK(launch_project_count(x->indptr, x->indices, n, d_map.as<int32_t>(), counts.as<int64_t>(), st, sms));
+    flags.alloc(16);
+    CK(cudaMemsetAsync(flags.p, 0, 16, st));
+    if (n == 0)  // no row to count: the row pointers are still checked
+      CK(launch_check_indices(x->indptr, x->indices, n, x->n_vars, x->nnz, flags.as<int32_t>(), st, sms));
+    CK(launch_project_count(x->indptr, x->indices, n, x->n_vars, x->nnz, bits, before, counts.as<int64_t>(),
+                            flags.as<int32_t>(), st, sms));
     CK(launch_exclusive_scan_i64(counts.as<int64_t>(), n, out_indptr, st));
-    CK(cudaMemcpyAsync(nnz_out, out_indptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+    int32_t hf[4];
+    int64_t kept = 0;
+    CK(cudaMemcpyAsync(hf, flags.p, 16, cudaMemcpyDeviceToHost, st));
+    CK(cudaMemcpyAsync(&kept, out_indptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    if (out_indices)
-      CK(launch_project_fill(x->indptr, x->indices, static_cast<const float*>(x->values), n, d_map.as<int32_t>(),
+    check_csr_flags(hf);
+    *nnz_out = kept;
+    if (out_indices) {
+      CK(launch_project_fill(x->indptr, x->indices, static_cast<const float*>(x->values), n, x->n_vars, bits, before,
                              out_indptr, out_indices, out_values, st, sms));
-    CK(cudaStreamSynchronize(st));
+      CK(cudaStreamSynchronize(st));
+    }
   });
 }
 

@@ -11,8 +11,6 @@
 // holding (cell, gene, stream, attempt), so the two passes (count, fill)
 // regenerate identical counts without storing them.  Gamma: Marsaglia & Tsang
 // (2000); Poisson: multiplication method below 12, PTRS (Hoermann 1993) above.
-#include <cub/device/device_scan.cuh>
-
 #include "common.cuh"
 #include "launch.h"
 
@@ -201,21 +199,6 @@ cudaError_t launch_synth_fill(uint64_t seed, int64_t n, int64_t g, double loc, d
   k_fill<<<grid_for(n * 32, 256, num_sms, 8), 256, 0, st>>>(seed, n, g, (float)(1.0 / disp), mu_g,
                                                            indptr, rowsum, idx, val);
   return cudaGetLastError();
-}
-
-// Exclusive prefix sum of n int64 counts into out[0..n] (out[n] = total).
-cudaError_t launch_exclusive_scan_i64(const int64_t* in, int64_t n, int64_t* out, cudaStream_t st) {
-  cudaError_t err = cudaMemsetAsync(out, 0, sizeof(int64_t), st);
-  if (err != cudaSuccess || n == 0) return err;
-  size_t temp = 0;
-  err = cub::DeviceScan::InclusiveSum(nullptr, temp, in, out + 1, n, st);
-  if (err != cudaSuccess) return err;
-  void* d_temp = nullptr;
-  err = cudaMallocAsync(&d_temp, temp, st);
-  if (err != cudaSuccess) return err;
-  err = cub::DeviceScan::InclusiveSum(d_temp, temp, in, out + 1, n, st);
-  cudaFreeAsync(d_temp, st);
-  return err;
 }
 
 }  // namespace scx

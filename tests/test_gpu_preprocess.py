@@ -98,3 +98,58 @@ def test_raw_counts_to_pca_on_device_matches_oracle():
     rel = np.abs(res.singular_values - ref["singular_values"]) / ref["singular_values"]
     assert rel.max() < 1e-4, rel.max()
     assert rpca.principal_angles(res.components.T, ref["components"].T).max() < 1e-3
+
+
+@pytest.mark.parametrize("g", [800, 200_000])  # the column table in shared memory, and in global memory
+def test_row_lengths_around_the_steps(g):
+    """Rows around the 32-entry and 128-entry steps and around what a warp holds
+    in registers (256 entries), projected bit for bit and normalised to the
+    FP64 restatement (1e-6, the bound of this file)."""
+    lengths = [0, 1, 31, 32, 33, 127, 128, 129, 255, 256, 257, 0, 700, 3]
+    rng = np.random.default_rng(g)
+    idx = np.concatenate([np.sort(rng.choice(g, m, replace=False)) for m in lengths]).astype(np.int32)
+    idx[-1] = g - 1  # the last column of the last word
+    c = rpca.Csr(np.r_[0, np.cumsum(lengths)].astype(np.int64), idx,
+                 rng.integers(1, 50, len(idx)).astype(np.float32), (len(lengths), g))
+    ip, ix, vv = _dev(c)
+    got = accel.preprocess(ip, ix, vv, c.shape)
+    np.testing.assert_allclose(got.cpu().numpy(), rpca.normalize_log1p(c, 1e4, True, None), rtol=1e-6, atol=0)
+    for cols in ([g - 1], np.flatnonzero(rng.random(g) < 0.4), np.arange(g)):
+        pip, pix, pvv, shape = accel.project_columns(ip, ix, vv, c.shape, cols)
+        want = rpca.project_columns(c, np.asarray(cols))
+        np.testing.assert_array_equal(pip.cpu().numpy(), want.indptr)
+        np.testing.assert_array_equal(pix.cpu().numpy(), want.indices)
+        np.testing.assert_array_equal(pvv.cpu().numpy(), want.data)
+
+
+@pytest.mark.parametrize("n", [1, 2047, 2048, 2049, 4096, 530_000])
+def test_row_pointers_of_many_rows(n):
+    """The projected row pointers are an exclusive scan in tiles of 2,048 rows
+    (and 256 tiles a step): whole tiles, one row off them, more than one step."""
+    per_row = np.random.default_rng(n).integers(0, 3, n)
+    indptr = np.r_[0, np.cumsum(per_row)].astype(np.int64)
+    starts = np.repeat(indptr[:-1], per_row)
+    idx = (np.arange(indptr[-1]) - starts).astype(np.int32)
+    c = rpca.Csr(indptr, idx, np.ones(len(idx), dtype=np.float32), (n, 40))
+    ip, ix, vv = _dev(c)
+    pip, pix, _, _ = accel.project_columns(ip, ix, vv, c.shape, [0, 39])
+    np.testing.assert_array_equal(pip.cpu().numpy(), np.r_[0, np.cumsum(per_row > 0)])
+    assert pix.numel() == (per_row > 0).sum() and not pix.any()
+
+
+def test_producers_refuse_a_bad_csr():
+    from scx_b200._lib import ScxPcaError
+
+    c = _raw_counts(n=300, g=60, seed=8)
+    for where, value, word in (("index", 60, "column index"), ("index", -1, "column index"), ("ptr", -5, "indptr"),
+                               ("last", 1, "indptr")):
+        ip, ix, vv = _dev(c)
+        if where == "index":
+            ix[ix.numel() - 1] = value
+        else:
+            at = 100 if where == "ptr" else len(ip) - 1
+            ip[at] += value * 1000 if where == "ptr" else value
+        for call in (lambda: accel.preprocess(ip, ix, vv, c.shape),
+                     lambda: accel.project_columns(ip, ix, vv, c.shape, [1, 5])):
+            with pytest.raises(ScxPcaError, match=word):
+                call()
