@@ -19,190 +19,146 @@ namespace scx {
 // bit-identical from run to run.  Restates ScxCsr::col_sums_and_sum_sq
 // (scx-sparse/src/csr.rs:570-580).
 //
-// Block b owns the stored entries [b * per, (b + 1) * per) and walks them in
-// windows of kStatsWindow entries.  Its kStatsWarps warps share one FP64
-// accumulator pair per gene, and warp w owns the genes j with (j - lo) %
-// kStatsWarps == w, so no two warps touch one accumulator and no atomics are
-// needed.  Each window is read into registers one window ahead (thread t of
-// warp w holds the window's 32-entry steps w, w + 4, ...), then bucketed by
-// owning warp with a stable partition (ballot counts per step, one scan, a
-// scatter into shared memory), so each warp then walks only its own entries,
-// in window order.  Inside one 32-entry step of a bucket two lanes may name
-// the same gene only across a row boundary (a sorted row holds a gene once);
-// the step is cut into runs of strictly increasing gene index, applied one
-// after another in lane order.  Every gene's adds therefore happen in entry
-// order, whatever the rows look like (unsorted rows and duplicates included).
-// Genes beyond the shared-memory accumulator take further passes over the
-// block's entries, kStatsPassGenes at a time.  Each block writes one partial
-// row pair [sum | sum sq] (n_vars each); reduce_rows_f64 adds the partials in
-// block order.
+// Warp b of the partition owns the stored entries [b * per, (b + 1) * per) and
+// one FP64 accumulator pair per gene in shared memory, and walks its entries 32
+// at a time; no other warp touches its accumulators, so there are no atomics
+// and no barriers.  Inside one 32-entry step two lanes may name the same gene
+// only across a row boundary (a sorted row holds a gene once); the step is cut
+// into runs of strictly increasing gene index, applied one after another in
+// lane order.  Every gene's adds therefore happen in entry order, whatever the
+// rows look like (unsorted rows and duplicates included).  Genes beyond the
+// shared-memory accumulators take further passes over the warp's entries,
+// kStatsPassGenes at a time.  Each warp writes one partial row pair
+// [sum | sum sq] (n_vars each); reduce_rows_f64 adds the partials in order.
+//
+// What bounds it is the latency of a step's read-modify-write of 32 scattered
+// 16-byte pairs.  As many warps run on an SM as have room for their own
+// accumulators (6 at 2,000 genes); a warp takes two steps at once where their 64
+// genes increase, so their updates cannot meet (most pairs: a row has some 190
+// entries), and loads eight steps ahead, as stored (a conversion in the load
+// would wait for it).  92M entries: 366 us FP32, 373 BF16, against 825 and 912
+// for one accumulator set per block, its genes dealt to four warps through a
+// bucket sort of every 1,024-entry window.  (One step at a time: 526.)
 // ---------------------------------------------------------------------------
-constexpr int kStatsWarps = 4;
-constexpr int kStatsWindow = 1024;
-constexpr int kStatsSteps = kStatsWindow / 32;  // 32-entry steps per window
-// shared bytes besides the accumulators: the bucketed window (index + value)
-// and the per-step bucket offsets
-constexpr size_t kStatsWindowBytes = (size_t)kStatsWindow * 8 + (size_t)kStatsSteps * kStatsWarps * 4 + 64;
-constexpr int kStatsPassGenes = (int)((kStatsSmemMax - kStatsWindowBytes) / 16);
-static_assert(kStatsSteps == 32, "the bucket scan gives one window step to each lane of a warp");
-static_assert(kStatsSteps % kStatsWarps == 0, "every warp holds the same number of window steps");
+constexpr int kStatsMaxWarps = 16;  // warps (parts) of a block
+constexpr int kStatsAhead = 8;      // 32-entry steps a warp loads at once, before it needs them
+constexpr int kStatsPassGenes = (int)(kStatsSmemMax / 16);
 
-// `value(p, j, first)` gives entry p's value (gene j) as float; `first` is
-// true in the first gene pass.
-template <typename Value>
-__device__ __forceinline__ void col_stats_body(const int32_t* __restrict__ idx, Value value, int64_t nnz, int32_t g,
-                                               int32_t pass_genes, int nparts, int block0,
-                                               double* __restrict__ partial) {
-  extern __shared__ double sm[];  // [2][pass_genes] accumulators, then the bucketed window
-  double* acc = sm;
-  int32_t* b_idx = reinterpret_cast<int32_t*>(sm + 2 * (int64_t)pass_genes);
-  float* b_val = reinterpret_cast<float*>(b_idx + kStatsWindow);
-  int32_t* base = reinterpret_cast<int32_t*>(b_val + kStatsWindow);  // [kStatsSteps][kStatsWarps]
-  int32_t* qbase = base + kStatsSteps * kStatsWarps;                 // [kStatsWarps + 1]
-  constexpr int kPer = kStatsSteps / kStatsWarps;                    // steps per warp
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned lanemask_lt = (1u << lane) - 1u;
+// Warps whose accumulators fit an SM's shared memory.
+static int stats_warps(int64_t g) {
+  const int64_t pass = std::min<int64_t>(std::max<int64_t>(g, 1), kStatsPassGenes);
+  return (int)std::min<int64_t>(kStatsMaxWarps, (int64_t)kStatsSmemMax / (16 * pass));
+}
+
+int col_stats_parts(int64_t g, int num_sms) { return num_sms * stats_warps(g); }
+
+template <typename ValT>
+__global__ void __launch_bounds__(kStatsMaxWarps * 32) k_col_stats(const int32_t* __restrict__ idx,
+                                                                   const ValT* __restrict__ val, int64_t nnz,
+                                                                   int32_t g, int32_t pass_genes, int nparts,
+                                                                   int part0, int part1, double* __restrict__ partial) {
+  extern __shared__ __align__(16) double2 stats_sm[];  // [warps][pass_genes]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const unsigned lanemask_le = 0xffffffffu >> (31 - lane);
-  // partition block b of nparts owns entries [b per, (b + 1) per); this
-  // launch runs blocks block0 .. block0 + gridDim.x - 1 of it
-  const int b = block0 + (int)blockIdx.x;
+  // this launch runs parts part0 .. part1 - 1 of the partition
+  const int b = part0 + (int)blockIdx.x * warps + warp;
+  if (b >= part1) return;
+  double2* acc = stats_sm + (int64_t)warp * pass_genes;
   const int64_t per = (nnz + nparts - 1) / nparts;
   const int64_t s = min(nnz, (int64_t)b * per);
   const int64_t e = min(nnz, s + per);
   double* out = partial + (int64_t)b * 2 * g;
   for (int32_t lo = 0; lo < g; lo += pass_genes) {
     const int32_t gp = min(pass_genes, g - lo);
-    for (int i = threadIdx.x; i < 2 * gp; i += blockDim.x) acc[i] = 0.0;
-    // step u of this thread is the window's step kStatsWarps u + warp
-    int32_t ri[kPer];
-    float rv[kPer];
+    for (int i = lane; i < gp; i += 32) acc[i] = make_double2(0.0, 0.0);
+    int32_t nj[kStatsAhead];
+    ValT nx[kStatsAhead];
     auto load = [&](int64_t w) {
-      const int c = (int)min((int64_t)kStatsWindow, e - w);
 #pragma unroll
-      for (int u = 0; u < kPer; ++u) {
-        const int t = (kStatsWarps * u + warp) * 32 + lane;
-        ri[u] = t < c ? __ldg(idx + w + t) : -1;
-        rv[u] = t < c ? value(w + t, ri[u], lo == 0) : 0.f;
+      for (int u = 0; u < kStatsAhead; ++u) {
+        const int64_t p = w + 32 * u + lane;
+        nj[u] = p < e ? __ldg(idx + p) : INT32_MAX;
+        nx[u] = p < e ? val[p] : ValT();
       }
     };
-    if (s < e) load(s);
-    for (int64_t w0 = s; w0 < e; w0 += kStatsWindow) {
-      // owning warp of each held entry (kStatsWarps: not in this pass)
-      int own[kPer];
+    auto in_pass = [&](int32_t j) { return j >= lo && j - lo < gp; };  // (an index out of range is in no pass)
+    auto add = [](double2& a, double x) {
+      a.x += x;
+      a.y += x * x;
+    };
+    load(s);
+    __syncwarp();  // the accumulators are zeroed
+    for (int64_t w0 = s; w0 < e; w0 += 32 * kStatsAhead) {
+      int32_t cj[kStatsAhead];
+      double cx[kStatsAhead];
+      unsigned starts[kStatsAhead];  // lanes whose gene is not above the lane before's
+      bool follows[kStatsAhead];     // the step's first gene is above the last one of the step before
 #pragma unroll
-      for (int u = 0; u < kPer; ++u) {
-        const int32_t jr = ri[u] - lo;
-        own[u] = (ri[u] >= 0 && jr >= 0 && jr < gp) ? jr % kStatsWarps : kStatsWarps;
+      for (int u = 0; u < kStatsAhead; ++u) {
+        cj[u] = nj[u];
+        cx[u] = (double)to_f32(nx[u]);
       }
-      __syncthreads();  // the previous window's buckets are consumed (and the accumulators zeroed)
-      // per-step bucket sizes
+      load(w0 + 32 * kStatsAhead);
 #pragma unroll
-      for (int u = 0; u < kPer; ++u) {
-        const int step = kStatsWarps * u + warp;
-#pragma unroll
-        for (int q = 0; q < kStatsWarps; ++q) {
-          const unsigned m = __ballot_sync(0xffffffffu, own[u] == q);
-          if (lane == 0) base[step * kStatsWarps + q] = __popc(m);
-        }
+      for (int u = 0; u < kStatsAhead; ++u) {
+        const int32_t jl = __shfl_up_sync(0xffffffffu, cj[u], 1);
+        starts[u] = __ballot_sync(0xffffffffu, lane > 0 && cj[u] != INT32_MAX && cj[u] <= jl);
+        follows[u] = u > 0 && __shfl_sync(0xffffffffu, cj[u], 0) > __shfl_sync(0xffffffffu, cj[u ? u - 1 : 0], 31);
       }
-      __syncthreads();
-      // exclusive scan over the steps, bucket by bucket (warp 0; lane = step)
-      if (warp == 0) {
-        int cnt[kStatsWarps], inc[kStatsWarps];
 #pragma unroll
-        for (int q = 0; q < kStatsWarps; ++q) {
-          cnt[q] = base[lane * kStatsWarps + q];
-          inc[q] = cnt[q];
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, inc[q], o);
-            if (lane >= o) inc[q] += y;
+      for (int u = 0; u < kStatsAhead; u += 2) {
+        const bool in0 = in_pass(cj[u]), in1 = in_pass(cj[u + 1]);
+        if (starts[u] == 0 && starts[u + 1] == 0 && follows[u + 1]) {
+          // 64 increasing genes: the two steps' updates do not meet
+          double2 a0, a1;
+          if (in0) a0 = acc[cj[u] - lo];
+          if (in1) a1 = acc[cj[u + 1] - lo];
+          if (in0) {
+            add(a0, cx[u]);
+            acc[cj[u] - lo] = a0;
           }
-        }
-        int off = 0;
-#pragma unroll
-        for (int q = 0; q < kStatsWarps; ++q) {
-          const int total = __shfl_sync(0xffffffffu, inc[q], 31);
-          base[lane * kStatsWarps + q] = off + inc[q] - cnt[q];
-          if (lane == 0) qbase[q] = off;
-          off += total;
-        }
-        if (lane == 0) qbase[kStatsWarps] = off;
-      }
-      __syncthreads();
-      // stable scatter into the buckets
-#pragma unroll
-      for (int u = 0; u < kPer; ++u) {
-        const int step = kStatsWarps * u + warp;
-        const int q = own[u];
-        const unsigned m = __match_any_sync(0xffffffffu, q);
-        if (q < kStatsWarps) {
-          const int pos = base[step * kStatsWarps + q] + __popc(m & lanemask_lt);
-          b_idx[pos] = ri[u] - lo;
-          b_val[pos] = rv[u];
-        }
-      }
-      __syncthreads();
-      // the next window's loads are in flight while the buckets are applied
-      if (w0 + kStatsWindow < e) load(w0 + kStatsWindow);
-      const int q0 = qbase[warp], q1 = qbase[warp + 1];
-      for (int p0 = q0; p0 < q1; p0 += 32) {
-        const int t = p0 + lane;
-        const bool in = t < q1;
-        const int32_t jr = in ? b_idx[t] : -1;
-        const int32_t jl = __shfl_up_sync(0xffffffffu, jr, 1);
-        const unsigned starts = __ballot_sync(0xffffffffu, lane > 0 && in && jr <= jl);
-        const double x = in ? (double)b_val[t] : 0.0;
-        if (starts == 0) {
-          if (in) {
-            acc[jr] += x;
-            acc[gp + jr] += x * x;
+          if (in1) {
+            add(a1, cx[u + 1]);
+            acc[cj[u + 1] - lo] = a1;
           }
           __syncwarp();  // the next step's lanes see these updates
         } else {
-          const int run = __popc(starts & lanemask_le);
-          const int runs = __popc(starts) + 1;
-          for (int r = 0; r < runs; ++r) {
-            if (in && run == r) {
-              acc[jr] += x;
-              acc[gp + jr] += x * x;
+#pragma unroll
+          for (int v = u; v < u + 2; ++v) {
+            const int run = __popc(starts[v] & lanemask_le);
+            const int runs = __popc(starts[v]) + 1;
+            for (int r = 0; r < runs; ++r) {
+              if ((v == u ? in0 : in1) && run == r) {
+                double2 a = acc[cj[v] - lo];
+                add(a, cx[v]);
+                acc[cj[v] - lo] = a;
+              }
+              __syncwarp();
             }
-            __syncwarp();
           }
         }
       }
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < gp; i += blockDim.x) {
-      out[lo + i] = acc[i];
-      out[g + lo + i] = acc[gp + i];
+    for (int i = lane; i < gp; i += 32) {
+      out[lo + i] = acc[i].x;
+      out[g + lo + i] = acc[i].y;
     }
-    __syncthreads();
+    __syncwarp();
   }
-}
-
-template <typename ValT>
-__global__ void __launch_bounds__(kStatsWarps * 32) k_col_stats(const int32_t* __restrict__ idx,
-                                                                const ValT* __restrict__ val, int64_t nnz,
-                                                                int32_t g, int32_t pass_genes, int nparts,
-                                                                int block0, double* __restrict__ partial) {
-  col_stats_body(idx, [&](int64_t p, int32_t, bool) { return to_f32(val[p]); }, nnz, g, pass_genes, nparts, block0,
-                 partial);
 }
 
 // The value transform of one entry (k_transform_values, below): the working
 // value as stored.
 template <typename InT, typename OutT>
-__device__ __forceinline__ OutT transform_value(InT v, int32_t j, int mode, const double* __restrict__ mu,
-                                                const double* __restrict__ inv_std,
-                                                const double* __restrict__ cshift, double clip) {
+__device__ __forceinline__ OutT transform_value(InT v, int32_t j, int mode, const double* mu, const double* inv_std,
+                                                const double* cshift, double clip) {
   double x = (double)to_f32(v);
   if (mode != 0) {
-    const double is = __ldg(inv_std + j);
+    const double is = inv_std[j];
     if (mode == 1) {
-      double sv = (x - __ldg(mu + j)) * is;
+      double sv = (x - mu[j]) * is;
       if (clip > 0.0) sv = fmin(fmax(sv, -clip), clip);
-      x = sv - __ldg(cshift + j);
+      x = sv - cshift[j];
     } else {
       x = x * is;
       if (clip > 0.0) x = fmin(x, clip);
@@ -384,14 +340,42 @@ cudaError_t launch_reduce_rows_f64_batch(const GramTask* tasks, int ntasks, int 
 // c_g = clip(-mu * inv_std) is the value every stored zero takes, so the dense
 // scaled matrix is P + 1 c^T with P on X's sparsity pattern.
 // ---------------------------------------------------------------------------
-template <typename InT, typename OutT>
-__global__ void k_transform_values(const int32_t* __restrict__ idx, const InT* __restrict__ in,
-                                   OutT* __restrict__ out, int64_t nnz, int mode,
-                                   const double* __restrict__ mu, const double* __restrict__ inv_std,
-                                   const double* __restrict__ cshift, double clip) {
-  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz;
-       p += (int64_t)gridDim.x * blockDim.x)
-    out[p] = transform_value<InT, OutT>(in[p], mode != 0 ? __ldg(idx + p) : 0, mode, mu, inv_std, cshift, clip);
+// Four entries a thread, their loads in flight together.  With SMEM a block
+// stages the three per-gene vectors (mode != 0): an entry's three lookups are
+// random genes, and 32 of them cost the L1 a tag lookup per line touched
+// (92M FP32 entries to scaled BF16: 234 us against 282).
+template <typename InT, typename OutT, bool SMEM>
+__global__ void __launch_bounds__(512) k_transform_values(const int32_t* __restrict__ idx, const InT* __restrict__ in,
+                                                          OutT* __restrict__ out, int64_t nnz, int32_t g, int mode,
+                                                          const double* __restrict__ mu,
+                                                          const double* __restrict__ inv_std,
+                                                          const double* __restrict__ cshift, double clip) {
+  extern __shared__ double vec_sm[];  // [3][g]
+  if (SMEM) {
+    for (int i = threadIdx.x; i < g; i += blockDim.x) {
+      vec_sm[i] = mu[i];
+      vec_sm[g + i] = inv_std[i];
+      vec_sm[2 * g + i] = cshift[i];
+    }
+    __syncthreads();
+    mu = vec_sm;
+    inv_std = vec_sm + g;
+    cshift = vec_sm + 2 * g;
+  }
+  const int64_t nt = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < nnz; p += 4 * nt) {
+    int32_t j[4];
+    InT x[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool ok = p + u * nt < nnz;
+      j[u] = ok && mode != 0 ? __ldg(idx + p + u * nt) : 0;
+      x[u] = ok ? in[p + u * nt] : InT();
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (p + u * nt < nnz) out[p + u * nt] = transform_value<InT, OutT>(x[u], j[u], mode, mu, inv_std, cshift, clip);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -548,16 +532,19 @@ __global__ void __launch_bounds__(512) k_spmm_t(const int64_t* __restrict__ indp
 // Host launchers
 // ---------------------------------------------------------------------------
 template <typename ValT>
-static cudaError_t col_stats_blocks_t(const int32_t* idx, const void* val, int64_t nnz, int32_t g,
-                                      double* partial, int nparts, int block0, int nblocks, cudaStream_t st) {
-  if (nblocks <= 0) return cudaSuccess;
+static cudaError_t col_stats_blocks_t(const int32_t* idx, const void* val, int64_t nnz, int32_t g, double* partial,
+                                      int nparts, int part0, int count, cudaStream_t st, int num_sms) {
+  if (count <= 0) return cudaSuccess;
   const ValT* v = static_cast<const ValT*>(val);
   const int32_t pass_genes = std::min<int32_t>(g, kStatsPassGenes);
-  const size_t smem = (size_t)2 * pass_genes * sizeof(double) + kStatsWindowBytes;
+  // one block per SM, of as few warps as spread the parts over all of them
+  const int warps = std::max(1, std::min(stats_warps(g), (count + num_sms - 1) / num_sms));
+  const size_t smem = (size_t)warps * pass_genes * sizeof(double2);
   if (smem > 48 * 1024) {
     if (cudaError_t e = allow_smem(k_col_stats<ValT>, smem); e != cudaSuccess) return e;
   }
-  k_col_stats<ValT><<<nblocks, kStatsWarps * 32, smem, st>>>(idx, v, nnz, g, pass_genes, nparts, block0, partial);
+  k_col_stats<ValT><<<(count + warps - 1) / warps, warps * 32, smem, st>>>(idx, v, nnz, g, pass_genes, nparts, part0,
+                                                                          part0 + count, partial);
   note_launches(1);
   return cudaGetLastError();
 }
@@ -568,11 +555,12 @@ int64_t col_stats_block_begin(int64_t nnz, int nparts, int b) {
 }
 
 cudaError_t launch_col_stats_blocks(int dtype, const int32_t* idx, const void* val, int64_t nnz, int32_t g,
-                                    double* partial, int nparts, int block0, int nblocks, cudaStream_t st) {
+                                    double* partial, int nparts, int part0, int count, cudaStream_t st,
+                                    int num_sms) {
   switch (dtype) {
-    case 0: return col_stats_blocks_t<float>(idx, val, nnz, g, partial, nparts, block0, nblocks, st);
-    case 1: return col_stats_blocks_t<__nv_bfloat16>(idx, val, nnz, g, partial, nparts, block0, nblocks, st);
-    default: return col_stats_blocks_t<__half>(idx, val, nnz, g, partial, nparts, block0, nblocks, st);
+    case 0: return col_stats_blocks_t<float>(idx, val, nnz, g, partial, nparts, part0, count, st, num_sms);
+    case 1: return col_stats_blocks_t<__nv_bfloat16>(idx, val, nnz, g, partial, nparts, part0, count, st, num_sms);
+    default: return col_stats_blocks_t<__half>(idx, val, nnz, g, partial, nparts, part0, count, st, num_sms);
   }
 }
 
@@ -587,35 +575,52 @@ cudaError_t launch_col_stats_reduce(const double* partial, int nparts, int32_t g
 cudaError_t launch_col_stats(int dtype, const int32_t* idx, const void* val, int64_t nnz,
                              int32_t g, double* partial, int nparts, double* out,
                              cudaStream_t st, int num_sms, int accumulate) {
-  cudaError_t e = launch_col_stats_blocks(dtype, idx, val, nnz, g, partial, nparts, 0, nparts, st);
+  cudaError_t e = launch_col_stats_blocks(dtype, idx, val, nnz, g, partial, nparts, 0, nparts, st, num_sms);
   if (e != cudaSuccess) return e;
   return launch_col_stats_reduce(partial, nparts, g, out, st, num_sms, accumulate);
 }
 
-template <typename InT>
-static cudaError_t transform_in(int out_dtype, const int32_t* idx, const void* in, void* out,
-                                int64_t nnz, int mode, const double* mu, const double* inv_std,
-                                const double* cshift, double clip, cudaStream_t st, int num_sms) {
-  const InT* src = static_cast<const InT*>(in);
-  int grid = grid_for(nnz, 256, num_sms);
-  note_launches(1);
-  switch (out_dtype) {
-    case 0: k_transform_values<InT, float><<<grid, 256, 0, st>>>(idx, src, (float*)out, nnz, mode, mu, inv_std, cshift, clip); break;
-    case 1: k_transform_values<InT, __nv_bfloat16><<<grid, 256, 0, st>>>(idx, src, (__nv_bfloat16*)out, nnz, mode, mu, inv_std, cshift, clip); break;
-    default: k_transform_values<InT, __half><<<grid, 256, 0, st>>>(idx, src, (__half*)out, nnz, mode, mu, inv_std, cshift, clip); break;
-  }
-  return cudaGetLastError();
+template <typename InT, typename OutT>
+static cudaError_t transform_io(const int32_t* idx, const void* in, void* out, int64_t nnz, int32_t g, int mode,
+                                const double* mu, const double* inv_std, const double* cshift, double clip,
+                                cudaStream_t st, int num_sms) {
+  auto go = [&](auto kern, size_t smem, int blocks_per_sm) {
+    if (smem > 48 * 1024)
+      if (cudaError_t e = allow_smem(kern, smem); e != cudaSuccess) return e;
+    note_launches(1);
+    kern<<<grid_for(nnz, 2048, num_sms, blocks_per_sm), 512, smem, st>>>(idx, static_cast<const InT*>(in),
+                                                                         static_cast<OutT*>(out), nnz, g, mode, mu,
+                                                                         inv_std, cshift, clip);
+    return cudaGetLastError();
+  };
+  // the vectors in shared memory while two blocks of an SM can hold them
+  const size_t smem = 3 * sizeof(double) * (size_t)g;
+  if (mode != 0 && smem <= 100 * 1024)
+    return go(k_transform_values<InT, OutT, true>, smem, (int)std::min<size_t>(4, 200 * 1024 / smem));
+  return go(k_transform_values<InT, OutT, false>, 0, 4);
 }
 
-cudaError_t launch_transform_values(int in_dtype, int out_dtype, const int32_t* idx, const void* in,
-                                    void* out, int64_t nnz, int mode, const double* mu,
-                                    const double* inv_std, const double* cshift, double clip,
-                                    cudaStream_t st, int num_sms) {
+template <typename InT>
+static cudaError_t transform_in(int out_dtype, const int32_t* idx, const void* in, void* out, int64_t nnz, int32_t g,
+                                int mode, const double* mu, const double* inv_std, const double* cshift, double clip,
+                                cudaStream_t st, int num_sms) {
+  switch (out_dtype) {
+    case 0: return transform_io<InT, float>(idx, in, out, nnz, g, mode, mu, inv_std, cshift, clip, st, num_sms);
+    case 1:
+      return transform_io<InT, __nv_bfloat16>(idx, in, out, nnz, g, mode, mu, inv_std, cshift, clip, st, num_sms);
+    default: return transform_io<InT, __half>(idx, in, out, nnz, g, mode, mu, inv_std, cshift, clip, st, num_sms);
+  }
+}
+
+cudaError_t launch_transform_values(int in_dtype, int out_dtype, const int32_t* idx, const void* in, void* out,
+                                    int64_t nnz, int32_t g, int mode, const double* mu, const double* inv_std,
+                                    const double* cshift, double clip, cudaStream_t st, int num_sms) {
   if (nnz == 0) return cudaSuccess;
   switch (in_dtype) {
-    case 0: return transform_in<float>(out_dtype, idx, in, out, nnz, mode, mu, inv_std, cshift, clip, st, num_sms);
-    case 1: return transform_in<__nv_bfloat16>(out_dtype, idx, in, out, nnz, mode, mu, inv_std, cshift, clip, st, num_sms);
-    default: return transform_in<__half>(out_dtype, idx, in, out, nnz, mode, mu, inv_std, cshift, clip, st, num_sms);
+    case 0: return transform_in<float>(out_dtype, idx, in, out, nnz, g, mode, mu, inv_std, cshift, clip, st, num_sms);
+    case 1:
+      return transform_in<__nv_bfloat16>(out_dtype, idx, in, out, nnz, g, mode, mu, inv_std, cshift, clip, st, num_sms);
+    default: return transform_in<__half>(out_dtype, idx, in, out, nnz, g, mode, mu, inv_std, cshift, clip, st, num_sms);
   }
 }
 

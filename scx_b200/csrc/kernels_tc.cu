@@ -91,73 +91,142 @@ __host__ __device__ __forceinline__ int padded4(int x) { return (x + 3) & ~3; }
 // ---------------------------------------------------------------------------
 // format build
 // ---------------------------------------------------------------------------
-__global__ void k_tile_count(const int64_t* __restrict__ indptr, const int32_t* __restrict__ idx,
-                             int64_t n, int64_t n_tiles, int nc, int64_t* __restrict__ counts) {
+// Rows are sorted, so a row's entries of one chunk are neighbours: a run of
+// lanes with the same chunk counts through its first lane.  Four loads per lane
+// are in flight (92M entries: 144 us against 184).
+__global__ void __launch_bounds__(256) k_tile_count(const int64_t* __restrict__ indptr,
+                                                    const int32_t* __restrict__ idx, int64_t n, int64_t n_tiles,
+                                                    int nc, int64_t* __restrict__ counts) {
   extern __shared__ int cnt[];
+  const int lane = threadIdx.x & 31;
   for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
     for (int c = threadIdx.x; c < nc; c += blockDim.x) cnt[c] = 0;
     __syncthreads();
     const int64_t r0 = t * TM, r1 = min(n, r0 + TM);
-    for (int64_t p = indptr[r0] + threadIdx.x; p < indptr[r1]; p += blockDim.x)
-      atomicAdd(&cnt[__ldg(idx + p) >> 6], 1);
+    const int64_t e = indptr[r1];
+    for (int64_t b = indptr[r0] + (threadIdx.x & ~31); b < e; b += 4 * blockDim.x) {
+      int c[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int64_t p = b + (int64_t)u * blockDim.x + lane;
+        c[u] = p < e ? __ldg(idx + p) >> 6 : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int before = __shfl_up_sync(0xffffffffu, c[u], 1);
+        const bool first = lane == 0 || before != c[u];
+        const unsigned starts = __ballot_sync(0xffffffffu, first);
+        const unsigned behind = lane == 31 ? 0u : starts >> (lane + 1);
+        if (first && c[u] >= 0) atomicAdd(&cnt[c[u]], behind ? __ffs(behind) : 32 - lane);
+      }
+    }
     __syncthreads();
     for (int c = threadIdx.x; c < nc; c += blockDim.x) counts[t * nc + c] = padded4(cnt[c]);
     __syncthreads();
   }
 }
 
-__global__ void k_tile_fill(const int64_t* __restrict__ indptr, const int32_t* __restrict__ idx,
-                            const uint16_t* __restrict__ val, int64_t n, int64_t n_tiles, int nc,
-                            const int64_t* __restrict__ seg, uint32_t* __restrict__ ent,
-                            SegMeta* __restrict__ meta) {
+// One block per tile.  A row's first entry of every chunk falls out of its
+// sorted indices (no counters); a warp per chunk turns the rows' counts into
+// each row's first place in the chunk's segment; then every entry goes to its
+// place.  Entries are read 128 of a row at a time (four loads per lane in
+// flight), and the offsets take 16 KB at 2,000 genes, so four blocks share an
+// SM (92M entries: 450 us against 880 with two blocks, a shared atomic per
+// entry, one load in flight and a serial scan per row and per chunk).
+__global__ void __launch_bounds__(512) k_tile_fill(const int64_t* __restrict__ indptr, const int32_t* __restrict__ idx,
+                                                   const uint16_t* __restrict__ val, int64_t n, int64_t n_tiles,
+                                                   int nc, const int64_t* __restrict__ seg, uint32_t* __restrict__ ent,
+                                                   SegMeta* __restrict__ meta) {
   extern __shared__ int sm[];
-  int* colpre = sm;            // [TM][nc]: entries of chunk c in rows before r
-  int* rowpre = sm + TM * nc;  // [TM][nc]: entries of row r in chunks before c
+  // [TM][nc + 1]: a row's entries in chunks before c; then the place, from the
+  // tile's first entry word, that an entry of row r and chunk c takes less its
+  // position in the row
+  const int W = nc + 1;
+  int* place = sm;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x) {
-    for (int i = threadIdx.x; i < TM * nc; i += blockDim.x) colpre[i] = 0;
-    __syncthreads();
     const int64_t r0 = t * TM;
     const int rows = (int)min((int64_t)TM, n - r0);
-    for (int r = warp; r < rows; r += nw)
-      for (int64_t p = indptr[r0 + r] + lane; p < indptr[r0 + r + 1]; p += 32)
-        atomicAdd(&colpre[r * nc + (__ldg(idx + p) >> 6)], 1);
-    __syncthreads();
-    for (int r = threadIdx.x; r < TM; r += blockDim.x) {
-      int run = 0;
-      for (int c = 0; c < nc; ++c) {
-        rowpre[r * nc + c] = run;
-        run += colpre[r * nc + c];
+    for (int r = warp; r < TM; r += nw) {
+      const int64_t s = r < rows ? indptr[r0 + r] : 0, e = r < rows ? indptr[r0 + r + 1] : 0;
+      int before = -1;  // the chunk in front of the step's first entry
+      for (int64_t b = s; b < e; b += 128) {
+        int c[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int64_t p = b + 32 * u + lane;
+          c[u] = p < e ? __ldg(idx + p) >> 6 : nc;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          int prev = __shfl_up_sync(0xffffffffu, c[u], 1);
+          if (lane == 0) prev = before;
+          before = __shfl_sync(0xffffffffu, c[u], 31);
+          const int at = (int)(min(b + 32 * u + lane, e) - s);
+          for (int k = prev + 1; k <= c[u]; ++k) place[r * W + k] = at;
+        }
       }
+      // chunks past the last entry's (all of them in an empty row)
+      for (int k = before + 1 + lane; k <= nc; k += 32) place[r * W + k] = (int)(e - s);
     }
     __syncthreads();
-    for (int c = threadIdx.x; c < nc; c += blockDim.x) {
+    const int64_t base = seg[t * nc];
+    for (int c = warp; c < nc; c += nw) {
+      // lane l takes rows 4 l .. 4 l + 3: quarter q of the tile is lanes 8 q .. 8 q + 7
+      int at[4], cnt[4], sum = 0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        at[u] = place[(4 * lane + u) * W + c];
+        cnt[u] = place[(4 * lane + u) * W + c + 1] - at[u];
+        sum += cnt[u];
+      }
+      int incl = sum;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+      }
+      const int64_t start = seg[t * nc + c];
       SegMeta m;
-      m.start = seg[t * nc + c];
-      int run = 0;
-      for (int r = 0; r < TM; ++r) {
-        const int v = colpre[r * nc + c];
-        colpre[r * nc + c] = run;
-        run += v;
-        if (r == 31 || r == 63 || r == 95) m.q[r >> 5] = (uint16_t)run;
+      m.start = start;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) m.q[q] = (uint16_t)__shfl_sync(0xffffffffu, incl, 8 * q + 7);
+      if (lane == 0) meta[t * nc + c] = m;
+      // the chunk's column is read by the chunk in front of it as well: its new
+      // values wait in the column of a second table
+      int run = (int)(start - base) + incl - sum;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        sm[TM * W + (4 * lane + u) * nc + c] = run - at[u];
+        run += cnt[u];
       }
-      m.q[3] = (uint16_t)run;
-      meta[t * nc + c] = m;
     }
     __syncthreads();
+    const int* off = sm + TM * W;
     for (int r = warp; r < rows; r += nw) {
-      const int64_t s = indptr[r0 + r];
-      for (int64_t p = s + lane; p < indptr[r0 + r + 1]; p += 32) {
-        const int32_t j = __ldg(idx + p);
-        const int c = j >> 6;
-        const int64_t dst = seg[t * nc + c] + colpre[r * nc + c] + ((p - s) - rowpre[r * nc + c]);
-        ent[dst] = (uint32_t)val[p] | (sw128_offset((uint32_t)r, (uint32_t)(j & 63)) << 16);
+      const int64_t s = indptr[r0 + r], e = indptr[r0 + r + 1];
+      uint32_t* to = ent + base;
+      for (int64_t b = s; b < e; b += 128) {
+        int32_t j[4];
+        uint32_t x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int64_t p = b + 32 * u + lane;
+          j[u] = p < e ? __ldg(idx + p) : 0;
+          x[u] = p < e ? (uint32_t)val[p] : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int64_t p = b + 32 * u + lane;
+          if (p < e)
+            to[off[r * nc + (j[u] >> 6)] + (int)(p - s)] =
+                x[u] | (sw128_offset((uint32_t)r, (uint32_t)(j[u] & 63)) << 16);
+        }
       }
     }
     __syncthreads();
   }
 }
-
 
 // ---------------------------------------------------------------------------
 // shared pieces of the two product kernels
@@ -1695,7 +1764,7 @@ cudaError_t tile_format_count(const int64_t* indptr, const int32_t* idx, int64_t
                               int64_t* counts, cudaStream_t st, int num_sms) {
   const int64_t n_tiles = (n + TM - 1) / TM;
   note_launches(1);
-  k_tile_count<<<grid_for(n_tiles, 1, num_sms, 8), 256, nc * sizeof(int), st>>>(indptr, idx, n, n_tiles,
+  k_tile_count<<<grid_for(n_tiles, 1, num_sms, 64), 256, nc * sizeof(int), st>>>(indptr, idx, n, n_tiles,
                                                                                nc, counts);
   return cudaGetLastError();
 }
@@ -1704,10 +1773,10 @@ cudaError_t tile_format_fill(const int64_t* indptr, const int32_t* idx, const vo
                              int nc, const int64_t* seg, uint32_t* ent, void* meta, cudaStream_t st,
                              int num_sms) {
   const int64_t n_tiles = (n + TM - 1) / TM;
-  size_t smem = (size_t)2 * TM * nc * sizeof(int);
+  size_t smem = (size_t)TM * (2 * nc + 1) * sizeof(int);
   if (cudaError_t e = allow_smem(k_tile_fill, smem); e != cudaSuccess) return e;
   note_launches(1);
-  k_tile_fill<<<grid_for(n_tiles, 1, num_sms, 2), 512, smem, st>>>(
+  k_tile_fill<<<grid_for(n_tiles, 1, num_sms, 64), 512, smem, st>>>(
       indptr, idx, static_cast<const uint16_t*>(val16), n, n_tiles, nc, seg, ent,
       static_cast<SegMeta*>(meta));
   return cudaGetLastError();

@@ -25,17 +25,20 @@ constexpr int kTransposeGeneBlock = 256;       // genes per block, CUDA-core tra
 cudaError_t launch_col_stats(int dtype, const int32_t* idx, const void* val, int64_t nnz,
                              int32_t g, double* partial, int nparts, double* out,
                              cudaStream_t st, int num_sms, int accumulate = 0);
-// The same statistics in two halves: blocks [block0, block0 + nblocks) of the
-// nparts-block partition write their partials (block b reads entries
+// Parts that fill the device: as many warps per SM as hold their own accumulators.
+int col_stats_parts(int64_t g, int num_sms);
+// The same statistics in two halves: parts [part0, part0 + count) of the
+// partition write their partials (part b reads entries
 // [col_stats_block_begin(b), col_stats_block_begin(b + 1))), then one reduce.
 // Launching the partition in pieces gives the bits of one launch.
 int64_t col_stats_block_begin(int64_t nnz, int nparts, int b);
 cudaError_t launch_col_stats_blocks(int dtype, const int32_t* idx, const void* val, int64_t nnz, int32_t g,
-                                    double* partial, int nparts, int block0, int nblocks, cudaStream_t st);
+                                    double* partial, int nparts, int part0, int count, cudaStream_t st,
+                                    int num_sms);
 cudaError_t launch_col_stats_reduce(const double* partial, int nparts, int32_t g, double* out, cudaStream_t st,
                                     int num_sms, int accumulate = 0);
 cudaError_t launch_transform_values(int in_dtype, int out_dtype, const int32_t* idx,
-                                    const void* in, void* out, int64_t nnz, int mode,
+                                    const void* in, void* out, int64_t nnz, int32_t g, int mode,
                                     const double* mu, const double* inv_std,
                                     const double* cshift, double clip, cudaStream_t st,
                                     int num_sms);

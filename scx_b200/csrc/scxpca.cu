@@ -483,7 +483,7 @@ void compute_total_variance(scxpca_plan* pl) {
   DevBuf dz, d1;
   upload(dz, zero, pl->stream);
   upload(d1, one, pl->stream);
-  CK(launch_transform_values(pl->dtype, 0, pl->idx, pl->val, shifted.p, pl->nnz, 1, dmu.as<double>(),
+  CK(launch_transform_values(pl->dtype, 0, pl->idx, pl->val, shifted.p, pl->nnz, (int32_t)pl->g, 1, dmu.as<double>(),
                              d1.as<double>(), dz.as<double>(), 0.0, pl->stream, pl->num_sms));
   std::vector<double> s1, s2;
   stats_pass(pl, shifted.p, 0, s1, s2);
@@ -610,7 +610,7 @@ const void* shard_prepare(scxpca_plan* pl, size_t s, int k, bool work, int pack)
   const void* vals = sl.vin.p;
   if (work && pl->stream_transform) {
     CK(launch_transform_values(pl->in_dtype, pl->dtype, sl.idx.as<int32_t>(), sl.vin.p, sl.vwork.p, cnt,
-                               pl->stream_mode, pl->t_mu.as<double>(), pl->t_inv_std.as<double>(),
+                               (int32_t)pl->g, pl->stream_mode, pl->t_mu.as<double>(), pl->t_inv_std.as<double>(),
                                pl->t_cshift.as<double>(), pl->clip, st, pl->num_sms));
     vals = sl.vwork.p;
   }
@@ -775,7 +775,7 @@ void setup_streaming(scxpca_plan* pl, const scxpca_csr* x, size_t limit) {
   // what stays resident: the tall buffers (Y; the 16-bit image), the gene-side
   // and statistics buffers; the rest of `limit` is the two shard slots
   const double resident = (double)n * ld * 4 * (pl->use_tc ? 2 : 1) + (double)n * pl->nc * 4 +
-                          (double)g * ld * 8 * 8 + (double)2 * g * 8 * (2 * pl->num_sms + 1) + (64 << 20);
+                          (double)g * ld * 8 * 8 + (double)2 * g * 8 * (col_stats_parts(g, pl->num_sms) + 1) + (64 << 20);
   const double per_entry = slot_bytes_per_entry(pl, pl->use_tc) + (pl->use_tc ? 0.0 : 1.0);
   const double room = ((double)limit / 1.1 - resident) / 2.0;
   int64_t cap = (int64_t)std::min<double>((double)kShardEntriesMax, room / per_entry);
@@ -815,7 +815,7 @@ void setup_streaming(scxpca_plan* pl, const scxpca_csr* x, size_t limit) {
   phase_mark(SCXPCA_PHASE_UPLOAD, st);
 
   // ---- validation, input statistics (and gene counts) over the shards ----
-  pl->stats_parts = 4 * pl->num_sms;
+  pl->stats_parts = col_stats_parts(g, pl->num_sms);
   pl->stats_part.alloc(sizeof(double) * 2 * g * pl->stats_parts);
   pl->stats_out.alloc(sizeof(double) * 2 * g);
   DevBuf flags, counts;
@@ -896,7 +896,7 @@ void setup_streaming(scxpca_plan* pl, const scxpca_csr* x, size_t limit) {
         const int64_t cnt = sh.p1 - sh.p0;
         const void* vals = shard_prepare(pl, s, k, true, 0);
         CK(launch_transform_values(pl->stream_transform ? pl->dtype : pl->in_dtype, 0, sl.idx.as<int32_t>(), vals,
-                                   shifted.p, cnt, 1, d_shift.as<double>(), d_one.as<double>(), d_zero.as<double>(),
+                                   shifted.p, cnt, (int32_t)g, 1, d_shift.as<double>(), d_one.as<double>(), d_zero.as<double>(),
                                    0.0, st, pl->num_sms));
         CK(launch_col_stats(0, sl.idx.as<int32_t>(), shifted.p, cnt, (int32_t)g, pl->stats_part.as<double>(),
                             pl->stats_parts, pl->stats_out.as<double>(), st, pl->num_sms, s > 0 ? 1 : 0));
@@ -1098,7 +1098,7 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
 
     // ---- resident CSR ----
     const bool dev_in = x->memory == SCXPCA_MEM_DEVICE;
-    pl->stats_parts = 4 * pl->num_sms;
+    pl->stats_parts = col_stats_parts(g, pl->num_sms);
     pl->stats_part.alloc(sizeof(double) * 2 * g * pl->stats_parts);
     pl->stats_out.alloc(sizeof(double) * 2 * g);
     const void* vin = x->values;
@@ -1143,7 +1143,7 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
           CK(cudaEventRecord(landed[c], cs));
           CK(cudaStreamWaitEvent(st, landed[c], 0));
           CK(launch_col_stats_blocks(pl->in_dtype, pl->idx, vin, nnz, (int32_t)g, pl->stats_part.as<double>(),
-                                     parts, b0, b1 - b0, st));
+                                     parts, b0, b1 - b0, st, pl->num_sms));
         }
         for (auto& e : landed) CK(cudaEventDestroy(e));  // released once the pending work completes
         stats_queued = true;
@@ -1257,7 +1257,7 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
       upload(pl->d_mu, mu, st);
       upload(pl->d_inv_std, inv_std, st);
       upload(pl->d_cshift, cshift, st);
-      CK(launch_transform_values(pl->in_dtype, pl->dtype, pl->idx, vin, pl->b_val.p, nnz, mode,
+      CK(launch_transform_values(pl->in_dtype, pl->dtype, pl->idx, vin, pl->b_val.p, nnz, (int32_t)g, mode,
                                  pl->d_mu.as<double>(), pl->d_inv_std.as<double>(),
                                  pl->d_cshift.as<double>(), pl->clip, st, pl->num_sms));
       pl->val = pl->b_val.p;
