@@ -371,8 +371,8 @@ cudaError_t launch_split16(const float* in, int64_t count, uint16_t* img, int fm
 cudaError_t launch_colsum_f32(const float* A, int64_t n, int ld, int ncols, double* part, int nparts,
                               double* out, cudaStream_t st, int num_sms);
 // T (ld x ld) = A^T B over g rows, first ka x kb block (FP64).
-cudaError_t launch_atb(const double* A, const double* B, int64_t g, int ld, int ka, int kb, double* T,
-                       cudaStream_t st);
+cudaError_t launch_atb(const double* A, const double* B, int64_t g, int ld, int ka, int kb, double* part,
+                       int max_parts, double* T, cudaStream_t st, int num_sms);
 // M = E diag(1 / sqrt(evals)) over the first k columns.
 cudaError_t launch_ritz_scale(const double* E, const double* evals, int k, int ld, double* M, cudaStream_t st);
 // Phi[j][i] = T[j][i] / (evals[i] - evals[j]), j < k, i < c, j != i.

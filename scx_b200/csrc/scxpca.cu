@@ -985,7 +985,7 @@ void setup_streaming(scxpca_plan* pl, const scxpca_csr* x, size_t limit) {
 // The dense work buffers of a run (tall Y, gene-side factors, k x k FP64).
 void alloc_work_buffers(scxpca_plan* pl) {
   const int64_t n = pl->n, g = pl->g, ld = pl->ld;
-  pl->gram_parts = 2 * pl->num_sms;
+  pl->gram_parts = pl->num_sms;  // the Gram's registers leave room for one block per SM
   pl->gram_parts_small = (int)std::max<int64_t>(1, std::min<int64_t>(2 * pl->num_sms, (g + 31) / 32));
   pl->Y.alloc(sizeof(float) * n * ld);
   pl->W.alloc(sizeof(double) * g * ld);
@@ -2015,7 +2015,7 @@ void backward(scxpca_plan* pl, const float* S, const float* GS, int iters, float
   colsum(Y, ld, ld, sG);
   apply_t(1, H);
   // inside the sketch subspace: A_in = Vk Phi, Phi_ji = (Vk^T H)_ji / (lambda_i - lambda_j)
-  CK(launch_atb(Vk, H, g, ld, k, c, T, st));
+  CK(launch_atb(Vk, H, g, ld, k, c, pl->gpart.as<double>(), pl->gram_parts, T, st, pl->num_sms));
   CK(launch_phi(T, evals, k, c, ld, M, st));
   CK(launch_center_apply(Vk, g, ld, nullptr, nullptr, M, A, st));
   // outside it: (lambda_i I - X~^T X~) x_i = r_i on the complement, r = H - Vk (Vk^T H), by CG
@@ -2027,7 +2027,7 @@ void backward(scxpca_plan* pl, const float* S, const float* GS, int iters, float
   for (int m = 0; m < iters; ++m) {
     apply_f(P);
     apply_t(0, H);  // H <- X~^T X~ P
-    CK(launch_atb(Vk, H, g, ld, k, c, T, st));
+    CK(launch_atb(Vk, H, g, ld, k, c, pl->gpart.as<double>(), pl->gram_parts, T, st, pl->num_sms));
     CK(launch_center_apply(Vk, g, ld, nullptr, nullptr, T, Proj, st));
     CK(launch_cg_ap(P, H, Proj, evals, g, ld, c, Ap, st));
     CK(launch_coldot(P, Ap, g, ld, c, pAp, st));

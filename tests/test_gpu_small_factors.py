@@ -55,3 +55,25 @@ def test_singular_values_widths(matrix, k):
     rel = np.abs(res.singular_values - ref["singular_values"]) / ref["singular_values"]
     assert rel.max() < 1e-4
     assert np.abs(res.components @ res.components.T - np.eye(k)).max() < 1e-5
+
+
+@pytest.mark.parametrize("m", (128, 129, 130, 131, 1187, 9473))  # 9,473 rows: 32 a block, and one over
+@pytest.mark.parametrize("k", (20, 60, 90, 128))
+def test_qr_row_counts(matrix, m, k):
+    """The Gram behind a factor takes four rows at a time, a row group per block:
+    every remainder, blocks with no row, one row over.  The bound of
+    test_qr_factor_widths; the square case (m = k = 128) only keeps its
+    columns orthogonal, cond(A)^2 being past FP32 there."""
+    import torch
+
+    c = matrix
+    plan = accel.Plan(c.indptr, c.indices, c.data, c.shape, n_components=k, n_oversamples=0)
+    a = np.random.default_rng(m + k).standard_normal((m, k)).astype(np.float32)
+    q = plan.qr(torch.from_numpy(a).cuda()).cpu().numpy().astype(np.float64)
+    plan.close()
+    assert np.abs(q.T @ q - np.eye(k)).max() < 2e-6
+    if m > 2 * k:
+        a64 = a.astype(np.float64)
+        r = np.linalg.cholesky(a64.T @ a64).T
+        want = np.linalg.solve(r.T, a64.T).T
+        assert np.abs(q - want).max() < 2e-6 * np.abs(want).max() * np.linalg.cond(a64)
