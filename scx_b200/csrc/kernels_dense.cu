@@ -1081,6 +1081,17 @@ cudaError_t launch_apply_right_f64(double* A, int64_t g, int ld, const double* M
   return launch_center_apply(A, g, ld, nullptr, nullptr, M, A, st);
 }
 
+__global__ void k_identity(double* __restrict__ M, int ld) {
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < ld * ld; t += gridDim.x * blockDim.x)
+    M[t] = t / ld == t % ld ? 1.0 : 0.0;
+}
+
+cudaError_t launch_identity(double* M, int ld, cudaStream_t st) {
+  note_launches(1);
+  k_identity<<<(ld * ld + 1023) / 1024, 256, 0, st>>>(M, ld);
+  return cudaGetLastError();
+}
+
 __global__ void k_round_v(const double* __restrict__ A, int64_t g, int ld, float* __restrict__ Vf) {
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < g * ld;
        t += (int64_t)gridDim.x * blockDim.x)

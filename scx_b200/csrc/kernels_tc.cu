@@ -192,6 +192,9 @@ __global__ void __launch_bounds__(512) k_tile_fill(const int64_t* __restrict__ i
 #pragma unroll
       for (int q = 0; q < 4; ++q) m.q[q] = (uint16_t)__shfl_sync(0xffffffffu, incl, 8 * q + 7);
       if (lane == 0) meta[t * nc + c] = m;
+      // the padding of the segment's last entry word
+      const int total = __shfl_sync(0xffffffffu, incl, 31);
+      if (lane < padded4(total) - total) ent[start + total + lane] = 0u;
       // the chunk's column is read by the chunk in front of it as well: its new
       // values wait in the column of a second table
       int run = (int)(start - base) + incl - sum;
@@ -1348,10 +1351,11 @@ __device__ __forceinline__ void fwd_swap_body(const Src& src, int nc, int fmt) {
           float* ydst = Y ? Y + c0 * LD + j : nullptr;
 #pragma unroll
           for (int i = 0; i < 32; i += 2) {
+            // each lane gives the other the half it does not need (one exchange
+            // for two cells)
             const float x0 = __uint_as_float(r[i]), x1 = __uint_as_float(r[i + 1]);
-            const float s0 = x0 + __shfl_xor_sync(0xffffffffu, x0, 1) - mcj;
-            const float s1 = x1 + __shfl_xor_sync(0xffffffffu, x1, 1) - mcj;
-            const float sm = p ? s1 : s0;
+            const float other = __shfl_xor_sync(0xffffffffu, p ? x0 : x1, 1);
+            const float sm = (p ? x1 : x0) + other - mcj;
             if (i + p < lim) {
               dst[(i + p) * 64] = hilo16(sm, fmt);
               if (ydst) ydst[(i + p) * LD] = sm;

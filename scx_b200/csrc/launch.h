@@ -244,6 +244,7 @@ cudaError_t launch_center_apply(const double* W, int64_t g, int ld, const double
 cudaError_t launch_apply_right_f64(double* A, int64_t g, int ld, const double* M,
                                    cudaStream_t st);
 //   Vf = (float)A ; mc = A^T mu (float, from the rounded Vf) ; mu may be null
+cudaError_t launch_identity(double* M, int ld, cudaStream_t st);  // M = I (ld x ld)
 cudaError_t launch_round_v(const double* A, int64_t g, int ld, const double* mu, float* Vf,
                            float* mc, cudaStream_t st);
 //   mc = Vf^T mu for a float V (mu may be null -> zeros)

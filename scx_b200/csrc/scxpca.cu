@@ -23,6 +23,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/scxpca.h"
@@ -88,6 +89,7 @@ struct DeviceGuard {
 // against the stream that uses the memory by events.  The pool's memory
 // stays reserved by the process until it exits.
 struct DevicePool {
+  int dev = 0;
   cudaMemPool_t pool = nullptr;
   cudaStream_t st = nullptr;  // allocation stream
 };
@@ -99,6 +101,7 @@ DevicePool& pool_for(int dev) {
   if (dev < 0 || dev >= 256) fail(SCXPCA_INVALID_ARGUMENT, "device ordinal out of range");
   DevicePool& dp = pools[dev];
   if (!dp.pool) {
+    dp.dev = dev;
     cudaMemPoolProps props{};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
@@ -111,13 +114,151 @@ DevicePool& pool_for(int dev) {
   return dp;
 }
 
-// Order `to` after the work enqueued so far on `from`.
-void stream_fence(cudaStream_t from, cudaStream_t to) {
-  cudaEvent_t e;
-  CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  CK(cudaEventRecord(e, from));
-  CK(cudaStreamWaitEvent(to, e, 0));
-  cudaEventDestroy(e);
+// Order `to` after the work enqueued so far on `from`.  A thread keeps one
+// event per device for this (a record and a wait, no creation): a wait takes
+// the state of the record before it, so the event can be recorded again at once.
+struct FenceEvents {
+  cudaEvent_t e[256] = {};
+  ~FenceEvents() {
+    for (cudaEvent_t ev : e)
+      if (ev) cudaEventDestroy(ev);
+  }
+};
+thread_local FenceEvents t_fence;
+
+cudaError_t try_stream_fence(int dev, cudaStream_t from, cudaStream_t to) {
+  cudaEvent_t& ev = t_fence.e[dev & 255];
+  cudaError_t e = ev ? cudaSuccess : cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventRecord(ev, from);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(to, ev, 0);
+  return e;
+}
+
+// Streams of plans that make their own: given back when the plan goes and
+// handed to the next one (creating and destroying one costs 180 us of a
+// one-shot call).  At most kIdleStreams wait per device.
+constexpr size_t kIdleStreams = 16;
+struct StreamPool {
+  std::mutex mu;
+  std::vector<cudaStream_t> idle;
+};
+StreamPool& stream_pool(int dev) {
+  static StreamPool* pools = new StreamPool[256];  // never destroyed: plans may outlive static objects
+  return pools[dev & 255];
+}
+cudaStream_t take_stream(int dev) {
+  {
+    StreamPool& sp = stream_pool(dev);
+    std::lock_guard<std::mutex> lock(sp.mu);
+    if (!sp.idle.empty()) {
+      cudaStream_t st = sp.idle.back();
+      sp.idle.pop_back();
+      return st;
+    }
+  }
+  cudaStream_t st = nullptr;
+  CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+  return st;
+}
+void give_stream(int dev, cudaStream_t st) {
+  if (!st) return;
+  {
+    StreamPool& sp = stream_pool(dev);
+    std::lock_guard<std::mutex> lock(sp.mu);
+    if (sp.idle.size() < kIdleStreams) {
+      sp.idle.push_back(st);
+      return;
+    }
+  }
+  cudaStreamDestroy(st);
+}
+
+// Page-locked staging of small results: device-to-host copies into it run
+// without the driver's own staging and its wait per copy, and one
+// synchronisation serves them all.  Buffers go back to a list that keeps at most
+// kStageHeld bytes; a buffer whose copies may still run is waited for first.
+constexpr size_t kStageMost = size_t(16) << 20;  // larger results are copied directly
+constexpr size_t kStageHeld = size_t(64) << 20;
+struct StageList {
+  std::mutex mu;
+  std::vector<std::pair<void*, size_t>> idle;
+  size_t held = 0;
+};
+StageList& stage_list() {
+  static StageList* l = new StageList;
+  return *l;
+}
+struct Staging {
+  char* p = nullptr;
+  size_t bytes = 0;
+  cudaStream_t busy = nullptr;  // stream whose copies into the buffer have not been waited for
+  bool pending = false;
+  explicit Staging(size_t need, cudaStream_t st) : busy(st) {
+    StageList& l = stage_list();
+    {
+      std::lock_guard<std::mutex> lock(l.mu);
+      size_t best = l.idle.size();
+      for (size_t i = 0; i < l.idle.size(); ++i)
+        if (l.idle[i].second >= need && (best == l.idle.size() || l.idle[i].second < l.idle[best].second)) best = i;
+      if (best < l.idle.size()) {
+        p = static_cast<char*>(l.idle[best].first);
+        bytes = l.idle[best].second;
+        l.held -= bytes;
+        l.idle.erase(l.idle.begin() + best);
+        return;
+      }
+    }
+    bytes = size_t(1) << 16;
+    while (bytes < need) bytes *= 2;
+    void* q = nullptr;
+    CK(cudaHostAlloc(&q, bytes, cudaHostAllocPortable));
+    p = static_cast<char*>(q);
+  }
+  Staging(const Staging&) = delete;
+  Staging& operator=(const Staging&) = delete;
+  void fetch(size_t at, const void* src, size_t n) {
+    pending = true;
+    CK(cudaMemcpyAsync(p + at, src, n, cudaMemcpyDeviceToHost, busy));
+  }
+  void wait() {
+    CK(cudaStreamSynchronize(busy));
+    pending = false;
+  }
+  template <typename T> const T* at(size_t o) const { return reinterpret_cast<const T*>(p + o); }
+  ~Staging() {
+    if (pending) cudaStreamSynchronize(busy);
+    StageList& l = stage_list();
+    {
+      std::lock_guard<std::mutex> lock(l.mu);
+      if (l.held + bytes <= kStageHeld) {
+        l.idle.emplace_back(p, bytes);
+        l.held += bytes;
+        return;
+      }
+    }
+    cudaFreeHost(p);
+  }
+};
+
+// Copy between host buffers; a large one by four threads (most of it is the
+// destination's first touch, page by page).
+void host_copy(void* dst, const void* src, size_t bytes) {
+  constexpr size_t kEach = size_t(1) << 20;
+  const int parts = (int)std::min<size_t>(4, bytes / kEach);
+  if (parts < 2) {
+    memcpy(dst, src, bytes);
+    return;
+  }
+  const size_t per = bytes / parts;
+  std::vector<std::thread> threads;
+  int started = 0;
+  try {
+    for (; started + 1 < parts; ++started)
+      threads.emplace_back([=] { memcpy((char*)dst + started * per, (const char*)src + started * per, per); });
+  } catch (...) {  // no thread to be had: the rest here
+  }
+  memcpy((char*)dst + started * per, (const char*)src + started * per, bytes - started * per);
+  for (std::thread& t : threads) t.join();
 }
 
 // Phase timing of the calling thread's one-shot call (scxpca_randomized):
@@ -165,6 +306,15 @@ struct AllocCtx {
 };
 thread_local AllocCtx t_alloc;
 
+// A stream the calling thread has waited for and enqueues nothing more on:
+// buffers used on it are freed without an event each (a plan being destroyed).
+thread_local cudaStream_t t_idle_stream = nullptr;
+struct IdleStreamScope {
+  cudaStream_t prev;
+  explicit IdleStreamScope(cudaStream_t st) : prev(t_idle_stream) { t_idle_stream = st; }
+  ~IdleStreamScope() { t_idle_stream = prev; }
+};
+
 struct PoolScope {
   AllocCtx prev;
   PoolScope(int dev, cudaStream_t use) : prev(t_alloc) { t_alloc = AllocCtx{&pool_for(dev), use}; }
@@ -184,12 +334,7 @@ struct DevBuf {
   void release() {
     if (p) {
       if (pooled) {  // after the work already enqueued on the using stream
-        cudaEvent_t e;
-        if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess) {
-          cudaEventRecord(e, st);
-          cudaStreamWaitEvent(dp->st, e, 0);
-          cudaEventDestroy(e);
-        }
+        if (st != t_idle_stream || !t_idle_stream) try_stream_fence(dp->dev, st, dp->st);
         cudaFreeAsync(p, dp->st);
       } else {
         cudaFree(p);
@@ -210,7 +355,7 @@ struct DevBuf {
         dp = t_alloc.dp;
         st = t_alloc.use;
         pooled = true;
-        stream_fence(dp->st, st);  // the using stream starts after the allocation
+        CK(try_stream_fence(dp->dev, dp->st, st));  // the using stream starts after the allocation
       }
     } else {
       e = cudaMalloc(&p, b);
@@ -378,7 +523,7 @@ struct scxpca_plan {
     for (cudaEvent_t e : events) cudaEventDestroy(e);
     if (copy_stream) {
       cudaStreamSynchronize(copy_stream);
-      cudaStreamDestroy(copy_stream);
+      give_stream(device, copy_stream);
     }
     for (int i = 0; i < 2; ++i) {
       if (ev_copied[i]) cudaEventDestroy(ev_copied[i]);
@@ -422,29 +567,26 @@ void validate_params(const scxpca_csr* x, const scxpca_params* p) {
 // Pieces a host matrix's entries are copied in (statistics overlap the copy).
 constexpr int kUploadPieces = 8;
 
-// Reduce the statistics partials already written to stats_part and bring
-// the column sums and sums of squares to the host.
-void stats_finish(scxpca_plan* pl, std::vector<double>& sums, std::vector<double>& sq) {
-  CK(launch_col_stats_reduce(pl->stats_part.as<double>(), pl->stats_parts, (int32_t)pl->g,
-                             pl->stats_out.as<double>(), pl->stream, pl->num_sms));
-  std::vector<double> host(2 * pl->g);
-  CK(cudaMemcpyAsync(host.data(), pl->stats_out.p, sizeof(double) * 2 * pl->g,
-                     cudaMemcpyDeviceToHost, pl->stream));
-  CK(cudaStreamSynchronize(pl->stream));
-  sums.assign(host.begin(), host.begin() + pl->g);
-  sq.assign(host.begin() + pl->g, host.end());
-}
+// Column sums and sums of squares on their way to the host.
+struct StatsFetch {
+  Staging h;
+  int64_t g;
+  StatsFetch(scxpca_plan* pl) : h(sizeof(double) * 2 * pl->g + 16, pl->stream), g(pl->g) {
+    h.fetch(0, pl->stats_out.p, sizeof(double) * 2 * g);
+  }
+  void take(std::vector<double>& sums, std::vector<double>& sq) {  // after h.wait()
+    sums.assign(h.at<double>(0), h.at<double>(0) + g);
+    sq.assign(h.at<double>(0) + g, h.at<double>(0) + 2 * g);
+  }
+};
 
 void stats_pass(scxpca_plan* pl, const void* val, int dtype, std::vector<double>& sums,
                 std::vector<double>& sq) {
   CK(launch_col_stats(dtype, pl->idx, val, pl->nnz, (int32_t)pl->g, pl->stats_part.as<double>(),
                       pl->stats_parts, pl->stats_out.as<double>(), pl->stream, pl->num_sms));
-  std::vector<double> host(2 * pl->g);
-  CK(cudaMemcpyAsync(host.data(), pl->stats_out.p, sizeof(double) * 2 * pl->g,
-                     cudaMemcpyDeviceToHost, pl->stream));
-  CK(cudaStreamSynchronize(pl->stream));
-  sums.assign(host.begin(), host.begin() + pl->g);
-  sq.assign(host.begin() + pl->g, host.end());
+  StatsFetch f(pl);
+  f.h.wait();
+  f.take(sums, sq);
 }
 
 void upload(DevBuf& buf, const std::vector<double>& v, cudaStream_t st) {
@@ -619,7 +761,6 @@ const void* shard_prepare(scxpca_plan* pl, size_t s, int k, bool work, int pack)
     CK(tile_format_count(sl.ip.as<int64_t>(), sl.idx.as<int32_t>(), rows, pl->n_chunks, sl.counts.as<int64_t>(), st,
                          pl->num_sms));
     CK(launch_exclusive_scan_i64(sl.counts.as<int64_t>(), nseg, sl.seg.as<int64_t>(), st));
-    CK(cudaMemsetAsync(sl.ent.p, 0, sizeof(uint32_t) * (size_t)(cnt + 3 * nseg + 4), st));
     CK(tile_format_fill(sl.ip.as<int64_t>(), sl.idx.as<int32_t>(), vals, rows, pl->n_chunks, sl.seg.as<int64_t>(),
                         sl.ent.as<uint32_t>(), sl.meta.p, st, pl->num_sms));
   } else if (pack == 2) {
@@ -801,7 +942,7 @@ void setup_streaming(scxpca_plan* pl, const scxpca_csr* x, size_t limit) {
   if (room <= 0.0 || (double)pl->shard_nnz_max * per_entry > room * 1.5)
     fail(SCXPCA_OUT_OF_MEMORY, "streamed GPU PCA: the device budget of " + std::to_string(limit >> 20) +
                                    " MB does not hold the resident buffers and two shard slots");
-  CK(cudaStreamCreateWithFlags(&pl->copy_stream, cudaStreamNonBlocking));
+  pl->copy_stream = take_stream(pl->device);
   for (int i = 0; i < 2; ++i) {
     CK(cudaEventCreateWithFlags(&pl->ev_copied[i], cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&pl->ev_free[i], cudaEventDisableTiming));
@@ -1004,10 +1145,8 @@ void alloc_work_buffers(scxpca_plan* pl) {
   pl->comps.alloc(sizeof(float) * pl->nc * g);
   pl->M_emb.alloc(sizeof(float) * ld * pl->nc);
   pl->status.alloc(sizeof(int) * 4);
-  std::vector<double> eye(ld * ld, 0.0);
-  for (int64_t i = 0; i < ld; ++i) eye[i * ld + i] = 1.0;
-  upload(pl->eye, eye, pl->stream);
-  CK(cudaStreamSynchronize(pl->stream));  // `eye` goes out of scope
+  pl->eye.alloc(sizeof(double) * ld * ld);
+  CK(launch_identity(pl->eye.as<double>(), (int)ld, pl->stream));
 }
 
 // The baseline of a PFlog plan: the working matrix's last column holds b.
@@ -1044,7 +1183,7 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
     if (p->stream) {
       pl->stream = static_cast<cudaStream_t>(p->stream);
     } else {
-      CK(cudaStreamCreateWithFlags(&pl->stream, cudaStreamNonBlocking));
+      pl->stream = take_stream(pl->device);
       pl->own_stream = true;
     }
     cudaStream_t st = pl->stream;
@@ -1059,22 +1198,24 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
                     (size_t)nnz * 4 + (size_t)n * ldp * 8 + (size_t)n * pl->nc * 4 + (size_t)n * 36 +
                     (size_t)g * ldp * 4 * 400;
       size_t fr = 0, tot = 0;
-      CK(cudaMemGetInfo(&fr, &tot));
-      {  // memory our pool holds but does not use is free for this plan
+      const double with_headroom = (double)need * 1.1;
+      const char* res_env = getenv("SCXPCA_RESIDENT");
+      const bool force_stream = res_env && res_env[0] == '0';
+      {  // memory our pool holds but does not use is free for this plan; where
+         // that is enough the device is not asked (80 us, milliseconds at times)
         uint64_t reserved = 0, used = 0;
         cudaMemPool_t pool = pool_for(pl->device).pool;
         CK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved));
         CK(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
-        if (reserved > used) fr += (size_t)(reserved - used);
+        const size_t slack = reserved > used ? (size_t)(reserved - used) : 0;
+        if (force_stream || with_headroom > (double)slack) CK(cudaMemGetInfo(&fr, &tot));
+        fr += slack;
       }
-      double with_headroom = (double)need * 1.1;
       // A host matrix that does not fit (the free memory, or the caller's
       // device budget) is streamed from host memory instead of held resident
       // (gpu_pca.rs:520-590); SCXPCA_RESIDENT=0 forces it.
       size_t limit = fr;
       if (p->device_budget > 0) limit = std::min(limit, (size_t)p->device_budget);
-      const char* res_env = getenv("SCXPCA_RESIDENT");
-      const bool force_stream = res_env && res_env[0] == '0';
       if (x->memory != SCXPCA_MEM_DEVICE && !aff && !pf && (force_stream || with_headroom > (double)limit)) {
         if (pl->k > kMaxK)
           fail(SCXPCA_UNSUPPORTED, "a sketch wider than " + std::to_string(kMaxK) +
@@ -1122,7 +1263,7 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
         const size_t vs = dtype_size(pl->in_dtype);
         pl->b_stage.alloc(vs * nnz);
         vin = pl->b_stage.p;
-        if (!pl->copy_stream) CK(cudaStreamCreateWithFlags(&pl->copy_stream, cudaStreamNonBlocking));
+        if (!pl->copy_stream) pl->copy_stream = take_stream(pl->device);
         cudaStream_t cs = pl->copy_stream;
         const int parts = pl->stats_parts;
         const int pieces = std::min(kUploadPieces, parts);
@@ -1151,16 +1292,28 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
     }
     phase_mark(SCXPCA_PHASE_UPLOAD, st);
 
-    // ---- validation ----
+    // ---- validation, and the statistics of the input behind it (their kernel
+    // checks every index it reads, so both come back in one wait) ----
+    std::vector<double> sx, sxx;
     {
       DevBuf flags;
       flags.alloc(16);
       CK(cudaMemsetAsync(flags.p, 0, 16, st));
       CK(launch_validate_csr(pl->in_dtype, pl->indptr, pl->idx, vin, n, g, nnz, flags.as<int32_t>(),
                              st, pl->num_sms));
+      phase_mark(SCXPCA_PHASE_VALIDATE, st);
+      if (stats_queued)
+        CK(launch_col_stats_reduce(pl->stats_part.as<double>(), pl->stats_parts, (int32_t)g,
+                                   pl->stats_out.as<double>(), st, pl->num_sms));
+      else
+        CK(launch_col_stats(pl->in_dtype, pl->idx, vin, nnz, (int32_t)g, pl->stats_part.as<double>(),
+                            pl->stats_parts, pl->stats_out.as<double>(), st, pl->num_sms));
+      StatsFetch stats(pl);
+      stats.h.fetch(sizeof(double) * 2 * g, flags.p, 16);
+      stats.h.wait();
+      stats.take(sx, sxx);
       int32_t hf[4];
-      CK(cudaMemcpyAsync(hf, flags.p, 16, cudaMemcpyDeviceToHost, st));
-      CK(cudaStreamSynchronize(st));
+      memcpy(hf, stats.h.at<int32_t>(sizeof(double) * 2 * g), 16);
       if (hf[0]) fail(SCXPCA_INVALID_CSR, "invalid CSR: indptr is not monotone within [0, nnz]");
       if (hf[1]) fail(SCXPCA_INVALID_CSR, "invalid CSR: column index out of range [0, n_vars)");
       if (hf[3]) fail(SCXPCA_INVALID_CSR, "invalid CSR: non-finite value");
@@ -1195,14 +1348,7 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
       pl->fmt16 = pl->dtype == SCXPCA_BF16 ? 1 : 0;
     }
     const int64_t ld = pl->ld;
-    phase_mark(SCXPCA_PHASE_VALIDATE, st);
-
-    // ---- statistics of the input ----
-    std::vector<double> sx, sxx;
-    if (stats_queued && !pl->rows_resorted)
-      stats_finish(pl, sx, sxx);
-    else
-      stats_pass(pl, vin, pl->in_dtype, sx, sxx);
+    if (pl->rows_resorted) stats_pass(pl, vin, pl->in_dtype, sx, sxx);  // in the order of the sorted rows
     pl->mean_x.resize(g);
     for (int64_t j = 0; j < g; ++j) pl->mean_x[j] = sx[j] / (double)n;
     phase_mark(SCXPCA_PHASE_STATS, st);
@@ -1332,11 +1478,8 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
       seg.alloc(sizeof(int64_t) * (nseg + 1));
       CK(tile_format_count(pl->indptr, pl->idx, n, pl->n_chunks, counts.as<int64_t>(), st, pl->num_sms));
       CK(launch_exclusive_scan_i64(counts.as<int64_t>(), nseg, seg.as<int64_t>(), st));
-      int64_t padded_nnz = 0;
-      CK(cudaMemcpyAsync(&padded_nnz, seg.as<int64_t>() + nseg, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
-      CK(cudaStreamSynchronize(st));
-      pl->tf_ent.alloc(sizeof(uint32_t) * std::max<int64_t>(padded_nnz, 4));
-      CK(cudaMemsetAsync(pl->tf_ent.p, 0, sizeof(uint32_t) * std::max<int64_t>(padded_nnz, 4), st));
+      // every segment is padded to four entries: at most three more each
+      pl->tf_ent.alloc(sizeof(uint32_t) * (size_t)(nnz + 3 * nseg + 4));
       pl->tf_meta.alloc(tile_meta_bytes(n, pl->n_chunks));
       CK(tile_format_fill(pl->indptr, pl->idx, pl->val, n, pl->n_chunks, seg.as<int64_t>(),
                           pl->tf_ent.as<uint32_t>(), pl->tf_meta.p, st, pl->num_sms));
@@ -1371,8 +1514,6 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
     alloc_work_buffers(pl);
     phase_mark(SCXPCA_PHASE_BUFFERS, st);
     CK(cudaStreamSynchronize(st));
-    size_t fr = 0, tot = 0;
-    CK(cudaMemGetInfo(&fr, &tot));
     pl->device_bytes = pl->b_indptr.bytes + pl->b_idx.bytes + pl->b_val.bytes + pl->stats_part.bytes +
                        pl->rbp.bytes + pl->wpart.bytes + pl->Y.bytes + pl->gpart.bytes +
                        pl->W.bytes + pl->Z.bytes + pl->V.bytes + pl->csc_tptr.bytes + pl->csc_row.bytes +
@@ -1381,9 +1522,10 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
   } catch (...) {
     // the buffers are freed in the stream's order: delete the plan first
     const bool own = pl->own_stream;
+    const int dev = pl->device;
     cudaStream_t st = pl->stream;
     delete pl;
-    if (own && st) cudaStreamDestroy(st);
+    if (own) give_stream(dev, st);
     throw;
   }
 }
@@ -1594,15 +1736,19 @@ void forward(scxpca_plan* pl, bool f32 = true, bool split_v = true) {
 }
 
 // Raise the error a tensor-core kernel recorded (a bounded wait that ran out).
+void raise_tc_error(scxpca_plan* pl, int e) {
+  if (e != 0) {
+    CK(cudaMemsetAsync(pl->tc_err.p, 0, sizeof(int), pl->stream));
+    fail(SCXPCA_TIMEOUT, "tensor-core pipeline wait timed out (site " + std::to_string(e) + ")");
+  }
+}
+
 void check_tc_error(scxpca_plan* pl) {
   if (!pl->use_tc) return;
   int e = 0;
   CK(cudaMemcpyAsync(&e, pl->tc_err.p, sizeof(int), cudaMemcpyDeviceToHost, pl->stream));
   CK(cudaStreamSynchronize(pl->stream));
-  if (e != 0) {
-    CK(cudaMemsetAsync(pl->tc_err.p, 0, sizeof(int), pl->stream));
-    fail(SCXPCA_TIMEOUT, "tensor-core pipeline wait timed out (site " + std::to_string(e) + ")");
-  }
+  raise_tc_error(pl, e);
 }
 
 // V = Omega (seeded, or the caller's), zero-padded to g x ld; V's mean
@@ -1928,18 +2074,28 @@ void run_plan(scxpca_plan* pl, const scxpca_params* over, scxpca_result* out) {
   if (host_out)
     CK(cudaMemcpyAsync(out->embeddings, U, sizeof(float) * pl->n * pl->nc, cudaMemcpyDeviceToHost, st));
 
-  int hstatus[4];
-  std::vector<double> sigma(pl->k);
-  CK(cudaMemcpyAsync(hstatus, pl->status.p, sizeof(int) * 4, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(sigma.data(), pl->sigma.p, sizeof(double) * pl->k, cudaMemcpyDeviceToHost, st));
-  if (out->components)  // the first g_user loadings of every component row
-    CK(cudaMemcpy2DAsync(out->components, sizeof(float) * pl->g_user, pl->comps.p, sizeof(float) * pl->g,
-                         sizeof(float) * pl->g_user, pl->nc, cudaMemcpyDeviceToHost, st));
+  // status, error flag, sigma and (unless they are large) the first g_user
+  // loadings of every component row come back through one page-locked buffer
+  const size_t comp_bytes = out->components ? sizeof(float) * (size_t)pl->nc * pl->g_user : 0;
+  const bool staged = comp_bytes <= kStageMost;
+  const size_t at_err = 16, at_sigma = 64, at_comps = (at_sigma + sizeof(double) * pl->k + 63) / 64 * 64;
+  Staging h(at_comps + (staged ? comp_bytes : 0), st);
+  h.fetch(0, pl->status.p, sizeof(int) * 4);
+  if (pl->use_tc) h.fetch(at_err, pl->tc_err.p, sizeof(int));
+  h.fetch(at_sigma, pl->sigma.p, sizeof(double) * pl->k);
+  if (comp_bytes) {
+    if (staged && pl->g_user == pl->g)
+      h.fetch(at_comps, pl->comps.p, comp_bytes);
+    else
+      CK(cudaMemcpy2DAsync(staged ? h.p + at_comps : (char*)out->components, sizeof(float) * pl->g_user, pl->comps.p,
+                           sizeof(float) * pl->g, sizeof(float) * pl->g_user, pl->nc, cudaMemcpyDeviceToHost, st));
+  }
   phase_mark(SCXPCA_PHASE_DOWNLOAD, st);
-  CK(cudaStreamSynchronize(st));
+  h.wait();
   collect_stages(pl);
-  check_tc_error(pl);
-  finish_result(pl, hstatus, sigma.data(), out);
+  if (pl->use_tc) raise_tc_error(pl, *h.at<int>(at_err));
+  finish_result(pl, h.at<int>(0), h.at<double>(at_sigma), out);
+  if (comp_bytes && staged) memcpy(out->components, h.p + at_comps, comp_bytes);
 }
 
 // ---------------------------------------------------------------------------
@@ -2620,7 +2776,7 @@ void batch_collect(scxpca_batch* b, float* components, double* singular_values, 
       if (variance_explained) variance_explained[q * b->nc + c] = ve[c];
     }
   }
-  if (components) memcpy(components, b->h_comps, sizeof(float) * (size_t)ns * b->nc * b->n_vars);
+  if (components) host_copy(components, b->h_comps, sizeof(float) * (size_t)ns * b->nc * b->n_vars);
 }
 
 // Plain reference execution: one synchronising plan run per segment.
@@ -2925,10 +3081,14 @@ void scxpca_plan_destroy(scxpca_plan* plan) {
   cudaGetDevice(&prev);
   cudaSetDevice(plan->device);
   cudaStreamSynchronize(plan->stream);
-  bool own = plan->own_stream;
+  const bool own = plan->own_stream;
+  const int dev = plan->device;
   cudaStream_t st = plan->stream;
-  delete plan;
-  if (own) cudaStreamDestroy(st);
+  {
+    IdleStreamScope idle(st);
+    delete plan;
+  }
+  if (own) give_stream(dev, st);
   if (prev >= 0) cudaSetDevice(prev);
 }
 
