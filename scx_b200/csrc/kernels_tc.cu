@@ -39,10 +39,21 @@
 // thread; warp 21 loads the dense operand by TMA; warp 22 copies segment
 // metadata per tile (or band of two tiles) and prefetches their entries into
 // L2.  Each densify warp reads its quarter of a segment straight from global
-// memory with 16-byte loads, keeping the loads of its group's next segment
-// in flight in registers while the current one is scattered, so many warps
-// -- not one issuing thread -- keep the entry stream moving.  All waits are
-// bounded (tc.cuh).
+// memory, keeping the loads of its group's next segments in flight in
+// registers while the current one is scattered, so many warps -- not one
+// issuing thread -- keep the entry stream moving.  All waits are bounded
+// (tc.cuh).
+//
+// What bounds the ld-64 pair: the stage, 256 cells x 64 genes of the forward
+// kernel, takes about 930 cycles at 9 % stored (1,000,000 x 2,000: 450 us
+// forward, 410 us transposed), of which the MMAs need 512 of the tensor pipe
+// and zeroing, scattering and operand reads about 75 % of the shared-memory
+// pipe; left out of the kernel by themselves, MMAs are worth 80 us, bank
+// conflicts of the scatter 35 and the latency of the entry loads 40.  Before
+// loads ran two stages ahead, a wait cost a vote instead of a shuffle, the
+// image shared the stage's barriers and the epilogue went in passes, the two
+// took 585 and 527 us.  Zeroing the tiles by TMA (boxes outside the tensor)
+// takes the stores away but lengthens the chain of a stage: 494 us forward.
 #include <algorithm>
 
 #include "common.cuh"
@@ -274,6 +285,25 @@ __device__ __forceinline__ uint32_t hilo16(float x, int fmt) {
   return h | (l << 16);
 }
 
+// hilo16 of 16 values, two at a time, with one branch on the format.
+template <bool BF>
+__device__ __forceinline__ void hilo16_block_as(const float (&v)[16], uint32_t (&w)[16]) {
+#pragma unroll
+  for (int i = 0; i < 16; i += 2) {
+    const uint32_t h = pack16x2(v[i], v[i + 1], BF);
+    const uint32_t l =
+        pack16x2(v[i] - unpack16(h & 0xFFFFu, BF), v[i + 1] - unpack16(h >> 16, BF), BF);
+    w[i] = __byte_perm(h, l, 0x5410);
+    w[i + 1] = __byte_perm(h, l, 0x7632);
+  }
+}
+__device__ __forceinline__ void hilo16_block(const float (&v)[16], uint32_t (&w)[16], int fmt) {
+  if (fmt)
+    hilo16_block_as<true>(v, w);
+  else
+    hilo16_block_as<false>(v, w);
+}
+
 // Zero rows 32q .. 32q+31 of a 128 x 64 16-bit swizzled tile, lane = row.
 // Iteration i writes physical chunk i ^ (row % 8): the 32 lanes of one store
 // cover all eight 16-byte bank groups, so every store is conflict-free.
@@ -341,6 +371,47 @@ __device__ __forceinline__ void span_scatter(uint32_t tile, const uint32_t* __re
 #pragma unroll
   for (int r = 0; r < R; ++r) scatter4(tile, w[r], 4 * (lane + 32 * r) - plo, n);
   for (int p = 4 * (lane + 32 * R); p < phi; p += 128) scatter4(tile, ldg_entries(ent + a0 + p), p - plo, n);
+}
+
+// The words of a densify warp's next segment quarter for one of its two stage
+// buffers (ld-64 kernels), in flight: word r of a lane is entry lane + 32 r, so
+// that one store instruction takes 32 neighbouring entries, five or six rows
+// of genes that differ within a row: fewer bank conflicts, and fewer
+// instructions, than 16-byte loads give, whose k-th words lie 4 apart
+// (1,000,000 x 2,000 at 9 %: forward 466 -> 451 us, transposed 450 -> 414).
+template <int R>
+struct DenseSlot {
+  uint32_t w[R];
+  const uint32_t* base;
+  int n;  // entries; < 0: no tile here
+};
+
+// The first R blocks of 32 entries, straight into the slot's registers: a lane
+// without one keeps what it had (the scatter does not look at it), so no
+// select sits between the load and its use two stages later.
+template <int R>
+__device__ __forceinline__ void slot_load(DenseSlot<R>& x, const uint32_t* __restrict__ ent, Span sp, int lane) {
+  x.base = ent + sp.lo;
+  x.n = (int)(sp.hi - sp.lo);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int p = lane + 32 * r;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.lt.s32 p, %2, %3;\n\t"
+        "@p ld.global.nc.u32 %0, [%1];\n\t}"
+        : "+r"(x.w[r])
+        : "l"(x.base + p), "r"(p), "r"(x.n));
+  }
+}
+
+// Scatter the slot's quarter into its rows of `tile`, which hold zeros.
+template <int R>
+__device__ __forceinline__ void slot_scatter(const DenseSlot<R>& x, uint32_t tile, int lane) {
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    if (lane + 32 * r < x.n) scatter_one(tile, x.w[r]);
+  for (int p = lane + 32 * R; p < x.n; p += 32) scatter_one(tile, __ldg(x.base + p));
 }
 
 // Meta loader: L2 prefetch of the entries of segments [c0, c1) of one tile
@@ -1153,11 +1224,11 @@ __global__ void k_split16_batch(const SplitTask* __restrict__ tasks, int64_t cou
 // 2 j + 1 hold the two halves of one output column and a lane shuffle adds
 // them.
 // ---------------------------------------------------------------------------
-constexpr int kSwapFwdStages = 4;  // pair stages: the two tiles of a band, one chunk
-constexpr int kSwapFwdSlots = 5;   // dense-operand ring (16 KB image chunks)
+constexpr int kSwapFwdStages = 4;  // one chunk: the two tiles of a band and the chunk of the image
+constexpr int kSwapRegs = 8;       // entries a densify lane has in flight per stage (x 32 a warp)
 
 __host__ __device__ constexpr size_t fwd_swap_smem() {
-  return 1024 + (size_t)kSwapFwdStages * 2 * (TM * CW * 2) + (size_t)kSwapFwdSlots * (CW * 128 * 2) +
+  return 1024 + (size_t)kSwapFwdStages * (2 * (TM * CW * 2) + CW * 128 * 2) +
          2 * 2 * (size_t)kMaxChunks * sizeof(SegMeta) + 64 * sizeof(uint64_t) + 64;
 }
 
@@ -1210,13 +1281,14 @@ struct FwdBatch {
   }
 };
 
-// A band is two consecutive row tiles.  Per band:
+// The image chunk of a stage lands on the stage's own barriers: the MMA thread
+// waits once and commits once a chunk (a ring of its own cost it about 200 of
+// 1,200 cycles).  A band is two consecutive row tiles.  Per band:
 // Y^T[m, its 256 cells] = sum over chunks c of Vimg_c^T (m x 64 genes) [A_(t0,c) | A_(t1,c)]^T.
 template <class Src>
 __device__ __forceinline__ void fwd_swap_body(const Src& src, int nc, int fmt) {
   constexpr int LD = 64;
   constexpr int S = kSwapFwdStages;
-  constexpr int NB = kSwapFwdSlots;
   constexpr int TILE = TM * CW * 2;      // one 128 x 64 tile, 16 KB
   constexpr int STAGE = 2 * TILE;        // the band's two tiles, 256 cell rows
   constexpr int B_BYTES = CW * 128 * 2;  // 64 genes x 128 image columns
@@ -1226,13 +1298,11 @@ __device__ __forceinline__ void fwd_swap_body(const Src& src, int nc, int fmt) {
   uint8_t* smem = align1024(smem_raw);
   uint8_t* As = smem;
   uint8_t* Bs = As + S * STAGE;
-  SegMeta* mring = reinterpret_cast<SegMeta*>(Bs + NB * B_BYTES);  // [2][2 * kMaxChunks]
+  SegMeta* mring = reinterpret_cast<SegMeta*>(Bs + S * B_BYTES);  // [2][2 * kMaxChunks]
   uint64_t* bars = reinterpret_cast<uint64_t*>(mring + 2 * MSLOT);
-  uint64_t* full = bars;            // [S]  stage densified (two groups x 4 warps)
-  uint64_t* empty = full + S;       // [S]  stage consumed (MMA commit)
-  uint64_t* bfull = empty + S;      // [NB] image chunk landed (TMA)
-  uint64_t* bempty = bfull + NB;    // [NB] image chunk consumed (MMA commit)
-  uint64_t* acc_full = bempty + NB;
+  uint64_t* full = bars;       // [S] stage densified (two groups x 4 warps) and its image chunk landed (TMA)
+  uint64_t* empty = full + S;  // [S] stage consumed (MMA commit)
+  uint64_t* acc_full = empty + S;
   uint64_t* acc_empty = acc_full + 2;
   uint64_t* mfull = acc_empty + 2;
   uint64_t* mempty = mfull + 2;
@@ -1243,12 +1313,8 @@ __device__ __forceinline__ void fwd_swap_body(const Src& src, int nc, int fmt) {
   const int64_t n_bands = src.bands();
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(&full[s], 8);
+      mbar_init(&full[s], 9);
       mbar_init(&empty[s], 1);
-    }
-    for (int b = 0; b < NB; ++b) {
-      mbar_init(&bfull[b], 1);
-      mbar_init(&bempty[b], 1);
     }
     for (int a = 0; a < 2; ++a) {
       mbar_init(&acc_full[a], 1);
@@ -1269,57 +1335,75 @@ __device__ __forceinline__ void fwd_swap_body(const Src& src, int nc, int fmt) {
   const uint32_t tmem = *tmem_slot;
 
   if (warp < W_EPI) {
-    // ---- densify: group (cc & 1, u) fills tile u of the stage of chunk
-    // counter cc; a band with one tile leaves its u = 1 groups idle, but they
-    // still take part in the stage handshake ----
+    // ---- densify: group (par, u) fills tile u of the stages of the chunk
+    // counters with that parity, which are the stages par and par + 2 in
+    // turn; a band with one tile leaves its u = 1 groups idle, but they still
+    // take part in the stage handshake.  The words of a segment are loaded as
+    // soon as the buffer's last one is scattered, two stages ahead ----
     const int group = warp >> 2, q = warp & 3;
     const int par = group >> 1, u = group & 1;
-    uint32_t cc = 0, bi = 0;
-    uint4 w[kFwdRegs];
-    Span pre{-1, -1};             // span whose loads are in flight in w
-    const uint32_t* pre_ent = nullptr;  // the entry array pre indexes
-    for (int64_t band = blockIdx.x; band < n_bands; band += gridDim.x, ++bi) {
+    const uint32_t tile0 = smem_u32(As + par * STAGE + u * TILE);
+    DenseSlot<kSwapRegs> sl[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+#pragma unroll
+      for (int r = 0; r < kSwapRegs; ++r) sl[k].w[r] = 0u;
+    }
+    // cursor: the next segment to load
+    int64_t band = blockIdx.x;
+    uint32_t bi = 0;
+    int c = par;
+    bool has = false, live = true;
+    const uint32_t* ent = nullptr;
+    int* err = nullptr;
+    auto enter = [&]() {
       const FwdBand bd = src.band(band);
-      int* err = bd.err;
-      const bool has = u < bd.tiles;
-      if (!warp_wait(&mfull[bi & 1u], (bi >> 1) & 1u, abort_flag, err, 11)) goto done;
-      const SegMeta* mt = mring + (bi & 1u) * MSLOT;
-      for (int c = 0; c < nc; ++c, ++cc) {
-        if ((int)(cc & 1u) != par) continue;
-        // the span loaded ahead (pre) is this segment's whenever one was loaded
-        const Span sp = !has ? Span{0, 0} : pre.lo >= 0 ? pre : quarter_span(mt[u * nc + c], q);
-        const uint32_t* sp_ent = pre.lo >= 0 ? pre_ent : bd.ent;
-        if (has && pre.lo < 0) span_load<kFwdRegs>(sp_ent, sp, lane, w);
-        const int s = cc % S;
-        if (!warp_wait(&empty[s], ((cc / S) & 1u) ^ 1u, abort_flag, err, 12)) goto done;
-        if (has) {
-          const uint32_t tile = smem_u32(As + s * STAGE + u * TILE);
+      ent = bd.ent;
+      err = bd.err;
+      has = u < bd.tiles;
+      return warp_wait(&mfull[bi & 1u], (bi >> 1) & 1u, abort_flag, err, 11);
+    };
+    auto fetch = [&](DenseSlot<kSwapRegs>& x) {
+      while (c >= nc) {  // leave the band
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&mempty[bi & 1u]);
+        c -= nc;
+        band += gridDim.x;
+        ++bi;
+        if (band >= n_bands) {
+          live = false;
+          c = -1;
+          return true;
+        }
+        if (!enter()) return false;
+      }
+      x.n = -1;
+      if (has) slot_load(x, ent, quarter_span(mring[(bi & 1u) * MSLOT + u * nc + c], q), lane);
+      c += 2;
+      return true;
+    };
+    if (band >= n_bands || !enter() || !fetch(sl[0])) goto done;
+    bool more0 = live, more1;
+    if (live && !fetch(sl[1])) goto done;
+    more1 = live;
+    for (uint32_t i = 0; more0; ++i) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        if (k == 1 && !more1) break;
+        const int s = par + 2 * k;
+        if (!warp_wait(&empty[s], (i & 1u) ^ 1u, abort_flag, err, 12)) goto done;
+        if (sl[k].n >= 0) {
+          const uint32_t tile = tile0 + 2 * k * STAGE;
           zero_rows(tile, q, lane);
           __syncwarp();
-          span_scatter<kFwdRegs>(tile, sp_ent, sp, lane, w);
+          slot_scatter(sl[k], tile, lane);
         }
-        // the group's next segment: chunk c + 2 of this band, or of the next
-        pre = Span{-1, -1};
-        if (c + 2 < nc) {
-          if (has) {
-            pre = quarter_span(mt[u * nc + c + 2], q);
-            pre_ent = bd.ent;
-          }
-        } else if (band + gridDim.x < n_bands && c + 2 - nc < nc) {
-          const FwdBand nx = src.band(band + gridDim.x);
-          if (u < nx.tiles) {
-            if (!warp_wait(&mfull[(bi + 1) & 1u], ((bi + 1) >> 1) & 1u, abort_flag, err, 11)) goto done;
-            pre = quarter_span(mring[((bi + 1) & 1u) * MSLOT + u * nc + (c + 2 - nc)], q);
-            pre_ent = nx.ent;
-          }
-        }
-        if (pre.lo >= 0) span_load<kFwdRegs>(pre_ent, pre, lane, w);
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) mbar_arrive(&full[s]);
+        if (live && !fetch(sl[k])) goto done;
+        (k ? more1 : more0) = live;
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&mempty[bi & 1u]);
     }
   } else if (warp < W_MMA) {
     // ---- epilogue: lane pair (2 j, 2 j + 1) -> column j of Y and its image ----
@@ -1346,20 +1430,30 @@ __device__ __forceinline__ void fwd_swap_body(const Src& src, int nc, int fmt) {
           tmem_wait_ld();
           const int64_t c0 = row0 + cb * 32;
           const int lim = (int)min((int64_t)32, n - c0);  // cells of this block inside the matrix
-          // word j of an image row holds (hi, lo) of column j; lane p handles cell i + p
-          uint32_t* dst = reinterpret_cast<uint32_t*>(Yimg) + c0 * 64 + 16 * q + (lane >> 1);
-          float* ydst = Y ? Y + c0 * LD + j : nullptr;
+          // word j of an image row holds (hi, lo) of column j; lane p handles
+          // cells 2 i + p.  Each lane gives the other the halves it does not
+          // need, one exchange for two cells, and the exchanges, conversions
+          // and stores of the block go in passes of their own: sixteen
+          // independent chains, where cell after cell would stall on each.
+          float v[16];
 #pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            // each lane gives the other the half it does not need (one exchange
-            // for two cells)
-            const float x0 = __uint_as_float(r[i]), x1 = __uint_as_float(r[i + 1]);
+          for (int i = 0; i < 16; ++i) {
+            const float x0 = __uint_as_float(r[2 * i]), x1 = __uint_as_float(r[2 * i + 1]);
             const float other = __shfl_xor_sync(0xffffffffu, p ? x0 : x1, 1);
-            const float sm = (p ? x1 : x0) + other - mcj;
-            if (i + p < lim) {
-              dst[(i + p) * 64] = hilo16(sm, fmt);
-              if (ydst) ydst[(i + p) * LD] = sm;
-            }
+            v[i] = (p ? x1 : x0) + other - mcj;
+          }
+          const int left = lim - p;  // cell 2 i + p is inside the matrix iff 2 i < left
+          uint32_t* dst = reinterpret_cast<uint32_t*>(Yimg) + (c0 + p) * 64 + j;
+          uint32_t img[16];
+          hilo16_block(v, img, fmt);
+#pragma unroll
+          for (int i = 0; i < 16; ++i)
+            if (2 * i < left) dst[i * 128] = img[i];
+          if (Y) {
+            float* ydst = Y + (c0 + p) * LD + j;
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+              if (2 * i < left) ydst[i * 2 * LD] = v[i];
           }
         }
       }
@@ -1385,28 +1479,26 @@ __device__ __forceinline__ void fwd_swap_body(const Src& src, int nc, int fmt) {
         tc_fence_after();
         const uint32_t d = tmem + a * 256;
         for (int c = 0; c < nc; ++c, ++cc) {
-          const int b = cc % NB, s = cc % S;
-          if (!mbar_wait(&bfull[b], (cc / NB) & 1u, abort_flag, err, 16) ||
-              !mbar_wait(&full[s], (cc / S) & 1u, abort_flag, err, 16)) {
+          const int s = cc % S;
+          if (!mbar_wait(&full[s], (cc / S) & 1u, abort_flag, err, 16)) {
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint64_t vd = vdesc0 + (uint64_t)(b * (B_BYTES >> 4));
+          const uint64_t vd = vdesc0 + (uint64_t)(s * (B_BYTES >> 4));
           const uint64_t td = tdesc0 + (uint64_t)(s * (STAGE >> 4));
           umma_f16(d, vd, td, idesc, c != 0);
 #pragma unroll
           for (int kk = 1; kk < CW / 16; ++kk)  // K steps of 16 genes: +2 KB down the image, +32 B along the tiles
             umma_f16(d, vd + 128 * kk, td + 2 * kk, idesc, 1u);
           umma_commit(&empty[s]);
-          umma_commit(&bempty[b]);
         }
         if (ok) umma_commit(&acc_full[a]);
       }
     }
     __syncwarp();
   } else if (warp == W_DENSE) {
-    // ---- dense loader: image chunks into the ring, up to NB ahead ----
+    // ---- dense loader: the image chunk of each stage ----
     if (lane == 0) {
       uint32_t cc = 0;
       bool ok = true;
@@ -1415,15 +1507,15 @@ __device__ __forceinline__ void fwd_swap_body(const Src& src, int nc, int fmt) {
         int* err = bd.err;
         if (Src::kGlobalMaps) tmap_acquire(bd.vmap);
         for (int c = 0; c < nc; ++c, ++cc) {
-          const int b = cc % NB;
-          if (!mbar_wait(&bempty[b], ((cc / NB) & 1u) ^ 1u, abort_flag, err, 19)) {
+          const int s = cc % S;
+          if (!mbar_wait(&empty[s], ((cc / S) & 1u) ^ 1u, abort_flag, err, 19)) {
             ok = false;
             break;
           }
-          uint8_t* bb = Bs + b * B_BYTES;
-          mbar_arrive_expect_tx(&bfull[b], B_BYTES);
-          tma_load_2d(bb, bd.vmap, &bfull[b], 0, CW * c);
-          tma_load_2d(bb + CW * 128, bd.vmap, &bfull[b], 64, CW * c);
+          uint8_t* bb = Bs + s * B_BYTES;
+          mbar_arrive_expect_tx(&full[s], B_BYTES);
+          tma_load_2d(bb, bd.vmap, &full[s], 0, CW * c);
+          tma_load_2d(bb + CW * 128, bd.vmap, &full[s], 64, CW * c);
         }
       }
     }
@@ -1554,65 +1646,65 @@ __device__ __forceinline__ void rmat_swap_body(const RmatJob& job, int nc, int64
 
   if (warp < W_EPI) {
     // ---- densify: team h (warps 8 h .. 8 h + 7) fills the half-tile stages
-    // of cells 64 h .. 64 h + 63; warp (c, r) of a team takes chunk 4 qd + c,
-    // quarter 2 h + r of the tile ----
+    // of cells 64 h .. 64 h + 63, stages h and h + 2 in turn; warp (c, r) of a
+    // team takes chunk 4 qd + c, quarter 2 h + r of the tile.  Words are
+    // loaded two stages ahead, as in the forward kernel ----
     const int h = warp >> 3, cofs = (warp >> 1) & 3, q = 2 * h + (warp & 1);
+    // entry offsets address the whole 128-row tile: rows 64 h.. start 8 KB before the half
+    const uint32_t tile0 = smem_u32(As + h * STAGE + cofs * HSUB) - h * HSUB;
+    DenseSlot<kSwapRegs> sl[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+#pragma unroll
+      for (int r = 0; r < kSwapRegs; ++r) sl[k].w[r] = 0u;
+    }
+    // cursor: the next segment to load
+    int jq = 0;
     uint32_t ti = 0;
-    uint4 w[kRmatRegs];
-    Span pre{-1, -1};     // span whose loads are in flight in w
-    bool zeroed = false;  // this warp's rows of its next stage were zeroed ahead
-    if (have_work)
-      for (int64_t t = t0; t < t1; ++t, ++ti) {
-        if (!warp_wait(&mfull[ti & 1u], (ti >> 1) & 1u, abort_flag, err, 21)) goto done;
-        const SegMeta* mt = mring + (ti & 1u) * kMaxChunks;
-        for (int jq = 0; jq < nq; ++jq) {
-          const uint32_t it = (ti * (uint32_t)nq + jq) * 2u + h;  // this stage in the MMA's order
-          const int ch = 4 * (qd0 + jq) + cofs;
-          const bool has = ch < nc;
-          // the span loaded ahead (pre) is this segment's whenever one was loaded
-          const Span sp = !has ? Span{0, 0} : pre.lo >= 0 ? pre : quarter_span(mt[ch], q);
-          if (has && pre.lo < 0) span_load<kRmatRegs>(ent, sp, lane, w);
-          const int s = it % S;
-          if (!warp_wait(&empty[s], ((it / S) & 1u) ^ 1u, abort_flag, err, 22)) goto done;
-          if (has) {
-            // entry offsets address the whole 128-row tile: rows 64 h.. start 8 KB before the half
-            const uint32_t tile = smem_u32(As + s * STAGE + cofs * HSUB) - h * HSUB;
-            if (!zeroed) zero_rows(tile, q, lane);
+    const uint32_t ntl = have_work ? (uint32_t)(t1 - t0) : 0u;
+    bool live = true;
+    auto fetch = [&](DenseSlot<kSwapRegs>& x) {
+      if (jq == nq) {  // leave the tile
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&mempty[ti & 1u]);
+        jq = 0;
+        if (++ti == ntl) {
+          live = false;
+          return true;
+        }
+      }
+      if (jq == 0 && !warp_wait(&mfull[ti & 1u], (ti >> 1) & 1u, abort_flag, err, 21)) return false;
+      const int ch = 4 * (qd0 + jq) + cofs;
+      x.n = -1;
+      if (ch < nc) slot_load(x, ent, quarter_span(mring[(ti & 1u) * kMaxChunks + ch], q), lane);
+      ++jq;
+      return true;
+    };
+    if (have_work) {
+      if (!fetch(sl[0])) goto done;
+      bool more0 = live, more1;
+      if (!fetch(sl[1])) goto done;
+      more1 = live;
+      for (uint32_t i = 0; more0; ++i) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          if (k == 1 && !more1) break;
+          const int s = h + 2 * k;
+          if (!warp_wait(&empty[s], (i & 1u) ^ 1u, abort_flag, err, 22)) goto done;
+          if (sl[k].n >= 0) {
+            const uint32_t tile = tile0 + 2 * k * STAGE;
+            zero_rows(tile, q, lane);
             __syncwarp();
-            span_scatter<kRmatRegs>(tile, ent, sp, lane, w);
+            slot_scatter(sl[k], tile, lane);
           }
-          // the warp's next segment: the next quad of this tile, or the first of the next tile
-          pre = Span{-1, -1};
-          bool next = false;
-          if (jq + 1 < nq) {
-            next = ch + 4 < nc;
-            if (next) pre = quarter_span(mt[ch + 4], q);
-          } else if (t + 1 < t1 && 4 * qd0 + cofs < nc) {
-            next = true;
-            if (!warp_wait(&mfull[(ti + 1) & 1u], ((ti + 1) >> 1) & 1u, abort_flag, err, 21)) goto done;
-            pre = quarter_span(mring[((ti + 1) & 1u) * kMaxChunks + 4 * qd0 + cofs], q);
-          }
-          if (pre.lo >= 0) span_load<kRmatRegs>(ent, pre, lane, w);
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) mbar_arrive(&full[s]);
-          // Zero this warp's rows of its next stage now, so the stores drain
-          // while the next segment's metadata and entries are fetched and the
-          // warp barrier before the next scatter finds them done (measured:
-          // -9 % on this kernel; the forward kernel, whose stage holds two
-          // tiles of one chunk, gained nothing and zeroes in place).
-          zeroed = false;
-          if (next) {
-            const uint32_t itn = it + 2;  // this team's next stage
-            const int sn = itn % S;
-            if (!warp_wait(&empty[sn], ((itn / S) & 1u) ^ 1u, abort_flag, err, 22)) goto done;
-            zero_rows(smem_u32(As + sn * STAGE + cofs * HSUB) - h * HSUB, q, lane);
-            zeroed = true;
-          }
+          if (live && !fetch(sl[k])) goto done;
+          (k ? more1 : more0) = live;
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&mempty[ti & 1u]);
       }
+    }
   } else if (warp < W_MMA) {
     // ---- epilogue: lane pair (2 j, 2 j + 1) -> column j of the partial ----
     const int q = warp & 3;

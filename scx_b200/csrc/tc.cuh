@@ -96,14 +96,16 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
-// Warp-uniform bounded wait: lane 0 waits, the result is broadcast, so every
-// lane of the warp leaves (or continues) together.
+// Warp-uniform bounded wait.  Every lane tries once, and a vote (which, unlike
+// a shuffle, does not queue behind the warp's shared-memory accesses: 8 % of
+// k_rmat_swap) settles the common case; otherwise lane 0 waits and all lanes
+// leave (or continue) together.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           int* err, int code) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   int ok = 1;
   if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, abort_flag, err, code) ? 1 : 0;
-  ok = __shfl_sync(0xffffffffu, ok, 0);
-  return ok != 0;
+  return __all_sync(0xffffffffu, ok) != 0;
 }
 
 // ---------------------------------------------------------------------------

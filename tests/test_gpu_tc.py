@@ -140,3 +140,48 @@ def test_tensor_core_embeddings_match_cuda_core_product(monkeypatch, n, nc, over
     err = np.linalg.norm(tc.embeddings - cc.embeddings) / np.linalg.norm(cc.embeddings)
     assert err < 2e-4, err
     assert np.abs(tc.embeddings - cc.embeddings).max() < 2e-3 * np.abs(cc.embeddings).max()
+
+
+@pytest.mark.parametrize("n,g,mode", [
+    (300, 64, "mixed_bf16"),       # one chunk, a last band of one ragged tile
+    (80000, 60, "mixed_f16"),      # one chunk, several bands per SM
+    (80111, 130, "mixed_bf16"),    # three chunks: the chunk counter's parity alternates from band to band
+    (20000, 1100, "mixed_bf16"),   # five quads of chunks, three gene groups
+])
+def test_tc_quarters_of_every_size(n, g, mode):
+    """32 x 64 blocks that hold no entry, fewer and more than a warp's store
+    takes (32) and than a lane keeps in flight (256 a warp), and all 2,048,
+    next to one another in every order; the tolerance is the module's."""
+    import torch
+
+    rng = np.random.default_rng(n + g)
+    sizes = np.array([0, 1, 31, 32, 33, 180, 255, 256, 257, 700, 2048])
+    nb, nc = (n + 31) // 32, (g + 63) // 64
+    fill = rng.choice(sizes, size=(nb, nc), p=[.2, .1, .1, .1, .1, .1, .08, .08, .08, .04, .02])
+    rows, cols = [], []
+    for b in range(nb):
+        h = min(32, n - 32 * b)
+        for c in range(nc):
+            w = min(64, g - 64 * c)
+            at = rng.choice(h * w, size=min(int(fill[b, c]), h * w), replace=False)
+            rows.append(32 * b + at // w)
+            cols.append(64 * c + at % w)
+    rows, cols = np.concatenate(rows), np.concatenate(cols)
+    order = np.lexsort((cols, rows))
+    rows, cols = rows[order], cols[order].astype(np.int32)
+    indptr = np.r_[0, np.cumsum(np.bincount(rows, minlength=n))]
+    c = rpca.Csr(indptr, cols, rng.integers(1, 64, len(cols)).astype(np.float32) / 8, (n, g))  # exact in 16 bits
+    k = 20
+    plan = accel.Plan(c.indptr, c.indices, c.data, c.shape, n_components=k, n_oversamples=0, math_mode=mode)
+    assert plan.ld == 64
+    mu = rpca.col_sums_and_sum_sq(c)[0] / n
+    v = (rng.standard_normal((g, k)) / np.sqrt(g)).astype(np.float32)
+    q = (rng.standard_normal((n, k)) / np.sqrt(n)).astype(np.float32)
+    y_ref = rpca.spmm_forward(c, v.astype(np.float64), mu)
+    z_ref = rpca.spmm_transpose(c, q.astype(np.float64), mu)
+    for _ in range(2):
+        y = plan.matmat(torch.from_numpy(v).cuda()).cpu().numpy().astype(np.float64)
+        z = plan.rmatmat(torch.from_numpy(q).cuda()).cpu().numpy().astype(np.float64)
+        assert np.linalg.norm(y - y_ref) / np.linalg.norm(y_ref) < 1e-4
+        assert np.linalg.norm(z - z_ref) / np.linalg.norm(z_ref) < 1e-4
+    plan.close()
