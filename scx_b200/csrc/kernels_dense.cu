@@ -936,12 +936,16 @@ cudaError_t launch_apply_right_split(const float* In, int64_t n, int ld, const f
 
 // ---------------------------------------------------------------------------
 // Gene-side FP64 ops: Z = (W - mu s^T) M for a g x LD matrix W and an LD x LD
-// M (mu null: Z = W M; Z may be W).  A block of 256 threads stages M once and
-// then 64 rows of W at a time; thread (ty, tx) of the 16 x 16 grid owns rows
-// ty + 16 i (i < 4) and columns tx + 16 v (v < LD / 16) of the 64-row block,
-// so every shared value it reads feeds 4 or LD / 16 FMAs (one value per FMA
-// made the kernel shared-memory bound at 256 segments).  Each output is one
-// FMA chain over l = 0 .. LD-1 in order.
+// M (mu null: Z = W M; Z may be W), on the FP64 matrix instruction (8 x 8 x 4).
+// A block of eight warps stages M once and then RB rows of W at a time; row
+// strips and column ranges are dealt to the warps, and a warp keeps its tiles of
+// Z in registers over the whole of l.  Rows of both staged matrices are LD + 4
+// values apart, which puts the 4 x 8 values of one operand load into different
+// banks.  At 64 matrices of 2,000 x 64 the FP64 pipe's floor is 29 us and the
+// memory's 25; scalar FMAs, which read a shared value for every 1.6 of them,
+// took 70 us, this takes 60: the chain of a block (M in, rows in, products,
+// rows out) with three blocks an SM.  One matrix of 3,001 x 128: 24 -> 11 us,
+// of 2,000 x 64: 5.1 -> 3.6.
 // ---------------------------------------------------------------------------
 // Rows per block step: 16 for one matrix (125 blocks at 2,000 genes, a
 // latency-bound launch); 64 when a launch covers the segments of a batch
@@ -949,17 +953,21 @@ cudaError_t launch_apply_right_split(const float* In, int64_t n, int ld, const f
 constexpr int kApplyRows = 16, kApplyRowsBatch = 64;
 
 __host__ __device__ constexpr size_t center_apply_smem(int ld, int rb) {
-  return ((size_t)ld * ld + (size_t)rb * (ld + 1)) * sizeof(double);
+  return ((size_t)ld + rb) * (ld + 4) * sizeof(double);
 }
 
 // Block b of nb (of one matrix's grid) takes the row blocks b, b + nb, ...
-template <int LD, int kApplyRows>
+template <int LD, int RB>
 __device__ __forceinline__ void center_apply_body(const double* W, int64_t g, const double* mu, const double* s,
                                                   const double* M, double* Z, int b, int nb) {
-  constexpr int TT = LD / 16, RP = LD + 1;  // odd row stride: rows ty and ty + 1 sit in different banks
+  constexpr int ST = LD + 4;
+  constexpr int RS = RB / 16 == 1 ? 1 : 2;        // 8-row strips of a warp
+  constexpr int NS = RB / (8 * RS);               // warps along the rows: 2 or 4
+  constexpr int CT = LD / 8 / (8 / NS);           // 8-column tiles of a warp
+  static_assert(NS * RS * 8 == RB && CT * 8 * (8 / NS) == LD, "eight warps cover the block's rows and columns");
   extern __shared__ double sm[];
-  double* Ms = sm;             // [LD][LD]
-  double* rows = sm + LD * LD;  // [kApplyRows][LD + 1]
+  double* Ms = sm;               // [LD][ST]
+  double* rows = sm + LD * ST;   // [RB][ST]
   {
     // every load of M in flight before the first shared store: one L2 round
     // trip per block instead of one per element the thread stages
@@ -968,12 +976,16 @@ __device__ __forceinline__ void center_apply_body(const double* W, int64_t g, co
 #pragma unroll
     for (int u = 0; u < PT; ++u) mv[u] = M[threadIdx.x + 256 * u];
 #pragma unroll
-    for (int u = 0; u < PT; ++u) Ms[threadIdx.x + 256 * u] = mv[u];
+    for (int u = 0; u < PT; ++u) {
+      const int t = threadIdx.x + 256 * u;
+      Ms[t / LD * ST + t % LD] = mv[u];
+    }
   }
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  for (int64_t j0 = (int64_t)b * kApplyRows; j0 < g; j0 += (int64_t)nb * kApplyRows) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kr = lane & 3, m = lane >> 2;
+  const int r0 = warp % NS * (8 * RS), c0 = warp / NS * (8 * CT);
+  for (int64_t j0 = (int64_t)b * RB; j0 < g; j0 += (int64_t)nb * RB) {
     __syncthreads();  // M staged; the previous block's rows consumed
-    constexpr int RT = kApplyRows * LD / 256;  // row elements per thread
+    constexpr int RT = RB * LD / 256;  // row elements per thread
     double wv[RT];
 #pragma unroll
     for (int u = 0; u < RT; ++u) {
@@ -988,33 +1000,33 @@ __device__ __forceinline__ void center_apply_body(const double* W, int64_t g, co
       const int64_t j = j0 + r;
       double v = wv[u];
       if (j < g && mu) v -= mu[j] * s[c];
-      rows[r * RP + c] = v;
+      rows[r * ST + c] = v;
     }
     __syncthreads();
-    constexpr int RI = kApplyRows / 16;  // rows per thread
-    double acc[RI][TT];
+    double acc[RS][CT][2];
 #pragma unroll
-    for (int i = 0; i < RI; ++i)
+    for (int i = 0; i < RS; ++i)
 #pragma unroll
-      for (int v = 0; v < TT; ++v) acc[i][v] = 0.0;
+      for (int v = 0; v < CT; ++v) acc[i][v][0] = acc[i][v][1] = 0.0;
 #pragma unroll 4
-    for (int l = 0; l < LD; ++l) {
-      double a[RI], m[TT];
+    for (int l = 0; l < LD; l += 4) {
+      double a[RS], bm[CT];
 #pragma unroll
-      for (int i = 0; i < RI; ++i) a[i] = rows[(ty + 16 * i) * RP + l];
+      for (int i = 0; i < RS; ++i) a[i] = rows[(r0 + 8 * i + m) * ST + l + kr];
 #pragma unroll
-      for (int v = 0; v < TT; ++v) m[v] = Ms[l * LD + tx + 16 * v];
+      for (int v = 0; v < CT; ++v) bm[v] = Ms[(l + kr) * ST + c0 + 8 * v + m];
 #pragma unroll
-      for (int i = 0; i < RI; ++i)
+      for (int i = 0; i < RS; ++i)
 #pragma unroll
-        for (int v = 0; v < TT; ++v) acc[i][v] = fma(a[i], m[v], acc[i][v]);
+        for (int v = 0; v < CT; ++v) mma_f64(acc[i][v], a[i], bm[v]);
     }
 #pragma unroll
-    for (int i = 0; i < RI; ++i) {
-      const int64_t j = j0 + ty + 16 * i;
+    for (int i = 0; i < RS; ++i) {
+      const int64_t j = j0 + r0 + 8 * i + m;
       if (j < g)
 #pragma unroll
-        for (int v = 0; v < TT; ++v) Z[j * LD + tx + 16 * v] = acc[i][v];
+        for (int v = 0; v < CT; ++v)
+          *reinterpret_cast<double2*>(Z + j * LD + c0 + 8 * v + 2 * kr) = make_double2(acc[i][v][0], acc[i][v][1]);
     }
   }
 }
@@ -1028,7 +1040,7 @@ __global__ void __launch_bounds__(256) k_center_apply(const double* W, int64_t g
 
 // One matrix per grid row y (batched segments).
 template <int LD>
-__global__ void __launch_bounds__(256) k_center_apply_batch(const ApplyTask* __restrict__ tasks, int64_t g) {
+__global__ void __launch_bounds__(256, LD <= 64 ? 3 : 1) k_center_apply_batch(const ApplyTask* __restrict__ tasks, int64_t g) {
   const ApplyTask t = tasks[blockIdx.y];
   center_apply_body<LD, kApplyRowsBatch>(t.W, g, t.mu, t.s, t.M, t.Z, blockIdx.x, gridDim.x);
 }
@@ -1041,7 +1053,8 @@ static cudaError_t center_apply_t(const ApplyTask* tasks, int ntasks, const doub
   if (tasks) {
     const size_t smem = center_apply_smem(LD, kApplyRowsBatch);
     if (cudaError_t e = allow_smem(k_center_apply_batch<LD>, smem); e != cudaSuccess) return e;
-    // up to 16 blocks per matrix (two 64-row steps each at 2,000 genes), M staged once per block
+    // up to 16 blocks per matrix (two 64-row steps each at 2,000 genes), M
+    // staged once per block; one wave of longer blocks took 67 us against 60
     const int64_t blocks = (g + kApplyRowsBatch - 1) / kApplyRowsBatch;
     const dim3 grid((unsigned)std::min<int64_t>(blocks, 16), (unsigned)ntasks);
     k_center_apply_batch<LD><<<grid, 256, smem, st>>>(tasks, g);
@@ -1126,9 +1139,44 @@ __global__ void k_mean_prefactor(const float* __restrict__ Vf, int64_t g, int ld
   mean_prefactor_body(Vf, g, ld, mu, mc, blockIdx.x);
 }
 
-__global__ void k_mean_prefactor_batch(const RoundTask* __restrict__ tasks, int64_t g, int ld) {
+// The same sums for every segment of a batch, eight columns per block: row group
+// r = 4 w + lane / 8 keeps, for its lane's column, the eight partial sums that
+// the threads 8 r .. 8 r + 7 of k_mean_prefactor hold.  So rows are read a full
+// 32-byte sector at a time (a block per column read 4 bytes of each: 64
+// segments of 2,000 x 64 took 40 us, 13 us now) and the bits are the same.
+__global__ void __launch_bounds__(256) k_mean_prefactor_batch(const RoundTask* __restrict__ tasks, int64_t g, int ld) {
   const RoundTask tk = tasks[blockIdx.y];
-  mean_prefactor_body(tk.Vf, g, ld, tk.mu, tk.mc, blockIdx.x);
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, c = blockIdx.x * 8 + (lane & 7);
+  double acc[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) acc[i] = 0.0;
+  if (tk.mu)
+    for (int64_t j0 = 8 * (4 * w + (lane >> 3)); j0 < g; j0 += 256)
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        if (j0 + i < g) acc[i] += tk.mu[j0 + i] * (double)tk.Vf[(j0 + i) * ld + c];
+  __shared__ double red[4][8][32];
+#pragma unroll
+  for (int h = 4; h > 0; h >>= 1) {  // warps w and w + h
+    if (w >= h && w < 2 * h)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) red[w - h][i][lane] = acc[i];
+    __syncthreads();
+    if (w < h)
+#pragma unroll
+      for (int i = 0; i < 8; ++i) acc[i] += red[w][i][lane];
+    __syncthreads();
+  }
+  if (w > 0) return;
+#pragma unroll
+  for (int o = 16; o >= 8; o >>= 1)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] += __shfl_down_sync(0xffffffffu, acc[i], o);
+#pragma unroll
+  for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+    for (int i = 0; i < h; ++i) acc[i] += acc[i + h];
+  if (lane < 8) tk.mc[c] = (float)acc[0];
 }
 
 cudaError_t launch_round_v_batch(const RoundTask* tasks, int ntasks, int64_t g, int ld, cudaStream_t st) {
@@ -1136,7 +1184,7 @@ cudaError_t launch_round_v_batch(const RoundTask* tasks, int ntasks, int64_t g, 
   note_launches(2);
   const int gx = (int)std::min<int64_t>((g * ld + 255) / 256, 64);
   k_round_v_batch<<<dim3((unsigned)gx, (unsigned)ntasks), 256, 0, st>>>(tasks, g, ld);
-  k_mean_prefactor_batch<<<dim3((unsigned)ld, (unsigned)ntasks), 256, 0, st>>>(tasks, g, ld);
+  k_mean_prefactor_batch<<<dim3((unsigned)(ld / 8), (unsigned)ntasks), 256, 0, st>>>(tasks, g, ld);
   return cudaGetLastError();
 }
 
@@ -1182,7 +1230,7 @@ cudaError_t launch_zero_status(const OutTask* tasks, int ntasks, cudaStream_t st
 cudaError_t launch_mean_prefactor_batch(const RoundTask* tasks, int ntasks, int64_t g, int ld, cudaStream_t st) {
   if (ntasks <= 0) return cudaSuccess;
   note_launches(1);
-  k_mean_prefactor_batch<<<dim3((unsigned)ld, (unsigned)ntasks), 256, 0, st>>>(tasks, g, ld);
+  k_mean_prefactor_batch<<<dim3((unsigned)(ld / 8), (unsigned)ntasks), 256, 0, st>>>(tasks, g, ld);
   return cudaGetLastError();
 }
 
@@ -1751,6 +1799,119 @@ __device__ __forceinline__ void ritz_finish_body(const double* __restrict__ B, i
   }
 }
 
+// The same at ld <= 128, where E's columns fit beside the rows: both products
+// on the FP64 matrix instruction.  A block stages E (zero past row k and column
+// nc) and takes strips of 32 rows at a time, first those of M_emb, then the
+// genes of the components; a warp owns eight rows of a strip and half of the
+// columns.  Scalar FMAs read E from shared memory once per FMA and a row of B
+// through a broadcast load: 2,000 genes, k = 60, 50 components 20 us, 8 now;
+// 64 segments with k = 40 and 30 components 164 -> 58; 3,001 genes, k = 110,
+// 100 components 72 -> 23.
+constexpr int kRitzRows = 32;
+
+template <int LD>
+__device__ __forceinline__ void ritz_mma_body(const double* __restrict__ B, int64_t g, int k, int nc,
+                                              const double* __restrict__ evals, const double* __restrict__ E,
+                                              const double* __restrict__ Rinv2, double* __restrict__ sigma,
+                                              float* __restrict__ comps, float* __restrict__ M_emb, int b, int nb) {
+  constexpr int ST = LD + 4, CT = LD / 16;  // 8-column tiles of a warp
+  extern __shared__ double sm[];
+  double* Es = sm;              // [LD][ST]
+  double* rows = sm + LD * ST;  // [kRitzRows][ST]
+  __shared__ double sg[LD];
+  for (int t = threadIdx.x; t < LD * LD; t += 256) {
+    const int l = t / LD, c = t % LD;
+    Es[l * ST + c] = l < k && c < nc ? E[t] : 0.0;
+  }
+  for (int c = threadIdx.x; c < LD; c += 256) sg[c] = c < k ? sqrt(fmax(evals[c], 0.0)) : 0.0;
+  __syncthreads();
+  if (b == 0)
+    for (int c = threadIdx.x; c < k; c += 256) sigma[c] = sg[c];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kr = lane & 3, m = lane >> 2;
+  const int r0 = warp % 4 * 8, c0 = warp / 4 * (8 * CT);
+  constexpr int emb_strips = LD / kRitzRows;
+  const int64_t strips = emb_strips + (g + kRitzRows - 1) / kRitzRows;
+  for (int64_t strip = b; strip < strips; strip += nb) {
+    const bool emb = strip < emb_strips;
+    const int64_t j0 = (emb ? strip : strip - emb_strips) * kRitzRows, jn = emb ? LD : g;
+    const double* from = emb ? Rinv2 : B;
+    __syncthreads();  // the previous strip's rows consumed
+    constexpr int RT = kRitzRows * LD / 256;
+    double v[RT];
+#pragma unroll
+    for (int u = 0; u < RT; ++u) {
+      const int t = threadIdx.x + 256 * u;
+      const int64_t j = j0 + t / LD;
+      v[u] = j < jn && t % LD < k ? from[j * LD + t % LD] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < RT; ++u) {
+      const int t = threadIdx.x + 256 * u;
+      rows[t / LD * ST + t % LD] = v[u];
+    }
+    __syncthreads();
+    if (c0 >= nc) continue;
+    double acc[CT][2];
+#pragma unroll
+    for (int f = 0; f < CT; ++f) acc[f][0] = acc[f][1] = 0.0;
+#pragma unroll 4
+    for (int l = 0; l < LD; l += 4) {
+      const double a = rows[(r0 + m) * ST + l + kr];
+#pragma unroll
+      for (int f = 0; f < CT; ++f) mma_f64(acc[f], a, Es[(l + kr) * ST + c0 + 8 * f + m]);
+    }
+    const int64_t j = j0 + r0 + m;
+    if (j >= jn) continue;
+#pragma unroll
+    for (int f = 0; f < CT; ++f)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int c = c0 + 8 * f + 2 * kr + e;
+        if (c >= nc) continue;
+        if (emb)
+          M_emb[j * nc + c] = (float)(acc[f][e] * sg[c]);
+        else
+          comps[(int64_t)c * g + j] = sg[c] > 0.0 ? (float)(acc[f][e] / sg[c]) : 0.f;
+      }
+  }
+}
+
+__host__ __device__ constexpr size_t ritz_mma_smem(int ld) {
+  return (size_t)(ld + kRitzRows) * (ld + 4) * sizeof(double);
+}
+
+// One matrix, or with `tasks` one segment of a batch per grid row y.
+template <int LD>
+__global__ void __launch_bounds__(256) k_ritz_mma(const RitzTask* __restrict__ tasks, RitzTask one, int64_t g, int k,
+                                                  int nc) {
+  const RitzTask t = tasks ? tasks[blockIdx.y] : one;
+  ritz_mma_body<LD>(t.B, g, k, nc, t.evals, t.evecs, t.Rinv2, t.sigma, t.comps, t.M_emb, blockIdx.x, gridDim.x);
+}
+
+template <int LD>
+static cudaError_t ritz_mma_go(const RitzTask* tasks, int ntasks, const RitzTask& one, int64_t g, int k, int nc,
+                               cudaStream_t st) {
+  constexpr size_t smem = ritz_mma_smem(LD);
+  if (cudaError_t e = allow_smem(k_ritz_mma<LD>, smem); e != cudaSuccess) return e;
+  // one matrix: a strip per block; a batch: a few strips per staged E
+  const int64_t strips = LD / kRitzRows + (g + kRitzRows - 1) / kRitzRows;
+  const dim3 grid((unsigned)std::min<int64_t>(strips, tasks ? 16 : 148), (unsigned)(tasks ? ntasks : 1));
+  note_launches(1);
+  k_ritz_mma<LD><<<grid, 256, smem, st>>>(tasks, one, g, k, nc);
+  return cudaGetLastError();
+}
+
+static cudaError_t ritz_mma(const RitzTask* tasks, int ntasks, const RitzTask& one, int64_t g, int ld, int k, int nc,
+                            cudaStream_t st) {
+  switch (ld) {
+    case 32: return ritz_mma_go<32>(tasks, ntasks, one, g, k, nc, st);
+    case 64: return ritz_mma_go<64>(tasks, ntasks, one, g, k, nc, st);
+    case 96: return ritz_mma_go<96>(tasks, ntasks, one, g, k, nc, st);
+    case 128: return ritz_mma_go<128>(tasks, ntasks, one, g, k, nc, st);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
 __global__ void __launch_bounds__(128) k_ritz_finish(const double* __restrict__ B, int64_t g, int ld, int k,
                                                      int nc, int c0, int ncc, const double* __restrict__ evals,
                                                      const double* __restrict__ E,
@@ -1778,6 +1939,9 @@ static int ritz_cols(int ld, int nc, size_t* smem) {
 cudaError_t launch_ritz_finish(const double* B, int64_t g, int ld, int k, int nc,
                                const double* evals, const double* evecs, const double* Rinv2,
                                double* sigma, float* components, float* M_emb, cudaStream_t st) {
+  if (ld <= kMaxK)
+    return ritz_mma(nullptr, 0,
+                    RitzTask{B, evals, evecs, Rinv2, sigma, components, M_emb}, g, ld, k, nc, st);
   size_t smem = 0;
   const int ncc = ritz_cols(ld, nc, &smem);
   if (cudaError_t e = allow_smem(k_ritz_finish, smem); e != cudaSuccess) return e;
@@ -1794,6 +1958,7 @@ cudaError_t launch_ritz_finish(const double* B, int64_t g, int ld, int k, int nc
 cudaError_t launch_ritz_finish_batch(const RitzTask* tasks, int ntasks, int64_t g, int ld, int k, int nc,
                                      cudaStream_t st) {
   if (ntasks <= 0) return cudaSuccess;
+  if (ld <= kMaxK) return ritz_mma(tasks, ntasks, RitzTask{}, g, ld, k, nc, st);
   size_t smem = 0;
   const int ncc = ritz_cols(ld, nc, &smem);
   if (cudaError_t e = allow_smem(k_ritz_finish_batch, smem); e != cudaSuccess) return e;

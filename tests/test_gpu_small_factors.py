@@ -77,3 +77,30 @@ def test_qr_row_counts(matrix, m, k):
         r = np.linalg.cholesky(a64.T @ a64).T
         want = np.linalg.solve(r.T, a64.T).T
         assert np.abs(q - want).max() < 2e-6 * np.abs(want).max() * np.linalg.cond(a64)
+
+
+@pytest.mark.parametrize("n,g,nc,over", [
+    (300, 20, 5, 15),      # ld 32; components end inside the first half of the columns
+    (300, 64, 33, 31),     # both halves
+    (400, 95, 95, 0),      # ld 96, as many components as columns
+    (500, 127, 70, 57),    # ld 128
+    (32, 5003, 9, 22),     # more strips of genes than blocks, a ragged last one
+    (120, 4801, 65, 54),
+])
+def test_finish_is_consistent(n, g, nc, over):
+    """A sketch as wide as the centred matrix's rank spans its range, so the
+    embeddings are the matrix times the components, and these are orthonormal:
+    FP32 factors of a well-conditioned sketch, 2e-5 of the largest singular value."""
+    rng = np.random.default_rng(n + g)
+    x = rng.standard_normal((n, g)).astype(np.float32) * (rng.random((n, g)) < 0.4)
+    rows, cols = np.nonzero(x)
+    indptr = np.r_[0, np.cumsum(np.bincount(rows, minlength=n))]
+    res = accel.randomized_pca(indptr, cols.astype(np.int32), x[rows, cols], (n, g), n_components=nc,
+                               n_oversamples=over, n_power_iterations=2)
+    xc = x.astype(np.float64) - x.astype(np.float64).mean(axis=0)
+    comps = np.asarray(res.components, dtype=np.float64)
+    emb = np.asarray(res.embeddings, dtype=np.float64)
+    s = np.linalg.svd(xc, compute_uv=False)[:nc]
+    assert np.abs(comps @ comps.T - np.eye(nc)).max() < 2e-5
+    assert np.abs(res.singular_values - s).max() < 2e-5 * s[0]
+    assert np.abs(emb - xc @ comps.T).max() < 2e-5 * s[0]
