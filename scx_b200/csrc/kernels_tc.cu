@@ -29,9 +29,8 @@
 // A tcgen05.mma at M = 128 costs about the same to issue whatever its N, so
 // spanning two row tiles (forward) or four gene chunks (transposed) in
 // N = 256 halves the instructions per segment against N = 128.  At ld 128
-// (k_fwd_tc, k_rmat_tc) the image is the B operand (N = 256) and the tiles
-// the A:
-//   forward    Y(128 cells x 256) += A(cells x 64 genes, K-major) Vimg_c
+// k_fwd_tc does the same for either half of the 256 image columns; k_rmat_tc
+// takes the image as the B operand (N = 256) and the tiles as the A:
 //   transposed Z(128 genes x 256) += A^T(genes x cells, MN-major) Qimg_t
 //
 // Warp roles (23 warps): warps 0-15 densify in four groups of four; warps
@@ -80,22 +79,20 @@ struct SegMeta {
 static_assert(sizeof(SegMeta) == 16, "segment metadata is one 16-byte record");
 
 // Pipeline shapes of the ld-128 kernels (k_fwd_tc, k_rmat_tc; ld 64 has its
-// own, next to k_fwd_swap / k_rmat_swap).  In the forward kernel densify group
-// g takes the stages it with it % G == g and owns A stage buffers g and g + G
-// (S == 2 G), so it densifies its next segment while the MMAs read the
-// previous one.  In the transposed kernel a stage (two 64-gene sub-tiles) is
-// filled by a pair of groups, one sub-tile each; pair p takes the stages it
-// with it % 2 == p.  Either way each waiter runs at most one barrier phase
-// ahead of the phase it waits for, which is what a parity wait can
+// own, next to k_fwd_swap / k_rmat_swap).  Densify group g takes the 16 KB
+// stages it with it % kGroups == g and owns stage buffer g: a tile's chunk in the
+// forward kernel, half a tile of two chunks in the transposed one (a whole tile
+// per stage and two buffers left a pair of groups one stage's time for a stage:
+// 120,000 x 3,001, k = 110: 169 us, now 145).  Each waiter runs at most one
+// barrier phase ahead of the phase it waits for, which is what a parity wait can
 // distinguish.  The forward kernel's dense operand has its own ring of
 // fwd_bslots(LD) chunk buffers, filled ahead of the MMAs.
-__host__ __device__ constexpr int fwd_stages(int LD) { return 2 * kGroups; }
-__host__ __device__ constexpr int fwd_bslots(int LD) { return 2; }
-__host__ __device__ constexpr int rmat_stages(int LD) { return 2; }
-// 16-byte entry words a densify lane keeps in flight per segment quarter
-// (x 128 entries per warp); a larger quarter loads the rest on demand.
-constexpr int kFwdRegs = 4;
-constexpr int kRmatRegs = 4;
+__host__ __device__ constexpr int fwd_stages(int LD) { return kGroups; }
+__host__ __device__ constexpr int fwd_bslots(int LD) { return 4; }
+__host__ __device__ constexpr int rmat_stages(int LD) { return kGroups; }
+// Entries a densify lane keeps in flight per stage (x 32 a warp); a larger
+// segment quarter loads the rest on demand.
+constexpr int kDenseRegs = 8;
 
 __host__ __device__ __forceinline__ int padded4(int x) { return (x + 3) & ~3; }
 
@@ -255,15 +252,6 @@ __device__ __forceinline__ void sts_u16(uint32_t addr, uint32_t v) {
 __device__ __forceinline__ void sts_zero16(uint32_t addr) {
   asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(addr), "r"(0u) : "memory");
 }
-// 16 bytes of entries, read-only path (the packed matrix never changes during a launch).
-__device__ __forceinline__ uint4 ldg_entries(const uint32_t* p) {
-  uint4 v;
-  asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-               : "l"(p));
-  return v;
-}
-
 // Two floats as a pair of 16-bit values (fmt 1 = bf16, 0 = f16), low word first.
 __device__ __forceinline__ uint32_t pack16x2(float a, float b, int fmt) {
   if (fmt) {
@@ -285,11 +273,11 @@ __device__ __forceinline__ uint32_t hilo16(float x, int fmt) {
   return h | (l << 16);
 }
 
-// hilo16 of 16 values, two at a time, with one branch on the format.
-template <bool BF>
-__device__ __forceinline__ void hilo16_block_as(const float (&v)[16], uint32_t (&w)[16]) {
+// hilo16 of N values, two at a time, with one branch on the format.
+template <bool BF, int N>
+__device__ __forceinline__ void hilo16_block_as(const float (&v)[N], uint32_t (&w)[N]) {
 #pragma unroll
-  for (int i = 0; i < 16; i += 2) {
+  for (int i = 0; i < N; i += 2) {
     const uint32_t h = pack16x2(v[i], v[i + 1], BF);
     const uint32_t l =
         pack16x2(v[i] - unpack16(h & 0xFFFFu, BF), v[i + 1] - unpack16(h >> 16, BF), BF);
@@ -297,7 +285,8 @@ __device__ __forceinline__ void hilo16_block_as(const float (&v)[16], uint32_t (
     w[i + 1] = __byte_perm(h, l, 0x7632);
   }
 }
-__device__ __forceinline__ void hilo16_block(const float (&v)[16], uint32_t (&w)[16], int fmt) {
+template <int N>
+__device__ __forceinline__ void hilo16_block(const float (&v)[N], uint32_t (&w)[N], int fmt) {
   if (fmt)
     hilo16_block_as<true>(v, w);
   else
@@ -334,45 +323,6 @@ __device__ __forceinline__ Span quarter_span(const SegMeta& m, int q) {
   return Span{start + (int64_t)lo, start + (int64_t)hi};
 }
 
-// Issue the first R 16-byte loads of a span (its start rounded down to a
-// 16-byte boundary; segments start on one and are padded to one, so a load
-// never leaves its segment).  Lane L holds words 4 (L + 32 r) .. + 3.
-template <int R>
-__device__ __forceinline__ void span_load(const uint32_t* __restrict__ ent, Span sp, int lane, uint4 (&w)[R]) {
-  const int64_t a0 = sp.lo & ~int64_t(3);
-  const int phi = (int)(sp.hi - a0);
-  const uint32_t* base = ent + a0;
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int p = 4 * (lane + 32 * r);
-    w[r] = p < phi ? ldg_entries(base + p) : make_uint4(0u, 0u, 0u, 0u);
-  }
-}
-
-// The four words at span positions p .. p + 3 (counted from the span's 16-byte
-// aligned start); those outside [plo, phi) belong to the neighbouring spans.
-// With d = p - plo and n = phi - plo, word k is in the span iff
-// (unsigned)(d + k) < n: one 32-bit compare per word.
-__device__ __forceinline__ void scatter4(uint32_t tile, const uint4& w, int d, unsigned n) {
-  if ((unsigned)d < n) scatter_one(tile, w.x);
-  if ((unsigned)(d + 1) < n) scatter_one(tile, w.y);
-  if ((unsigned)(d + 2) < n) scatter_one(tile, w.z);
-  if ((unsigned)(d + 3) < n) scatter_one(tile, w.w);
-}
-
-// Scatter a span into `tile` (already zeroed): the R words in flight first,
-// then whatever lies beyond them, loaded here.
-template <int R>
-__device__ __forceinline__ void span_scatter(uint32_t tile, const uint32_t* __restrict__ ent, Span sp, int lane,
-                                             const uint4 (&w)[R]) {
-  const int64_t a0 = sp.lo & ~int64_t(3);
-  const int plo = (int)(sp.lo - a0), phi = (int)(sp.hi - a0);  // a quarter holds at most 2,048 entries
-  const unsigned n = (unsigned)(phi - plo);
-#pragma unroll
-  for (int r = 0; r < R; ++r) scatter4(tile, w[r], 4 * (lane + 32 * r) - plo, n);
-  for (int p = 4 * (lane + 32 * R); p < phi; p += 128) scatter4(tile, ldg_entries(ent + a0 + p), p - plo, n);
-}
-
 // The words of a densify warp's next segment quarter for one of its two stage
 // buffers (ld-64 kernels), in flight: word r of a lane is entry lane + 32 r, so
 // that one store instruction takes 32 neighbouring entries, five or six rows
@@ -385,6 +335,14 @@ struct DenseSlot {
   const uint32_t* base;
   int n;  // entries; < 0: no tile here
 };
+
+template <int R>
+__device__ __forceinline__ void slots_init(DenseSlot<R> (&x)[2]) {
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+#pragma unroll
+    for (int r = 0; r < R; ++r) x[k].w[r] = 0u;
+}
 
 // The first R blocks of 32 entries, straight into the slot's registers: a lane
 // without one keeps what it had (the scatter does not look at it), so no
@@ -436,8 +394,56 @@ __device__ __forceinline__ bool load_meta(const SegMeta* __restrict__ src, int r
   return true;
 }
 
+// Epilogue of the forward kernels, whose accumulators hold image columns in
+// the TMEM lanes and the cells of `tiles` tiles (from row0 of n) in the columns:
+// the warp's lane pair with p = 0, 1 holds the hi and lo halves of column j,
+// which go to Y (unless null) and, as a (hi, lo) word, to its image.  Each lane
+// gives the other the halves it does not need, one exchange for two cells, and
+// the exchanges, conversions and stores of 32 cells go in passes of their own:
+// sixteen independent chains, where cell after cell would stall on each.
+template <int LD>
+__device__ __forceinline__ void swap_tile_out(uint32_t tbase, int tiles, int64_t row0, int64_t n,
+                                              const float* __restrict__ mc, int j, int p, float* __restrict__ Y,
+                                              uint16_t* __restrict__ Yimg, int fmt) {
+  const float mcj = __ldg(mc + j);
+#pragma unroll 1
+  for (int cb = 0; cb < tiles * (TM / 32); ++cb) {  // 32 cells per TMEM load
+    uint32_t r[32];
+    tmem_ld32(tbase + cb * 32, r);
+    tmem_wait_ld();
+    const int64_t c0 = row0 + cb * 32 + p;  // lane p handles cells c0 + 2 i
+    float v[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const float x0 = __uint_as_float(r[2 * i]), x1 = __uint_as_float(r[2 * i + 1]);
+      const float other = __shfl_xor_sync(0xffffffffu, p ? x0 : x1, 1);
+      v[i] = (p ? x1 : x0) + other - mcj;
+    }
+    const int left = (int)min((int64_t)32, n - c0);  // cell 2 i is inside the matrix iff 2 i < left
+    uint32_t* dst = reinterpret_cast<uint32_t*>(Yimg) + c0 * LD + j;
+    uint32_t img[16];
+    hilo16_block(v, img, fmt);
+#pragma unroll
+    for (int i = 0; i < 16; ++i)
+      if (2 * i < left) dst[i * 2 * LD] = img[i];
+    if (Y) {
+      float* ydst = Y + c0 * LD + j;
+#pragma unroll
+      for (int i = 0; i < 16; ++i)
+        if (2 * i < left) ydst[i * 2 * LD] = v[i];
+    }
+  }
+}
+
 // ---------------------------------------------------------------------------
-// forward: Y[tile rows, :LD] = A_tile (Vhi + Vlo) - mc   (persistent over tiles)
+// forward, ld 128: as k_fwd_swap, with the 256 image columns as two halves of
+// M = 128 and the two tiles of a band (256 cells) as N.  CTA b takes the tiles
+// [tc_range_begin(b), tc_range_begin(b + 1)), two at a time, so that each 32 KB
+// image chunk serves two tiles; the two accumulators fill TMEM.  The MMAs alone
+// take about 140 us at 120,000 x 3,001, k = 110 (175 cycles each, 8 per chunk
+// and band); an image chunk per tile as the MMA's B operand, double-buffered,
+// took 217 us, of which 195 the MMAs (282 cycles each with an MN-major B) and a
+// two-slot image ring; this takes 194, the epilogues of the bands included.
 // ---------------------------------------------------------------------------
 template <int LD>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -445,18 +451,18 @@ __global__ void __launch_bounds__(kThreads, 1)
              int64_t n, const __grid_constant__ CUtensorMap vmap, const float* __restrict__ mc,
              float* __restrict__ Y, uint16_t* __restrict__ Yimg, int fmt, int* err) {
   constexpr int N2 = 2 * LD;                // [hi | lo] columns
-  constexpr int S = fwd_stages(LD);         // A stages, two per densify group
-  constexpr int G = kGroups;
+  constexpr int S = fwd_stages(LD);         // A stages, one per densify group
   constexpr int NB = fwd_bslots(LD);        // dense-operand ring
   constexpr int A_BYTES = TM * CW * 2;      // 16 KB
   constexpr int B_BYTES = CW * N2 * 2;      // 64 genes x N2 image columns
-  static_assert(S == 2 * G, "two A stages per densify group");
+  static_assert(S == kGroups, "group = stage");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = align1024(smem_raw);
   uint8_t* As = smem;
   uint8_t* Bs = As + S * A_BYTES;
-  SegMeta* mring = reinterpret_cast<SegMeta*>(Bs + NB * B_BYTES);  // [2][kMaxChunks]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(mring + 2 * kMaxChunks);
+  constexpr int MSLOT = 2 * kMaxChunks;
+  SegMeta* mring = reinterpret_cast<SegMeta*>(Bs + NB * B_BYTES);  // [2][2 * kMaxChunks]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(mring + 2 * MSLOT);
   uint64_t* full = bars;            // [S]  A stage densified (4 warp arrivals)
   uint64_t* empty = full + S;       // [S]  A stage consumed (MMA commit)
   uint64_t* bfull = empty + S;      // [NB] dense chunk landed (TMA)
@@ -469,6 +475,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t t0 = tc_range_begin(blockIdx.x, gridDim.x, n_tiles), t1 = tc_range_begin(blockIdx.x + 1, gridDim.x, n_tiles);
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
       mbar_init(&full[s], 4);  // one arrival per warp of the stage's densify group
@@ -497,80 +504,79 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tmem = *tmem_slot;
 
   if (warp < W_EPI) {
-    // ---- densify: group (warp / 4) takes stages it % G == group ----
+    // ---- densify: group (warp / 4) takes the stages it with it % S == group;
+    // words are loaded two stages ahead ----
     const int group = warp >> 2, q = warp & 3;
-    uint32_t it = 0, ti = 0;
-    uint4 w[kFwdRegs];
-    Span pre{-1, -1};  // span whose loads are in flight in w
-    for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x, ++ti) {
-      if (!warp_wait(&mfull[ti & 1u], (ti >> 1) & 1u, abort_flag, err, 11)) goto done;
-      const SegMeta* mt = mring + (ti & 1u) * kMaxChunks;
-      for (int c = 0; c < nc; ++c, ++it) {
-        if ((int)(it % G) != group) continue;
-        const Span sp = quarter_span(mt[c], q);
-        if (sp.lo != pre.lo || sp.hi != pre.hi) span_load<kFwdRegs>(ent, sp, lane, w);
-        const int s = it % S;
-        if (!warp_wait(&empty[s], ((it / S) & 1u) ^ 1u, abort_flag, err, 12)) goto done;
-        const uint32_t tile = smem_u32(As + s * A_BYTES);
-        zero_rows(tile, q, lane);
+    const uint32_t tile = smem_u32(As + group * A_BYTES);
+    DenseSlot<kDenseRegs> sl[2];
+    slots_init(sl);
+    // cursor: the next segment to load, number j = 2 chunk + tile of its band
+    int64_t t = t0;
+    uint32_t bi = 0;
+    int tiles = 0, j = group;
+    bool live = true;
+    auto enter = [&]() {
+      tiles = (int)min((int64_t)2, t1 - t);
+      return warp_wait(&mfull[bi & 1u], (bi >> 1) & 1u, abort_flag, err, 11);
+    };
+    auto fetch = [&](DenseSlot<kDenseRegs>& x) {
+      while (j >= 2 * nc) {  // leave the band
         __syncwarp();
-        span_scatter<kFwdRegs>(tile, ent, sp, lane, w);
-        // put the group's next segment in flight: chunk c + G of this tile, or
-        // of the next tile once its metadata is in
-        pre = Span{-1, -1};
-        const int cn = c + G;
-        if (cn < nc) {
-          pre = quarter_span(mt[cn], q);
-        } else if (cn - nc < nc && t + gridDim.x < n_tiles) {
-          if (!warp_wait(&mfull[(ti + 1) & 1u], ((ti + 1) >> 1) & 1u, abort_flag, err, 11)) goto done;
-          pre = quarter_span(mring[((ti + 1) & 1u) * kMaxChunks + (cn - nc)], q);
+        if (lane == 0) mbar_arrive(&mempty[bi & 1u]);
+        j -= 2 * nc;
+        t += 2;
+        ++bi;
+        if (t >= t1) {
+          live = false;
+          return true;
         }
-        if (pre.lo >= 0) span_load<kFwdRegs>(ent, pre, lane, w);
+        if (!enter()) return false;
+      }
+      x.n = -1;
+      if ((j & 1) < tiles) slot_load(x, ent, quarter_span(mring[(bi & 1u) * MSLOT + (j & 1) * nc + (j >> 1)], q), lane);
+      j += S;
+      return true;
+    };
+    if (t0 >= t1) goto done;
+    if (!enter() || !fetch(sl[0])) goto done;
+    bool more0 = live, more1;
+    if (live && !fetch(sl[1])) goto done;
+    more1 = live;
+    for (; more0;) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        if (k == 1 && !more1) break;
+        if (!warp_wait(&empty[group], (uint32_t)(k ^ 1), abort_flag, err, 12)) goto done;
+        if (sl[k].n >= 0) {
+          zero_rows(tile, q, lane);
+          __syncwarp();
+          slot_scatter(sl[k], tile, lane);
+        }
         // every lane's shared stores -> async proxy, then one arrival per warp
         fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&full[s]);
+        if (lane == 0) mbar_arrive(&full[group]);
+        if (live && !fetch(sl[k])) goto done;
+        (k ? more1 : more0) = live;
       }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&mempty[ti & 1u]);
     }
   } else if (warp < W_MMA) {
-    // ---- epilogue: TMEM (hi, lo) column pairs -> Y (FP32) and its 16-bit image ----
-    const int q = warp & 3;
-    const uint32_t row = 32u * q + lane;
+    // ---- epilogue: lane pair (2 i, 2 i + 1) of half h -> column 64 h + i of Y
+    // and its image; a half goes back to the MMAs as soon as it is read ----
+    const int q = warp & 3, p = lane & 1;
     uint32_t k = 0;
-    for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x, ++k) {
-      const uint32_t a = k & 1u, ph = (k >> 1) & 1u;
-      if (!warp_wait(&acc_full[a], ph, abort_flag, err, 14)) goto done;
-      tc_fence_after();
-      const uint32_t tbase = tmem + ((32u * q) << 16) + a * N2;
-      const int64_t grow = t * TM + row;
-#pragma unroll 1
-      for (int cb = 0; cb < N2 / 16; ++cb) {  // 16 image columns = 8 output columns
-        uint32_t r[16];
-        tmem_ld16(tbase + cb * 16, r);
-        tmem_wait_ld();
-        if (grow < n) {
-          float o[8];
-          uint32_t w[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            o[i] = __uint_as_float(r[2 * i]) + __uint_as_float(r[2 * i + 1]) - __ldg(mc + cb * 8 + i);
-            w[i] = hilo16(o[i], fmt);
-          }
-          if (Y) {  // the FP32 copy only when the caller reads it
-            float4* yr = reinterpret_cast<float4*>(Y + grow * LD + cb * 8);
-            yr[0] = make_float4(o[0], o[1], o[2], o[3]);
-            yr[1] = make_float4(o[4], o[5], o[6], o[7]);
-          }
-          uint4* ir = reinterpret_cast<uint4*>(Yimg + grow * N2 + cb * 16);
-          ir[0] = make_uint4(w[0], w[1], w[2], w[3]);
-          ir[1] = make_uint4(w[4], w[5], w[6], w[7]);
-        }
+    for (int64_t t = t0; t < t1; t += 2, ++k) {
+      const int tiles = (int)min((int64_t)2, t1 - t);
+      for (int h = 0; h < 2; ++h) {
+        const int j = 64 * h + 16 * q + (lane >> 1);
+        if (!warp_wait(&acc_full[h], k & 1u, abort_flag, err, 14)) goto done;
+        tc_fence_after();
+        const uint32_t tbase = tmem + ((32u * q) << 16) + h * 256;
+        swap_tile_out<LD>(tbase, tiles, t * TM, n, mc, j, p, Y, Yimg, fmt);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[h]);
       }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&acc_empty[a]);
     }
   } else if (warp == W_MMA) {
     // ---- MMA issuer ----
@@ -578,36 +584,43 @@ __global__ void __launch_bounds__(kThreads, 1)
       // The issue loop is the pipeline's critical path: descriptors are
       // formed once and advanced by constant offsets (their address field is
       // in 16-byte units; shared addresses stay below 256 KB, so no carry).
-      const uint32_t idesc = idesc_f16(128, N2, fmt, 0, 1);
-      const uint64_t adesc0 = sdesc_sw128(smem_u32(As), 16, 1024);
-      const uint64_t bdesc0 = sdesc_sw128(smem_u32(Bs), CW * 128, 1024);
+      const uint32_t idesc2 = idesc_f16(128, 256, fmt, 1, 0);
+      const uint32_t idesc1 = idesc_f16(128, 128, fmt, 1, 0);
+      const uint64_t tdesc0 = sdesc_sw128(smem_u32(As), 16, 1024);        // K-major, 256 cell rows
+      const uint64_t vdesc0 = sdesc_sw128(smem_u32(Bs), CW * 128, 1024);  // MN-major, 64-column blocks
       static_assert((S & (S - 1)) == 0 && (NB & (NB - 1)) == 0, "power-of-two rings");
-      uint32_t it = 0, k = 0;
-      for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x, ++k) {
-        const uint32_t a = k & 1u, ph = (k >> 1) & 1u;
-        if (!mbar_wait(&acc_empty[a], ph ^ 1u, abort_flag, err, 15)) break;
-        tc_fence_after();
-        const uint32_t d = tmem + a * N2;
-        bool ok = true;
-        for (int c = 0; c < nc; ++c, ++it) {
-          const int s = it % S, b = it % NB;
-          if (!mbar_wait(&bfull[b], (it / NB) & 1u, abort_flag, err, 16) ||
-              !mbar_wait(&full[s], (it / S) & 1u, abort_flag, err, 16)) {
+      uint32_t cc = 0, k = 0;
+      bool ok = true;
+      for (int64_t t = t0; t < t1 && ok; t += 2, ++k) {
+        const uint32_t idesc = t1 - t >= 2 ? idesc2 : idesc1;
+        for (int c = 0; c < nc; ++c, ++cc) {
+          const int b = cc % NB, s = 2 * cc % S;
+          if (!mbar_wait(&bfull[b], (cc / NB) & 1u, abort_flag, err, 16) ||
+              !mbar_wait(&full[s], (2 * cc / S) & 1u, abort_flag, err, 16) ||
+              !mbar_wait(&full[s + 1], (2 * cc / S) & 1u, abort_flag, err, 16)) {
             ok = false;
             break;
           }
-          tc_fence_after();
-          const uint64_t ad = adesc0 + (uint64_t)(s * (A_BYTES >> 4));
-          const uint64_t bd = bdesc0 + (uint64_t)(b * (B_BYTES >> 4));
-          umma_f16(d, ad, bd, idesc, c != 0);
+          const uint64_t td = tdesc0 + (uint64_t)(s * (A_BYTES >> 4));
 #pragma unroll
-          for (int kk = 1; kk < CW / 16; ++kk)  // K steps: +32 B along A's rows, +2 KB down B
-            umma_f16(d, ad + 2 * kk, bd + 128 * kk, idesc, 1u);
+          for (int h = 0; h < 2; ++h) {  // image columns 128 h ..
+            if (c == 0 && !mbar_wait(&acc_empty[h], (k & 1u) ^ 1u, abort_flag, err, 15)) {
+              ok = false;
+              break;
+            }
+            tc_fence_after();
+            const uint64_t vd = vdesc0 + (uint64_t)((b * B_BYTES + h * (2 * CW * 128)) >> 4);
+            umma_f16(tmem + h * 256, vd, td, idesc, c != 0);
+#pragma unroll
+            for (int kk = 1; kk < CW / 16; ++kk)  // K steps of 16 genes: +2 KB down the image, +32 B along the tiles
+              umma_f16(tmem + h * 256, vd + 128 * kk, td + 2 * kk, idesc, 1u);
+            if (c == nc - 1) umma_commit(&acc_full[h]);
+          }
+          if (!ok) break;
           umma_commit(&empty[s]);
+          umma_commit(&empty[s + 1]);
           umma_commit(&bempty[b]);
         }
-        if (!ok) break;
-        umma_commit(&acc_full[a]);
       }
     }
     __syncwarp();
@@ -616,7 +629,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (lane == 0) {
       uint32_t it = 0;
       bool ok = true;
-      for (int64_t t = blockIdx.x; t < n_tiles && ok; t += gridDim.x) {
+      for (int64_t t = t0; t < t1 && ok; t += 2) {
         for (int c = 0; c < nc; ++c, ++it) {
           const int b = it % NB;
           if (!mbar_wait(&bempty[b], ((it / NB) & 1u) ^ 1u, abort_flag, err, 19)) {
@@ -632,13 +645,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     __syncwarp();
   } else if (warp == W_META) {
-    // ---- meta loader: tile metadata, and the tile's entries into L2 ----
+    // ---- meta loader: band metadata, and the band's entries into L2 ----
     if (lane == 0) {
-      uint32_t ti = 0;
-      for (int64_t t = blockIdx.x; t < n_tiles; t += gridDim.x, ++ti) {
-        if (!load_meta(meta + t * nc, nc, mring, kMaxChunks, mfull, mempty, ti, abort_flag, err, 17)) break;
-        if (!mbar_wait(&mfull[ti & 1u], (ti >> 1) & 1u, abort_flag, err, 18)) break;
-        prefetch_segments(ent, mring + (ti & 1u) * kMaxChunks, 0, nc);
+      uint32_t bi = 0;
+      for (int64_t t = t0; t < t1; t += 2, ++bi) {
+        const int records = nc * (int)min((int64_t)2, t1 - t);  // consecutive in `meta`
+        if (!load_meta(meta + t * nc, records, mring, MSLOT, mfull, mempty, bi, abort_flag, err, 17)) break;
+        if (!mbar_wait(&mfull[bi & 1u], (bi >> 1) & 1u, abort_flag, err, 18)) break;
+        prefetch_segments(ent, mring + (bi & 1u) * MSLOT, 0, records);
       }
     }
     __syncwarp();
@@ -666,9 +680,10 @@ __global__ void __launch_bounds__(kThreads, 1)
               int64_t g, int n_gene_groups, const __grid_constant__ CUtensorMap qmap, float* __restrict__ part,
               int fmt, int* err) {
   constexpr int N2 = 2 * LD;
-  constexpr int S = rmat_stages(LD);     // A stages, one per pair of densify groups
-  constexpr int SUB = TM * CW * 2;       // one 64-gene sub-tile, 16 KB
-  constexpr int A_BYTES = 2 * SUB;       // 128 genes
+  constexpr int S = rmat_stages(LD);     // A stages, one per densify group
+  static_assert(S == kGroups, "group = stage");
+  constexpr int HSUB = 64 * CW * 2;      // half a chunk tile (64 cells x 64 genes), 8 KB
+  constexpr int A_BYTES = 2 * HSUB;      // 64 cells x 128 genes
   constexpr int Q_BYTES = TM * N2 * 2;   // 128 cells x N2 image columns
   constexpr int SPG = 512 / N2;          // 128-gene super-chunks per CTA (TMEM columns)
   extern __shared__ uint8_t smem_raw[];
@@ -699,7 +714,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
-      mbar_init(&full[s], 8);  // one arrival per warp of the stage's two densify groups
+      mbar_init(&full[s], 4);  // one arrival per warp of the stage's densify group
       mbar_init(&empty[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
@@ -722,54 +737,61 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tmem = *tmem_slot;
 
   if (warp < W_EPI) {
-    // ---- densify: a stage (128-gene super-chunk) is split over a pair of
-    // groups, one 64-gene sub-tile each: group g fills sub-tile g & 1 of the
-    // stages it with it % 2 == g >> 1, so each pair owns every other stage
-    // buffer and has its next stage in hand while the MMAs read this one ----
-    const int group = warp >> 2, q = warp & 3;
-    const int h = group & 1, pg = group >> 1;
-    uint32_t it = 0, ti = 0;
-    uint4 w[kRmatRegs];
-    Span pre{-1, -1};  // span whose loads are in flight in w
-    if (have_work)
-      for (int64_t t = t0; t < t1; ++t, ++ti) {
-        if (!warp_wait(&mfull[ti & 1u], (ti >> 1) & 1u, abort_flag, err, 21)) goto done;
-        const SegMeta* mt = mring + (ti & 1u) * kMaxChunks;
-        for (int sc = sc0; sc < sc1; ++sc, ++it) {
-          if ((int)(it & 1u) != pg) continue;
-          const int ch = 2 * sc + h;
-          const Span sp = ch < nc ? quarter_span(mt[ch], q) : Span{0, 0};
-          if (sp.lo != pre.lo || sp.hi != pre.hi) span_load<kRmatRegs>(ent, sp, lane, w);
-          const int s = it % S;
-          if (!warp_wait(&empty[s], ((it / S) & 1u) ^ 1u, abort_flag, err, 22)) goto done;
-          const uint32_t tile = smem_u32(As + s * A_BYTES) + h * SUB;
-          zero_rows(tile, q, lane);
-          __syncwarp();
-          span_scatter<kRmatRegs>(tile, ent, sp, lane, w);
-          // the pair's next stage: super-chunk sc + 2 of this tile, or of the next
-          pre = Span{-1, -1};
-          const int scn = sc + 2;
-          const SegMeta* mn = nullptr;
-          int scx = 0;
-          if (scn < sc1) {
-            mn = mt;
-            scx = scn;
-          } else if (scn - nsc < sc1 && t + 1 < t1) {
-            if (!warp_wait(&mfull[(ti + 1) & 1u], ((ti + 1) >> 1) & 1u, abort_flag, err, 21)) goto done;
-            mn = mring + ((ti + 1) & 1u) * kMaxChunks;
-            scx = scn - nsc;
-          }
-          if (mn && 2 * scx + h < nc) {
-            pre = quarter_span(mn[2 * scx + h], q);
-            span_load<kRmatRegs>(ent, pre, lane, w);
-          }
-          fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(&full[s]);
-        }
+    // ---- densify: group (warp / 4) takes the stages it with it % S == group,
+    // one half (64 cells) of a tile for the two chunks of a super-chunk: warp
+    // (chunk, quarter) of the group fills 32 cells of one chunk.  Words are
+    // loaded two stages ahead ----
+    const int group = warp >> 2, cofs = (warp >> 1) & 1, r = warp & 1;
+    const uint32_t stage0 = smem_u32(As + group * A_BYTES + cofs * HSUB);
+    DenseSlot<kDenseRegs> sl[2];
+    slots_init(sl);
+    int hs[2] = {0, 0};  // the half of each slot's segment
+    // cursor: the next segment to load, number j = 2 (super-chunk) + half of its tile
+    const uint32_t ntl = have_work ? (uint32_t)(t1 - t0) : 0u;
+    uint32_t ti = 0;
+    int j = group;
+    bool live = true;
+    auto fetch = [&](DenseSlot<kDenseRegs>& x, int& hx) {
+      while (j >= 2 * nsc) {  // leave the tile
         __syncwarp();
         if (lane == 0) mbar_arrive(&mempty[ti & 1u]);
+        j -= 2 * nsc;
+        if (++ti == ntl) {
+          live = false;
+          return true;
+        }
+        if (!warp_wait(&mfull[ti & 1u], (ti >> 1) & 1u, abort_flag, err, 21)) return false;
       }
+      hx = j & 1;
+      const int ch = 2 * (sc0 + (j >> 1)) + cofs;
+      x.n = 0;
+      if (ch < nc) slot_load(x, ent, quarter_span(mring[(ti & 1u) * kMaxChunks + ch], 2 * hx + r), lane);
+      j += S;
+      return true;
+    };
+    if (have_work) {
+      if (!warp_wait(&mfull[0], 0u, abort_flag, err, 21) || !fetch(sl[0], hs[0])) goto done;
+      bool more0 = live, more1;
+      if (live && !fetch(sl[1], hs[1])) goto done;
+      more1 = live;
+      for (; more0;) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+          if (k == 1 && !more1) break;
+          if (!warp_wait(&empty[group], (uint32_t)(k ^ 1), abort_flag, err, 22)) goto done;
+          // entry offsets address the whole 128-row tile: rows 64.. start 8 KB before the half
+          const uint32_t tile = stage0 - hs[k] * HSUB;
+          zero_rows(tile, 2 * hs[k] + r, lane);
+          __syncwarp();
+          slot_scatter(sl[k], tile, lane);
+          fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&full[group]);
+          if (live && !fetch(sl[k], hs[k])) goto done;
+          (k ? more1 : more0) = live;
+        }
+      }
+    }
   } else if (warp < W_MMA) {
     // ---- epilogue: accumulators (hi + lo halves) -> partials ----
     const int q = warp & 3;
@@ -803,9 +825,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else if (warp == W_MMA) {
     // ---- MMA issuer ----
     if (lane == 0 && have_work) {
-      // descriptors formed once and advanced by constant offsets (see k_fwd_tc)
+      // descriptors formed once and advanced by constant offsets
       const uint32_t idesc = idesc_f16(128, N2, fmt, 1, 1);
-      const uint64_t adesc0 = sdesc_sw128(smem_u32(As), SUB, 1024);
+      const uint64_t adesc0 = sdesc_sw128(smem_u32(As), HSUB, 1024);
       const uint64_t qdesc0 = sdesc_sw128(smem_u32(Qs), TM * 128, 1024);
       uint32_t it = 0, ti = 0;
       bool ok = true;
@@ -817,19 +839,20 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         tc_fence_after();
         const uint64_t qd = qdesc0 + (uint64_t)(b * (Q_BYTES >> 4));
-        for (int sc = sc0; sc < sc1; ++sc, ++it) {
-          const int s = it % S;
+        for (int j = 0; j < 2 * nsc; ++j, ++it) {  // super-chunk j / 2, half tile j % 2
+          const int s = it % S, h = j & 1;
           if (!mbar_wait(&full[s], (it / S) & 1u, abort_flag, err, 26)) {
             ok = false;
             break;
           }
           tc_fence_after();
           const uint64_t ad = adesc0 + (uint64_t)(s * (A_BYTES >> 4));
-          const uint32_t d = tmem + (sc - sc0) * N2;
-          umma_f16(d, ad, qd, idesc, ti != 0);
+          const uint64_t qh = qd + (uint64_t)(h * (64 * 128 >> 4));  // cells 64 h.. of the image tile
+          const uint32_t d = tmem + (j >> 1) * N2;
+          umma_f16(d, ad, qh, idesc, (ti | h) != 0);
 #pragma unroll
-          for (int kk = 1; kk < TM / 16; ++kk)  // K steps of 16 cells: +2 KB down both operands
-            umma_f16(d, ad + 128 * kk, qd + 128 * kk, idesc, 1u);
+          for (int kk = 1; kk < 64 / 16; ++kk)  // K steps of 16 cells: +2 KB down both operands
+            umma_f16(d, ad + 128 * kk, qh + 128 * kk, idesc, 1u);
           umma_commit(&empty[s]);
         }
         if (!ok) break;
@@ -1225,7 +1248,6 @@ __global__ void k_split16_batch(const SplitTask* __restrict__ tasks, int64_t cou
 // them.
 // ---------------------------------------------------------------------------
 constexpr int kSwapFwdStages = 4;  // one chunk: the two tiles of a band and the chunk of the image
-constexpr int kSwapRegs = 8;       // entries a densify lane has in flight per stage (x 32 a warp)
 
 __host__ __device__ constexpr size_t fwd_swap_smem() {
   return 1024 + (size_t)kSwapFwdStages * (2 * (TM * CW * 2) + CW * 128 * 2) +
@@ -1343,12 +1365,8 @@ __device__ __forceinline__ void fwd_swap_body(const Src& src, int nc, int fmt) {
     const int group = warp >> 2, q = warp & 3;
     const int par = group >> 1, u = group & 1;
     const uint32_t tile0 = smem_u32(As + par * STAGE + u * TILE);
-    DenseSlot<kSwapRegs> sl[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-#pragma unroll
-      for (int r = 0; r < kSwapRegs; ++r) sl[k].w[r] = 0u;
-    }
+    DenseSlot<kDenseRegs> sl[2];
+    slots_init(sl);
     // cursor: the next segment to load
     int64_t band = blockIdx.x;
     uint32_t bi = 0;
@@ -1363,7 +1381,7 @@ __device__ __forceinline__ void fwd_swap_body(const Src& src, int nc, int fmt) {
       has = u < bd.tiles;
       return warp_wait(&mfull[bi & 1u], (bi >> 1) & 1u, abort_flag, err, 11);
     };
-    auto fetch = [&](DenseSlot<kSwapRegs>& x) {
+    auto fetch = [&](DenseSlot<kDenseRegs>& x) {
       while (c >= nc) {  // leave the band
         __syncwarp();
         if (lane == 0) mbar_arrive(&mempty[bi & 1u]);
@@ -1413,50 +1431,10 @@ __device__ __forceinline__ void fwd_swap_body(const Src& src, int nc, int fmt) {
     for (int64_t band = blockIdx.x; band < n_bands; band += gridDim.x, ++k) {
       const FwdBand bd = src.band(band);
       int* err = bd.err;
-      const int64_t n = bd.n;
-      const float mcj = __ldg(bd.mc + j);
-      uint16_t* Yimg = bd.Yimg;
-      float* Y = bd.Y;
       const uint32_t a = k & 1u, ph = (k >> 1) & 1u;
       if (!warp_wait(&acc_full[a], ph, abort_flag, err, 14)) goto done;
       tc_fence_after();
-      for (int u = 0; u < bd.tiles; ++u) {
-        const uint32_t tbase = tmem + ((32u * q) << 16) + a * 256 + u * 128;
-        const int64_t row0 = bd.row0 + u * TM;
-#pragma unroll 1
-        for (int cb = 0; cb < TM / 32; ++cb) {  // 32 cells per TMEM load
-          uint32_t r[32];
-          tmem_ld32(tbase + cb * 32, r);
-          tmem_wait_ld();
-          const int64_t c0 = row0 + cb * 32;
-          const int lim = (int)min((int64_t)32, n - c0);  // cells of this block inside the matrix
-          // word j of an image row holds (hi, lo) of column j; lane p handles
-          // cells 2 i + p.  Each lane gives the other the halves it does not
-          // need, one exchange for two cells, and the exchanges, conversions
-          // and stores of the block go in passes of their own: sixteen
-          // independent chains, where cell after cell would stall on each.
-          float v[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const float x0 = __uint_as_float(r[2 * i]), x1 = __uint_as_float(r[2 * i + 1]);
-            const float other = __shfl_xor_sync(0xffffffffu, p ? x0 : x1, 1);
-            v[i] = (p ? x1 : x0) + other - mcj;
-          }
-          const int left = lim - p;  // cell 2 i + p is inside the matrix iff 2 i < left
-          uint32_t* dst = reinterpret_cast<uint32_t*>(Yimg) + (c0 + p) * 64 + j;
-          uint32_t img[16];
-          hilo16_block(v, img, fmt);
-#pragma unroll
-          for (int i = 0; i < 16; ++i)
-            if (2 * i < left) dst[i * 128] = img[i];
-          if (Y) {
-            float* ydst = Y + (c0 + p) * LD + j;
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-              if (2 * i < left) ydst[i * 2 * LD] = v[i];
-          }
-        }
-      }
+      swap_tile_out<LD>(tmem + ((32u * q) << 16) + a * 256, bd.tiles, bd.row0, bd.n, bd.mc, j, p, bd.Y, bd.Yimg, fmt);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&acc_empty[a]);
@@ -1652,18 +1630,14 @@ __device__ __forceinline__ void rmat_swap_body(const RmatJob& job, int nc, int64
     const int h = warp >> 3, cofs = (warp >> 1) & 3, q = 2 * h + (warp & 1);
     // entry offsets address the whole 128-row tile: rows 64 h.. start 8 KB before the half
     const uint32_t tile0 = smem_u32(As + h * STAGE + cofs * HSUB) - h * HSUB;
-    DenseSlot<kSwapRegs> sl[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-#pragma unroll
-      for (int r = 0; r < kSwapRegs; ++r) sl[k].w[r] = 0u;
-    }
+    DenseSlot<kDenseRegs> sl[2];
+    slots_init(sl);
     // cursor: the next segment to load
     int jq = 0;
     uint32_t ti = 0;
     const uint32_t ntl = have_work ? (uint32_t)(t1 - t0) : 0u;
     bool live = true;
-    auto fetch = [&](DenseSlot<kSwapRegs>& x) {
+    auto fetch = [&](DenseSlot<kDenseRegs>& x) {
       if (jq == nq) {  // leave the tile
         __syncwarp();
         if (lane == 0) mbar_arrive(&mempty[ti & 1u]);
@@ -1842,11 +1816,12 @@ __global__ void __launch_bounds__(kThreads, 1)
 }
 
 size_t smem_tail() { return 2 * kMaxChunks * sizeof(SegMeta) + 64 * sizeof(uint64_t) + 64; }
-size_t fwd_smem(int LD) {
-  return 1024 + (size_t)fwd_stages(LD) * (TM * CW * 2) + (size_t)fwd_bslots(LD) * (2 * CW * LD * 2) + smem_tail();
+size_t fwd_smem(int LD) {  // metadata of two tiles a slot
+  return 1024 + (size_t)fwd_stages(LD) * (TM * CW * 2) + (size_t)fwd_bslots(LD) * (2 * CW * LD * 2) + smem_tail() +
+         2 * kMaxChunks * sizeof(SegMeta);
 }
 size_t rmat_smem(int LD) {
-  return 1024 + (size_t)rmat_stages(LD) * (2 * TM * CW * 2) + 4 * (size_t)TM * LD * 2 + smem_tail();
+  return 1024 + (size_t)rmat_stages(LD) * (TM * CW * 2) + 4 * (size_t)TM * LD * 2 + smem_tail();
 }
 
 }  // namespace

@@ -142,13 +142,17 @@ def test_tensor_core_embeddings_match_cuda_core_product(monkeypatch, n, nc, over
     assert np.abs(tc.embeddings - cc.embeddings).max() < 2e-3 * np.abs(cc.embeddings).max()
 
 
-@pytest.mark.parametrize("n,g,mode", [
-    (300, 64, "mixed_bf16"),       # one chunk, a last band of one ragged tile
-    (80000, 60, "mixed_f16"),      # one chunk, several bands per SM
-    (80111, 130, "mixed_bf16"),    # three chunks: the chunk counter's parity alternates from band to band
-    (20000, 1100, "mixed_bf16"),   # five quads of chunks, three gene groups
+@pytest.mark.parametrize("n,g,mode,k", [
+    (300, 64, "mixed_bf16", 20),       # one chunk, a last band of one ragged tile
+    (80000, 60, "mixed_f16", 20),      # one chunk, several bands per SM
+    (80111, 130, "mixed_bf16", 20),    # three chunks: the chunk counter's parity alternates from band to band
+    (20000, 1100, "mixed_bf16", 20),   # five quads of chunks, three gene groups
+    (300, 128, "mixed_f16", 100),      # ld 128: one tile per SM, one super-chunk
+    (60000, 64, "mixed_f16", 57),      # ld 64 at its widest, one chunk
+    (60111, 65, "mixed_bf16", 65),     # ld 128: bands of two tiles and a single one, half a super-chunk
+    (60111, 330, "mixed_f16", 128),    # three super-chunks, two gene groups
 ])
-def test_tc_quarters_of_every_size(n, g, mode):
+def test_tc_quarters_of_every_size(n, g, mode, k):
     """32 x 64 blocks that hold no entry, fewer and more than a warp's store
     takes (32) and than a lane keeps in flight (256 a warp), and all 2,048,
     next to one another in every order; the tolerance is the module's."""
@@ -171,9 +175,8 @@ def test_tc_quarters_of_every_size(n, g, mode):
     rows, cols = rows[order], cols[order].astype(np.int32)
     indptr = np.r_[0, np.cumsum(np.bincount(rows, minlength=n))]
     c = rpca.Csr(indptr, cols, rng.integers(1, 64, len(cols)).astype(np.float32) / 8, (n, g))  # exact in 16 bits
-    k = 20
     plan = accel.Plan(c.indptr, c.indices, c.data, c.shape, n_components=k, n_oversamples=0, math_mode=mode)
-    assert plan.ld == 64
+    assert plan.ld == (64 if k <= 64 else 128)
     mu = rpca.col_sums_and_sum_sq(c)[0] / n
     v = (rng.standard_normal((g, k)) / np.sqrt(g)).astype(np.float32)
     q = (rng.standard_normal((n, k)) / np.sqrt(n)).astype(np.float32)
