@@ -101,8 +101,11 @@ cudaError_t launch_normalize_log1p(const int64_t* indptr, const float* in, float
 // entries in row order, each warp compacting by ballot prefix.  The passes take
 // 256 and 128 entries of a row at a time (eight and four loads per lane in
 // flight), in blocks enough that the last wave is short: 114M entries, 38M
-// kept: check and count 171 us, fill 264 (1.2 GB, 71 % of the measured copy
-// rate), against 260 + 274 us and 564 us before.
+// kept: check and count 129 us, fill 264 (1.2 GB, 71 % of the measured copy
+// rate), against 260 + 274 us and 564 us before.  Pass 1 is bound by its
+// instructions: whole blocks go without a bounds check per entry, indices are
+// compared unsigned, and one sum carries the kept entries and those inside the
+// columns (171 us without; loading a row ahead of the one counted gave 158).
 // ---------------------------------------------------------------------------
 // Entries at or past `words` words of the table are dropped columns.
 template <bool SMEM>
@@ -128,6 +131,8 @@ struct KeptColumns {
   }
 };
 
+constexpr int64_t kCountStep = 1 << 20;  // entries a warp counts in 16 bits per lane
+
 template <bool SMEM>
 __global__ void __launch_bounds__(256) k_project_count(const int64_t* __restrict__ indptr,
                                                        const int32_t* __restrict__ idx, int64_t n, int64_t g,
@@ -141,25 +146,40 @@ __global__ void __launch_bounds__(256) k_project_count(const int64_t* __restrict
   const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   bool bad_ptr = false, bad_idx = false;
+  const uint32_t columns = (uint32_t)min(g, (int64_t)0x7FFFFFFF + 1);  // no int32 index lies past them
   for (int64_t row = warp; row < n; row += nwarps) {
     const int64_t s = indptr[row], e = indptr[row + 1];
-    int c = 0;
     int64_t total = 0;
     if (s < 0 || e < s || e > nnz) {
       bad_ptr = true;
     } else {
-      for (int64_t b = s; b < e; b += 256) {
-        int32_t j[8];
+      for (int64_t b = s; b < e; b += kCountStep) {  // once, but for a row of a million entries
+        const int len = (int)min(e - b, (int64_t)kCountStep);
+        const int32_t* from = idx + b + lane;
+        // kept entries in the low half of the sum, entries inside the columns in the high half
+        uint32_t c = 0;
+        auto count = [&](uint32_t j) {
+          if (j < columns) c += (cols.bits[j >> 5] >> (j & 31u) & 1u) | 0x10000u;
+        };
+        int o = 0;
+        for (; o + 256 <= len; o += 256) {
+          uint32_t j[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) j[u] = b + 32 * u + lane < e ? __ldg(idx + b + 32 * u + lane) : -1;
+          for (int u = 0; u < 8; ++u) j[u] = (uint32_t)__ldg(from + o + 32 * u);
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const bool in = j[u] >= 0 && (int64_t)j[u] < g;
-          bad_idx |= !in && b + 32 * u + lane < e;
-          if (in && cols.kept(j[u])) ++c;
+          for (int u = 0; u < 8; ++u) count(j[u]);
         }
+        uint32_t j[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (o + 32 * u < len) j[u] = o + 32 * u + lane < len ? (uint32_t)__ldg(from + o + 32 * u) : 0xFFFFFFFFu;
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (o + 32 * u < len) count(j[u]);
+        const uint32_t kept = __reduce_add_sync(0xffffffffu, c & 0xFFFFu);
+        bad_idx |= (int)__reduce_add_sync(0xffffffffu, c >> 16) != len;
+        total += kept;
       }
-      total = (int64_t)__reduce_add_sync(0xffffffffu, (unsigned)c);
     }
     if (lane == 0) counts[row] = total;
   }

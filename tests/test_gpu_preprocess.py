@@ -153,3 +153,26 @@ def test_producers_refuse_a_bad_csr():
                      lambda: accel.project_columns(ip, ix, vv, c.shape, [1, 5])):
             with pytest.raises(ScxPcaError, match=word):
                 call()
+
+
+def test_counts_of_rows_of_a_million_entries():
+    """Kept entries of rows that end around the most that is summed at once
+    (2^20), and an index one past the columns as the last of the longest: refused."""
+    from scx_b200._lib import ScxPcaError
+
+    lengths = [(1 << 20) - 1, 1 << 20, (1 << 20) + 1, (1 << 20) + 300]
+    g = max(lengths) + 40
+    rng = np.random.default_rng(g)
+    idx = np.concatenate([np.sort(rng.choice(g, m, replace=False)) for m in lengths]).astype(np.int32)
+    c = rpca.Csr(np.r_[0, np.cumsum(lengths)].astype(np.int64), idx, np.arange(len(idx), dtype=np.float32),
+                 (len(lengths), g))
+    cols = np.flatnonzero(rng.random(g) < 0.3)
+    keep = np.isin(idx, cols)
+    ip, ix, vv = _dev(c)
+    pip, pix, pvv, _ = accel.project_columns(ip, ix, vv, c.shape, cols)
+    np.testing.assert_array_equal(pip.cpu().numpy(), np.r_[0, np.cumsum(keep)][c.indptr])
+    np.testing.assert_array_equal(pix.cpu().numpy(), np.searchsorted(cols, idx[keep]))
+    np.testing.assert_array_equal(pvv.cpu().numpy(), c.data[keep])
+    ix[ix.numel() - 1] = g
+    with pytest.raises(ScxPcaError, match="column index"):
+        accel.project_columns(ip, ix, vv, c.shape, cols)
