@@ -1133,7 +1133,8 @@ void alloc_work_buffers(scxpca_plan* pl) {
   pl->Z.alloc(sizeof(double) * g * ld);
   pl->V.alloc(sizeof(float) * g * ld);
   pl->mc.alloc(sizeof(float) * ld);
-  pl->gpart.alloc(sizeof(double) * pl->gram_parts * (ld * ld + ld));
+  // partials of the cell-side Gram (num_sms), the gene-side one and a batch segment's (up to twice as many)
+  pl->gpart.alloc(sizeof(double) * 2 * pl->num_sms * (ld * ld + ld));
   pl->G.alloc(sizeof(double) * (ld * ld + ld));
   pl->R.alloc(sizeof(double) * ld * ld);
   pl->Rinv.alloc(sizeof(double) * ld * ld);
@@ -2899,7 +2900,8 @@ scxpca_batch* create_batch(const scxpca_csr* x, const int64_t* offsets, int64_t 
           1, std::min<int64_t>(pl->gram_parts_small, (2 * pl->num_sms + n_segments - 1) / n_segments));
       if (pl->use_tc && !pl->streaming) {
         pl->tc_row_groups = (int)std::max<int64_t>(1, std::min<int64_t>(pl->tc_row_groups, (pl->n + 2047) / 2048));
-        pl->tc_gram_parts = (int)std::max<int64_t>(1, (pl->n + 1023) / 1024);  // eight row tiles each
+        // eight row tiles each, as many as gpart holds
+        pl->tc_gram_parts = (int)std::max<int64_t>(1, std::min<int64_t>(2 * pl->num_sms, (pl->n + 1023) / 1024));
       }
     }
     b->seg_ms.assign(n_segments, 1.0);

@@ -133,3 +133,29 @@ def test_lockstep_tensor_core_products_ld64(branches):
                                   True, om)
         rel = np.abs(sv_g[s] - ref["singular_values"]) / ref["singular_values"]
         assert rel.max() < 1e-4, (s, rel.max())
+
+
+def test_batch_with_large_segments():
+    """Segments of more than 148 and more than 296 Gram ranges of 1,024 cells: the
+    partials stay inside their buffer, and each segment matches the FP64 oracle
+    on its (BF16-exact) values with the same test matrix."""
+    import torch
+
+    sizes, g, per, nc, over = (160_000, 310_000, 500), 40, 5, 10, 10
+    offs = np.r_[0, np.cumsum(sizes)]
+    n = int(offs[-1])
+    rng = np.random.default_rng(3)
+    ix = ((rng.integers(0, 8, (n, 1)) + 8 * np.arange(per)) % g).astype(np.int32).ravel()
+    vv = rng.integers(1, 17, n * per).astype(np.float32)
+    ip = np.arange(n + 1, dtype=np.int64) * per
+    om = rpca.gaussian_omega(g, nc + over, 4)
+    b = accel.Batch(torch.from_numpy(ip).cuda(), torch.from_numpy(ix).cuda(),
+                    torch.from_numpy(vv).cuda().to(torch.bfloat16), (n, g), offs, n_components=nc,
+                    n_oversamples=over, n_power_iterations=2, seed=4, math_mode="mixed_bf16",
+                    branches=-1)
+    _, _, sv, _, _ = b.run()
+    b.close()
+    for q, (lo, hi) in enumerate(zip(offs[:-1], offs[1:])):
+        c = rpca.Csr(ip[lo:hi + 1] - lo * per, ix[lo * per:hi * per], vv[lo * per:hi * per], (int(hi - lo), g))
+        ref = rpca.randomized_pca(c, nc, over, 2, True, om)
+        np.testing.assert_allclose(sv[q], ref["singular_values"], rtol=1e-4)
