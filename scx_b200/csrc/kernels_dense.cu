@@ -605,10 +605,15 @@ __device__ __forceinline__ TallBatch tall_batch(const TallTask* tasks, int ntask
                    (int64_t)(blockIdx.x + 1) * total_tiles / gridDim.x};
 }
 
-template <int OUTB, class Src>
+// NT threads, thread (ty, tx) of NT / 16 x 16 taking rows ty + NT / 16 i and
+// four columns of every 64.  UPPER: M is upper triangular, so columns 64 h ..
+// need its rows below 64 (h + 1) only.  At OUTB 128 one block fills an SM's
+// shared memory and needs 16 warps to keep the FMAs fed (120,000 x 128 by
+// 128 x 128: 256 threads 138 us; 512 threads 123, and 112 with an upper M).
+template <int OUTB, int NT, bool UPPER, class Src>
 __device__ __forceinline__ void tall_mm_body(const Src& src, int K, int ldi, int ldm, int cnt, int ldo, int fmt) {
   constexpr int H = OUTB / 64;
-  constexpr int RPT = kTallRows / 16;  // rows per thread
+  constexpr int RS = NT / 16, RPT = kTallRows / RS;  // rows per thread
   extern __shared__ __align__(16) float sm_f[];
   const int KP = K + 4;
   float* Ms = sm_f;  // [K][OUTB]
@@ -654,32 +659,36 @@ __device__ __forceinline__ void tall_mm_body(const Src& src, int K, int ldi, int
     for (int i = 0; i < RPT; ++i)
 #pragma unroll
       for (int o = 0; o < 4 * H; ++o) acc[i][o] = 0.f;
-    for (int l = 0; l < K; l += 4) {
-      float4 a[RPT];
+    auto terms = [&](int l0, int l1, auto first) {  // rows l0 .. l1 - 1 of M, its columns from 64 first on
+      for (int l = l0; l < l1; l += 4) {
+        float4 a[RPT];
 #pragma unroll
-      for (int i = 0; i < RPT; ++i) a[i] = *reinterpret_cast<const float4*>(T + (ty + 16 * i) * KP + l);
+        for (int i = 0; i < RPT; ++i) a[i] = *reinterpret_cast<const float4*>(T + (ty + RS * i) * KP + l);
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < 4; ++u) {
 #pragma unroll
-        for (int h = 0; h < H; ++h) {
-          const float4 m = *reinterpret_cast<const float4*>(Ms + (l + u) * OUTB + 64 * h + 4 * tx);
+          for (int h = decltype(first)::value; h < H; ++h) {
+            const float4 m = *reinterpret_cast<const float4*>(Ms + (l + u) * OUTB + 64 * h + 4 * tx);
 #pragma unroll
-          for (int i = 0; i < RPT; ++i) {
-            const float x = u == 0 ? a[i].x : u == 1 ? a[i].y : u == 2 ? a[i].z : a[i].w;
-            acc[i][4 * h + 0] = fmaf(x, m.x, acc[i][4 * h + 0]);
-            acc[i][4 * h + 1] = fmaf(x, m.y, acc[i][4 * h + 1]);
-            acc[i][4 * h + 2] = fmaf(x, m.z, acc[i][4 * h + 2]);
-            acc[i][4 * h + 3] = fmaf(x, m.w, acc[i][4 * h + 3]);
+            for (int i = 0; i < RPT; ++i) {
+              const float x = u == 0 ? a[i].x : u == 1 ? a[i].y : u == 2 ? a[i].z : a[i].w;
+              acc[i][4 * h + 0] = fmaf(x, m.x, acc[i][4 * h + 0]);
+              acc[i][4 * h + 1] = fmaf(x, m.y, acc[i][4 * h + 1]);
+              acc[i][4 * h + 2] = fmaf(x, m.z, acc[i][4 * h + 2]);
+              acc[i][4 * h + 3] = fmaf(x, m.w, acc[i][4 * h + 3]);
+            }
           }
         }
       }
-    }
+    };
+    terms(0, UPPER && H == 2 ? 64 : K, std::integral_constant<int, 0>{});
+    if constexpr (UPPER && H == 2) terms(64, K, std::integral_constant<int, 1>{});
     const int64_t r0 = (tile - tk.tile0) * kTallRows;
     float* Out = tk.Out;
     uint16_t* img = tk.img;
 #pragma unroll
     for (int i = 0; i < RPT; ++i) {
-      const int64_t row = r0 + ty + 16 * i;
+      const int64_t row = r0 + ty + RS * i;
       if (row >= tk.n) continue;
 #pragma unroll
       for (int h = 0; h < H; ++h) {
@@ -712,19 +721,19 @@ __device__ __forceinline__ void tall_mm_body(const Src& src, int K, int ldi, int
   asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-template <int OUTB>
-__global__ void __launch_bounds__(256, 2) k_tall_mm(const float* In, int64_t n, int K, int ldi,
-                                                    const float* __restrict__ M, int ldm, int cnt, float* Out,
-                                                    int ldo, uint16_t* __restrict__ img, int fmt) {
-  tall_mm_body<OUTB>(TallOne{TallTask{In, Out, img, M, n, 0}, (n + kTallRows - 1) / kTallRows}, K, ldi, ldm, cnt,
-                     ldo, fmt);
+template <int OUTB, int NT, bool UPPER>
+__global__ void __launch_bounds__(NT, NT == 256 ? 2 : 1)
+    k_tall_mm(const float* In, int64_t n, int K, int ldi, const float* __restrict__ M, int ldm, int cnt, float* Out,
+              int ldo, uint16_t* __restrict__ img, int fmt) {
+  tall_mm_body<OUTB, NT, UPPER>(TallOne{TallTask{In, Out, img, M, n, 0}, (n + kTallRows - 1) / kTallRows}, K, ldi,
+                                ldm, cnt, ldo, fmt);
 }
 
 template <int OUTB>
 __global__ void __launch_bounds__(256, 2) k_tall_mm_batch(const TallTask* __restrict__ tasks, int ntasks,
                                                           int64_t total_tiles, int K, int ldi, int ldm, int cnt,
                                                           int ldo, int fmt) {
-  tall_mm_body<OUTB>(tall_batch(tasks, ntasks, total_tiles), K, ldi, ldm, cnt, ldo, fmt);
+  tall_mm_body<OUTB, 256, false>(tall_batch(tasks, ntasks, total_tiles), K, ldi, ldm, cnt, ldo, fmt);
 }
 
 // ---------------------------------------------------------------------------
@@ -892,24 +901,24 @@ cudaError_t launch_embed_batch(const TallTask* tasks, int ntasks, int64_t total_
   return cudaGetLastError();
 }
 
+// upper: M is upper triangular (told apart at more than 64 columns only).
 static cudaError_t tall_mm(const float* In, int64_t n, int K, int ldi, const float* M, int ldm, int cnt,
                            float* Out, int ldo, uint16_t* img, int fmt, cudaStream_t st,
-                           int num_sms) {
+                           int num_sms, bool upper = false) {
   if (n == 0) return cudaSuccess;
   if ((K & 3) || (ldi & 3)) return cudaErrorInvalidValue;
   const int outb = cnt <= 64 ? 64 : 128;
   const size_t smem = ((size_t)K * outb + 2 * (size_t)kTallRows * (K + 4)) * sizeof(float);
-  const int per_sm = (int)std::max<size_t>(1, std::min<size_t>(2, (220 * 1024) / smem));
+  const int per_sm = outb == 64 ? (int)std::max<size_t>(1, std::min<size_t>(2, (220 * 1024) / smem)) : 1;
   const int grid = grid_for(n, kTallRows, num_sms, per_sm);
-  note_launches(1);
-  if (outb == 64) {
-    if (cudaError_t e = allow_smem(k_tall_mm<64>, smem); e != cudaSuccess) return e;
-    k_tall_mm<64><<<grid, 256, smem, st>>>(In, n, K, ldi, M, ldm, cnt, Out, ldo, img, fmt);
-  } else {
-    if (cudaError_t e = allow_smem(k_tall_mm<128>, smem); e != cudaSuccess) return e;
-    k_tall_mm<128><<<grid, 256, smem, st>>>(In, n, K, ldi, M, ldm, cnt, Out, ldo, img, fmt);
-  }
-  return cudaGetLastError();
+  auto go = [&](auto kern, int threads) {
+    if (cudaError_t e = allow_smem(kern, smem); e != cudaSuccess) return e;
+    note_launches(1);
+    kern<<<grid, threads, smem, st>>>(In, n, K, ldi, M, ldm, cnt, Out, ldo, img, fmt);
+    return cudaGetLastError();
+  };
+  if (outb == 64) return go(k_tall_mm<64, 256, false>, 256);
+  return upper ? go(k_tall_mm<128, 512, true>, 512) : go(k_tall_mm<128, 512, false>, 512);
 }
 
 cudaError_t launch_apply_right_f32(const float* In, int64_t n, int ld, const float* M, float* Out,
@@ -924,14 +933,14 @@ cudaError_t launch_apply_right_f32(const float* In, int64_t n, int ld, const flo
     return cudaSuccess;
   }
   if (ld == 64) return tall_mm_upper64(In, n, M, Out, nullptr, 0, st, num_sms);
-  return tall_mm(In, n, ld, ld, M, ld, ld, Out, ld, nullptr, 0, st, num_sms);
+  return tall_mm(In, n, ld, ld, M, ld, ld, Out, ld, nullptr, 0, st, num_sms, true);
 }
 
 cudaError_t launch_apply_right_split(const float* In, int64_t n, int ld, const float* M, float* Out,
                                      uint16_t* img, int fmt, cudaStream_t st, int num_sms) {
   if (ld > kMaxK) return cudaErrorInvalidValue;  // the 16-bit image belongs to the tensor-core path (ld <= 128)
   if (ld == 64) return tall_mm_upper64(In, n, M, Out, img, fmt, st, num_sms);
-  return tall_mm(In, n, ld, ld, M, ld, ld, Out, ld, img, fmt, st, num_sms);
+  return tall_mm(In, n, ld, ld, M, ld, ld, Out, ld, img, fmt, st, num_sms, true);
 }
 
 // ---------------------------------------------------------------------------
