@@ -147,10 +147,12 @@ __device__ __forceinline__ float4 lds128(unsigned addr) {
 // position order; with LIMIT it stops at the first entry whose row is not in
 // the table (idx[p] >= j0 + rows; the list is sorted).  Returns where it
 // stopped.  `tab` is the shared address of the lane's first piece of row 0.
-// Entries of a step that are not the list's read the row of zeros behind the
-// table, so a step is the same instructions for a full and for a ragged one
-// and the lists of a warp stay together.  (Indices are validated when
-// the plan is built; one that is out of range reads that row as well.)
+// Entries of a step that are not the list's count as zeros and read the row of
+// zeros behind the table, so a step is the same instructions for a full and for
+// a ragged one and the lists of a warp stay together.  (Their values are cleared
+// too: a neighbouring list's may be an infinity, where a finite value does not
+// fit the 16-bit working type.  Indices are validated when the plan is built;
+// one that is out of range reads that row as well.)
 template <bool VEC, bool LIMIT, int NV, typename IdxT, typename ValT>
 __device__ __forceinline__ int64_t walk(float (&acc)[4 * NV], const IdxT* __restrict__ idx,
                                         const ValT* __restrict__ val, int64_t s, int64_t e, int64_t lim, int j0,
@@ -168,7 +170,7 @@ __device__ __forceinline__ int64_t walk(float (&acc)[4 * NV], const IdxT* __rest
   }
   while (true) {
     Oct<IdxT> cj = j1;
-    const Oct<ValT> cx = x1;
+    Oct<ValT> cx = x1;
     j1 = j2;
     x1 = x2;
     const int64_t left = e - p;  // entries from the step's first position to the list's end
@@ -191,7 +193,10 @@ __device__ __forceinline__ int64_t walk(float (&acc)[4 * NV], const IdxT* __rest
     if (valid != 0xffu) {
 #pragma unroll
       for (int u = 0; u < 8; ++u)
-        if (!(valid >> u & 1)) cj.v[u] = (IdxT)(j0 + rows);
+        if (!(valid >> u & 1)) {
+          cj.v[u] = (IdxT)(j0 + rows);
+          cx.v[u] = from_f32<ValT>(0.f);
+        }
     }
 #pragma unroll
     for (int half = 0; half < 8; half += 4) {

@@ -220,3 +220,51 @@ def test_strict_products_across_tables(n, g, k):
     z_ref = rpca.spmm_transpose(c, q.astype(np.float64), mu)
     assert np.linalg.norm(got[0][0] - y_ref) / np.linalg.norm(y_ref) < OP_RTOL
     assert np.linalg.norm(got[0][1] - z_ref) / np.linalg.norm(z_ref) < OP_RTOL
+
+
+@pytest.mark.parametrize("n,g,k", [
+    (300, 70, 20),      # 32-column blocks
+    (38016, 260, 60),   # 64-column blocks
+    (500, 1700, 30),    # V in two gene chunks
+])
+@pytest.mark.parametrize("offset", [0, 1])  # the index array at a vector boundary and off it
+def test_overflowed_values_stay_in_their_row_and_gene(n, g, k, offset, monkeypatch):
+    """A value that does not fit the 16-bit working type is an infinity there.
+    It belongs to the sums of its own row and gene: every other row of P V and
+    gene of P^T Q is the FP64 product of the rounded values, within the FP32
+    sums of this file."""
+    import torch
+
+    monkeypatch.setenv("SCXPCA_TC", "0")  # 16-bit values on the CUDA cores
+    c = _csr(n, g, seed=7)
+    data = c.data.copy()
+    length = np.diff(c.indptr)
+    rows = [r for r in (3, n // 2, n - 4) if length[r] > 0]
+    ends = [c.indptr[r] for r in rows] + [c.indptr[r + 1] - 1 for r in rows]  # beside the rows before and behind
+    data[ends] = 1e5
+    genes = np.unique(c.indices[ends])
+    ok_rows, ok_genes = np.ones(n, dtype=bool), np.ones(g, dtype=bool)
+    ok_rows[rows], ok_genes[genes] = False, False
+    with np.errstate(over="ignore"):
+        rounded = data.astype(np.float16)
+    d = rpca.Csr(c.indptr, c.indices, np.where(np.isfinite(rounded), rounded, 0).astype(np.float32), c.shape)
+    ix = torch.zeros(len(c.indices) + offset, dtype=torch.int32, device="cuda")
+    ix[offset:] = torch.from_numpy(c.indices).cuda()
+    ip, vv = torch.from_numpy(c.indptr).cuda(), torch.from_numpy(data).cuda()
+    rng = np.random.default_rng(5)
+    v = rng.standard_normal((g, k)).astype(np.float32)
+    q = rng.standard_normal((n, k)).astype(np.float32)
+    y_ref = rpca.spmm_forward(d, v.astype(np.float64), None)
+    for center in (False, True):
+        torch.cuda.synchronize()
+        plan = accel.Plan(ip, ix[offset:], vv, c.shape, n_components=k, n_oversamples=0, math_mode="mixed_f16",
+                          zero_center=center)
+        z = plan.rmatmat(torch.from_numpy(q).cuda()).cpu().numpy()
+        mu = rpca.col_sums_and_sum_sq(d)[0] / n if center else None
+        z_ref = rpca.spmm_transpose(d, q.astype(np.float64), mu)
+        assert np.linalg.norm((z - z_ref)[ok_genes]) / np.linalg.norm(z_ref[ok_genes]) < OP_RTOL
+        if not center:  # (the mean of an overflowed gene is infinite, and so is a centred product)
+            y = plan.matmat(torch.from_numpy(v).cuda()).cpu().numpy().astype(np.float64)
+            assert np.linalg.norm((y - y_ref)[ok_rows]) / np.linalg.norm(y_ref[ok_rows]) < OP_RTOL
+            assert not np.isfinite(y[rows]).any()
+        plan.close()
