@@ -19,95 +19,118 @@ namespace scx {
 // bit-identical from run to run.  Restates ScxCsr::col_sums_and_sum_sq
 // (scx-sparse/src/csr.rs:570-580).
 //
-// Warp b of the partition owns the stored entries [b * per, (b + 1) * per) and
-// one FP64 accumulator pair per gene in shared memory, and walks its entries 32
-// at a time; no other warp touches its accumulators, so there are no atomics
-// and no barriers.  Inside one 32-entry step two lanes may name the same gene
-// only across a row boundary (a sorted row holds a gene once); the step is cut
-// into runs of strictly increasing gene index, applied one after another in
-// lane order.  Every gene's adds therefore happen in entry order, whatever the
-// rows look like (unsorted rows and duplicates included).  Genes beyond the
-// shared-memory accumulators take further passes over the warp's entries,
-// kStatsPassGenes at a time.  Each warp writes one partial row pair
+// Part b of the partition owns the stored entries [b * per, (b + 1) * per) and
+// one FP64 accumulator pair per gene in shared memory.  A warp walks the part's
+// entries 32 at a time; where few parts fit an SM, several warps walk the same
+// part, each adding its own range of the genes.  No two warps touch one
+// accumulator, so there are no atomics and no barriers.  Inside one 32-entry
+// step two lanes may name the same gene only across a row boundary (a sorted row
+// holds a gene once); the step is cut into runs of strictly increasing gene
+// index, applied one after another in lane order.  Every gene's adds therefore
+// happen in entry order, whatever the rows look like (unsorted rows and
+// duplicates included) and however many warps share the part.  Genes beyond the
+// shared-memory accumulators take further passes over the part's entries, of at
+// most kStatsPassGenes genes each.  Each part writes one partial row pair
 // [sum | sum sq] (n_vars each); reduce_rows_f64 adds the partials in order.
 //
-// What bounds it is the latency of a step's read-modify-write of 32 scattered
-// 16-byte pairs.  As many warps run on an SM as have room for their own
-// accumulators (6 at 2,000 genes); a warp takes two steps at once where their 64
-// genes increase, so their updates cannot meet (most pairs: a row has some 190
-// entries), and loads eight steps ahead, as stored (a conversion in the load
-// would wait for it).  92M entries: 366 us FP32, 373 BF16, against 825 and 912
-// for one accumulator set per block, its genes dealt to four warps through a
-// bucket sort of every 1,024-entry window.  (One step at a time: 526.)
+// What bounds it is latency: of a step's read-modify-write of 32 scattered
+// 16-byte pairs, and of the loads when few warps run.  As many parts run on an
+// SM as have room for their accumulators (6 at 2,000 genes); a warp takes two
+// steps at once where their 64 genes increase, so their updates cannot meet
+// (most pairs: a row has some 190 entries), and loads eight steps ahead, as
+// stored (a conversion in the load would wait for it).  92M entries: 366 us
+// FP32, 373 BF16, against 825 and 912 for one accumulator set per block, its
+// genes dealt to four warps through a bucket sort of every 1,024-entry window.
+// (One step at a time: 526.)
+//
+// Above 4,266 genes at most two parts fit.  Their warps are made up to
+// kStatsLeast by ranges and load sixteen steps ahead, and there are four parts
+// per SM, in turn, so that a piece of an upload still fills half of the SMs.
+// 46M entries, one warp a part and eight steps against this: 8,000 genes 850 ->
+// 660 us, 12,800 855 -> 656, 30,000 2,468 -> 1,627 (the bucket sort: 1,071,
+// 1,608, 2,146); a plan from host memory at 30,000 genes 39.2 -> 29.3 ms
+// (the bucket sort 37.3).  Ranges without the longer loads gain nothing, the
+// loads alone 17 % at 30,000 genes and nothing at 12,800; with three parts an
+// SM neither gains.
 // ---------------------------------------------------------------------------
-constexpr int kStatsMaxWarps = 16;  // warps (parts) of a block
-constexpr int kStatsAhead = 8;      // 32-entry steps a warp loads at once, before it needs them
+constexpr int kStatsMaxWarps = 16;  // warps of a block
 constexpr int kStatsPassGenes = (int)(kStatsSmemMax / 16);
+constexpr int kStatsLeast = 4;      // warps of a block whose parts are shared
+constexpr int kStatsOwn = 3;        // parts of a block from which on each has one warp
 
-// Warps whose accumulators fit an SM's shared memory.
-static int stats_warps(int64_t g) {
+// Parts whose accumulators fit an SM's shared memory.
+static int stats_sets(int64_t g) {
   const int64_t pass = std::min<int64_t>(std::max<int64_t>(g, 1), kStatsPassGenes);
   return (int)std::min<int64_t>(kStatsMaxWarps, (int64_t)kStatsSmemMax / (16 * pass));
 }
 
-int col_stats_parts(int64_t g, int num_sms) { return num_sms * stats_warps(g); }
+int col_stats_parts(int64_t g, int num_sms) {
+  const int sets = stats_sets(g);
+  return num_sms * (sets >= kStatsOwn ? sets : 4);
+}
 
-template <typename ValT>
-__global__ void __launch_bounds__(kStatsMaxWarps * 32) k_col_stats(const int32_t* __restrict__ idx,
-                                                                   const ValT* __restrict__ val, int64_t nnz,
-                                                                   int32_t g, int32_t pass_genes, int nparts,
-                                                                   int part0, int part1, double* __restrict__ partial) {
-  extern __shared__ __align__(16) double2 stats_sm[];  // [warps][pass_genes]
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+// SHARED: `ranges` warps walk a part, and a step may hold none of a warp's genes.
+template <typename ValT, bool SHARED>
+__global__ void __launch_bounds__(SHARED ? kStatsLeast * 32 : kStatsMaxWarps * 32)
+    k_col_stats(const int32_t* __restrict__ idx, const ValT* __restrict__ val, int64_t nnz, int32_t g,
+                int32_t pass_genes, int ranges, int nparts, int part0, int part1, double* __restrict__ partial) {
+  constexpr int AHEAD = SHARED ? 16 : 8;  // 32-entry steps a warp loads at once, before it needs them
+  extern __shared__ __align__(16) double2 stats_sm[];  // [parts of the block][pass_genes]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, set = warp / ranges, range = warp % ranges;
   const unsigned lanemask_le = 0xffffffffu >> (31 - lane);
   // this launch runs parts part0 .. part1 - 1 of the partition
-  const int b = part0 + (int)blockIdx.x * warps + warp;
+  const int b = part0 + (int)blockIdx.x * ((int)(blockDim.x >> 5) / ranges) + set;
   if (b >= part1) return;
-  double2* acc = stats_sm + (int64_t)warp * pass_genes;
+  double2* acc = stats_sm + (int64_t)set * pass_genes;
   const int64_t per = (nnz + nparts - 1) / nparts;
   const int64_t s = min(nnz, (int64_t)b * per);
   const int64_t e = min(nnz, s + per);
   double* out = partial + (int64_t)b * 2 * g;
   for (int32_t lo = 0; lo < g; lo += pass_genes) {
     const int32_t gp = min(pass_genes, g - lo);
-    for (int i = lane; i < gp; i += 32) acc[i] = make_double2(0.0, 0.0);
-    int32_t nj[kStatsAhead];
-    ValT nx[kStatsAhead];
+    // the warp's genes of this pass, lo + [i0, i1): the same accumulators in
+    // every pass, as the part's other warps may be a pass behind
+    const int32_t i0 = min(gp, pass_genes * range / ranges), i1 = min(gp, pass_genes * (range + 1) / ranges);
+    for (int i = i0 + lane; i < i1; i += 32) acc[i] = make_double2(0.0, 0.0);
+    int32_t nj[AHEAD];
+    ValT nx[AHEAD];
     auto load = [&](int64_t w) {
 #pragma unroll
-      for (int u = 0; u < kStatsAhead; ++u) {
+      for (int u = 0; u < AHEAD; ++u) {
         const int64_t p = w + 32 * u + lane;
         nj[u] = p < e ? __ldg(idx + p) : INT32_MAX;
         nx[u] = p < e ? val[p] : ValT();
       }
     };
-    auto in_pass = [&](int32_t j) { return j >= lo && j - lo < gp; };  // (an index out of range is in no pass)
+    // (an index out of range is no warp's)
+    auto in_range = [&](int32_t j) { return j >= lo + i0 && j - lo < i1; };
     auto add = [](double2& a, double x) {
       a.x += x;
       a.y += x * x;
     };
     load(s);
     __syncwarp();  // the accumulators are zeroed
-    for (int64_t w0 = s; w0 < e; w0 += 32 * kStatsAhead) {
-      int32_t cj[kStatsAhead];
-      double cx[kStatsAhead];
-      unsigned starts[kStatsAhead];  // lanes whose gene is not above the lane before's
-      bool follows[kStatsAhead];     // the step's first gene is above the last one of the step before
+    for (int64_t w0 = s; w0 < e; w0 += 32 * AHEAD) {
+      int32_t cj[AHEAD];
+      double cx[AHEAD];
+      unsigned starts[AHEAD];  // lanes whose gene is not above the lane before's
+      bool follows[AHEAD];     // the step's first gene is above the last one of the step before
 #pragma unroll
-      for (int u = 0; u < kStatsAhead; ++u) {
+      for (int u = 0; u < AHEAD; ++u) {
         cj[u] = nj[u];
         cx[u] = (double)to_f32(nx[u]);
       }
-      load(w0 + 32 * kStatsAhead);
+      load(w0 + 32 * AHEAD);
 #pragma unroll
-      for (int u = 0; u < kStatsAhead; ++u) {
+      for (int u = 0; u < AHEAD; ++u) {
         const int32_t jl = __shfl_up_sync(0xffffffffu, cj[u], 1);
         starts[u] = __ballot_sync(0xffffffffu, lane > 0 && cj[u] != INT32_MAX && cj[u] <= jl);
         follows[u] = u > 0 && __shfl_sync(0xffffffffu, cj[u], 0) > __shfl_sync(0xffffffffu, cj[u ? u - 1 : 0], 31);
       }
 #pragma unroll
-      for (int u = 0; u < kStatsAhead; u += 2) {
-        const bool in0 = in_pass(cj[u]), in1 = in_pass(cj[u + 1]);
+      for (int u = 0; u < AHEAD; u += 2) {
+        const bool in0 = in_range(cj[u]), in1 = in_range(cj[u + 1]);
+        if (SHARED && !__any_sync(0xffffffffu, in0 || in1)) continue;
         if (starts[u] == 0 && starts[u + 1] == 0 && follows[u + 1]) {
           // 64 increasing genes: the two steps' updates do not meet
           double2 a0, a1;
@@ -139,7 +162,7 @@ __global__ void __launch_bounds__(kStatsMaxWarps * 32) k_col_stats(const int32_t
         }
       }
     }
-    for (int i = lane; i < gp; i += 32) {
+    for (int i = i0 + lane; i < i1; i += 32) {
       out[lo + i] = acc[i].x;
       out[g + lo + i] = acc[i].y;
     }
@@ -536,17 +559,21 @@ static cudaError_t col_stats_blocks_t(const int32_t* idx, const void* val, int64
                                       int nparts, int part0, int count, cudaStream_t st, int num_sms) {
   if (count <= 0) return cudaSuccess;
   const ValT* v = static_cast<const ValT*>(val);
-  const int32_t pass_genes = std::min<int32_t>(g, kStatsPassGenes);
-  // one block per SM, of as few warps as spread the parts over all of them
-  const int warps = std::max(1, std::min(stats_warps(g), (count + num_sms - 1) / num_sms));
-  const size_t smem = (size_t)warps * pass_genes * sizeof(double2);
-  if (smem > 48 * 1024) {
-    if (cudaError_t e = allow_smem(k_col_stats<ValT>, smem); e != cudaSuccess) return e;
-  }
-  k_col_stats<ValT><<<(count + warps - 1) / warps, warps * 32, smem, st>>>(idx, v, nnz, g, pass_genes, nparts, part0,
-                                                                          part0 + count, partial);
-  note_launches(1);
-  return cudaGetLastError();
+  const int32_t passes = std::max(1, (int32_t)(((int64_t)g + kStatsPassGenes - 1) / kStatsPassGenes));
+  const int32_t pass_genes = (g + passes - 1) / passes;
+  // one block per SM, of as few parts as spread them over all SMs
+  const int sets = std::max(1, std::min(stats_sets(g), (count + num_sms - 1) / num_sms));
+  const int ranges = sets >= kStatsOwn ? 1 : kStatsLeast / sets;
+  const size_t smem = (size_t)sets * pass_genes * sizeof(double2);
+  auto go = [&](auto kern) {
+    if (smem > 48 * 1024)
+      if (cudaError_t e = allow_smem(kern, smem); e != cudaSuccess) return e;
+    note_launches(1);
+    kern<<<(count + sets - 1) / sets, sets * ranges * 32, smem, st>>>(idx, v, nnz, g, pass_genes, ranges, nparts,
+                                                                      part0, part0 + count, partial);
+    return cudaGetLastError();
+  };
+  return ranges == 1 ? go(k_col_stats<ValT, false>) : go(k_col_stats<ValT, true>);
 }
 
 int64_t col_stats_block_begin(int64_t nnz, int nparts, int b) {

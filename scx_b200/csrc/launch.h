@@ -16,7 +16,7 @@ namespace scx {
 void note_launches(int n);
 int64_t launches_total();
 
-constexpr size_t kStatsSmemMax = 200 * 1024;  // per-block FP64 gene accumulators
+constexpr size_t kStatsSmemMax = 200 * 1024;  // FP64 gene accumulators of a block
 constexpr int kTransposeGeneBlock = 256;       // genes per block, CUDA-core transposed product
 
 // ---- sparse side (kernels_sparse.cu) ----
@@ -25,7 +25,7 @@ constexpr int kTransposeGeneBlock = 256;       // genes per block, CUDA-core tra
 cudaError_t launch_col_stats(int dtype, const int32_t* idx, const void* val, int64_t nnz,
                              int32_t g, double* partial, int nparts, double* out,
                              cudaStream_t st, int num_sms, int accumulate = 0);
-// Parts that fill the device: as many warps per SM as hold their own accumulators.
+// Parts that fill the device: as many per SM as hold their own accumulators, four of wide matrices.
 int col_stats_parts(int64_t g, int num_sms);
 // The same statistics in two halves: parts [part0, part0 + count) of the
 // partition write their partials (part b reads entries

@@ -65,3 +65,33 @@ def test_col_stats_orders(kind, g, dtype):
         _lib.check(lib.scxpca_col_stats_noalloc(0, C.byref(x), C.c_void_p(out.data_ptr()), None, err, len(err)), err)
         got = out.cpu().numpy()
     assert np.all(np.abs(got - want) <= RTOL * np.maximum(mag, 1e-300))
+
+
+@pytest.mark.parametrize("g", [3200, 3201, 4267, 6400, 6401, 12801, 30011])
+def test_col_stats_of_wide_matrices(g):
+    """Widths around those where fewer parts fit an SM and several warps share
+    one, each with its own genes: a plan's sums, and the means of the same
+    matrix uploaded from the host, whose statistics run in pieces and have the
+    bits of one launch."""
+    import torch
+
+    from scx_b200 import accel
+
+    rng = np.random.default_rng(g)
+    rows = _rows("sorted", g, rng) + [np.arange(g), np.arange(0, g, 7), np.arange(g)[-40:]]
+    idx = np.concatenate(rows).astype(np.int32)
+    indptr = np.r_[0, np.cumsum([len(r) for r in rows])].astype(np.int64)
+    val = rng.standard_normal(len(idx)).astype(np.float32)
+    v64 = val.astype(np.float64)
+    want = np.r_[np.bincount(idx, weights=v64, minlength=g), np.bincount(idx, weights=v64 * v64, minlength=g)]
+    mag = np.r_[np.bincount(idx, weights=np.abs(v64), minlength=g), want[g:]]
+    on_device = [torch.from_numpy(a).cuda() for a in (indptr, idx, val)]
+    torch.cuda.synchronize()
+    means = []
+    for csr in (on_device, (indptr, idx, val)):
+        plan = accel.Plan(*csr, (len(rows), g), n_components=2, n_oversamples=0, n_power_iterations=0)
+        got = np.concatenate(plan.col_stats())
+        assert np.all(np.abs(got - want) <= RTOL * np.maximum(mag, 1e-300))
+        means.append(plan.run().mean)
+        plan.close()
+    assert np.array_equal(means[0], means[1])
