@@ -7,7 +7,7 @@
 // cudaMalloc/cudaFree would add implicit device-wide synchronisation between
 // their streams.  scxpca_col_stats_noalloc serves them: the caller passes the
 // device CSR and the device output, and the only scratch the computation
-// needs -- the per-block partial sums of k_col_stats and four validation
+// needs -- the partial sums of k_col_stats's parts and four validation
 // flags -- lives in the file-scope array below, which every GPU that loads
 // the library holds (kNoAllocScratchBytes, 8 MiB) until the process exits.
 //
@@ -37,7 +37,7 @@ constexpr size_t kFlagBytes = 256;  // four int32 flags, padded to keep the part
 constexpr int64_t kPartialDoubles = (int64_t)((kNoAllocScratchBytes - kFlagBytes) / sizeof(double));
 constexpr int kMaxDevices = 256;
 static_assert(kPartialDoubles / (2 * SCXPCA_NOALLOC_MAX_VARS) >= 32,
-              "the scratch must hold at least 32 per-block partials at the widest matrix");
+              "the scratch must hold at least 32 partials at the widest matrix");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
@@ -114,7 +114,10 @@ void col_stats_noalloc(int32_t dev, const scxpca_csr* x, double* out, cudaStream
   int32_t* flags = reinterpret_cast<int32_t*>(base);
   double* partial = reinterpret_cast<double*>(base + kFlagBytes);
   const int64_t g = x->n_vars;
-  const int nparts = (int)std::min<int64_t>(2 * (int64_t)sms, kPartialDoubles / (2 * g));
+  // the parts of a plan, or as many as the scratch holds (46M entries: 500 genes
+  // 0.93 ms the call with 2 x SMs parts, 0.44 so; the 40 parts at 12,800 genes
+  // have four warps each, 3.05 -> 2.24)
+  const int nparts = (int)std::min<int64_t>(col_stats_parts(g, sms), kPartialDoubles / (2 * g));
 
   // Once work is queued, an error must not release the lock while our
   // kernels may still touch the shared array: wait for the stream first
