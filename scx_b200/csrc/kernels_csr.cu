@@ -210,8 +210,13 @@ __device__ __forceinline__ int64_t block_inclusive(int64_t x, int64_t* warp_sums
   return x;
 }
 
-__global__ void __launch_bounds__(256) k_scan_sums(const int64_t* __restrict__ in, int64_t n, int64_t* out) {
+// `flags` (may be null): with flags[0] or flags[1] set, nothing is written.
+__device__ __forceinline__ bool refused(const int32_t* flags) { return flags && (flags[0] | flags[1]); }
+
+__global__ void __launch_bounds__(256) k_scan_sums(const int64_t* __restrict__ in, int64_t n, int64_t* out,
+                                                   const int32_t* __restrict__ flags) {
   __shared__ int64_t warp_sums[8];
+  if (refused(flags)) return;
   const int64_t b = (int64_t)blockIdx.x * kScanTile, e = min(n, b + kScanTile);
   int64_t x = 0;
   for (int64_t i = b + threadIdx.x; i < e; i += 256) x += in[i];
@@ -219,9 +224,10 @@ __global__ void __launch_bounds__(256) k_scan_sums(const int64_t* __restrict__ i
   if (threadIdx.x == 255) out[e] = x;
 }
 
-__global__ void __launch_bounds__(256) k_scan_tops(int64_t n, int64_t* out) {
+__global__ void __launch_bounds__(256) k_scan_tops(int64_t n, int64_t* out, const int32_t* __restrict__ flags) {
   __shared__ int64_t warp_sums[8];
   __shared__ int64_t total;
+  if (refused(flags)) return;
   const int64_t tiles = (n + kScanTile - 1) / kScanTile;
   if (threadIdx.x == 0) {
     out[0] = 0;
@@ -238,8 +244,10 @@ __global__ void __launch_bounds__(256) k_scan_tops(int64_t n, int64_t* out) {
   }
 }
 
-__global__ void __launch_bounds__(256) k_scan_tiles(const int64_t* __restrict__ in, int64_t n, int64_t* out) {
+__global__ void __launch_bounds__(256) k_scan_tiles(const int64_t* __restrict__ in, int64_t n, int64_t* out,
+                                                    const int32_t* __restrict__ flags) {
   __shared__ int64_t warp_sums[8];
+  if (refused(flags)) return;
   const int64_t b = (int64_t)blockIdx.x * kScanTile;
   const int64_t base = out[b];  // the tile in front writes this place too, with the value it holds
   const int64_t i0 = b + threadIdx.x * 8;
@@ -257,13 +265,13 @@ __global__ void __launch_bounds__(256) k_scan_tiles(const int64_t* __restrict__ 
   }
 }
 
-cudaError_t launch_exclusive_scan_i64(const int64_t* in, int64_t n, int64_t* out, cudaStream_t st) {
-  if (n == 0) return cudaMemsetAsync(out, 0, sizeof(int64_t), st);
+cudaError_t launch_exclusive_scan_i64(const int64_t* in, int64_t n, int64_t* out, cudaStream_t st,
+                                      const int32_t* flags) {
   const unsigned tiles = (unsigned)((n + kScanTile - 1) / kScanTile);
-  note_launches(3);
-  k_scan_sums<<<tiles, 256, 0, st>>>(in, n, out);
-  k_scan_tops<<<1, 256, 0, st>>>(n, out);
-  k_scan_tiles<<<tiles, 256, 0, st>>>(in, n, out);
+  note_launches(tiles ? 3 : 1);
+  if (tiles) k_scan_sums<<<tiles, 256, 0, st>>>(in, n, out, flags);
+  k_scan_tops<<<1, 256, 0, st>>>(n, out, flags);
+  if (tiles) k_scan_tiles<<<tiles, 256, 0, st>>>(in, n, out, flags);
   return cudaGetLastError();
 }
 

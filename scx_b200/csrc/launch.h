@@ -96,7 +96,9 @@ cudaError_t launch_reduce_rows_f64(const double* part, int nparts, int64_t len, 
 
 // ---- prefix sums, CSR validation (kernels_csr.cu) ----
 // out[0..n] = exclusive prefix sums of n counts (out[n] the total); in and out do not overlap.
-cudaError_t launch_exclusive_scan_i64(const int64_t* in, int64_t n, int64_t* out, cudaStream_t st);
+// With `flags`, out is left alone where flags[0] or flags[1] is set (a refused CSR).
+cudaError_t launch_exclusive_scan_i64(const int64_t* in, int64_t n, int64_t* out, cudaStream_t st,
+                                      const int32_t* flags = nullptr);
 // flags[0] and flags[1] of launch_validate_csr alone.
 cudaError_t launch_check_indices(const int64_t* indptr, const int32_t* idx, int64_t n, int64_t g, int64_t nnz,
                                  int32_t* flags, cudaStream_t st, int num_sms);

@@ -3392,7 +3392,8 @@ int32_t scxpca_project_columns(int32_t device_ordinal, const scxpca_csr* x, cons
       CK(launch_check_indices(x->indptr, x->indices, n, x->n_vars, x->nnz, flags.as<int32_t>(), st, sms));
     CK(launch_project_count(x->indptr, x->indices, n, x->n_vars, x->nnz, bits, before, counts.as<int64_t>(),
                             flags.as<int32_t>(), st, sms));
-    CK(launch_exclusive_scan_i64(counts.as<int64_t>(), n, out_indptr, st));
+    // (a refused CSR leaves out_indptr as it was: the scan reads the flags too)
+    CK(launch_exclusive_scan_i64(counts.as<int64_t>(), n, out_indptr, st, flags.as<int32_t>()));
     int32_t hf[4];
     int64_t kept = 0;
     CK(cudaMemcpyAsync(hf, flags.p, 16, cudaMemcpyDeviceToHost, st));

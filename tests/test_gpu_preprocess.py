@@ -176,3 +176,34 @@ def test_counts_of_rows_of_a_million_entries():
     ix[ix.numel() - 1] = g
     with pytest.raises(ScxPcaError, match="column index"):
         accel.project_columns(ip, ix, vv, c.shape, cols)
+
+
+@pytest.mark.parametrize("n,where,value", [(300, "index", 60), (300, "index", -1), (5000, "ptr", -5000),
+                                           (300, "last", 1), (0, "last", 2)])
+def test_a_refused_projection_leaves_its_outputs(n, where, value):
+    """The caller's row pointers and count are written for an accepted CSR only."""
+    import ctypes as C
+
+    import torch
+
+    from scx_b200 import _lib
+
+    c = _raw_counts(n=n or 300, g=60, seed=8)
+    ip, ix, vv = _dev(c)
+    if n == 0:
+        ip, ix, vv = ip[:1].clone(), ix[:0], vv[:0]
+    if where == "index":
+        ix[ix.numel() - 1] = value
+    else:
+        ip[100 if where == "ptr" else len(ip) - 1] += value
+    cols = np.array([1, 5], dtype=np.int32)
+    out_ip = torch.full((n + 1,), -7, dtype=torch.int64, device="cuda")
+    nnz = C.c_int64(-7)
+    torch.cuda.synchronize()
+    csr = _lib.Csr(n, 60, int(ix.numel()), ip.data_ptr(), ix.data_ptr(), vv.data_ptr(), _lib.F32, _lib.MEM_DEVICE)
+    err = _lib.errbuf()
+    st = _lib.load().scxpca_project_columns(0, C.byref(csr), cols.ctypes.data, 2, out_ip.data_ptr(), None, None,
+                                            C.byref(nnz), None, err, len(err))
+    assert st == _lib.INVALID_CSR
+    assert nnz.value == -7
+    assert (out_ip == -7).all()
