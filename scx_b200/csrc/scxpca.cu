@@ -30,6 +30,7 @@
 #include "common.cuh"
 #include "launch.h"
 #include "power_loop.h"
+#include "staging.h"
 
 using namespace scx;
 
@@ -172,73 +173,6 @@ void give_stream(int dev, cudaStream_t st) {
   }
   cudaStreamDestroy(st);
 }
-
-// Page-locked staging of small results: device-to-host copies into it run
-// without the driver's own staging and its wait per copy, and one
-// synchronisation serves them all.  Buffers go back to a list that keeps at most
-// kStageHeld bytes; a buffer whose copies may still run is waited for first.
-constexpr size_t kStageMost = size_t(16) << 20;  // larger results are copied directly
-constexpr size_t kStageHeld = size_t(64) << 20;
-struct StageList {
-  std::mutex mu;
-  std::vector<std::pair<void*, size_t>> idle;
-  size_t held = 0;
-};
-StageList& stage_list() {
-  static StageList* l = new StageList;
-  return *l;
-}
-struct Staging {
-  char* p = nullptr;
-  size_t bytes = 0;
-  cudaStream_t busy = nullptr;  // stream whose copies into the buffer have not been waited for
-  bool pending = false;
-  explicit Staging(size_t need, cudaStream_t st) : busy(st) {
-    StageList& l = stage_list();
-    {
-      std::lock_guard<std::mutex> lock(l.mu);
-      size_t best = l.idle.size();
-      for (size_t i = 0; i < l.idle.size(); ++i)
-        if (l.idle[i].second >= need && (best == l.idle.size() || l.idle[i].second < l.idle[best].second)) best = i;
-      if (best < l.idle.size()) {
-        p = static_cast<char*>(l.idle[best].first);
-        bytes = l.idle[best].second;
-        l.held -= bytes;
-        l.idle.erase(l.idle.begin() + best);
-        return;
-      }
-    }
-    bytes = size_t(1) << 16;
-    while (bytes < need) bytes *= 2;
-    void* q = nullptr;
-    CK(cudaHostAlloc(&q, bytes, cudaHostAllocPortable));
-    p = static_cast<char*>(q);
-  }
-  Staging(const Staging&) = delete;
-  Staging& operator=(const Staging&) = delete;
-  void fetch(size_t at, const void* src, size_t n) {
-    pending = true;
-    CK(cudaMemcpyAsync(p + at, src, n, cudaMemcpyDeviceToHost, busy));
-  }
-  void wait() {
-    CK(cudaStreamSynchronize(busy));
-    pending = false;
-  }
-  template <typename T> const T* at(size_t o) const { return reinterpret_cast<const T*>(p + o); }
-  ~Staging() {
-    if (pending) cudaStreamSynchronize(busy);
-    StageList& l = stage_list();
-    {
-      std::lock_guard<std::mutex> lock(l.mu);
-      if (l.held + bytes <= kStageHeld) {
-        l.idle.emplace_back(p, bytes);
-        l.held += bytes;
-        return;
-      }
-    }
-    cudaFreeHost(p);
-  }
-};
 
 // Copy between host buffers; a large one by four threads (most of it is the
 // destination's first touch, page by page).
@@ -572,7 +506,7 @@ struct StatsFetch {
   Staging h;
   int64_t g;
   StatsFetch(scxpca_plan* pl) : h(sizeof(double) * 2 * pl->g + 16, pl->stream), g(pl->g) {
-    h.fetch(0, pl->stats_out.p, sizeof(double) * 2 * g);
+    CK(h.fetch(0, pl->stats_out.p, sizeof(double) * 2 * g));
   }
   void take(std::vector<double>& sums, std::vector<double>& sq) {  // after h.wait()
     sums.assign(h.at<double>(0), h.at<double>(0) + g);
@@ -585,7 +519,7 @@ void stats_pass(scxpca_plan* pl, const void* val, int dtype, std::vector<double>
   CK(launch_col_stats(dtype, pl->idx, val, pl->nnz, (int32_t)pl->g, pl->stats_part.as<double>(),
                       pl->stats_parts, pl->stats_out.as<double>(), pl->stream, pl->num_sms));
   StatsFetch f(pl);
-  f.h.wait();
+  CK(f.h.wait());
   f.take(sums, sq);
 }
 
@@ -1310,8 +1244,8 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
         CK(launch_col_stats(pl->in_dtype, pl->idx, vin, nnz, (int32_t)g, pl->stats_part.as<double>(),
                             pl->stats_parts, pl->stats_out.as<double>(), st, pl->num_sms));
       StatsFetch stats(pl);
-      stats.h.fetch(sizeof(double) * 2 * g, flags.p, 16);
-      stats.h.wait();
+      CK(stats.h.fetch(sizeof(double) * 2 * g, flags.p, 16));
+      CK(stats.h.wait());
       stats.take(sx, sxx);
       int32_t hf[4];
       memcpy(hf, stats.h.at<int32_t>(sizeof(double) * 2 * g), 16);
@@ -2081,18 +2015,18 @@ void run_plan(scxpca_plan* pl, const scxpca_params* over, scxpca_result* out) {
   const bool staged = comp_bytes <= kStageMost;
   const size_t at_err = 16, at_sigma = 64, at_comps = (at_sigma + sizeof(double) * pl->k + 63) / 64 * 64;
   Staging h(at_comps + (staged ? comp_bytes : 0), st);
-  h.fetch(0, pl->status.p, sizeof(int) * 4);
-  if (pl->use_tc) h.fetch(at_err, pl->tc_err.p, sizeof(int));
-  h.fetch(at_sigma, pl->sigma.p, sizeof(double) * pl->k);
+  CK(h.fetch(0, pl->status.p, sizeof(int) * 4));
+  if (pl->use_tc) CK(h.fetch(at_err, pl->tc_err.p, sizeof(int)));
+  CK(h.fetch(at_sigma, pl->sigma.p, sizeof(double) * pl->k));
   if (comp_bytes) {
     if (staged && pl->g_user == pl->g)
-      h.fetch(at_comps, pl->comps.p, comp_bytes);
+      CK(h.fetch(at_comps, pl->comps.p, comp_bytes));
     else
       CK(cudaMemcpy2DAsync(staged ? h.p + at_comps : (char*)out->components, sizeof(float) * pl->g_user, pl->comps.p,
                            sizeof(float) * pl->g, sizeof(float) * pl->g_user, pl->nc, cudaMemcpyDeviceToHost, st));
   }
   phase_mark(SCXPCA_PHASE_DOWNLOAD, st);
-  h.wait();
+  CK(h.wait());
   collect_stages(pl);
   if (pl->use_tc) raise_tc_error(pl, *h.at<int>(at_err));
   finish_result(pl, h.at<int>(0), h.at<double>(at_sigma), out);
