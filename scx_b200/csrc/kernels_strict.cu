@@ -593,11 +593,8 @@ StrictGeometry strict_geometry(int64_t n, int ld, int num_sms) {
   return geo;
 }
 
-// The per-warp slot counters of the chunk-CSC build have to fit shared memory.
-bool strict_csc_fits(int64_t g, int ld) {
-  const int64_t unit = ld <= 64 ? 256 : 128;
-  return sizeof(int32_t) * (size_t)((g + unit - 1) / unit * unit + 1) <= kStatsSmemMax;
-}
+// One warp's slot counters of the chunk-CSC build have to fit shared memory.
+bool strict_csc_fits(int64_t g) { return g <= kStrictMaxGenes; }
 
 cudaError_t launch_gene_counts(const int32_t* idx, int64_t nnz, int32_t g, int32_t* counts, cudaStream_t st,
                                int num_sms) {
@@ -625,8 +622,8 @@ template <typename ValT>
 static cudaError_t chunk_csc_t(const int64_t* indptr, const int32_t* idx, const void* val, int64_t n,
                                const StrictGeometry& geo, const int32_t* gene2slot, int32_t g, int32_t* tptr,
                                uint16_t* row, void* cval, cudaStream_t st) {
+  if (!strict_csc_fits(g)) return cudaErrorInvalidValue;
   const size_t per_warp = sizeof(int32_t) * (size_t)g;
-  if (per_warp > kStatsSmemMax) return cudaErrorInvalidValue;
   int warps = (int)std::min<size_t>(16, kStatsSmemMax / per_warp);
   warps = std::max(1, std::min(warps, (geo.rows + 3) / 4));
   // the slot map beside the counters where it fits (a gather per entry from L1

@@ -68,8 +68,9 @@ struct StrictGeometry {
 };
 // Geometry for n cells and a column panel of width ld.
 StrictGeometry strict_geometry(int64_t n, int ld, int num_sms);
-// Whether the chunk-CSC copy can be built for g genes at panel width ld.
-bool strict_csc_fits(int64_t g, int ld);
+// Whether the chunk-CSC copy can be built for g genes.
+constexpr int64_t kStrictMaxGenes = kStatsSmemMax / sizeof(int32_t);
+bool strict_csc_fits(int64_t g);
 cudaError_t launch_gene_counts(const int32_t* idx, int64_t nnz, int32_t g, int32_t* counts, cudaStream_t st,
                                int num_sms);
 // Genes in decreasing order of stored entries: gene -> slot and slot -> gene.

@@ -1031,9 +1031,9 @@ void setup_streaming(scxpca_plan* pl, const scxpca_csr* x, size_t limit) {
     if (r1 || r2)
       fail(SCXPCA_CUDA_ERROR, "cuTensorMapEncodeTiled failed (" + std::to_string(r1) + ", " + std::to_string(r2) + ")");
   } else {
-    if (!strict_csc_fits(g, (int)ld))
-      fail(SCXPCA_UNSUPPORTED, "a streamed CUDA-core PCA takes at most " +
-                                   std::to_string(kStatsSmemMax / sizeof(int32_t) - 1) + " genes");
+    if (!strict_csc_fits(g))
+      fail(SCXPCA_UNSUPPORTED,
+           "a streamed CUDA-core PCA takes at most " + std::to_string(kStrictMaxGenes) + " genes");
     pl->d_gene2slot.alloc(sizeof(int32_t) * g);
     pl->d_slot2gene.alloc(sizeof(int32_t) * g);
     CK(launch_rank_genes(counts.as<int32_t>(), (int32_t)g, pl->d_gene2slot.as<int32_t>(),
@@ -1437,7 +1437,7 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
     pl->nchunks = std::max(1, (2 * pl->num_sms + pl->nb - 1) / pl->nb);
     pl->nchunks = (int)std::min<int64_t>(pl->nchunks, n);
     pl->rows_per_chunk = (n + pl->nchunks - 1) / pl->nchunks;
-    if (!pl->use_tc) pl->strict_csc = strict_csc_fits(g, panel_width(pl));
+    if (!pl->use_tc) pl->strict_csc = strict_csc_fits(g);
     if (pl->ld > kMaxK && !pl->strict_csc)
       fail(SCXPCA_UNSUPPORTED, "a sketch wider than " + std::to_string(kMaxK) + " columns needs the chunk-CSC "
                                "copy, whose per-gene offsets exceed shared memory at n_vars = " + std::to_string(g));

@@ -85,3 +85,39 @@ def test_streamed_operator_seam_matches_oracle(mode, rounder, tol):
     s_ref, sq_ref = rpca.col_sums_and_sum_sq(cr)
     np.testing.assert_allclose(s, s_ref, rtol=1e-10, atol=1e-10 * np.abs(s_ref).max())
     plan.close()
+
+
+@pytest.mark.parametrize("k", [20, 60, 90])
+@pytest.mark.parametrize("g", [51_200, 51_201])
+def test_most_genes_of_a_streamed_cuda_core_plan(g, k, monkeypatch):
+    """One warp's slot counters fit shared memory up to 51,200 genes at every
+    sketch width: products there equal FP64 to 1e-5, and one gene more is
+    refused with that number."""
+    import torch
+
+    from scx_b200._lib import ScxPcaError
+
+    monkeypatch.setenv("SCXPCA_RESIDENT", "0")
+    n = 300
+    rng = np.random.default_rng(g)
+    lengths = rng.integers(0, 200, n)
+    ix = np.concatenate([np.sort(rng.choice(g, m, replace=False)) for m in lengths]).astype(np.int32)
+    ix[-1] = g - 1
+    c = rpca.Csr(np.r_[0, np.cumsum(lengths)].astype(np.int64), ix,
+                 rng.standard_normal(len(ix)).astype(np.float32), (n, g))
+    kw = dict(n_components=k, n_oversamples=0, math_mode="strict_fp32")
+    if g > 51_200:
+        with pytest.raises(ScxPcaError, match="at most 51200 genes"):
+            accel.Plan(c.indptr, c.indices, c.data, c.shape, **kw)
+        return
+    plan = accel.Plan(c.indptr, c.indices, c.data, c.shape, **kw)
+    mu = rpca.col_sums_and_sum_sq(c)[0] / n
+    v = rng.standard_normal((g, k)).astype(np.float32)
+    q = rng.standard_normal((n, k)).astype(np.float32)
+    y = plan.matmat(torch.from_numpy(v).cuda()).cpu().numpy().astype(np.float64)
+    y_ref = rpca.spmm_forward(c, v.astype(np.float64), mu)
+    assert np.linalg.norm(y - y_ref) / np.linalg.norm(y_ref) < 1e-5
+    z = plan.rmatmat(torch.from_numpy(q).cuda()).cpu().numpy()
+    z_ref = rpca.spmm_transpose(c, q.astype(np.float64), mu)
+    assert np.linalg.norm(z - z_ref) / np.linalg.norm(z_ref) < 1e-5
+    plan.close()
