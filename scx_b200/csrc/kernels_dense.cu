@@ -322,7 +322,7 @@ __global__ void __launch_bounds__(kCholThreads) k_cholesky(const double* __restr
   __shared__ double piv[KP], dg[KP];
   __shared__ double maxdiag_s;
   __shared__ int fail_s;
-  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, warp = tid >> 5;
   for (int j = tid; j < k; j += NT) dg[j] = G[(int64_t)j * ld + j];
   __syncthreads();
   if (tid < 32) {
@@ -1768,16 +1768,17 @@ cudaError_t launch_jacobi_eig_batch(const JacobiTask* tasks, int ntasks, int k, 
 // Rayleigh-Ritz finish: sigma, the components and M_emb from B (g x k, in
 // Z), the eigenpairs of B^T B and R2^{-1}.
 // ---------------------------------------------------------------------------
-// Components c0 .. c0 + ncc - 1 of nc per launch (E's columns staged in
-// shared memory); one launch takes them all when E[:, :nc] fits.  Block b of
+// Sketches wider than one panel (ld > 128), one matrix: components c0 .. c0 +
+// ncc - 1 of nc per launch (E's columns staged in shared memory).  Block b of
 // nb takes the rows l = b, b + nb, ... of M_emb and the genes j = b, b + nb,
 // ... of the components, its 128 threads spread over (row, component) pairs.
 // Each output is one FMA chain in index order.
-__device__ __forceinline__ void ritz_finish_body(const double* __restrict__ B, int64_t g, int ld, int k, int nc,
-                                                 int c0, int ncc, const double* __restrict__ evals,
-                                                 const double* __restrict__ E, const double* __restrict__ Rinv2,
-                                                 double* __restrict__ sigma, float* __restrict__ comps,
-                                                 float* __restrict__ M_emb, int b, int nb) {
+__global__ void __launch_bounds__(128) k_ritz_finish(const double* __restrict__ B, int64_t g, int ld, int k,
+                                                     int nc, int c0, int ncc, const double* __restrict__ evals,
+                                                     const double* __restrict__ E,
+                                                     const double* __restrict__ Rinv2, double* __restrict__ sigma,
+                                                     float* __restrict__ comps, float* __restrict__ M_emb) {
+  const int b = blockIdx.x, nb = gridDim.x;
   extern __shared__ double sm[];
   double* Es = sm;              // [ld][ncc]: columns c0 .. c0 + ncc - 1 of E
   double* sg = sm + ld * ncc;   // [ncc]
@@ -1921,22 +1922,6 @@ static cudaError_t ritz_mma(const RitzTask* tasks, int ntasks, const RitzTask& o
   }
 }
 
-__global__ void __launch_bounds__(128) k_ritz_finish(const double* __restrict__ B, int64_t g, int ld, int k,
-                                                     int nc, int c0, int ncc, const double* __restrict__ evals,
-                                                     const double* __restrict__ E,
-                                                     const double* __restrict__ Rinv2, double* __restrict__ sigma,
-                                                     float* __restrict__ comps, float* __restrict__ M_emb) {
-  ritz_finish_body(B, g, ld, k, nc, c0, ncc, evals, E, Rinv2, sigma, comps, M_emb, blockIdx.x, gridDim.x);
-}
-
-// One segment per grid row y (batched segments).
-__global__ void __launch_bounds__(128) k_ritz_finish_batch(const RitzTask* __restrict__ tasks, int64_t g, int ld,
-                                                           int k, int nc, int c0, int ncc) {
-  const RitzTask t = tasks[blockIdx.y];
-  ritz_finish_body(t.B, g, ld, k, nc, c0, ncc, t.evals, t.evecs, t.Rinv2, t.sigma, t.comps, t.M_emb, blockIdx.x,
-                   gridDim.x);
-}
-
 // Components staged per launch, and the launch's shared bytes.
 static int ritz_cols(int ld, int nc, size_t* smem) {
   constexpr size_t kStage = 160 * 1024;  // shared bytes for the staged columns of E
@@ -1949,8 +1934,7 @@ cudaError_t launch_ritz_finish(const double* B, int64_t g, int ld, int k, int nc
                                const double* evals, const double* evecs, const double* Rinv2,
                                double* sigma, float* components, float* M_emb, cudaStream_t st) {
   if (ld <= kMaxK)
-    return ritz_mma(nullptr, 0,
-                    RitzTask{B, evals, evecs, Rinv2, sigma, components, M_emb}, g, ld, k, nc, st);
+    return ritz_mma(nullptr, 0, RitzTask{B, evals, evecs, Rinv2, sigma, components, M_emb}, g, ld, k, nc, st);
   size_t smem = 0;
   const int ncc = ritz_cols(ld, nc, &smem);
   if (cudaError_t e = allow_smem(k_ritz_finish, smem); e != cudaSuccess) return e;
@@ -1967,17 +1951,7 @@ cudaError_t launch_ritz_finish(const double* B, int64_t g, int ld, int k, int nc
 cudaError_t launch_ritz_finish_batch(const RitzTask* tasks, int ntasks, int64_t g, int ld, int k, int nc,
                                      cudaStream_t st) {
   if (ntasks <= 0) return cudaSuccess;
-  if (ld <= kMaxK) return ritz_mma(tasks, ntasks, RitzTask{}, g, ld, k, nc, st);
-  size_t smem = 0;
-  const int ncc = ritz_cols(ld, nc, &smem);
-  if (cudaError_t e = allow_smem(k_ritz_finish_batch, smem); e != cudaSuccess) return e;
-  const int gx = (int)std::max<int64_t>(1, std::min<int64_t>(std::max<int64_t>(g, ld), 8));
-  for (int c0 = 0; c0 < nc; c0 += ncc) {
-    note_launches(1);
-    k_ritz_finish_batch<<<dim3((unsigned)gx, (unsigned)ntasks), 128, smem, st>>>(tasks, g, ld, k, nc, c0,
-                                                                                  std::min(ncc, nc - c0));
-  }
-  return cudaGetLastError();
+  return ritz_mma(tasks, ntasks, RitzTask{}, g, ld, k, nc, st);
 }
 
 // Embeddings U = Q M_emb (n x nc row-major).

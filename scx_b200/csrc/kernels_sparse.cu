@@ -402,73 +402,6 @@ __global__ void __launch_bounds__(512) k_transform_values(const int32_t* __restr
 }
 
 // ---------------------------------------------------------------------------
-// Forward product Y[i, :] = sum_p x_p V[j_p, :] - mc.  One warp per row; lane
-// l owns columns l + 32 c.  Nonzeros are fetched 32 at a time (coalesced) and
-// broadcast by shuffle; V rows are read through the read-only cache (V is
-// n_vars x ld x 4 bytes, L2-resident).
-// Restates spmm_forward_row (scx-accel/src/pca/cpu.rs:1500-1523) with the
-// mean correction of forward_mean_prefactor (scx-gpu/src/gpu_pca.rs:218-237).
-// ---------------------------------------------------------------------------
-template <int C, typename ValT>
-__global__ void __launch_bounds__(256) k_spmm_fwd(const int64_t* __restrict__ indptr,
-                                                  const int32_t* __restrict__ idx,
-                                                  const ValT* __restrict__ val, int64_t n_obs,
-                                                  const float* __restrict__ V, int ldv,
-                                                  const float* __restrict__ mc,
-                                                  float* __restrict__ Y, int ldy) {
-  const int lane = threadIdx.x & 31;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  float m[C];
-#pragma unroll
-  for (int c = 0; c < C; ++c) m[c] = mc ? mc[lane + 32 * c] : 0.f;
-  for (int64_t row = warp; row < n_obs; row += nwarps) {
-    const int64_t s = indptr[row], e = indptr[row + 1];
-    float acc[C];
-#pragma unroll
-    for (int c = 0; c < C; ++c) acc[c] = 0.f;
-    for (int64_t base = s; base < e; base += 32) {
-      const int64_t p = base + lane;
-      int32_t j = 0;
-      float x = 0.f;
-      if (p < e) {
-        j = __ldg(idx + p);
-        x = to_f32(val[p]);
-      }
-      const int cnt = (int)min((int64_t)32, e - base);
-      int t = 0;
-      for (; t + 4 <= cnt; t += 4) {
-        int jj[4];
-        float xx[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          jj[u] = __shfl_sync(0xffffffffu, j, t + u);
-          xx[u] = __shfl_sync(0xffffffffu, x, t + u);
-        }
-        float vv[4][C];
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int c = 0; c < C; ++c) vv[u][c] = __ldg(V + (int64_t)jj[u] * ldv + lane + 32 * c);
-#pragma unroll
-        for (int u = 0; u < 4; ++u)
-#pragma unroll
-          for (int c = 0; c < C; ++c) acc[c] = fmaf(xx[u], vv[u][c], acc[c]);
-      }
-      for (; t < cnt; ++t) {
-        const int jt = __shfl_sync(0xffffffffu, j, t);
-        const float xt = __shfl_sync(0xffffffffu, x, t);
-#pragma unroll
-        for (int c = 0; c < C; ++c) acc[c] = fmaf(xt, __ldg(V + (int64_t)jt * ldv + lane + 32 * c), acc[c]);
-      }
-    }
-    float* yr = Y + row * (int64_t)ldy;
-#pragma unroll
-    for (int c = 0; c < C; ++c) yr[lane + 32 * c] = acc[c] - m[c];
-  }
-}
-
-// ---------------------------------------------------------------------------
 // Row-block pointer table for the transposed product: for row i and gene
 // block b, rbp[i * (nb + 1) + b] = offset (from indptr[i]) of the first stored
 // entry of row i whose gene is >= b * gb.  Rows must be sorted by gene.
@@ -649,40 +582,6 @@ cudaError_t launch_transform_values(int in_dtype, int out_dtype, const int32_t* 
     case 1:
       return transform_in<__nv_bfloat16>(out_dtype, idx, in, out, nnz, g, mode, mu, inv_std, cshift, clip, st, num_sms);
     default: return transform_in<__half>(out_dtype, idx, in, out, nnz, g, mode, mu, inv_std, cshift, clip, st, num_sms);
-  }
-}
-
-template <int C, typename ValT>
-static cudaError_t fwd_c(const int64_t* indptr, const int32_t* idx, const void* val, int64_t n,
-                         const float* V, int ldv, const float* mc, float* Y, int ldy,
-                         cudaStream_t st, int num_sms) {
-  int grid = grid_for(n * 32, 256, num_sms, 8);
-  note_launches(1);
-  k_spmm_fwd<C, ValT><<<grid, 256, 0, st>>>(indptr, idx, static_cast<const ValT*>(val), n, V, ldv,
-                                            mc, Y, ldy);
-  return cudaGetLastError();
-}
-
-template <typename ValT>
-static cudaError_t fwd_t(int ld, const int64_t* indptr, const int32_t* idx, const void* val,
-                         int64_t n, const float* V, int ldv, const float* mc, float* Y, int ldy,
-                         cudaStream_t st, int num_sms) {
-  switch (ld) {
-    case 32: return fwd_c<1, ValT>(indptr, idx, val, n, V, ldv, mc, Y, ldy, st, num_sms);
-    case 64: return fwd_c<2, ValT>(indptr, idx, val, n, V, ldv, mc, Y, ldy, st, num_sms);
-    case 96: return fwd_c<3, ValT>(indptr, idx, val, n, V, ldv, mc, Y, ldy, st, num_sms);
-    default: return fwd_c<4, ValT>(indptr, idx, val, n, V, ldv, mc, Y, ldy, st, num_sms);
-  }
-}
-
-cudaError_t launch_spmm_fwd(int dtype, int ld, const int64_t* indptr, const int32_t* idx,
-                            const void* val, int64_t n, const float* V, const float* mc,
-                            float* Y, cudaStream_t st, int num_sms) {
-  if (n == 0) return cudaSuccess;
-  switch (dtype) {
-    case 0: return fwd_t<float>(ld, indptr, idx, val, n, V, ld, mc, Y, ld, st, num_sms);
-    case 1: return fwd_t<__nv_bfloat16>(ld, indptr, idx, val, n, V, ld, mc, Y, ld, st, num_sms);
-    default: return fwd_t<__half>(ld, indptr, idx, val, n, V, ld, mc, Y, ld, st, num_sms);
   }
 }
 

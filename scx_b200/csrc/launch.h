@@ -7,8 +7,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <vector>
-
 namespace scx {
 
 // Process-wide count of kernels launched by this library (every launcher
@@ -42,9 +40,6 @@ cudaError_t launch_transform_values(int in_dtype, int out_dtype, const int32_t* 
                                     const double* mu, const double* inv_std,
                                     const double* cshift, double clip, cudaStream_t st,
                                     int num_sms);
-cudaError_t launch_spmm_fwd(int dtype, int ld, const int64_t* indptr, const int32_t* idx,
-                            const void* val, int64_t n, const float* V, const float* mc,
-                            float* Y, cudaStream_t st, int num_sms);
 cudaError_t launch_row_block_ptr(const int64_t* indptr, const int32_t* idx, int64_t n, int nb,
                                  int gb, int32_t* rbp, cudaStream_t st, int num_sms);
 cudaError_t launch_spmm_t(int dtype, int ld, const int64_t* indptr, const int32_t* idx,
@@ -246,8 +241,9 @@ cudaError_t launch_center_apply(const double* W, int64_t g, int ld, const double
 //   A = A * M  in place (FP64)
 cudaError_t launch_apply_right_f64(double* A, int64_t g, int ld, const double* M,
                                    cudaStream_t st);
+//   M = I (ld x ld)
+cudaError_t launch_identity(double* M, int ld, cudaStream_t st);
 //   Vf = (float)A ; mc = A^T mu (float, from the rounded Vf) ; mu may be null
-cudaError_t launch_identity(double* M, int ld, cudaStream_t st);  // M = I (ld x ld)
 cudaError_t launch_round_v(const double* A, int64_t g, int ld, const double* mu, float* Vf,
                            float* mc, cudaStream_t st);
 //   mc = Vf^T mu for a float V (mu may be null -> zeros)

@@ -320,15 +320,6 @@ struct DevBuf {
 
 size_t dtype_size(int dt) { return dt == SCXPCA_F32 ? 4 : 2; }
 
-bool is_device_ptr(const void* p) {
-  cudaPointerAttributes a;
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
-    cudaGetLastError();
-    return false;
-  }
-  return a.type == cudaMemoryTypeDevice || a.type == cudaMemoryTypeManaged;
-}
-
 }  // namespace
 
 struct scxpca_plan {
@@ -1758,10 +1749,6 @@ struct DeviceOperator {
   void rmatmat_products() {
     rmatmat_raw(pl, pl->Y.as<float>(), 0);
     if (pl->pflog) CK(launch_aug_fold(pl->W.as<double>(), (int32_t)pl->g_user, (int)pl->ld, pl->stream, pl->num_sms));
-  }
-  ApplyTask rmatmat_task() const {
-    return ApplyTask{pl->W.as<double>(), mu, sY, closing ? pl->R2inv.as<double>() : pl->Rinv.as<double>(),
-                     pl->Z.as<double>()};
   }
   void qr(Buf b) {
     if (b == Buf::kY) {
