@@ -1900,24 +1900,24 @@ __global__ void __launch_bounds__(256) k_ritz_mma(const RitzTask* __restrict__ t
 
 template <int LD>
 static cudaError_t ritz_mma_go(const RitzTask* tasks, int ntasks, const RitzTask& one, int64_t g, int k, int nc,
-                               cudaStream_t st) {
+                               cudaStream_t st, int num_sms) {
   constexpr size_t smem = ritz_mma_smem(LD);
   if (cudaError_t e = allow_smem(k_ritz_mma<LD>, smem); e != cudaSuccess) return e;
-  // one matrix: a strip per block; a batch: a few strips per staged E
+  // one matrix: a strip per block, as many blocks as SMs; a batch: a few strips per staged E
   const int64_t strips = LD / kRitzRows + (g + kRitzRows - 1) / kRitzRows;
-  const dim3 grid((unsigned)std::min<int64_t>(strips, tasks ? 16 : 148), (unsigned)(tasks ? ntasks : 1));
+  const dim3 grid((unsigned)std::min<int64_t>(strips, tasks ? 16 : num_sms), (unsigned)(tasks ? ntasks : 1));
   note_launches(1);
   k_ritz_mma<LD><<<grid, 256, smem, st>>>(tasks, one, g, k, nc);
   return cudaGetLastError();
 }
 
 static cudaError_t ritz_mma(const RitzTask* tasks, int ntasks, const RitzTask& one, int64_t g, int ld, int k, int nc,
-                            cudaStream_t st) {
+                            cudaStream_t st, int num_sms) {
   switch (ld) {
-    case 32: return ritz_mma_go<32>(tasks, ntasks, one, g, k, nc, st);
-    case 64: return ritz_mma_go<64>(tasks, ntasks, one, g, k, nc, st);
-    case 96: return ritz_mma_go<96>(tasks, ntasks, one, g, k, nc, st);
-    case 128: return ritz_mma_go<128>(tasks, ntasks, one, g, k, nc, st);
+    case 32: return ritz_mma_go<32>(tasks, ntasks, one, g, k, nc, st, num_sms);
+    case 64: return ritz_mma_go<64>(tasks, ntasks, one, g, k, nc, st, num_sms);
+    case 96: return ritz_mma_go<96>(tasks, ntasks, one, g, k, nc, st, num_sms);
+    case 128: return ritz_mma_go<128>(tasks, ntasks, one, g, k, nc, st, num_sms);
     default: return cudaErrorInvalidValue;
   }
 }
@@ -1932,9 +1932,10 @@ static int ritz_cols(int ld, int nc, size_t* smem) {
 
 cudaError_t launch_ritz_finish(const double* B, int64_t g, int ld, int k, int nc,
                                const double* evals, const double* evecs, const double* Rinv2,
-                               double* sigma, float* components, float* M_emb, cudaStream_t st) {
+                               double* sigma, float* components, float* M_emb, cudaStream_t st, int num_sms) {
   if (ld <= kMaxK)
-    return ritz_mma(nullptr, 0, RitzTask{B, evals, evecs, Rinv2, sigma, components, M_emb}, g, ld, k, nc, st);
+    return ritz_mma(nullptr, 0, RitzTask{B, evals, evecs, Rinv2, sigma, components, M_emb}, g, ld, k, nc, st,
+                    num_sms);
   size_t smem = 0;
   const int ncc = ritz_cols(ld, nc, &smem);
   if (cudaError_t e = allow_smem(k_ritz_finish, smem); e != cudaSuccess) return e;
@@ -1951,7 +1952,7 @@ cudaError_t launch_ritz_finish(const double* B, int64_t g, int ld, int k, int nc
 cudaError_t launch_ritz_finish_batch(const RitzTask* tasks, int ntasks, int64_t g, int ld, int k, int nc,
                                      cudaStream_t st) {
   if (ntasks <= 0) return cudaSuccess;
-  return ritz_mma(tasks, ntasks, RitzTask{}, g, ld, k, nc, st);
+  return ritz_mma(tasks, ntasks, RitzTask{}, g, ld, k, nc, st, 0);
 }
 
 // Embeddings U = Q M_emb (n x nc row-major).

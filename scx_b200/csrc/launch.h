@@ -259,7 +259,7 @@ cudaError_t launch_jacobi_eig(const double* C, int k, int ld, double* evals, dou
 cudaError_t launch_ritz_finish(const double* B, int64_t g, int ld, int k, int nc,
                                const double* evals, const double* evecs, const double* Rinv2,
                                double* sigma, float* components, float* M_emb,
-                               cudaStream_t st);
+                               cudaStream_t st, int num_sms);
 // Embeddings U (n x nc row-major) = Q (n x ld) * M_emb (ld x nc).
 cudaError_t launch_embed(const float* Q, int64_t n, int ld, int k, const float* M_emb, int nc,
                          float* U, cudaStream_t st, int num_sms);

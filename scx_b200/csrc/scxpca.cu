@@ -1884,7 +1884,7 @@ void finish_after(scxpca_plan* pl, float* U) {
   const RitzTask t = ritz_task(pl);
   int s = stage_begin(pl);
   CK(launch_ritz_finish(t.B, pl->g, (int)pl->ld, (int)pl->k, (int)pl->nc, t.evals, t.evecs, t.Rinv2, t.sigma,
-                        t.comps, t.M_emb, pl->stream));
+                        t.comps, t.M_emb, pl->stream, pl->num_sms));
   stage_end(pl, SCXPCA_STAGE_SMALL, s);
   finish_embed(pl, U);
 }
