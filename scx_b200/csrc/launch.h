@@ -59,10 +59,12 @@ cudaError_t launch_reduce_panel_f32(const float* part, int nparts, int64_t rows,
 struct StrictGeometry {
   int cols = 32;  // columns a block takes
   int rows = 0, per_range = 1, ranges = 1;
+  int parts = 1;   // blocks that share the genes of a range
+  int splits = 1;  // blocks that build a chunk of the copy
   int64_t chunks = 0;
 };
-// Geometry for n cells and a column panel of width ld.
-StrictGeometry strict_geometry(int64_t n, int ld, int num_sms);
+// Geometry for n cells, g genes (0: of a streamed shard) and a column panel of width ld.
+StrictGeometry strict_geometry(int64_t n, int64_t g, int ld, int num_sms);
 // Whether the chunk-CSC copy can be built for g genes.
 constexpr int64_t kStrictMaxGenes = kStatsSmemMax / sizeof(int32_t);
 bool strict_csc_fits(int64_t g);
@@ -71,10 +73,12 @@ cudaError_t launch_gene_counts(const int32_t* idx, int64_t nnz, int32_t g, int32
 // Genes in decreasing order of stored entries: gene -> slot and slot -> gene.
 cudaError_t launch_rank_genes(const int32_t* counts, int32_t g, int32_t* gene2slot, int32_t* slot2gene,
                               cudaStream_t st);
-// Chunk-CSC copy of a row-sorted CSR: tptr [chunks][g + 1], row/cval [nnz].
+// Chunk-CSC copy of a row-sorted CSR: tptr [chunks][g + 1], row/cval [nnz];
+// `scratch` holds chunk_csc_scratch bytes until the launches are done.
+size_t chunk_csc_scratch(const StrictGeometry& geo, int64_t g);
 cudaError_t launch_chunk_csc(int dtype, const int64_t* indptr, const int32_t* idx, const void* val, int64_t n,
-                             const StrictGeometry& geo, const int32_t* gene2slot, int32_t g, int32_t* tptr,
-                             uint16_t* row, void* cval, cudaStream_t st);
+                             const StrictGeometry& geo, const int32_t* gene2slot, int32_t g, int32_t* scratch,
+                             int32_t* tptr, uint16_t* row, void* cval, cudaStream_t st);
 // Y (n x ld) = P V - 1 mc^T (mc may be null) from a row-sorted CSR.  `ld` is
 // the width of the column panel taken (32, 64, 96 or 128); V, mc and Y point
 // at its first column and `lds` is the row stride of V and Y in floats

@@ -615,12 +615,14 @@ void build_chunk_csc(scxpca_plan* pl) {
   CK(cudaMemsetAsync(counts.p, 0, sizeof(int32_t) * g, st));
   CK(launch_gene_counts(pl->idx, nnz, (int32_t)g, counts.as<int32_t>(), st, pl->num_sms));
   CK(launch_rank_genes(counts.as<int32_t>(), (int32_t)g, d_g2s.as<int32_t>(), pl->d_slot2gene.as<int32_t>(), st));
-  pl->geo = strict_geometry(n, pw, pl->num_sms);
+  pl->geo = strict_geometry(n, g, pw, pl->num_sms);
   pl->csc_tptr.alloc(sizeof(int32_t) * (size_t)pl->geo.chunks * (g + 1));
   pl->csc_row.alloc(sizeof(uint16_t) * std::max<int64_t>(nnz, 1));
   pl->csc_val.alloc(dtype_size(pl->dtype) * std::max<int64_t>(nnz, 1));
+  DevBuf scratch;
+  if (const size_t b = chunk_csc_scratch(pl->geo, g)) scratch.alloc(b);
   CK(launch_chunk_csc(pl->dtype, pl->indptr, pl->idx, pl->val, n, pl->geo, d_g2s.as<int32_t>(), (int32_t)g,
-                      pl->csc_tptr.as<int32_t>(), pl->csc_row.as<uint16_t>(), pl->csc_val.p, st));
+                      scratch.as<int32_t>(), pl->csc_tptr.as<int32_t>(), pl->csc_row.as<uint16_t>(), pl->csc_val.p, st));
   pl->wpart.alloc(sizeof(float) * (size_t)pl->geo.ranges * g * pw);
 }
 
@@ -690,8 +692,8 @@ const void* shard_prepare(scxpca_plan* pl, size_t s, int k, bool work, int pack)
                         sl.ent.as<uint32_t>(), sl.meta.p, st, pl->num_sms));
   } else if (pack == 2) {
     CK(launch_chunk_csc(pl->dtype, sl.ip.as<int64_t>(), sl.idx.as<int32_t>(), vals, rows, sh.geo,
-                        pl->d_gene2slot.as<int32_t>(), (int32_t)pl->g, sl.tptr.as<int32_t>(), sl.row.as<uint16_t>(),
-                        sl.cval.p, st));
+                        pl->d_gene2slot.as<int32_t>(), (int32_t)pl->g, nullptr, sl.tptr.as<int32_t>(),
+                        sl.row.as<uint16_t>(), sl.cval.p, st));
   }
   return vals;
 }
@@ -1032,7 +1034,7 @@ void setup_streaming(scxpca_plan* pl, const scxpca_csr* x, size_t limit) {
     int ranges_max = 1;
     int64_t chunks_max = 1;
     for (auto& sh : pl->shards) {
-      sh.geo = strict_geometry(sh.r1 - sh.r0, (int)ld, pl->num_sms);
+      sh.geo = strict_geometry(sh.r1 - sh.r0, 0, (int)ld, pl->num_sms);
       ranges_max = std::max(ranges_max, sh.geo.ranges);
       chunks_max = std::max(chunks_max, sh.geo.chunks);
     }

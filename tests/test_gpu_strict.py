@@ -268,3 +268,30 @@ def test_overflowed_values_stay_in_their_row_and_gene(n, g, k, offset, monkeypat
             assert np.linalg.norm((y - y_ref)[ok_rows]) / np.linalg.norm(y_ref[ok_rows]) < OP_RTOL
             assert not np.isfinite(y[rows]).any()
         plan.close()
+
+
+@pytest.mark.parametrize("n,g,k,loc", [
+    (64, 128, 20, -2.0),      # one range, the genes of one block
+    (70, 129, 20, -2.0),      # two ranges, one gene over
+    (300, 20011, 20, -2.0),   # many blocks a range and two a chunk of the copy, the last one short
+    (1000, 30011, 90, -4.0),  # three slices of columns; one warp builds
+    (15000, 6400, 20, -5.0),  # chunks of 307 rows
+    (9472, 300, 20, -2.0),    # a range on every SM
+    (9473, 300, 20, -2.0),    # longer ranges, fewer than SMs
+])
+def test_transposed_product_of_few_cells(n, g, k, loc):
+    """Where a small matrix's row ranges leave SMs idle, several blocks share a
+    range's genes and several build a chunk of the copy: each gene's sum against
+    FP64, alone and over all."""
+    import torch
+
+    c = _csr(n, g, seed=g, loc=loc)
+    plan = accel.Plan(c.indptr, c.indices, c.data, c.shape, n_components=k, n_oversamples=0, math_mode="strict_fp32")
+    q = np.random.default_rng(7).standard_normal((n, k)).astype(np.float32)
+    z = plan.rmatmat(torch.from_numpy(q).cuda()).cpu().numpy()
+    plan.close()
+    mu = rpca.col_sums_and_sum_sq(c)[0] / n
+    z_ref = rpca.spmm_transpose(c, q.astype(np.float64), mu)
+    assert np.linalg.norm(z - z_ref) / np.linalg.norm(z_ref) < OP_RTOL
+    rel = np.linalg.norm(z - z_ref, axis=1) / np.maximum(np.linalg.norm(z_ref, axis=1), 1e-3 * np.abs(z_ref).max())
+    assert rel.max() < 1e-4
