@@ -363,13 +363,69 @@ __device__ __forceinline__ void slot_load(DenseSlot<R>& x, const uint32_t* __res
   }
 }
 
+// The entries of a quarter beyond those in flight: `m` of them from `from`.  Not
+// inlined, so that the kernels' own registers are those of quarters without any.
+// A few are loaded at once; more in rounds of 512, 4 bytes a lane, or, DENSE, 16
+// (their k-th words lie 4 apart, which costs bank conflicts but takes a quarter
+// of the loads).  A load after another left most of a dense tile's time to
+// latency.  40,000 x 2,000, k = 50, forward (us): 15 % stored one by one 53, 4-byte
+// rounds 51, 16-byte 51; 20 % 79, 62, 66; 30 % 152, 88, 78; 100 % 699, 270, 173
+// (loads of 16 bytes for all entries, one stage ahead: 63, 66, 87, 190).  With
+// the 16-byte rounds the transposed product takes 2 % longer at 9 %, where they
+// hardly run, so there are two instances of each kernel (tc_dense).
+template <bool DENSE>
+__device__ __noinline__ void scatter_rest(uint32_t tile, const uint32_t* __restrict__ from, int m, int lane) {
+  if (m <= 128) {
+    uint32_t w[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) w[r] = lane + 32 * r < m ? __ldg(from + lane + 32 * r) : 0u;
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      if (lane + 32 * r < m) scatter_one(tile, w[r]);
+    return;
+  }
+  if (!DENSE) {
+    for (int b = lane; b < m; b += 512) {
+      uint32_t w[16];
+#pragma unroll
+      for (int r = 0; r < 16; ++r) w[r] = b + 32 * r < m ? __ldg(from + b + 32 * r) : 0u;
+#pragma unroll
+      for (int r = 0; r < 16; ++r)
+        if (b + 32 * r < m) scatter_one(tile, w[r]);
+    }
+    return;
+  }
+  // the words before a 16-byte boundary, then whole 16-byte loads (a segment is
+  // padded to four entries: a load never leaves it)
+  const int head = (int)((16u - (uint32_t)reinterpret_cast<uintptr_t>(from)) >> 2) & 3;
+  if (lane < head) scatter_one(tile, __ldg(from + lane));
+  const uint4* v = reinterpret_cast<const uint4*>(from + head);
+  m -= head;
+  for (int b = 0; b < m; b += 512) {
+    uint4 w[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int p = b + 4 * (lane + 32 * u);
+      w[u] = p < m ? __ldg(v + (p >> 2)) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int left = m - (b + 4 * (lane + 32 * u));
+      if (left > 0) scatter_one(tile, w[u].x);
+      if (left > 1) scatter_one(tile, w[u].y);
+      if (left > 2) scatter_one(tile, w[u].z);
+      if (left > 3) scatter_one(tile, w[u].w);
+    }
+  }
+}
+
 // Scatter the slot's quarter into its rows of `tile`, which hold zeros.
-template <int R>
+template <bool DENSE, int R>
 __device__ __forceinline__ void slot_scatter(const DenseSlot<R>& x, uint32_t tile, int lane) {
 #pragma unroll
   for (int r = 0; r < R; ++r)
     if (lane + 32 * r < x.n) scatter_one(tile, x.w[r]);
-  for (int p = lane + 32 * R; p < x.n; p += 32) scatter_one(tile, __ldg(x.base + p));
+  if (x.n > 32 * R) scatter_rest<DENSE>(tile, x.base + 32 * R, x.n - 32 * R, lane);
 }
 
 // Meta loader: L2 prefetch of the entries of segments [c0, c1) of one tile
@@ -445,7 +501,7 @@ __device__ __forceinline__ void swap_tile_out(uint32_t tbase, int tiles, int64_t
 // took 217 us, of which 195 the MMAs (282 cycles each with an MN-major B) and a
 // two-slot image ring; this takes 194, the epilogues of the bands included.
 // ---------------------------------------------------------------------------
-template <int LD>
+template <int LD, bool DENSE>
 __global__ void __launch_bounds__(kThreads, 1)
     k_fwd_tc(const uint32_t* __restrict__ ent, const SegMeta* __restrict__ meta, int64_t n_tiles, int nc,
              int64_t n, const __grid_constant__ CUtensorMap vmap, const float* __restrict__ mc,
@@ -550,7 +606,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         if (sl[k].n >= 0) {
           zero_rows(tile, q, lane);
           __syncwarp();
-          slot_scatter(sl[k], tile, lane);
+          slot_scatter<DENSE>(sl[k], tile, lane);
         }
         // every lane's shared stores -> async proxy, then one arrival per warp
         fence_proxy_async_smem();
@@ -674,7 +730,7 @@ done:
 // A_tile^T (Qhi_tile + Qlo_tile).  grid = G gene groups x R row groups; one
 // CTA per SM (the accumulators fill TMEM).
 // ---------------------------------------------------------------------------
-template <int LD>
+template <int LD, bool DENSE>
 __global__ void __launch_bounds__(kThreads, 1)
     k_rmat_tc(const uint32_t* __restrict__ ent, const SegMeta* __restrict__ meta, int64_t n_tiles, int nc,
               int64_t g, int n_gene_groups, const __grid_constant__ CUtensorMap qmap, float* __restrict__ part,
@@ -783,7 +839,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           const uint32_t tile = stage0 - hs[k] * HSUB;
           zero_rows(tile, 2 * hs[k] + r, lane);
           __syncwarp();
-          slot_scatter(sl[k], tile, lane);
+          slot_scatter<DENSE>(sl[k], tile, lane);
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) mbar_arrive(&full[group]);
@@ -1307,7 +1363,7 @@ struct FwdBatch {
 // waits once and commits once a chunk (a ring of its own cost it about 200 of
 // 1,200 cycles).  A band is two consecutive row tiles.  Per band:
 // Y^T[m, its 256 cells] = sum over chunks c of Vimg_c^T (m x 64 genes) [A_(t0,c) | A_(t1,c)]^T.
-template <class Src>
+template <bool DENSE, class Src>
 __device__ __forceinline__ void fwd_swap_body(const Src& src, int nc, int fmt) {
   constexpr int LD = 64;
   constexpr int S = kSwapFwdStages;
@@ -1414,7 +1470,7 @@ __device__ __forceinline__ void fwd_swap_body(const Src& src, int nc, int fmt) {
           const uint32_t tile = tile0 + 2 * k * STAGE;
           zero_rows(tile, q, lane);
           __syncwarp();
-          slot_scatter(sl[k], tile, lane);
+          slot_scatter<DENSE>(sl[k], tile, lane);
         }
         fence_proxy_async_smem();
         __syncwarp();
@@ -1523,18 +1579,20 @@ done:
   }
 }
 
+template <bool DENSE>
 __global__ void __launch_bounds__(kThreads, 1)
     k_fwd_swap(const uint32_t* __restrict__ ent, const SegMeta* __restrict__ meta, int64_t n_tiles, int nc,
                int64_t n, const __grid_constant__ CUtensorMap vmap, const float* __restrict__ mc,
                float* __restrict__ Y, uint16_t* __restrict__ Yimg, int fmt, int* err) {
-  fwd_swap_body(FwdOne{ent, meta, &vmap, mc, Y, Yimg, err, n_tiles, n, nc}, nc, fmt);
+  fwd_swap_body<DENSE>(FwdOne{ent, meta, &vmap, mc, Y, Yimg, err, n_tiles, n, nc}, nc, fmt);
 }
 
 // Every band of every segment of a batch in one persistent launch.
+template <bool DENSE>
 __global__ void __launch_bounds__(kThreads, 1)
     k_fwd_swap_batch(const TcSegment* __restrict__ segs, const int32_t* __restrict__ band_seg, int64_t n_bands,
                      int nc, int write_y, int fmt) {
-  fwd_swap_body(FwdBatch{segs, band_seg, n_bands, nc, write_y}, nc, fmt);
+  fwd_swap_body<DENSE>(FwdBatch{segs, band_seg, n_bands, nc, write_y}, nc, fmt);
 }
 
 constexpr int kSwapRmatStages = 4;  // stages: one half tile (64 cells) of a quad's four chunks
@@ -1563,7 +1621,7 @@ struct RmatJob {
   int gg, rg;
 };
 
-template <bool kGlobalMaps>
+template <bool kGlobalMaps, bool DENSE>
 __device__ __forceinline__ void rmat_swap_body(const RmatJob& job, int nc, int64_t g, int fmt) {
   constexpr int LD = 64;
   constexpr int S = kSwapRmatStages;
@@ -1669,7 +1727,7 @@ __device__ __forceinline__ void rmat_swap_body(const RmatJob& job, int nc, int64
             const uint32_t tile = tile0 + 2 * k * STAGE;
             zero_rows(tile, q, lane);
             __syncwarp();
-            slot_scatter(sl[k], tile, lane);
+            slot_scatter<DENSE>(sl[k], tile, lane);
           }
           fence_proxy_async_smem();
           __syncwarp();
@@ -1792,6 +1850,7 @@ done:
 
 // CTA b = (row group b / gene groups, gene group b % gene groups); the row
 // groups split the tiles evenly (tc_range_begin).
+template <bool DENSE>
 __global__ void __launch_bounds__(kThreads, 1)
     k_rmat_swap(const uint32_t* __restrict__ ent, const SegMeta* __restrict__ meta, int64_t n_tiles, int nc,
                 int64_t g, int n_gene_groups, const __grid_constant__ CUtensorMap qmap, float* __restrict__ part,
@@ -1800,11 +1859,12 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int R = gridDim.x / n_gene_groups;
   const RmatJob job{ent, meta, &qmap, part, err, tc_range_begin(rg, R, n_tiles), tc_range_begin(rg + 1, R, n_tiles),
                     gg, rg};
-  rmat_swap_body<false>(job, nc, g, fmt);
+  rmat_swap_body<false, DENSE>(job, nc, g, fmt);
 }
 
 // One item (segment, gene group, row group, tile range) per CTA, over every
 // segment of a batch.
+template <bool DENSE>
 __global__ void __launch_bounds__(kThreads, 1)
     k_rmat_swap_batch(const TcSegment* __restrict__ segs, const TcItem* __restrict__ items, int nc, int64_t g,
                       int fmt) {
@@ -1812,7 +1872,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const TcSegment& sg = segs[it.seg];
   const RmatJob job{sg.ent, static_cast<const SegMeta*>(sg.meta), sg.qmap, sg.part, sg.err, it.t0, it.t1, it.gg,
                     it.slot};
-  rmat_swap_body<true>(job, nc, g, fmt);
+  rmat_swap_body<true, DENSE>(job, nc, g, fmt);
 }
 
 size_t smem_tail() { return 2 * kMaxChunks * sizeof(SegMeta) + 64 * sizeof(uint64_t) + 64; }
@@ -1888,23 +1948,28 @@ int make_tmap16(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, 
   return (int)r;
 }
 
+// Which instance of the products: the 16-byte rounds pay where most quarters
+// (2,048 places) hold more entries than the lanes keep in flight and a few
+// more; the two cross between 20 and 25 % stored (k = 50, 40,000 x 2,000, us: 20 %
+// 62 and 66, 25 % 74 and 71).
+bool tc_dense(int64_t nnz, int64_t n, int64_t g) { return (double)nnz > 0.22 * (double)n * (double)g; }
+
 cudaError_t launch_fwd_tc(int ld, const uint32_t* ent, const void* meta, int64_t n, int nc, const CUtensorMap* vmap,
-                          const float* mc, float* Y, uint16_t* Yimg, int fmt, int* err, cudaStream_t st, int num_sms) {
+                          const float* mc, float* Y, uint16_t* Yimg, int fmt, bool dense, int* err, cudaStream_t st,
+                          int num_sms) {
   const int64_t n_tiles = (n + TM - 1) / TM;
   const SegMeta* m = static_cast<const SegMeta*>(meta);
-  note_launches(1);
-  if (ld == 64) {
-    const int grid = (int)std::min<int64_t>((n_tiles + 1) / 2, (int64_t)num_sms);
-    const size_t smem = fwd_swap_smem();
-    if (cudaError_t e = allow_smem(k_fwd_swap, smem); e != cudaSuccess) return e;
-    k_fwd_swap<<<grid, kThreads, smem, st>>>(ent, m, n_tiles, nc, n, *vmap, mc, Y, Yimg, fmt, err);
-  } else {
-    const int grid = (int)std::min<int64_t>(n_tiles, (int64_t)num_sms);
-    const size_t smem = fwd_smem(128);
-    if (cudaError_t e = allow_smem(k_fwd_tc<128>, smem); e != cudaSuccess) return e;
-    k_fwd_tc<128><<<grid, kThreads, smem, st>>>(ent, m, n_tiles, nc, n, *vmap, mc, Y, Yimg, fmt, err);
-  }
-  return cudaGetLastError();
+  auto go = [&](auto kern, int64_t blocks, size_t smem) {
+    if (cudaError_t e = allow_smem(kern, smem); e != cudaSuccess) return e;
+    note_launches(1);
+    kern<<<(int)std::min<int64_t>(blocks, (int64_t)num_sms), kThreads, smem, st>>>(ent, m, n_tiles, nc, n, *vmap, mc,
+                                                                                   Y, Yimg, fmt, err);
+    return cudaGetLastError();
+  };
+  if (ld == 64)
+    return dense ? go(k_fwd_swap<true>, (n_tiles + 1) / 2, fwd_swap_smem())
+                 : go(k_fwd_swap<false>, (n_tiles + 1) / 2, fwd_swap_smem());
+  return dense ? go(k_fwd_tc<128, true>, n_tiles, fwd_smem(128)) : go(k_fwd_tc<128, false>, n_tiles, fwd_smem(128));
 }
 
 int rmat_tc_groups(int ld, int nc, int num_sms, int* gene_groups) {
@@ -1920,22 +1985,18 @@ int rmat_tc_groups(int ld, int nc, int num_sms, int* gene_groups) {
 }
 
 cudaError_t launch_rmat_tc(int ld, const uint32_t* ent, const void* meta, int64_t n, int nc, int64_t g,
-                           int gene_groups, int row_groups, const CUtensorMap* qmap, float* part, int fmt, int* err,
-                           cudaStream_t st) {
+                           int gene_groups, int row_groups, const CUtensorMap* qmap, float* part, int fmt, bool dense,
+                           int* err, cudaStream_t st) {
   const int64_t n_tiles = (n + TM - 1) / TM;
-  const int grid = gene_groups * row_groups;
   const SegMeta* m = static_cast<const SegMeta*>(meta);
-  note_launches(1);
-  if (ld == 64) {
-    const size_t smem = rmat_swap_smem();
-    if (cudaError_t e = allow_smem(k_rmat_swap, smem); e != cudaSuccess) return e;
-    k_rmat_swap<<<grid, kThreads, smem, st>>>(ent, m, n_tiles, nc, g, gene_groups, *qmap, part, fmt, err);
-  } else {
-    const size_t smem = rmat_smem(128);
-    if (cudaError_t e = allow_smem(k_rmat_tc<128>, smem); e != cudaSuccess) return e;
-    k_rmat_tc<128><<<grid, kThreads, smem, st>>>(ent, m, n_tiles, nc, g, gene_groups, *qmap, part, fmt, err);
-  }
-  return cudaGetLastError();
+  auto go = [&](auto kern, size_t smem) {
+    if (cudaError_t e = allow_smem(kern, smem); e != cudaSuccess) return e;
+    note_launches(1);
+    kern<<<gene_groups * row_groups, kThreads, smem, st>>>(ent, m, n_tiles, nc, g, gene_groups, *qmap, part, fmt, err);
+    return cudaGetLastError();
+  };
+  if (ld == 64) return dense ? go(k_rmat_swap<true>, rmat_swap_smem()) : go(k_rmat_swap<false>, rmat_swap_smem());
+  return dense ? go(k_rmat_tc<128, true>, rmat_smem(128)) : go(k_rmat_tc<128, false>, rmat_smem(128));
 }
 
 cudaError_t launch_split16_batch(const SplitTask* tasks, int ntasks, int64_t count, int fmt, cudaStream_t st) {
@@ -1984,24 +2045,26 @@ cudaError_t launch_embed_tc(int64_t n, const CUtensorMap* qmap, const float* M, 
 }
 
 cudaError_t launch_fwd_tc_batch(const TcSegment* segs, const int32_t* band_seg, int64_t n_bands, int nc,
-                                int write_y, int fmt, cudaStream_t st, int num_sms) {
+                                int write_y, int fmt, bool dense, cudaStream_t st, int num_sms) {
   if (n_bands <= 0) return cudaSuccess;
   const int grid = (int)std::min<int64_t>(n_bands, (int64_t)num_sms);
   const size_t smem = fwd_swap_smem();
-  if (cudaError_t e = allow_smem(k_fwd_swap_batch, smem); e != cudaSuccess) return e;
+  auto kern = dense ? k_fwd_swap_batch<true> : k_fwd_swap_batch<false>;
+  if (cudaError_t e = allow_smem(kern, smem); e != cudaSuccess) return e;
   note_launches(1);
-  k_fwd_swap_batch<<<grid, kThreads, smem, st>>>(segs, band_seg, n_bands, nc, write_y, fmt);
+  kern<<<grid, kThreads, smem, st>>>(segs, band_seg, n_bands, nc, write_y, fmt);
   return cudaGetLastError();
 }
 
 cudaError_t launch_rmat_tc_batch(const TcSegment* segs, const TcItem* items, int n_items, int nc, int64_t g,
-                                 int gene_groups, int fmt, cudaStream_t st) {
+                                 int gene_groups, int fmt, bool dense, cudaStream_t st) {
   (void)gene_groups;  // each item names its gene group
   if (n_items <= 0) return cudaSuccess;
   const size_t smem = rmat_swap_smem();
-  if (cudaError_t e = allow_smem(k_rmat_swap_batch, smem); e != cudaSuccess) return e;
+  auto kern = dense ? k_rmat_swap_batch<true> : k_rmat_swap_batch<false>;
+  if (cudaError_t e = allow_smem(kern, smem); e != cudaSuccess) return e;
   note_launches(1);
-  k_rmat_swap_batch<<<n_items, kThreads, smem, st>>>(segs, items, nc, g, fmt);
+  kern<<<n_items, kThreads, smem, st>>>(segs, items, nc, g, fmt);
   return cudaGetLastError();
 }
 

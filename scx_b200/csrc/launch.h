@@ -294,14 +294,17 @@ int make_tmap16(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, 
 // 2 j = hi(M[:, j]) = round16(M[:, j]), column 2 j + 1 = round16(M[:, j] - hi).
 // Y (n x ld, FP32; may be null) = A V - mc with V given by its image (map
 // vmap), plus the image of Y.
+// `dense`: the products' instance for well-filled matrices (tc_dense), same results.
+bool tc_dense(int64_t nnz, int64_t n, int64_t g);
 cudaError_t launch_fwd_tc(int ld, const uint32_t* ent, const void* meta, int64_t n, int nc, const CUtensorMap* vmap,
-                          const float* mc, float* Y, uint16_t* Yimg, int fmt, int* err, cudaStream_t st, int num_sms);
+                          const float* mc, float* Y, uint16_t* Yimg, int fmt, bool dense, int* err, cudaStream_t st,
+                          int num_sms);
 // Partials part[row_group][g][ld] of A^T Q, Q given by its image (map qmap);
 // returns row groups.
 int rmat_tc_groups(int ld, int nc, int num_sms, int* gene_groups);
 cudaError_t launch_rmat_tc(int ld, const uint32_t* ent, const void* meta, int64_t n, int nc, int64_t g,
-                           int gene_groups, int row_groups, const CUtensorMap* qmap, float* part, int fmt, int* err,
-                           cudaStream_t st);
+                           int gene_groups, int row_groups, const CUtensorMap* qmap, float* part, int fmt, bool dense,
+                           int* err, cudaStream_t st);
 // Gram partials [G (64 x 64), colsum (64)] of hi + lo from the image (ld 64)
 // on tensor cores; returns the number of partials written, or -1 on a launch
 // error.
@@ -346,9 +349,9 @@ struct TcItem {
 cudaError_t launch_embed_tc(int64_t n, const CUtensorMap* qmap, const float* M, int nc, float* U, int fmt, int* err,
                             cudaStream_t st, int num_sms);
 cudaError_t launch_fwd_tc_batch(const TcSegment* segs, const int32_t* band_seg, int64_t n_bands, int nc,
-                                int write_y, int fmt, cudaStream_t st, int num_sms);
+                                int write_y, int fmt, bool dense, cudaStream_t st, int num_sms);
 cudaError_t launch_rmat_tc_batch(const TcSegment* segs, const TcItem* items, int n_items, int nc, int64_t g,
-                                 int gene_groups, int fmt, cudaStream_t st);
+                                 int gene_groups, int fmt, bool dense, cudaStream_t st);
 cudaError_t launch_gram_tc_batch(const TcSegment* segs, const TcItem* items, int n_items, int fmt, cudaStream_t st);
 // Tile range [t0, t1) of CTA b of nb over n_tiles row tiles: the split every
 // launcher above uses.

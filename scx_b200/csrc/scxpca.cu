@@ -370,6 +370,7 @@ struct scxpca_plan {
   // operands and their TMA maps
   bool use_tc = false;
   int fmt16 = 1;  // 1 = bf16, 0 = f16
+  bool tc_dense = false;  // the products' instance (tc_dense)
   int n_chunks = 0, tc_gene_groups = 0, tc_row_groups = 0;
   int tc_gram_parts = 0;  // partials of the tensor-core Gram (0: one per SM)
   // embeddings on tensor cores from Q's 16-bit image (ld 64); a batch's plans
@@ -756,7 +757,7 @@ void stream_forward(scxpca_plan* pl, bool f32) {
     if (pl->use_tc) {
       CK(launch_fwd_tc((int)ld, sl.ent.as<uint32_t>(), sl.meta.p, rows, pl->n_chunks, &pl->vmap, pl->mc.as<float>(),
                        f32 ? pl->Y.as<float>() + sh.r0 * ld : nullptr, pl->Yimg.as<uint16_t>() + sh.r0 * 2 * ld,
-                       pl->fmt16, pl->tc_err.as<int>(), st, pl->num_sms));
+                       pl->fmt16, pl->tc_dense, pl->tc_err.as<int>(), st, pl->num_sms));
     } else {
       CK(launch_fwd_strict(pl->dtype, (int)ld, sl.ip.as<int64_t>(), sl.idx.as<int32_t>(), vals, rows, (int32_t)pl->g,
                            pl->V.as<float>(), pl->centered ? pl->mc.as<float>() : nullptr,
@@ -775,7 +776,8 @@ void stream_rmat(scxpca_plan* pl, const float* A) {
     shard_prepare(pl, s, k, true, pl->use_tc ? 1 : 2);
     if (pl->use_tc) {
       CK(launch_rmat_tc((int)ld, sl.ent.as<uint32_t>(), sl.meta.p, rows, pl->n_chunks, g, pl->tc_gene_groups,
-                        sh.row_groups, &sh.qmap, pl->tc_part.as<float>(), pl->fmt16, pl->tc_err.as<int>(), st));
+                        sh.row_groups, &sh.qmap, pl->tc_part.as<float>(), pl->fmt16, pl->tc_dense,
+                        pl->tc_err.as<int>(), st));
       CK(launch_reduce_rows_f32(pl->tc_part.as<float>(), sh.row_groups, g * ld, pl->W.as<double>(), s > 0 ? 1 : 0,
                                 st, pl->num_sms));
     } else {
@@ -839,6 +841,7 @@ void setup_streaming(scxpca_plan* pl, const scxpca_csr* x, size_t limit) {
   pl->use_tc = tc_allowed && pl->dtype != SCXPCA_F32 && g <= 64 * 128;
   if (pl->use_tc) pl->ld = (pl->k + 63) / 64 * 64;
   pl->fmt16 = pl->dtype == SCXPCA_BF16 ? 1 : 0;
+  pl->tc_dense = tc_dense(nnz, n, g);
   const int64_t ld = pl->ld;
   // what stays resident: the tall buffers (Y; the 16-bit image), the gene-side
   // and statistics buffers; the rest of `limit` is the two shard slots
@@ -1274,6 +1277,7 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
       pl->use_tc = tc_allowed && pl->dtype != SCXPCA_F32 && !duplicates && g <= 64 * 128 && pl->k <= kMaxK;
       if (pl->use_tc) pl->ld = (pl->k + 63) / 64 * 64;
       pl->fmt16 = pl->dtype == SCXPCA_BF16 ? 1 : 0;
+      pl->tc_dense = tc_dense(nnz, n, g);
     }
     const int64_t ld = pl->ld;
     if (pl->rows_resorted) stats_pass(pl, vin, pl->in_dtype, sx, sxx);  // in the order of the sorted rows
@@ -1581,7 +1585,7 @@ void rmatmat_raw(scxpca_plan* pl, float* A, int split) {
     s = stage_begin(pl);
     CK(launch_rmat_tc((int)pl->ld, pl->tf_ent.as<uint32_t>(), pl->tf_meta.p, pl->n, pl->n_chunks, pl->g,
                       pl->tc_gene_groups, pl->tc_row_groups, &pl->qmap, pl->tc_part.as<float>(), pl->fmt16,
-                      pl->tc_err.as<int>(), st));
+                      pl->tc_dense, pl->tc_err.as<int>(), st));
     stage_end(pl, SCXPCA_STAGE_TRANSPOSE, s);
     s = stage_begin(pl);
     CK(launch_reduce_rows_f32(pl->tc_part.as<float>(), pl->tc_row_groups, pl->g * pl->ld,
@@ -1651,7 +1655,7 @@ void forward(scxpca_plan* pl, bool f32 = true, bool split_v = true) {
     s = stage_begin(pl);
     CK(launch_fwd_tc((int)pl->ld, pl->tf_ent.as<uint32_t>(), pl->tf_meta.p, pl->n, pl->n_chunks, &pl->vmap,
                      pl->mc.as<float>(), f32 ? pl->Y.as<float>() : nullptr, pl->Yimg.as<uint16_t>(), pl->fmt16,
-                     pl->tc_err.as<int>(), st, pl->num_sms));
+                     pl->tc_dense, pl->tc_err.as<int>(), st, pl->num_sms));
     stage_end(pl, SCXPCA_STAGE_FORWARD, s);
     return;
   }
@@ -2202,6 +2206,7 @@ struct scxpca_batch {
   DevBuf tc_segs, tc_maps, band_seg, rmat_items, gram_items, rmat_sums, gram_sums;
   int64_t n_bands = 0;
   int n_rmat_items = 0, n_gram_items = 0;
+  bool tc_dense = false;  // the batched products' instance (tc_dense)
   // and the tall right-multiplications (Y R^{-1} with its image, the
   // embeddings) over the row tiles of every segment, one launch each
   DevBuf task_tall_q, task_tall_emb;
@@ -2315,13 +2320,13 @@ struct BatchOperator {
     const scxpca_plan* p = p0();
     CK(launch_split16_batch(b->task_split.as<SplitTask>(), ns(), p->g * p->ld, p->fmt16, b->main));
     CK(launch_fwd_tc_batch(b->tc_segs.as<TcSegment>(), b->band_seg.as<int32_t>(), b->n_bands, p->n_chunks,
-                           last ? 1 : 0, p->fmt16, b->main, p->num_sms));
+                           last ? 1 : 0, p->fmt16, b->tc_dense, b->main, p->num_sms));
   }
   // W = X^T Q (raw) for every segment: the partials, then their sums
   void rmat_all() {
     const scxpca_plan* p = p0();
     CK(launch_rmat_tc_batch(b->tc_segs.as<TcSegment>(), b->rmat_items.as<TcItem>(), b->n_rmat_items, p->n_chunks,
-                            p->g, p->tc_gene_groups, p->fmt16, b->main));
+                            p->g, p->tc_gene_groups, p->fmt16, b->tc_dense, b->main));
     CK(launch_reduce_rows_batch(1, b->rmat_sums.as<SumTask>(), ns(), p->g * p->ld, b->main));
   }
   // Y's Gram and column sums (from its image) for every segment
@@ -2544,6 +2549,9 @@ bool batch_prepare_tasks(scxpca_batch* b, BatchOperator& bop) {
     put(b->gram_sums, gs.data(), sizeof(SumTask) * ns);
     b->n_bands = band0;
     b->n_rmat_items = (int)ritems.size();
+    int64_t entries = 0;
+    for (const scxpca_plan* pl : b->plans) entries += pl->nnz;
+    b->tc_dense = tc_dense(entries, b->n_obs, b->n_vars);
     b->n_gram_items = (int)gitems.size();
   }
   bop.tc_batched = tc;

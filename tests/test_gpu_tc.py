@@ -188,3 +188,63 @@ def test_tc_quarters_of_every_size(n, g, mode, k):
         assert np.linalg.norm(y - y_ref) / np.linalg.norm(y_ref) < 1e-4
         assert np.linalg.norm(z - z_ref) / np.linalg.norm(z_ref) < 1e-4
     plan.close()
+
+
+def _filled(n, g, sizes, empty, seed):
+    """A matrix whose 32 x 64 blocks hold numbers of entries from `sizes`, or,
+    with probability `empty`, none; values exact in 16 bits."""
+    rng = np.random.default_rng(seed)
+    rows, cols = [], []
+    for r in range(0, n, 32):
+        for j in range(0, g, 64):
+            h, w = min(32, n - r), min(64, g - j)
+            m = 0 if rng.random() < empty else min(int(rng.choice(sizes)), h * w)
+            at = rng.choice(h * w, size=m, replace=False)
+            rows.append(r + at // w)
+            cols.append(j + at % w)
+    rows, cols = np.concatenate(rows), np.concatenate(cols)
+    order = np.lexsort((cols, rows))
+    rows, cols = rows[order], cols[order].astype(np.int32)
+    indptr = np.r_[0, np.cumsum(np.bincount(rows, minlength=n))]
+    return rpca.Csr(indptr, cols, rng.integers(1, 64, len(cols)).astype(np.float32) / 8, (n, g))
+
+
+# beyond a lane's entries in flight (256 a warp): up to 128 at once, then rounds
+# of 512, from a start on and off a 16-byte boundary
+FULL = (300, 383, 384, 385, 386, 387, 388, 512, 767, 768, 769, 1000, 1024, 1281, 1791, 2047, 2048)
+
+
+@pytest.mark.parametrize("empty", [0.0, 0.85])  # the instance for well-filled matrices, and the other
+@pytest.mark.parametrize("n,g,mode,k", [(9000, 330, "mixed_bf16", 20), (9011, 130, "mixed_f16", 60),
+                                        (9000, 257, "mixed_f16", 100)])
+def test_tc_well_filled_quarters(n, g, mode, k, empty):
+    """Blocks that hold many entries, in matrices that are full of them and in
+    matrices that are nearly empty elsewhere; the tolerance is the module's."""
+    import torch
+
+    c = _filled(n, g, FULL, empty, n + g)
+    assert (len(c.indices) > 0.22 * n * g) == (empty == 0.0)
+    plan = accel.Plan(c.indptr, c.indices, c.data, c.shape, n_components=k, n_oversamples=0, math_mode=mode)
+    rng = np.random.default_rng(k)
+    mu = rpca.col_sums_and_sum_sq(c)[0] / n
+    v = (rng.standard_normal((g, k)) / np.sqrt(g)).astype(np.float32)
+    q = (rng.standard_normal((n, k)) / np.sqrt(n)).astype(np.float32)
+    y_ref = rpca.spmm_forward(c, v.astype(np.float64), mu)
+    z_ref = rpca.spmm_transpose(c, q.astype(np.float64), mu)
+    y = plan.matmat(torch.from_numpy(v).cuda()).cpu().numpy().astype(np.float64)
+    z = plan.rmatmat(torch.from_numpy(q).cuda()).cpu().numpy().astype(np.float64)
+    assert np.linalg.norm(y - y_ref) / np.linalg.norm(y_ref) < 1e-4
+    assert np.linalg.norm(z - z_ref) / np.linalg.norm(z_ref) < 1e-4
+    plan.close()
+
+
+def test_tc_well_filled_batch_equals_plain_runs():
+    """The batched products of well-filled segments give the bits of each
+    segment's own launches."""
+    c = _filled(3000, 200, FULL, 0.0, 5)
+    b = accel.Batch(c.indptr, c.indices, c.data, c.shape, [0, 700, 1411, 3000], n_components=20, n_oversamples=20,
+                    branches=-1)
+    graph = [np.array(a) for a in b.run()[:3]]
+    plain = [np.array(a) for a in b.run(use_graph=False)[:3]]
+    b.close()
+    assert all(np.array_equal(x, y) for x, y in zip(graph, plain))
