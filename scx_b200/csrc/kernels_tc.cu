@@ -500,6 +500,10 @@ __device__ __forceinline__ void swap_tile_out(uint32_t tbase, int tiles, int64_t
 // and band); an image chunk per tile as the MMA's B operand, double-buffered,
 // took 217 us, of which 195 the MMAs (282 cycles each with an MN-major B) and a
 // two-slot image ring; this takes 194, the epilogues of the bands included.
+// A single tile, the last band of a CTA with an odd number of them, takes a stage
+// a chunk, so that all four groups fill it (with two stages a chunk half of them
+// had nothing to do: 40,000 x 2,000 at 30 % stored 104 us, now 95; the operand
+// order before 95).
 // ---------------------------------------------------------------------------
 template <int LD, bool DENSE>
 __global__ void __launch_bounds__(kThreads, 1)
@@ -566,7 +570,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     const uint32_t tile = smem_u32(As + group * A_BYTES);
     DenseSlot<kDenseRegs> sl[2];
     slots_init(sl);
-    // cursor: the next segment to load, number j = 2 chunk + tile of its band
+    // cursor: the next segment to load, number j = tiles x chunk + tile of its band
+    // (a single tile, the CTA's last, takes one stage a chunk)
     int64_t t = t0;
     uint32_t bi = 0;
     int tiles = 0, j = group;
@@ -576,10 +581,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       return warp_wait(&mfull[bi & 1u], (bi >> 1) & 1u, abort_flag, err, 11);
     };
     auto fetch = [&](DenseSlot<kDenseRegs>& x) {
-      while (j >= 2 * nc) {  // leave the band
+      while (j >= tiles * nc) {  // leave the band
         __syncwarp();
         if (lane == 0) mbar_arrive(&mempty[bi & 1u]);
-        j -= 2 * nc;
+        j -= tiles * nc;
         t += 2;
         ++bi;
         if (t >= t1) {
@@ -588,8 +593,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         if (!enter()) return false;
       }
-      x.n = -1;
-      if ((j & 1) < tiles) slot_load(x, ent, quarter_span(mring[(bi & 1u) * MSLOT + (j & 1) * nc + (j >> 1)], q), lane);
+      const int c = tiles == 2 ? j >> 1 : j, u = tiles == 2 ? j & 1 : 0;
+      slot_load(x, ent, quarter_span(mring[(bi & 1u) * MSLOT + u * nc + c], q), lane);
       j += S;
       return true;
     };
@@ -603,11 +608,9 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int k = 0; k < 2; ++k) {
         if (k == 1 && !more1) break;
         if (!warp_wait(&empty[group], (uint32_t)(k ^ 1), abort_flag, err, 12)) goto done;
-        if (sl[k].n >= 0) {
-          zero_rows(tile, q, lane);
-          __syncwarp();
-          slot_scatter<DENSE>(sl[k], tile, lane);
-        }
+        zero_rows(tile, q, lane);
+        __syncwarp();
+        slot_scatter<DENSE>(sl[k], tile, lane);
         // every lane's shared stores -> async proxy, then one arrival per warp
         fence_proxy_async_smem();
         __syncwarp();
@@ -645,15 +648,16 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint64_t tdesc0 = sdesc_sw128(smem_u32(As), 16, 1024);        // K-major, 256 cell rows
       const uint64_t vdesc0 = sdesc_sw128(smem_u32(Bs), CW * 128, 1024);  // MN-major, 64-column blocks
       static_assert((S & (S - 1)) == 0 && (NB & (NB - 1)) == 0, "power-of-two rings");
-      uint32_t cc = 0, k = 0;
+      uint32_t cc = 0, it = 0, k = 0;  // chunks, stages, bands so far
       bool ok = true;
       for (int64_t t = t0; t < t1 && ok; t += 2, ++k) {
-        const uint32_t idesc = t1 - t >= 2 ? idesc2 : idesc1;
-        for (int c = 0; c < nc; ++c, ++cc) {
-          const int b = cc % NB, s = 2 * cc % S;
+        const bool two = t1 - t >= 2;  // (only the last band has one tile: a pair of stages starts at an even one)
+        const uint32_t idesc = two ? idesc2 : idesc1;
+        for (int c = 0; c < nc; ++c, ++cc, it += two ? 2 : 1) {
+          const int b = cc % NB, s = it % S;
           if (!mbar_wait(&bfull[b], (cc / NB) & 1u, abort_flag, err, 16) ||
-              !mbar_wait(&full[s], (2 * cc / S) & 1u, abort_flag, err, 16) ||
-              !mbar_wait(&full[s + 1], (2 * cc / S) & 1u, abort_flag, err, 16)) {
+              !mbar_wait(&full[s], (it / S) & 1u, abort_flag, err, 16) ||
+              (two && !mbar_wait(&full[s + 1], (it / S) & 1u, abort_flag, err, 16))) {
             ok = false;
             break;
           }
@@ -674,7 +678,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           if (!ok) break;
           umma_commit(&empty[s]);
-          umma_commit(&empty[s + 1]);
+          if (two) umma_commit(&empty[s + 1]);
           umma_commit(&bempty[b]);
         }
       }
