@@ -659,8 +659,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 // 30,000, k = 110 653, 335, 760; 300 x 20,000, k = 30 the call 379, 93, 104.
 // Where this leaves one part (10,000 x 2,000, k = 60: 67 us) nothing changes.
 //
-// Long chunks are built by as many blocks as fill the SMs once: 256 rows, or 128
-// where the genes leave room for at most 12 warps a block.  A plan of 2,000 x
+// Long chunks are built by as many blocks as fill the SMs once: from 256 rows on,
+// or 64 where the genes leave room for at most 12 warps a block.  A plan of 2,000 x
 // 30,000 takes 5.9 ms (one block a 64-row chunk 8.8, 23.7 before), of 10,000 x
 // 30,000 4.0 (3.9, 10.9).  g = 0 (a streamed shard, whose copy is built for every
 // product): one block a range and a chunk.
@@ -684,7 +684,7 @@ StrictGeometry strict_geometry(int64_t n, int64_t g, int ld, int num_sms) {
   geo.ranges = (int)((geo.chunks + m - 1) / m);
   // the last ones: ranges of at least 64 rows may be fewer still
   geo.parts = (int)std::max<int64_t>(1, std::min<int64_t>(want / geo.ranges, (g + kLists - 1) / kLists));
-  if (parts > 1 && geo.rows >= (g > 4096 ? 128 : 256))
+  if (parts > 1 && geo.rows >= (g > 4096 ? 64 : 256))
     geo.splits = (int)std::max<int64_t>(1, std::min<int64_t>(geo.rows / 32, num_sms / geo.chunks));
   return geo;
 }
