@@ -44,8 +44,9 @@ namespace scx {
 // (One step at a time: 526.)
 //
 // Above 4,266 genes at most two parts fit.  Their warps are made up to
-// kStatsLeast by ranges and load sixteen steps ahead, and there are four parts
-// per SM, in turn, so that a piece of an upload still fills half of the SMs.
+// kStatsLeast by ranges and load sixteen steps ahead, and where the entries are
+// worth the partials there are four parts per SM, in turn, so that a piece of an
+// upload still fills half of the SMs.
 // 46M entries, one warp a part and eight steps against this: 8,000 genes 850 ->
 // 660 us, 12,800 855 -> 656, 30,000 2,468 -> 1,627 (the bucket sort: 1,071,
 // 1,608, 2,146); a plan from host memory at 30,000 genes 39.2 -> 29.3 ms
@@ -57,6 +58,7 @@ constexpr int kStatsMaxWarps = 16;  // warps of a block
 constexpr int kStatsPassGenes = (int)(kStatsSmemMax / 16);
 constexpr int kStatsLeast = 4;      // warps of a block whose parts are shared
 constexpr int kStatsOwn = 3;        // parts of a block from which on each has one warp
+constexpr int kStatsWorth = 16384;  // entries that are worth a partial of a wide matrix
 
 // Parts whose accumulators fit an SM's shared memory.
 static int stats_sets(int64_t g) {
@@ -64,9 +66,9 @@ static int stats_sets(int64_t g) {
   return (int)std::min<int64_t>(kStatsMaxWarps, (int64_t)kStatsSmemMax / (16 * pass));
 }
 
-int col_stats_parts(int64_t g, int num_sms) {
-  const int sets = stats_sets(g);
-  return num_sms * (sets >= kStatsOwn ? sets : 4);
+int col_stats_parts(int64_t g, int64_t nnz, int num_sms) {
+  const int sets = stats_sets(g), four = 4 * num_sms;
+  return sets < kStatsOwn && nnz >= (int64_t)four * kStatsWorth ? four : num_sms * sets;
 }
 
 // SHARED: `ranges` warps walk a part, and a step may hold none of a warp's genes.

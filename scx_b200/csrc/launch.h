@@ -23,8 +23,9 @@ constexpr int kTransposeGeneBlock = 256;       // genes per block, CUDA-core tra
 cudaError_t launch_col_stats(int dtype, const int32_t* idx, const void* val, int64_t nnz,
                              int32_t g, double* partial, int nparts, double* out,
                              cudaStream_t st, int num_sms, int accumulate = 0);
-// Parts that fill the device: as many per SM as hold their own accumulators, four of wide matrices.
-int col_stats_parts(int64_t g, int num_sms);
+// Parts that fill the device: as many per SM as hold their own accumulators, four
+// of a wide matrix with entries enough.
+int col_stats_parts(int64_t g, int64_t nnz, int num_sms);
 // The same statistics in two halves: parts [part0, part0 + count) of the
 // partition write their partials (part b reads entries
 // [col_stats_block_begin(b), col_stats_block_begin(b + 1))), then one reduce.

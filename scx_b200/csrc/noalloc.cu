@@ -114,10 +114,12 @@ void col_stats_noalloc(int32_t dev, const scxpca_csr* x, double* out, cudaStream
   int32_t* flags = reinterpret_cast<int32_t*>(base);
   double* partial = reinterpret_cast<double*>(base + kFlagBytes);
   const int64_t g = x->n_vars;
-  // the parts of a plan, or as many as the scratch holds (46M entries: 500 genes
-  // 0.93 ms the call with 2 x SMs parts, 0.44 so; the 40 parts at 12,800 genes
-  // have four warps each, 3.05 -> 2.24)
-  const int nparts = (int)std::min<int64_t>(col_stats_parts(g, sms), kPartialDoubles / (2 * g));
+  // the parts of a plan, or as many as the scratch holds, and no more than 2 x SMs
+  // of few entries (46M entries: 500 genes 0.93 ms the call with 2 x SMs parts, 0.44
+  // so; the 40 parts at 12,800 genes have four warps each, 3.05 -> 2.24)
+  const int64_t worth = std::max<int64_t>(2 * (int64_t)sms, x->nnz / 1024);
+  const int nparts =
+      (int)std::min(worth, std::min<int64_t>(col_stats_parts(g, x->nnz, sms), kPartialDoubles / (2 * g)));
 
   // Once work is queued, an error must not release the lock while our
   // kernels may still touch the shared array: wait for the stream first

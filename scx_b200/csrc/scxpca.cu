@@ -846,7 +846,7 @@ void setup_streaming(scxpca_plan* pl, const scxpca_csr* x, size_t limit) {
   // what stays resident: the tall buffers (Y; the 16-bit image), the gene-side
   // and statistics buffers; the rest of `limit` is the two shard slots
   const double resident = (double)n * ld * 4 * (pl->use_tc ? 2 : 1) + (double)n * pl->nc * 4 +
-                          (double)g * ld * 8 * 8 + (double)2 * g * 8 * (col_stats_parts(g, pl->num_sms) + 1) + (64 << 20);
+                          (double)g * ld * 8 * 8 + (double)2 * g * 8 * (col_stats_parts(g, nnz, pl->num_sms) + 1) + (64 << 20);
   const double per_entry = slot_bytes_per_entry(pl, pl->use_tc) + (pl->use_tc ? 0.0 : 1.0);
   const double room = ((double)limit / 1.1 - resident) / 2.0;
   int64_t cap = (int64_t)std::min<double>((double)kShardEntriesMax, room / per_entry);
@@ -886,7 +886,7 @@ void setup_streaming(scxpca_plan* pl, const scxpca_csr* x, size_t limit) {
   phase_mark(SCXPCA_PHASE_UPLOAD, st);
 
   // ---- validation, input statistics (and gene counts) over the shards ----
-  pl->stats_parts = col_stats_parts(g, pl->num_sms);
+  pl->stats_parts = col_stats_parts(g, nnz, pl->num_sms);
   pl->stats_part.alloc(sizeof(double) * 2 * g * pl->stats_parts);
   pl->stats_out.alloc(sizeof(double) * 2 * g);
   DevBuf flags, counts;
@@ -1170,7 +1170,7 @@ scxpca_plan* create_plan(const scxpca_csr* x, const scxpca_params* p, const Affi
 
     // ---- resident CSR ----
     const bool dev_in = x->memory == SCXPCA_MEM_DEVICE;
-    pl->stats_parts = col_stats_parts(g, pl->num_sms);
+    pl->stats_parts = col_stats_parts(g, nnz, pl->num_sms);
     pl->stats_part.alloc(sizeof(double) * 2 * g * pl->stats_parts);
     pl->stats_out.alloc(sizeof(double) * 2 * g);
     const void* vin = x->values;
