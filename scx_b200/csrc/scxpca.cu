@@ -1498,7 +1498,7 @@ void collect_stages(scxpca_plan* pl) {
 
 // The Gram (FP64, with column sums after it) of a tall A into G.  With
 // `from_image` (tensor-core path, ld 64) it is taken on tensor cores from the
-// 16-bit image of A held in Yimg; otherwise from the FP32 A with FP64 FMAs.
+// 16-bit image of A held in Yimg; otherwise from the FP32 A by the FP64 matrix instruction.
 void tall_gram(scxpca_plan* pl, const float* A, int64_t rows, bool from_image) {
   cudaStream_t st = pl->stream;
   const int ld = (int)pl->ld;
@@ -1560,8 +1560,7 @@ void small_qr(scxpca_plan* pl, double* A, int shift) {
   small_apply(pl, A);
 }
 
-// W = X^T A (raw, uncentred), FP64, for a tall float A (n x ld).
-// W = X^T A (raw, uncentred) into pl->W (FP64).  On the tensor-core path the
+// W = X^T A (raw, uncentred) into pl->W (FP64), for a tall float A (n x ld).  On the tensor-core path the
 // tall operand enters as its 16-bit image Yimg: `split` != 0 first writes
 // the image of the FP32 A; otherwise it already holds the image of A (the
 // forward product's, or the explicit Q's).
