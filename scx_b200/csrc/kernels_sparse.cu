@@ -49,10 +49,10 @@ namespace scx {
 // upload still fills half of the SMs.
 // 46M entries, one warp a part and eight steps against this: 8,000 genes 850 ->
 // 660 us, 12,800 855 -> 656, 30,000 2,468 -> 1,627 (the bucket sort: 1,071,
-// 1,608, 2,146); a plan from host memory at 30,000 genes 39.2 -> 29.3 ms
-// (the bucket sort 37.3).  Ranges without the longer loads gain nothing, the
-// loads alone 17 % at 30,000 genes and nothing at 12,800; with three parts an
-// SM neither gains.
+// 1,608, 2,146); in a plan from host memory at 30,000 genes they take 10 ms less,
+// as the pieces no longer outlast the copy.  Ranges without the longer loads
+// gain nothing, the loads alone 17 % at 30,000 genes and nothing at 12,800; with
+// three parts an SM neither gains.
 // ---------------------------------------------------------------------------
 constexpr int kStatsMaxWarps = 16;  // warps of a block
 constexpr int kStatsPassGenes = (int)(kStatsSmemMax / 16);
